@@ -370,20 +370,27 @@ int tb_read_scatt_indices(const char* path, int nlegs, const int32_t* nsplit, in
  * of the tuples with such points and a 64-bit mask per tuple, built at
  * creation when the channel has at most 64 Monte-Carlo points; same sums as
  * the full quadrature for finite f), else 0 (every point of every tuple).
+ * FP64 channels that TB_LAYOUT_AUTO resolved (2 or 3 legs, at most 64
+ * points, shared by fewer than 16 runs) report TB_LAYOUT_T64 and stages 0,
+ * pair 6 too: they are evaluated over packed rows of the same tuples and
+ * points, and their moment tensor is built only when a contraction schedule is
+ * pinned, or by tb_options.autotune, which keeps the faster of the two.
  * No counterpart in the reference. */
 int tb_channel_schedule(const tb_handle* h, int ch, int32_t* stages, int32_t* pair, double* seconds);
 
 /* Monte-Carlo channels: the tuples with at least one point inside the
  * simplices and the number of such (tuple, point) pairs, i.e. the work the
  * quadrature does per instance; -1, -1 when the channel has no such list
- * (moment-tensor layout, or more than 64 Monte-Carlo points).  On a sharded
+ * (a moment tensor, or more than 64 Monte-Carlo points).  On a sharded
  * handle, this handle's part.  No counterpart in the reference. */
 int tb_channel_points_inside(const tb_handle* h, int ch, int64_t* n_tuples, int64_t* n_points);
 
 /* Pins the contraction schedule of a channel's moment-tensor group (every
  * channel of that group): stages 1..2, pair as tb_channel_schedule reports it
  * (2..5 only for groups of 8..1024 runs with at most 3 legs).  Monte-Carlo
- * groups take stages 0 with pair 0 (every point) or 6 (points inside only).  The result is
+ * groups take stages 0 with pair 0 (every point) or 6 (points inside only);
+ * channels with packed rows take stages 0 with pair 6, or any contraction
+ * schedule, whose moment tensor is then built.  The result is
  * the same up to FP64 summation order; the time is not.  No counterpart in the
  * reference. */
 int tb_set_channel_schedule(tb_handle* h, int ch, int32_t stages, int32_t pair);

@@ -1,0 +1,154 @@
+"""The packed-row evaluation of channels with at most three legs (tb_rows.cu)
+against the oracle: the shapes where its dispatch, padding and sharing change.
+
+Tolerance: 1e-12 relative L2, the bound of every FP64 layout of this suite (the
+summation noise of a few thousand FP64 terms per coefficient is about 1e-14)."""
+import numpy as np
+import pytest
+
+import oracle
+from conftest import rel_l2
+from tortoise_b200 import engine as E
+from tortoise_b200 import workloads as W
+from tortoise_b200.model import FERMION, IN, OUT
+
+pytestmark = pytest.mark.gpu
+TOL = 1e-12
+
+
+def _material(names, dirs, nsplit=(6, 5), umklapp=0, n_mc=50, bands=("P", "D"), crossing=False, amp=1.0):
+    mat = W.build_material(max(nsplit), bands, (0.2,), ee=False, eph=False, field=(0.1, 0.0), rtol=1e-6, atol=1e-9,
+                           n_mc=n_mc, mesh_nsplit=nsplit)
+    if crossing:   # a tilted plane that crosses the parabola: two-leg channels with tuples
+        b = mat.addBand("el:X", -1.0, FERMION, mat.bands[0].mesh, lambda kx, ky: 0.6 * kx + 0.3 * ky + 0.2)
+        b.relativeErrorTolerance, b.absoluteErrorTolerance = 1e-6, 1e-9
+    for c in mat.addScatteringChannelsWildcards(names, dirs, umklapp):
+        c.amplitude = amp
+    return mat
+
+
+SHAPES = {
+    "in_in_out": dict(names=["el:*", "pn:*", "el:*"], dirs=[IN, IN, OUT]),
+    "in_out_out": dict(names=["el:*", "el:*", "pn:*"], dirs=[IN, OUT, OUT]),
+    "out_in_out": dict(names=["pn:*", "el:*", "el:*"], dirs=[OUT, IN, OUT]),
+    "two_legs": dict(names=["el:*", "el:*"], dirs=[IN, OUT], crossing=True, nsplit=(9, 7)),
+    "umklapp": dict(names=["el:*", "pn:*", "el:*"], dirs=[IN, IN, OUT], umklapp=1, nsplit=(5, 3)),
+    "one_row_meshes": dict(names=["el:*", "pn:*", "el:*"], dirs=[IN, IN, OUT], nsplit=(7, 1)),
+    "one_point": dict(names=["el:*", "pn:*", "el:*"], dirs=[IN, IN, OUT], n_mc=1),
+    "64_points": dict(names=["el:*", "pn:*", "el:*"], dirs=[IN, IN, OUT], n_mc=64, nsplit=(8, 8)),
+    "65_points": dict(names=["el:*", "pn:*", "el:*"], dirs=[IN, IN, OUT], n_mc=65),   # beyond the mask: the tensor
+    "many_rows": dict(names=["el:*", "pn:*", "el:*"], dirs=[IN, IN, OUT], nsplit=(20, 17)),
+}
+
+
+@pytest.mark.parametrize("deterministic", [False, True])
+@pytest.mark.parametrize("shape", sorted(SHAPES))
+def test_rhs_and_rates_match_the_oracle(gpu_lib, shape, deterministic):
+    mat = _material(**SHAPES[shape])
+    f = W.initial_status(mat, kT=0.15, seed=5).vec
+    o = oracle.Oracle(mat)
+    e = E.Engine(mat, deterministic=deterministic)
+    live = [c for c in range(len(mat.channels)) if o.num_tuples(c)]
+    try:
+        assert live
+        for c in live:   # without any point inside there are no rows
+            rows = shape != "65_points" and o.points_inside(c)[1] > 0
+            assert bool(e.schedule(c).get("inside_only")) == rows
+        assert rel_l2(e.rhs(f), o.rhs(f)) < TOL
+        assert rel_l2(e.scattering_rates(f), o.scattering_rates(f)) < TOL
+        for c in live:
+            if np.linalg.norm(o.channel_propagate(c, f)) > 0:
+                assert rel_l2(e.channel_propagate(c, f), o.channel_propagate(c, f)) < TOL
+            for leg in range(mat.channels[c].nlegs):
+                r = o.scattering_rates(f, c, leg)
+                if np.linalg.norm(r) > 0:
+                    assert rel_l2(e.scattering_rates(f, c, leg), r) < TOL
+        th = np.random.default_rng(3).standard_normal(f.size)
+        v = np.random.default_rng(4).standard_normal(f.size)
+        g, _ = e.rhs_vjp(f, th)
+        jv = (o.rhs(f + 1e-5 * v) - o.rhs(f - 1e-5 * v)) / 2e-5
+        assert abs(th @ jv - g @ v) <= 1e-8 * (abs(th @ jv) + 1e-6 * np.linalg.norm(th) * np.linalg.norm(jv))
+    finally:
+        e.close()
+
+
+@pytest.mark.parametrize("runs", [2, 15])
+def test_shared_rows_of_a_small_batch(gpu_lib, runs):
+    mats = [_material(SHAPES["in_in_out"]["names"], [IN, IN, OUT], amp=0.5 + 0.1 * r) for r in range(runs)]
+    states = [W.initial_status(m, kT=0.05 + 0.01 * r, seed=r).vec for r, m in enumerate(mats)]
+    be = E.BatchEngine(mats)
+    try:
+        be.set_amplitude(1, 0.0)   # a channel of the first run switched off
+        got = be.split(be.rhs(np.concatenate(states)))
+        rates = be.split(be.scattering_rates(np.concatenate(states)))
+        mats[0].channels[1].amplitude = 0.0
+        for m, f, g, s in zip(mats, states, got, rates):
+            o = oracle.Oracle(m)
+            assert rel_l2(g, o.rhs(f)) < TOL and rel_l2(s, o.scattering_rates(f)) < TOL
+    finally:
+        be.close()
+
+
+def test_amplitude_factors_and_pinned_schedules(gpu_lib):
+    """functAmplitude through the rows; then a contraction schedule, whose tensor is built on request, and back."""
+    mat = _material(**SHAPES["in_in_out"])
+    fn = lambda b: 1.0 + 0.3 * b[:, 0, 0] - 0.2 * b[:, 1, 1]  # noqa: E731
+    for c in mat.channels:
+        c.functAmplitude = fn
+    f = W.initial_status(mat, seed=2).vec
+    ref = oracle.Oracle(mat).rhs(f)
+    e = E.Engine(mat)
+    try:
+        assert rel_l2(e.rhs(f), ref) < TOL
+        for c in range(len(mat.channels)):
+            e.set_schedule(c, 1, pair=0)
+            assert e.schedule(c)["stages"] == 1
+        assert rel_l2(e.rhs(f), ref) < TOL
+        for c in range(len(mat.channels)):
+            e.set_schedule(c, 0, inside_only=True)
+        assert rel_l2(e.rhs(f), ref) < TOL
+        with pytest.raises(E.TortoiseError):
+            e.set_schedule(0, 0, inside_only=False)
+        for c in range(len(mat.channels)):
+            e.set_channel_amplitude(c, None)
+            mat.channels[c].functAmplitude = None
+        assert rel_l2(e.rhs(f), oracle.Oracle(mat).rhs(f)) < TOL
+    finally:
+        e.close()
+
+
+@pytest.mark.parametrize("value", [np.nan, np.inf])
+def test_non_finite_coefficients_reach_the_same_elements_as_the_tensor(gpu_lib, value):
+    """Also through tuples without a point inside, whose integrand the full quadrature multiplies by 0."""
+    mat = _material(**SHAPES["in_in_out"])
+    f = W.initial_status(mat, seed=2).vec
+    rows, tensor = E.Engine(mat), E.Engine(mat, layout=E.LAYOUT_T64)
+    try:
+        for k in (4, f.size // 2, f.size - 1):
+            g = f.copy()
+            g[k] = value
+            for call in ("rhs", "scattering_rates"):
+                a, b = getattr(rows, call)(g), getattr(tensor, call)(g)
+                assert np.array_equal(np.isfinite(a), np.isfinite(b)), (k, call)
+                ok = np.isfinite(b)
+                assert rel_l2(a[ok], b[ok]) < TOL
+    finally:
+        rows.close()
+        tensor.close()
+
+
+def test_row_wait_runs_out_and_the_handle_recovers(gpu_lib):
+    """The bounded wait for staged rows (see test_gpu_timeout.py)."""
+    mat = _material(**SHAPES["in_in_out"])
+    f = W.initial_status(mat, seed=2).vec
+    e = E.Engine(mat, deterministic=True)
+    try:
+        ref = e.rhs(f)
+        e.set_copy_wait_limit(0)
+        with pytest.raises(E.TortoiseError) as ex:
+            e.rhs(f)
+        assert ex.value.rc == 6
+        e.set_copy_wait_limit(1 << 22)
+        assert np.array_equal(e.rhs(f), ref)
+    finally:
+        e.close()

@@ -392,8 +392,8 @@ static int vjp_at(tb_handle* h, const double* Y, int flags) {
                                          A->u, A->g, A->gamp + A->gamp_off[gi], h->stream, h->fx, fa));
                 continue;
             }
-            if (G.layout == TB_LAYOUT_MC64 && G.theta.use)   // the tuples and points inside the simplices only
-                TB_TRY(launch_collision_vjp(G.dev, G.d_insts, int(G.insts.size()), G.layout, G.tensor, G.theta.ids,
+            if (G.use_rows || (G.layout == TB_LAYOUT_MC64 && G.theta.use))   // the tuples and points inside the simplices only
+                TB_TRY(launch_collision_vjp(G.dev, G.d_insts, int(G.insts.size()), TB_LAYOUT_MC64, G.tensor, G.theta.ids,
                                             G.theta.n, G.theta.n, Y, A->u, A->g, A->gamp + A->gamp_off[gi], h->stream,
                                             G.theta.mask, G.theta.perm, h->fx, fa));
             else

@@ -561,8 +561,23 @@ int build_runs(tb_handle* h, const tb_problem_desc* const* descs, int nruns) {
     {
         NvtxRange r("tb_create: points inside the simplices");
         for (auto& G : h->groups)
-            if (G.layout == TB_LAYOUT_MC64) TB_TRY(build_theta_list(G.dev, G.tup, G.theta, h->stream));
+            if (G.layout == TB_LAYOUT_MC64) {
+                TB_TRY(build_theta_list(G.dev, G.tup, G.theta, h->stream));
+                if (G.theta.built) TB_TRY(build_rows(G.dev, G.theta, G.rows, h->stream));
+                G.use_rows = G.rows.blk != nullptr;
+            }
     }
+    h->d_f4 = reinterpret_cast<double4*>(dev_alloc(h, size_t(h->ndofs / 3 * 4)));
+    {
+        void* p = nullptr;
+        if (!h->d_f4 || cudaMalloc(&p, sizeof(int) * size_t(h->ed.nblk)) != cudaSuccess) {
+            set_error("state allocation failed");
+            return TB_ERR_OOM;
+        }
+        h->dev_raw.push_back(p);
+        h->d_nf = static_cast<int*>(p);
+    }
+    TB_TRY(refresh_row_sets(h));
     if (h->opts.autotune) {
         NvtxRange r("tb_create: autotune");
         TB_TRY(autotune(h));
@@ -586,6 +601,75 @@ static int launch_group_mc(tb_handle* h, GroupChan& G, const InstDev* insts, int
                                148 * 32, rate_leg, nullptr, nullptr, h->fx);
 }
 
+static int row_dirs(const ChanDev& c) {
+    int d = 0;
+    for (int l = 0; l < c.L; ++l) d |= c.leg[l].dir > 0.0 ? 1 << l : 0;
+    return d;
+}
+
+static RowChan row_chan(const GroupChan& G) {
+    RowChan c{};
+    c.blk = G.rows.blk;
+    c.row_e0 = G.rows.row_e0;
+    c.perm = G.rows.perm;
+    c.mc = G.dev.mc;
+    c.tamp = G.dev.tamp;
+    c.insts = G.d_insts;
+    c.n_insts = int(G.insts.size());
+    c.nmc = G.dev.nmc;
+    for (int l = 0; l < G.L; ++l) c.leg[l] = G.dev.leg[l];
+    c.tup = G.tup.d;
+    c.stride = G.tup.cap;
+    c.n = G.tup.n;
+    return c;
+}
+
+int refresh_row_sets(tb_handle* h) {
+    for (auto& rs : h->row_sets) rs.release();
+    h->row_sets.clear();
+    std::vector<bool> done(h->groups.size(), false);
+    for (size_t a = 0; a < h->groups.size(); ++a) {
+        GroupChan& A = h->groups[a];
+        A.row_one.release();
+        if (!A.use_rows) continue;
+        TB_TRY(build_row_set(A.L, row_dirs(A.dev), {row_chan(A)}, {&A.rows}, A.row_one));
+        if (done[a]) continue;
+        std::vector<RowChan> chan;
+        std::vector<const PointRows*> rows;
+        for (size_t b = a; b < h->groups.size(); ++b) {
+            const GroupChan& B = h->groups[b];
+            if (done[b] || !B.use_rows || B.L != A.L || row_dirs(B.dev) != row_dirs(A.dev)) continue;
+            chan.push_back(row_chan(B));
+            rows.push_back(&B.rows);
+            done[b] = true;
+        }
+        h->row_sets.emplace_back();
+        TB_TRY(build_row_set(A.L, row_dirs(A.dev), chan, rows, h->row_sets.back()));
+    }
+    return TB_OK;
+}
+
+// The channels over packed rows: all of them in one launch per leg count, or
+// (only_inst >= 0) that instance's alone.  rate_leg: -1 every leg.
+static int launch_row_sets(tb_handle* h, const double* d_in, double* d_acc, const DPCtl* ctl, int only_inst, bool rate,
+                           int rate_leg) {
+    if (only_inst >= 0) {
+        const ChanInst& I = h->insts[only_inst];
+        GroupChan& G = h->groups[I.group];
+        if (!G.use_rows) return TB_OK;
+        TB_TRY(launch_rows_prepare(h->ed, d_in, h->d_f4, h->d_nf, ctl, h->stream));
+        return launch_rows(G.row_one, h->ed, h->d_f4, h->d_nf, d_acc, ctl, h->stream, rate, rate_leg, h->fx,
+                           h->d_err, G.dev.wait_polls, I.d_single);
+    }
+    if (h->row_sets.empty()) return TB_OK;
+    TB_TRY(launch_rows_prepare(h->ed, d_in, h->d_f4, h->d_nf, ctl, h->stream));
+    for (const RowSet& rs : h->row_sets)
+        if (rate_leg < rs.L)
+            TB_TRY(launch_rows(rs, h->ed, h->d_f4, h->d_nf, d_acc, ctl, h->stream, rate, rate_leg, h->fx, h->d_err,
+                               h->groups[0].dev.wait_polls));
+    return TB_OK;
+}
+
 // A streamed group over this handle's work items.  Outside an integration
 // (ctl == nullptr) the launch records its counts for tb_channel_info; the
 // attempts of an integration leave them alone.
@@ -600,9 +684,10 @@ static int launch_group_stream(tb_handle* h, GroupChan& G, const InstDev* insts,
 
 int run_rhs_acc(tb_handle* h, const double* d_in, double* d_acc, const DPCtl* ctl, int flags, int only_inst) {
     if (!(flags & TB_NO_COLLISIONS)) {
+        TB_TRY(launch_row_sets(h, d_in, d_acc, ctl, only_inst, false, -1));
         for (size_t gi = 0; gi < h->groups.size(); ++gi) {
             GroupChan& G = h->groups[gi];
-            if (G.tup.n == 0 && !G.stream) continue;
+            if ((G.tup.n == 0 && !G.stream) || G.use_rows) continue;
             const InstDev* insts = G.d_insts;
             int n_insts = int(G.insts.size());
             if (only_inst >= 0) {
@@ -633,22 +718,75 @@ int run_rhs_acc(tb_handle* h, const double* d_in, double* d_acc, const DPCtl* ct
     return TB_OK;
 }
 
+// AUTO evaluates FP64 channels of at most three legs and 64 points over packed
+// rows, unless this many runs share one: there the contraction reads its f
+// run-minor.  Up to here the rows were faster at every size measured (12x12 to
+// 40x40: 1 run 36 against 56 and 119 against 443 us, 7 runs 70 against 116 and
+// 596 against 1513 us, 12 runs 100 against 150 and 1003 against 2412 us).
+constexpr int ROWS_MAX_INSTS = 16;
+
 // Times every contraction schedule of every moment-tensor group on a
 // representative state (all coefficients 0.25; the cost does not depend on
 // the values) and keeps the fastest (tune_tensor).  The accumulator is
 // cleared afterwards.
+static int tune_rows(tb_handle* h, GroupChan& G) {
+    const int rc = ensure_tensor(h, G);
+    if (rc == TB_ERR_OOM) return TB_OK;   // no room for the tensor: the rows stay
+    TB_TRY(rc);
+    TB_TRY(tune_tensor(G.dev, G.d_insts, int(G.insts.size()), G.tensor, G.tup.d, G.tup.cap, G.tup.n, h->d_f, h->d_acc,
+                       h->stream));
+    cudaEvent_t e0, e1;
+    TB_CUDA(cudaEventCreate(&e0));
+    TB_CUDA(cudaEventCreate(&e1));
+    TB_TRY(launch_rows_prepare(h->ed, h->d_f, h->d_f4, h->d_nf, nullptr, h->stream));
+    constexpr int REPS = 3;
+    for (int r = 0; r <= REPS; ++r) {
+        if (r == 1) cudaEventRecord(e0, h->stream);   // after a warm-up launch
+        TB_TRY(launch_rows(G.row_one, h->ed, h->d_f4, h->d_nf, h->d_acc, nullptr, h->stream, false, -1, h->fx, h->d_err,
+                           G.dev.wait_polls));
+    }
+    cudaEventRecord(e1, h->stream);
+    TB_CUDA(cudaEventSynchronize(e1));
+    float ms = 0.f;
+    cudaEventElapsedTime(&ms, e0, e1);
+    cudaEventDestroy(e0);
+    cudaEventDestroy(e1);
+    G.rows_seconds = 1e-3 * double(ms) / REPS;
+    if (G.rows_seconds <= G.tensor.tuned_seconds) G.tensor.release();
+    else G.use_rows = false;
+    return TB_OK;
+}
+
 int autotune(tb_handle* h) {
     const size_t n = size_t(h->ndofs);
     std::vector<double> probe(n, 0.25);
     TB_CUDA(cudaMemcpyAsync(h->d_f, probe.data(), sizeof(double) * n, cudaMemcpyHostToDevice, h->stream));
     for (auto& G : h->groups) {
         if (G.layout == TB_LAYOUT_MC64 || G.tup.n == 0) continue;
+        if (G.use_rows) {
+            TB_TRY(tune_rows(h, G));
+            continue;
+        }
         TB_TRY(tune_tensor(G.dev, G.d_insts, int(G.insts.size()), G.tensor, G.tup.d, G.tup.cap, G.tup.n, h->d_f,
                            h->d_acc, h->stream));
     }
     TB_CUDA(cudaMemsetAsync(h->d_acc, 0, sizeof(double) * n, h->stream));
     TB_CUDA(cudaStreamSynchronize(h->stream));
-    return TB_OK;
+    return refresh_row_sets(h);
+}
+
+static int build_group_tensor(tb_handle* h, GroupChan& G, int kind) {
+    TB_TRY(build_tensor(G.dev, G.tup.d, G.tup.cap, G.tup.n, kind, G.tensor, h->stream));
+    std::vector<int> runs_of;
+    for (int id : G.insts) runs_of.push_back(h->insts[id].run);
+    std::sort(runs_of.begin(), runs_of.end());
+    const bool distinct = std::adjacent_find(runs_of.begin(), runs_of.end()) == runs_of.end();
+    return prepare_runs(G.dev, int(G.insts.size()), distinct, G.tensor, h->stream, h->opts.deterministic != 0);
+}
+
+int ensure_tensor(tb_handle* h, GroupChan& G) {
+    if (G.tensor.d) return TB_OK;
+    return build_group_tensor(h, G, TK_F64);
 }
 
 int choose_layouts(tb_handle* h) {
@@ -682,13 +820,16 @@ int choose_layouts(tb_handle* h) {
         }
         G.layout = want;
         if (want != TB_LAYOUT_MC64) {
-            TB_TRY(build_tensor(G.dev, G.tup.d, G.tup.cap, G.tup.n, kind, G.tensor, h->stream));
-            std::vector<int> runs_of;
-            for (int id : G.insts) runs_of.push_back(h->insts[id].run);
-            std::sort(runs_of.begin(), runs_of.end());
-            const bool distinct = std::adjacent_find(runs_of.begin(), runs_of.end()) == runs_of.end();
-            TB_TRY(prepare_runs(G.dev, int(G.insts.size()), distinct, G.tensor, h->stream,
-                                h->opts.deterministic != 0));
+            // AUTO's FP64 channels go over their packed rows; the tensor is
+            // built when a contraction schedule is asked for
+            if (h->opts.layout == TB_LAYOUT_AUTO && want == TB_LAYOUT_T64 && int(G.insts.size()) < ROWS_MAX_INSTS) {
+                TB_TRY(build_theta_list(G.dev, G.tup, G.theta, h->stream));
+                if (G.theta.built) TB_TRY(build_rows(G.dev, G.theta, G.rows, h->stream));
+                G.use_rows = G.rows.blk != nullptr;
+                if (G.use_rows) continue;
+                G.theta.release();
+            }
+            TB_TRY(build_group_tensor(h, G, kind));
         }
     }
     return TB_OK;
@@ -886,8 +1027,11 @@ int tb_destroy(tb_handle* h) {
         G.tup.release();
         G.tensor.release();
         G.theta.release();
+        G.rows.release();
+        G.row_one.release();
         if (G.d_tamp) cudaFree(G.d_tamp);
     }
+    for (auto& rs : h->row_sets) rs.release();
     for (double* p : h->dev_allocs) cudaFree(p);
     for (void* p : h->dev_raw) cudaFree(p);
     if (h->dp.dense) cudaFree(h->dp.dense);
@@ -955,7 +1099,7 @@ int tb_channel_points_inside(const tb_handle* h, int ch, int64_t* n_tuples, int6
         if (n_points) *n_points = int64_t(cnt[3]);
         return TB_OK;
     }
-    const bool has = G.layout == TB_LAYOUT_MC64 && G.theta.built;
+    const bool has = G.theta.built;
     if (n_tuples) *n_tuples = has ? G.theta.n : -1;
     if (n_points) *n_points = has ? G.theta.points : -1;
     return TB_OK;
@@ -970,17 +1114,17 @@ int tb_channel_schedule(const tb_handle* h, int ch, int32_t* stages, int32_t* pa
         if (seconds) *seconds = 0.0;
         return TB_OK;
     }
-    const bool tensor = G.layout != TB_LAYOUT_MC64;
+    const bool tensor = G.layout != TB_LAYOUT_MC64 && !G.use_rows;
     if (stages) *stages = tensor ? G.tensor.stages : 0;
     if (pair)
-        *pair = !tensor                ? (G.theta.use ? 6 : 0)
+        *pair = !tensor                ? (G.use_rows || G.theta.use ? 6 : 0)
                 : G.tensor.runs == 32 ? 2
                 : G.tensor.runs == 8  ? 3
                 : G.tensor.runs == 4  ? 4
                 : G.tensor.runs == 16 ? 5
                 : (G.L <= 3 && G.insts.size() > 1) ? G.tensor.pair
                                                    : 0;
-    if (seconds) *seconds = tensor ? G.tensor.tuned_seconds : 0.0;
+    if (seconds) *seconds = tensor ? G.tensor.tuned_seconds : G.rows_seconds;
     return TB_OK;
 }
 
@@ -1003,8 +1147,26 @@ int tb_set_channel_schedule(tb_handle* h, int ch, int32_t stages, int32_t pair) 
         TB_CUDA(cudaSetDevice(h->device));
         TB_CUDA(cudaStreamSynchronize(h->stream));
         G.theta.use = pair == 6;
+        G.use_rows = pair == 6 && G.rows.blk;
+        TB_TRY(refresh_row_sets(h));
         if (h->graph) { cudaGraphExecDestroy(h->graph); h->graph = nullptr; }
         return TB_OK;
+    }
+    if (G.rows.blk) {   // AUTO's FP64 channel: its rows, or a contraction whose tensor is built now
+        const bool rows = stages == 0 && pair == 6;
+        if (!rows && (stages < 1 || stages > 2 || pair < 0 || pair > 5)) {
+            set_error("stages must be 1..2 and pair 0..5, or stages 0 and pair 6 (packed rows)");
+            return TB_ERR_ARG;
+        }
+        TB_CUDA(cudaSetDevice(h->device));
+        TB_CUDA(cudaStreamSynchronize(h->stream));
+        if (!rows) TB_TRY(ensure_tensor(h, G));
+        if (rows || pair < 2 || G.tensor.fT) {
+            G.use_rows = rows;
+            TB_TRY(refresh_row_sets(h));
+            if (h->graph) { cudaGraphExecDestroy(h->graph); h->graph = nullptr; }
+            if (rows) return TB_OK;
+        }
     }
     if (stages < 1 || stages > 2 || pair < 0 || pair > 5) { set_error("stages must be 1..2 and pair 0..5"); return TB_ERR_ARG; }
     if (pair >= 2 && !G.tensor.fT) {
@@ -1140,6 +1302,7 @@ int tb_set_channel_amplitude_fn(tb_handle* h, int ch, tb_amplitude_fn fn, void* 
     const int64_t n = G.tup.n;
     if (G.d_tamp) { cudaFree(G.d_tamp); G.d_tamp = nullptr; }
     G.dev.tamp = nullptr;
+    if (G.use_rows) TB_TRY(refresh_row_sets(h));   // the sets hold the table's address
     if (fn && n > 0) {
         if (cudaMalloc(&G.d_tamp, sizeof(double) * size_t(n)) != cudaSuccess) {
             G.d_tamp = nullptr;
@@ -1171,6 +1334,7 @@ int tb_set_channel_amplitude_fn(tb_handle* h, int ch, tb_amplitude_fn fn, void* 
     if (G.layout != TB_LAYOUT_MC64 && G.tensor.d)
         TB_TRY(refill_tensor(G.dev, G.tup.d, G.tup.cap, G.tup.n, G.tensor, h->stream));
     TB_TRY(stream_wait(h));
+    if (G.use_rows) TB_TRY(refresh_row_sets(h));
     if (h->graph) { cudaGraphExecDestroy(h->graph); h->graph = nullptr; }   // kernels take the channel by value
     return TB_OK;
 }
@@ -1253,9 +1417,10 @@ int tb_scattering_rates(tb_handle* h, int ch, int leg, const double* f, double* 
         d_res = h->d_out;
     }
     TB_CUDA(cudaMemsetAsync(h->d_acc, 0, bytes, h->stream));
+    TB_TRY(launch_row_sets(h, d_in, h->d_acc, nullptr, ch, true, leg));
     for (size_t gi = 0; gi < h->groups.size(); ++gi) {
         GroupChan& G = h->groups[gi];
-        if (G.tup.n == 0 && !G.stream) continue;
+        if ((G.tup.n == 0 && !G.stream) || G.use_rows) continue;
         const InstDev* insts = G.d_insts;
         int n_insts = int(G.insts.size());
         if (ch >= 0) {

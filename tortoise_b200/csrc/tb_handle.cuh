@@ -10,6 +10,7 @@
 #include "tb_dp45.cuh"
 #include "tb_enumerate.cuh"
 #include "tb_kernels.cuh"
+#include "tb_rows.cuh"
 #include "tb_stream.cuh"
 #include "tb_tensor.cuh"
 #include "tb_theta.cuh"
@@ -31,7 +32,14 @@ struct GroupChan {
     int64_t diag[3] = {0, 0, 0};
     int layout = TB_LAYOUT_MC64;
     MomentTensor tensor;
-    ThetaList theta;              // Monte-Carlo layout: tuples with points inside the simplices, and which
+    ThetaList theta;              // tuples with points inside the simplices, and which (Monte-Carlo layout, rows)
+    // packed rows of those tuples (at most three legs; tb_rows.cuh): use_rows
+    // evaluates the channel over them, alone or with the handle's other such
+    // channels; row_one is the set of this channel only
+    PointRows rows;
+    bool use_rows = false;
+    double rows_seconds = 0.0;    // launch time the autotuner measured
+    RowSet row_one;
     // streamed channel (TB_LAYOUT_STREAM): the candidate walk and this
     // handle's part [item_begin, item_end) of its work items; counts of the
     // last evaluation (prefilter, determinant, survivors, points inside,
@@ -83,6 +91,11 @@ struct tb_handle {
     double* d_out = nullptr;
     double* d_acc = nullptr;
     double* d_part = nullptr;
+    // channels evaluated over packed rows, by leg count and directions; the
+    // state padded to four doubles an element, and its non-finite blocks
+    std::vector<tb::RowSet> row_sets;
+    double4* d_f4 = nullptr;
+    int* d_nf = nullptr;
     // deterministic mode: the exact accumulator behind d_acc (3 words per
     // dof and a poison word; w == nullptr otherwise)
     tb::FxAcc fx{};
@@ -120,6 +133,11 @@ struct tb_handle {
 namespace tb {
 
 double* dev_alloc(tb_handle* h, size_t n);
+// The row sets of the handle and of each channel, after a change of what they
+// hold (the stream must be idle).
+int refresh_row_sets(tb_handle* h);
+// The moment tensor of a channel that was evaluated over rows so far.
+int ensure_tensor(tb_handle* h, GroupChan& G);
 int run_rhs_acc(tb_handle* h, const double* d_in, double* d_acc, const DPCtl* ctl, int flags, int only_inst);
 int dp_alloc(tb_handle* h, int64_t max_dense);
 int ensure_graph(tb_handle* h, int flags);

@@ -1,0 +1,891 @@
+// tb_rows.cu -- the collision operator over packed rows of tuples.
+//
+// In scatteringIntegrationTypeB (include/Physics/Scattering/IntegratorCore.hpp:
+// 260-357) a tuple contributes through its Monte-Carlo points inside the
+// simplices only (tb_theta.cu), and everything but the legs' f is fixed for the
+// life of a handle.  A row keeps, for 32 tuples that share their leg-0 element,
+// the affine map of the constrained coordinates, the weight and the mask of
+// points inside, so an evaluation reads 120 bytes per three-leg tuple, in whole
+// lines, instead of the 864 bytes of its moments or the element tables of
+// three legs.
+//
+//   * One warp takes consecutive rows, one lane per tuple.  Rows of one leg-0
+//     element follow one another and their tuples are sorted by point count,
+//     so the lanes of a warp run nearly the same number of points, and leg 0's
+//     three sums stay in registers until the element changes.
+//   * A point's coordinates q are read from a shared-memory table that holds
+//     16 copies side by side, one per lane of a half warp: the lanes visit
+//     different points, and with one copy their 64-bit reads would collide.
+//   * The legs' linear forms and the test functions are affine in q, so the
+//     tuple's map is folded into the forms' coefficients once and the loop over
+//     the points accumulates 1 + R sums (of the integrand times 1 and q);
+//     the constrained legs' moments follow from those after the loop.
+//   * A warp's rows come by bulk copies into its own shared-memory stages, one
+//     row ahead, and the map is read there, so it takes no registers.
+//   * Legs 1 and 2 are staged in shared memory and added by consecutive lanes,
+//     so the three adds of an element fall into one or two sectors (added lane
+//     by lane they bound the kernel: 587 against 336 us at 64x64 e-ph).
+//   * All channels of a handle run in one launch; blocks are dealt out by cost.
+//
+// Measured (64x64 two-band e-ph, 8.7 M tuples, 50 M points, whole right-hand
+// side): 333 us against 1589 us through the FP64 moment tensor; three bands and
+// two phonons at 72x56: 689 against 3283 us; the rates of every leg at 40x24
+// with umklapp: 203 against 1797 us.  The kernel reads 3.4 TB/s and issues half
+// of the time, with 27 % of the FP64 pipe: fixed-latency dependencies of the
+// 16 warps on an SM bound it, then the shared-memory pipe (65 %).
+//
+// The deterministic mode keeps the arithmetic of the streamed and list kernels
+// (tb_mcpoint.cuh), operation for operation, and adds exactly (tb_exact.cuh);
+// there leg 0's sums are kept as exact integers in registers.
+#include <algorithm>
+#include <atomic>
+#include <cmath>
+
+#include "tb_bulk.cuh"
+#include "tb_dp45.cuh"
+#include "tb_geom.cuh"
+#include "tb_rows.cuh"
+
+namespace tb {
+
+constexpr int ROW_WARPS = 16;   // shares of rows that a block takes, one per warp
+// Warps of a block.  16 warps leave 128 registers a thread, which the
+// propagation and the exact variant fit; 20 spill (a 64x64 e-ph right-hand
+// side: 421 us against 336), 12 hide less latency (350).  The rates of every
+// leg take 12 (184 us against 210 at 16, 40x24 with umklapp).
+template <bool RATE, bool DET> struct RowCap { static constexpr int W = RATE && !DET ? 12 : ROW_WARPS; };
+constexpr int ROW_STAGES = 2;    // rows of a warp in shared memory
+constexpr int ROW_COPIES = 16;   // copies of the point table, one per lane of a half warp
+
+template <int L>
+struct RowDim {
+    static constexpr int R = 2 * (L - 2) + 1;
+    static constexpr int ND = 3 * (R + 1) + 1;   // doubles per tuple: a0, G, w
+    static constexpr int BYTES = 32 * (8 * ND + 8 + 4 * (L - 1));
+};
+
+size_t row_bytes(int L) { return L == 2 ? RowDim<2>::BYTES : RowDim<3>::BYTES; }
+
+void PointRows::release() {
+    if (blk) cudaFree(blk);
+    if (row_e0) cudaFree(row_e0);
+    if (perm) cudaFree(perm);
+    blk = nullptr;
+    row_e0 = nullptr;
+    perm = nullptr;
+    nrows = n = points = 0;
+    cost.clear();
+}
+
+void RowSet::release() {
+    if (d_chan) cudaFree(d_chan);
+    if (d_work) cudaFree(d_work);
+    d_chan = nullptr;
+    d_work = nullptr;
+    if (d_warp_row) cudaFree(d_warp_row);
+    d_warp_row = nullptr;
+    nblocks = 0;
+}
+
+// ------------------------------------------------------------------ build
+__global__ void k_rows_count(const int32_t* __restrict__ e0, int64_t n, int32_t* __restrict__ count) {
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+        atomicAdd(count + e0[i], 1);
+}
+
+// Tuple j of the sorted list goes to lane (j - first[e0]) % 32 of row
+// row0[e0] + (j - first[e0]) / 32.
+template <int L>
+__global__ void __launch_bounds__(256) k_rows_fill(ChanDev c, const int32_t* __restrict__ ids,
+                                                   const uint64_t* __restrict__ mask, const int32_t* __restrict__ perm,
+                                                   int64_t n, const int64_t* __restrict__ first,
+                                                   const int64_t* __restrict__ row0, unsigned char* __restrict__ blk,
+                                                   int32_t* __restrict__ row_e0, int32_t* __restrict__ row_perm,
+                                                   int32_t* __restrict__ row_pts) {
+    constexpr int R = RowDim<L>::R, ND = RowDim<L>::ND;
+    for (int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; j < n; j += (int64_t)gridDim.x * blockDim.x) {
+        int e[L];
+#pragma unroll
+        for (int l = 0; l < L; ++l) e[l] = ids[l * n + j];
+        const int u = ids[L * n + j];
+        TupleGeom<L> g;
+        tuple_geometry<L>(c, e, u, g);
+        double Ci[3][3];
+        dc_inverse<L>(g, Ci);
+        AlphaMap<L> am;
+        alpha_map<L>(g, Ci, am);
+        const int64_t k = j - first[e[0]];
+        const int64_t row = row0[e[0]] + k / 32;
+        const int lane = int(k % 32);
+        unsigned char* b = blk + row * RowDim<L>::BYTES;
+        double* d = reinterpret_cast<double*>(b) + lane;
+#pragma unroll
+        for (int r = 0; r < 3; ++r) {
+            d[32 * r] = am.a0[r];
+#pragma unroll
+            for (int q = 0; q < R; ++q) d[32 * (3 + r * R + q)] = am.G[r][q];
+        }
+        d[32 * (ND - 1)] = 1.0 / (c.fact * double(c.nmc) * fabs(g.det));
+        reinterpret_cast<uint64_t*>(b + 256 * ND)[lane] = mask[j];
+        int32_t* ei = reinterpret_cast<int32_t*>(b + 256 * (ND + 1));
+#pragma unroll
+        for (int l = 1; l < L; ++l) ei[32 * (l - 1) + lane] = e[l];
+        row_perm[row * 32 + lane] = perm[j];
+        atomicMax(row_pts + row, __popcll(mask[j]));
+        if (lane == 0) row_e0[row] = e[0];
+    }
+}
+
+namespace {
+struct Tmp {
+    std::vector<void*> p;
+    void* get(size_t bytes) {
+        void* q = nullptr;
+        if (cudaMalloc(&q, bytes + 16) != cudaSuccess) {
+            cudaGetLastError();
+            return nullptr;
+        }
+        p.push_back(q);
+        return q;
+    }
+    ~Tmp() {
+        for (void* q : p) cudaFree(q);
+    }
+};
+}  // namespace
+
+int build_rows(const ChanDev& c, const ThetaList& th, PointRows& rows, cudaStream_t s) {
+    rows.release();
+    const int64_t n = th.n;
+    if (n <= 0 || c.L > 3) return TB_OK;
+    const int ne = c.leg[0].ne;
+    Tmp tmp;
+    int32_t* d_cnt = static_cast<int32_t*>(tmp.get(sizeof(int32_t) * size_t(ne)));
+    int64_t* d_first = static_cast<int64_t*>(tmp.get(sizeof(int64_t) * size_t(ne)));
+    int64_t* d_row0 = static_cast<int64_t*>(tmp.get(sizeof(int64_t) * size_t(ne)));
+    if (!d_cnt || !d_first || !d_row0) return TB_OK;
+    TB_CUDA(cudaMemsetAsync(d_cnt, 0, sizeof(int32_t) * size_t(ne), s));
+    const unsigned blocks = unsigned(std::min<int64_t>((n + 255) / 256, 148 * 16));
+    k_rows_count<<<blocks, 256, 0, s>>>(th.ids, n, d_cnt);
+    TB_CUDA(cudaGetLastError());
+    std::vector<int32_t> cnt(size_t(ne), 0);
+    TB_CUDA(cudaMemcpyAsync(cnt.data(), d_cnt, sizeof(int32_t) * size_t(ne), cudaMemcpyDeviceToHost, s));
+    TB_CUDA(cudaStreamSynchronize(s));
+    std::vector<int64_t> first(size_t(ne), 0), row0(size_t(ne), 0);
+    int64_t at = 0, nrows = 0;
+    for (int e = 0; e < ne; ++e) {
+        first[size_t(e)] = at;
+        row0[size_t(e)] = nrows;
+        at += cnt[size_t(e)];
+        nrows += (cnt[size_t(e)] + 31) / 32;
+    }
+    int32_t* d_pts = static_cast<int32_t*>(tmp.get(sizeof(int32_t) * size_t(nrows)));
+    const size_t bytes = row_bytes(c.L) * size_t(nrows);
+    if (!d_pts || cudaMalloc(&rows.blk, bytes) != cudaSuccess ||
+        cudaMalloc(&rows.row_e0, sizeof(int32_t) * size_t(nrows)) != cudaSuccess ||
+        cudaMalloc(&rows.perm, sizeof(int32_t) * size_t(nrows) * 32) != cudaSuccess) {
+        cudaGetLastError();
+        rows.release();
+        return TB_OK;
+    }
+    TB_CUDA(cudaMemsetAsync(rows.blk, 0, bytes, s));   // padding: no points, element 0
+    TB_CUDA(cudaMemsetAsync(rows.perm, 0xff, sizeof(int32_t) * size_t(nrows) * 32, s));
+    TB_CUDA(cudaMemsetAsync(d_pts, 0, sizeof(int32_t) * size_t(nrows), s));
+    TB_CUDA(cudaMemcpyAsync(d_first, first.data(), sizeof(int64_t) * size_t(ne), cudaMemcpyHostToDevice, s));
+    TB_CUDA(cudaMemcpyAsync(d_row0, row0.data(), sizeof(int64_t) * size_t(ne), cudaMemcpyHostToDevice, s));
+    if (c.L == 2)
+        k_rows_fill<2><<<blocks, 256, 0, s>>>(c, th.ids, th.mask, th.perm, n, d_first, d_row0, rows.blk, rows.row_e0,
+                                              rows.perm, d_pts);
+    else
+        k_rows_fill<3><<<blocks, 256, 0, s>>>(c, th.ids, th.mask, th.perm, n, d_first, d_row0, rows.blk, rows.row_e0,
+                                              rows.perm, d_pts);
+    TB_CUDA(cudaGetLastError());
+    std::vector<int32_t> pts(size_t(nrows), 0);
+    TB_CUDA(cudaMemcpyAsync(pts.data(), d_pts, sizeof(int32_t) * size_t(nrows), cudaMemcpyDeviceToHost, s));
+    TB_CUDA(cudaStreamSynchronize(s));
+    rows.cost.assign(size_t(nrows) + 1, 0);
+    for (int64_t r = 0; r < nrows; ++r) rows.cost[size_t(r) + 1] = rows.cost[size_t(r)] + 6 + pts[size_t(r)];
+    rows.nrows = nrows;
+    rows.n = n;
+    rows.points = th.points;
+    return TB_OK;
+}
+
+// ----------------------------------------------------------------- prepare
+__global__ void __launch_bounds__(256) k_rows_prepare(ElemDev ed, const double* __restrict__ f, double4* __restrict__ f4,
+                                                      int* __restrict__ nf, const DPCtl* __restrict__ ctl) {
+    const int band = ed.blk_band[blockIdx.x];
+    const BandDev& bd = ed.bands[band];
+    bool bad = false;
+    const int e = (blockIdx.x - ed.blk_first[band]) * blockDim.x + threadIdx.x;
+    if (e < bd.ne && !(ctl && ctl[ed.band_run[band]].done)) {
+        const int64_t o = bd.off + 3 * (int64_t)e;
+        const double x = f[o], y = f[o + 1], z = f[o + 2];
+        f4[bd.off / 3 + e] = make_double4(x, y, z, 0.0);
+        bad = !(isfinite(x) && isfinite(y) && isfinite(z));
+    }
+    bad = __syncthreads_or(bad);
+    if (threadIdx.x == 0) nf[blockIdx.x] = bad ? 1 : 0;
+}
+
+int launch_rows_prepare(const ElemDev& ed, const double* f, double4* f4, int* nf, const DPCtl* ctl, cudaStream_t s) {
+    k_rows_prepare<<<ed.nblk, 256, 0, s>>>(ed, f, f4, nf, ctl);
+    TB_CUDA(cudaGetLastError());
+    return TB_OK;
+}
+
+// -------------------------------------------------------------- evaluation
+// The point table of one lane: entry j of point m at q[(m R + j) ROW_COPIES].
+struct RowTable {
+    const double* q;
+    __device__ __forceinline__ double operator()(int i) const { return q[i * ROW_COPIES]; }
+};
+
+// One tuple's map, from this lane's column of the staged row.
+template <int L>
+struct RowMap {
+    static constexpr int R = RowDim<L>::R;
+    double a0_[3], G_[3][R];
+    __device__ __forceinline__ explicit RowMap(const double* d) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            a0_[k] = d[32 * k];
+#pragma unroll
+            for (int j = 0; j < R; ++j) G_[k][j] = d[32 * (3 + k * R + j)];
+        }
+    }
+    __device__ __forceinline__ double a0(int k) const { return a0_[k]; }
+    __device__ __forceinline__ double G(int k, int j) const { return G_[k][j]; }
+};
+
+// The padded coefficients of one element in one 32-byte load.
+__device__ __forceinline__ double4 load_f4(const double4* p) {
+    double4 v;
+    asm("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(v.w) : "l"(p));
+    return v;
+}
+
+// The values a tuple adds to its legs' elements: v[l] = (1, x_l, y_l)
+// moments of the integrand, scaled.
+template <int L>
+struct RowOut {
+    double v[L][3];
+};
+
+// Whether leg l is ingoing: from the template's direction mask, or (DIRS < 0)
+// from the channel.
+template <int DIRS>
+__device__ __forceinline__ bool leg_in(const RowChan& c, int l) {
+    return DIRS >= 0 ? ((DIRS >> l) & 1) != 0 : c.leg[l].dir > 0.0;
+}
+
+// The legs' linear forms as affine functions of q.  Free leg l < L - 2 lies
+// at (q[2l], q[2l+1]), leg L - 2 at (q[R-1], al0), leg L - 1 at (al1, al2)
+// with al = a0 + G q (IntegratorCore.hpp:298-320).
+template <int L>
+struct RowForms {
+    static constexpr int R = RowDim<L>::R;
+    double fr[L > 2 ? L - 2 : 1][3];   // free legs
+    double p0, p[R], c0, c[R];
+    __device__ __forceinline__ void set(const RowMap<L>& m, const double4 (&f)[L]) {
+#pragma unroll
+        for (int l = 0; l < L - 2; ++l) { fr[l][0] = f[l].x; fr[l][1] = f[l].y; fr[l][2] = f[l].z; }
+        const double4 P = f[L - 2], C = f[L - 1];
+        p0 = fma(P.z, m.a0(0), P.x);
+        c0 = fma(C.z, m.a0(2), fma(C.y, m.a0(1), C.x));
+#pragma unroll
+        for (int j = 0; j < R; ++j) {
+            p[j] = j == R - 1 ? fma(P.z, m.G(0, j), P.y) : P.z * m.G(0, j);
+            c[j] = fma(C.z, m.G(2, j), C.y * m.G(1, j));
+        }
+    }
+    __device__ __forceinline__ void at(const double (&q)[R], double (&t)[L]) const {
+#pragma unroll
+        for (int l = 0; l < L - 2; ++l) t[l] = fma(fr[l][2], q[2 * l + 1], fma(fr[l][1], q[2 * l], fr[l][0]));
+        double a = p0, b = c0;
+#pragma unroll
+        for (int j = 0; j < R; ++j) { a = fma(p[j], q[j], a); b = fma(c[j], q[j], b); }
+        t[L - 2] = a;
+        t[L - 1] = b;
+    }
+};
+
+// Propagation of one tuple: the loss and gain forms of a leg
+// (ScatteringChannel.cpp:633-641) are t and 1 + s t (s the statistics), in
+// this order for an ingoing leg and swapped for an outgoing one; the loss
+// product carries leg 0's minus sign.
+template <int L, int DIRS>
+__device__ __forceinline__ void row_tuple(const RowChan& c, const RowMap<L>& m, uint64_t mk, const double4 (&f)[L],
+                                          const RowTable& tab, double scale, RowOut<L>& o) {
+    constexpr int R = RowDim<L>::R;
+    RowForms<L> F;
+    F.set(m, f);
+    double s0 = 0.0, sq[R];
+#pragma unroll
+    for (int j = 0; j < R; ++j) sq[j] = 0.0;
+    double st[L];
+#pragma unroll
+    for (int l = 0; l < L; ++l) st[l] = c.leg[l].stat;
+    auto product = [&](const double (&t)[L]) {
+        double pa = 1.0, pb = 1.0;
+#pragma unroll
+        for (int l = 0; l < L; ++l) {
+            const double u = fma(st[l], t[l], 1.0);
+            const bool in = leg_in<DIRS>(c, l);
+            const double a = in ? t[l] : u, b = in ? u : t[l];
+            pb = l ? pb * b : b;
+            if (l < L - 1) pa = l ? pa * a : a;
+            else pb = fma(-pa, a, pb);
+        }
+        return pb;
+    };
+    for (; mk; mk &= mk - 1) {
+        const int i = (__ffsll((long long)mk) - 1) * R;
+        double q[R], t[L];
+#pragma unroll
+        for (int j = 0; j < R; ++j) q[j] = tab(i + j);
+        F.at(q, t);
+        const double v = product(t);
+        s0 += v;
+#pragma unroll
+        for (int j = 0; j < R; ++j) sq[j] = fma(q[j], v, sq[j]);
+    }
+    s0 *= scale;
+#pragma unroll
+    for (int j = 0; j < R; ++j) sq[j] *= scale;
+    double y = m.a0(0) * s0, cx = m.a0(1) * s0, cy = m.a0(2) * s0;
+#pragma unroll
+    for (int j = 0; j < R; ++j) {
+        y = fma(m.G(0, j), sq[j], y);
+        cx = fma(m.G(1, j), sq[j], cx);
+        cy = fma(m.G(2, j), sq[j], cy);
+    }
+#pragma unroll
+    for (int l = 0; l < L; ++l) {
+        const bool in = leg_in<DIRS>(c, l);
+        const double x = l < L - 2 ? sq[l < L - 2 ? 2 * l : 0] : l == L - 2 ? sq[R - 1] : cx;
+        const double z = l < L - 2 ? sq[l < L - 2 ? 2 * l + 1 : 0] : l == L - 2 ? y : cy;
+        o.v[l][0] = in ? s0 : -s0;
+        o.v[l][1] = in ? x : -x;
+        o.v[l][2] = in ? z : -z;
+    }
+}
+
+// Scattering rates of one tuple: leg r's forms become the unit forms
+// (ScatteringChannel.cpp:562-564), for every leg r in one pass over the points.
+template <int L, int DIRS>
+__device__ __forceinline__ void row_tuple_rate(const RowChan& c, const RowMap<L>& m, uint64_t mk,
+                                               const double4 (&f)[L], const RowTable& tab, double scale,
+                                               RowOut<L>& o) {
+    constexpr int R = RowDim<L>::R;
+    RowForms<L> F;
+    F.set(m, f);
+    double s0[L], sq[L][R];
+#pragma unroll
+    for (int l = 0; l < L; ++l) {
+        s0[l] = 0.0;
+#pragma unroll
+        for (int j = 0; j < R; ++j) sq[l][j] = 0.0;
+    }
+    double st[L];
+#pragma unroll
+    for (int l = 0; l < L; ++l) st[l] = c.leg[l].stat;
+    for (; mk; mk &= mk - 1) {
+        const int i = (__ffsll((long long)mk) - 1) * R;
+        double q[R], t[L], a[L], b[L];
+#pragma unroll
+        for (int j = 0; j < R; ++j) q[j] = tab(i + j);
+        F.at(q, t);
+#pragma unroll
+        for (int l = 0; l < L; ++l) {
+            const double u = fma(st[l], t[l], 1.0);
+            const bool in = leg_in<DIRS>(c, l);
+            a[l] = in ? t[l] : u;
+            b[l] = in ? u : t[l];
+        }
+#pragma unroll
+        for (int r = 0; r < L; ++r) {
+            const bool in = leg_in<DIRS>(c, r);
+            double pa = in ? -2.0 : -2.0 * st[r], pb = in ? 2.0 * st[r] : 2.0;
+#pragma unroll
+            for (int l = 0; l < L; ++l)
+                if (l != r) { pa *= a[l]; pb *= b[l]; }
+            const double v = pa + pb;
+            s0[r] += v;
+#pragma unroll
+            for (int j = 0; j < R; ++j)
+                if (r >= L - 2 || j / 2 == r) sq[r][j] = fma(q[j], v, sq[r][j]);   // a free leg needs its own two
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < L; ++r) {
+        double x, z;
+        if (r < L - 2) {
+            x = sq[r][r < L - 2 ? 2 * r : 0];
+            z = sq[r][r < L - 2 ? 2 * r + 1 : 0];
+        } else {
+            const int y = r == L - 2 ? 0 : 2;
+            x = r == L - 2 ? sq[r][R - 1] : m.a0(1) * s0[r];
+            z = m.a0(y) * s0[r];
+#pragma unroll
+            for (int j = 0; j < R; ++j) {
+                if (r == L - 1) x = fma(m.G(1, j), sq[r][j], x);
+                z = fma(m.G(y, j), sq[r][j], z);
+            }
+        }
+        const double d = leg_in<DIRS>(c, r) ? -scale : scale;
+        o.v[r][0] = d * s0[r];
+        o.v[r][1] = d * x;
+        o.v[r][2] = d * z;
+    }
+}
+
+// The same two with the list and streamed kernels' operations in their order
+// (inside_point_sums, tb_mcpoint.cuh): the deterministic mode's bits.
+template <int L, bool RATE>
+__device__ __forceinline__ void row_tuple_listed(const RowChan& c, const RowMap<L>& m, uint64_t mk,
+                                                 const double4 (&f)[L], const RowTable& tab, double w, double ampt,
+                                                 RowOut<L>& o) {
+    constexpr int R = RowDim<L>::R;
+    constexpr int NR = RATE ? L : 1;
+    double s0[NR], sx[L], sy[L];
+#pragma unroll
+    for (int r = 0; r < NR; ++r) s0[r] = 0.0;
+#pragma unroll
+    for (int l = 0; l < L; ++l) { sx[l] = 0.0; sy[l] = 0.0; }
+    for (; mk; mk &= mk - 1) {
+        const int i = (__ffsll((long long)mk) - 1) * R;
+        double q[R], al[3], px[L], py[L], a[L], b[L];
+#pragma unroll
+        for (int j = 0; j < R; ++j) q[j] = tab(i + j);
+#pragma unroll
+        for (int r = 0; r < 3; ++r) {
+            double t = m.a0(r);
+#pragma unroll
+            for (int j = 0; j < R; ++j) t = fma(m.G(r, j), q[j], t);
+            al[r] = t;
+        }
+#pragma unroll
+        for (int l = 0; l < L - 2; ++l) { px[l] = q[2 * l]; py[l] = q[2 * l + 1]; }
+        px[L - 2] = q[R - 1]; py[L - 2] = al[0];
+        px[L - 1] = al[1]; py[L - 1] = al[2];
+#pragma unroll
+        for (int l = 0; l < L; ++l) {
+            const double t = fma(f[l].z, py[l], fma(f[l].y, px[l], f[l].x));
+            a[l] = fma(c.leg[l].fa, t, c.leg[l].fa0);
+            b[l] = fma(c.leg[l].fb, t, c.leg[l].fb0);
+        }
+#pragma unroll
+        for (int r = 0; r < NR; ++r) {
+            double pa = 1.0, pb = 1.0;
+#pragma unroll
+            for (int l = 0; l < L; ++l) {
+                double x = a[l], y = b[l];
+                if (RATE && l == r) {
+                    const double d = c.leg[l].dir, s = c.leg[l].stat;
+                    x = (l == 0 ? -1.0 : 1.0) * __dadd_rn(__dmul_rn(1. - d, s), 1. + d);
+                    y = __dadd_rn(__dmul_rn(1. + d, s), 1. - d);
+                }
+                pa = __dmul_rn(pa, x);
+                pb = __dmul_rn(pb, y);
+            }
+            const double v = __dadd_rn(pa, pb);
+            s0[r] += v;
+#pragma unroll
+            for (int l = 0; l < L; ++l)
+                if (!RATE || l == r) { sx[l] = fma(px[l], v, sx[l]); sy[l] = fma(py[l], v, sy[l]); }
+        }
+    }
+#pragma unroll
+    for (int l = 0; l < L; ++l) {
+        const double d = RATE ? -c.leg[l].dir : c.leg[l].dir;
+        o.v[l][0] = d * ((w * s0[RATE ? l : 0]) * ampt);
+        o.v[l][1] = d * ((w * sx[l]) * ampt);
+        o.v[l][2] = d * ((w * sy[l]) * ampt);
+    }
+}
+
+// v on the exact grid, as fx_add takes it; false: nothing to add.
+__device__ __forceinline__ bool fx_grid(const FxAcc& a, double v, Fx& x) {
+    if (!fx_of(v, x)) {
+        if (!isfinite(v) || !a.sat) {
+            atomicOr(a.poison, 1u);
+            return false;
+        }
+        atomicOr(a.sat, 1u);
+        fx_of(v < 0.0 ? -FX_CLAMP : FX_CLAMP, x);
+    }
+    return true;
+}
+
+// Leg 0's sums of one warp, kept until the element changes.
+template <bool DET>
+struct LegZero {
+    double v[3] = {0.0, 0.0, 0.0};
+    __device__ __forceinline__ void add(const double (&x)[3], const FxAcc&) {
+#pragma unroll
+        for (int j = 0; j < 3; ++j) v[j] += x[j];
+    }
+    __device__ __forceinline__ void flush(double* acc, int64_t key, const FxAcc&) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+            for (int j = 0; j < 3; ++j) v[j] += __shfl_xor_sync(0xffffffffu, v[j], o);
+        const int lane = threadIdx.x & 31;
+        if (lane < 3) atomicAdd(acc + key + lane, lane == 0 ? v[0] : lane == 1 ? v[1] : v[2]);
+        v[0] = v[1] = v[2] = 0.0;
+    }
+};
+
+template <>
+struct LegZero<true> {
+    unsigned long long w[3][3] = {};
+    __device__ __forceinline__ void add(const double (&x)[3], const FxAcc& fx) {
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+            Fx g;
+            if (fx_grid(fx, x[j], g)) fx_add_plain(w[j], g);
+        }
+    }
+    __device__ __forceinline__ void flush(double*, int64_t key, const FxAcc& fx) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+            for (int j = 0; j < 3; ++j) {
+                Fx g;
+                g.w0 = __shfl_xor_sync(0xffffffffu, w[j][0], o);
+                g.w1 = __shfl_xor_sync(0xffffffffu, w[j][1], o);
+                g.w2 = __shfl_xor_sync(0xffffffffu, w[j][2], o);
+                fx_add_plain(w[j], g);
+            }
+        const int lane = threadIdx.x & 31;
+        if (lane < 3) {
+            Fx g;
+            g.w0 = lane == 0 ? w[0][0] : lane == 1 ? w[1][0] : w[2][0];
+            g.w1 = lane == 0 ? w[0][1] : lane == 1 ? w[1][1] : w[2][1];
+            g.w2 = lane == 0 ? w[0][2] : lane == 1 ? w[1][2] : w[2][2];
+            if (g.w0 | g.w1 | g.w2) fx_atomic_add(fx.w + 3 * (key + lane), g);
+        }
+#pragma unroll
+        for (int j = 0; j < 3; ++j) w[j][0] = w[j][1] = w[j][2] = 0ull;
+    }
+};
+
+__device__ __forceinline__ bool finite4(const double4& v) { return isfinite(v.x) && isfinite(v.y) && isfinite(v.z); }
+
+// A state with non-finite coefficients: the full quadrature multiplies the
+// integrand of every tuple by its Theta, also by 0, so each tuple that touches
+// such an element makes its legs NaN, also one without a point inside.  Tuples
+// [t0, t1) of the whole list.
+template <int L>
+__device__ __noinline__ void spread_nonfinite(const RowChan& c, const InstDev* insts, int n_insts, int64_t t0,
+                                              int64_t t1, const double4* f4, double* acc, const DPCtl* ctl, bool rate,
+                                              int rate_leg, const FxAcc& fx) {
+    const double nan = __longlong_as_double(0x7ff8000000000000ll);
+    for (int64_t i = t0 + threadIdx.x; i < t1; i += blockDim.x) {
+        int e[L];
+#pragma unroll
+        for (int l = 0; l < L; ++l) e[l] = __ldg(c.tup + l * c.stride + i);
+        for (int k = 0; k < n_insts; ++k) {
+            const InstDev& in = insts[k];
+            if (in.amp_full == 0.0 || (ctl && ctl[in.run].done)) continue;
+            bool bad[L];
+            int nbad = 0;
+#pragma unroll
+            for (int l = 0; l < L; ++l) {
+                bad[l] = !finite4(f4[in.foff[l] / 3 + e[l]]);
+                nbad += bad[l] ? 1 : 0;
+            }
+            if (nbad == 0) continue;
+#pragma unroll
+            for (int l = 0; l < L; ++l) {
+                // a leg's rate does not depend on its own f
+                if (rate && ((rate_leg >= 0 && l != rate_leg) || nbad == (bad[l] ? 1 : 0))) continue;
+                if (fx.w) atomicOr(fx.poison, 1u);
+                else
+                    for (int j = 0; j < 3; ++j) atomicAdd(acc + in.foff[l] + 3 * (int64_t)e[l] + j, nan);
+            }
+        }
+    }
+}
+
+template <int L, int DIRS, bool RATE, bool DET, bool MULTI>
+__global__ void __launch_bounds__(RowCap<RATE, DET>::W * 32, 1) k_rows(const RowChan* __restrict__ chans,
+                                                            const RowWork* __restrict__ work,
+                                                            const int32_t* __restrict__ warp_row, int shares,
+                                                            const InstDev* __restrict__ one,
+                                                            const double4* __restrict__ f4,
+                                                            const int* __restrict__ nf, int n_nf,
+                                                            double* __restrict__ acc, const DPCtl* __restrict__ ctl,
+                                                            int rate_leg, FxAcc fx, int* __restrict__ err_flag,
+                                                            int wait_polls) {
+    constexpr int R = RowDim<L>::R, ND = RowDim<L>::ND;
+    constexpr uint32_t BYTES = RowDim<L>::BYTES;
+    extern __shared__ __align__(128) unsigned char s_raw[];
+    __shared__ RowChan c;
+    __shared__ __align__(8) uint64_t s_bar[RowCap<RATE, DET>::W][ROW_STAGES];
+    const RowWork w = work[blockIdx.x];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, n_warps = blockDim.x >> 5;
+    for (int i = tid; i < int(sizeof(RowChan) / sizeof(int)); i += blockDim.x)
+        reinterpret_cast<int*>(&c)[i] = reinterpret_cast<const int*>(chans + w.chan)[i];
+    __syncthreads();
+    const InstDev* insts = one ? one : c.insts;
+    const int n_insts = one ? 1 : c.n_insts;
+    {
+        // every instance off or its run finished: nothing to add
+        bool any = false;
+        for (int k = 0; k < n_insts && !any; ++k)
+            any = insts[k].amp_full != 0.0 && !(ctl && ctl[insts[k].run].done);
+        if (!any) return;
+    }
+    // this warp's rows, and the copies of its first ones
+    int r0 = warp_row[w.share0 + warp], r1 = warp_row[w.share0 + warp + 1];
+    unsigned char* const stage = s_raw + size_t(warp) * ROW_STAGES * BYTES;
+    uint64_t* const bar = s_bar[warp];
+    auto fetch = [&](int r, int s) {
+        mbar_expect_tx_arrive(&bar[s], BYTES);
+        bulk_g2s(stage + s * BYTES, c.blk + int64_t(r) * BYTES, BYTES, &bar[s]);
+    };
+    auto fetch_first = [&](int used) {
+        for (int k = 0; k < ROW_STAGES; ++k)
+            if (r0 + k < r1) fetch(r0 + k, (used + k) % ROW_STAGES);
+    };
+    if (lane == 0) {
+        for (int s = 0; s < ROW_STAGES; ++s) mbar_init(&bar[s], 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        fetch_first(0);
+    }
+    double* const s_v = reinterpret_cast<double*>(s_raw + size_t(n_warps) * ROW_STAGES * BYTES) + warp * 96 * (L - 1);
+    double* const s_q = reinterpret_cast<double*>(s_raw + size_t(n_warps) * (ROW_STAGES * BYTES + 768 * (L - 1)));
+    for (int i = tid; i < c.nmc * R * ROW_COPIES; i += blockDim.x) s_q[i] = __ldg(c.mc + i / ROW_COPIES);
+    __syncthreads();
+    const RowTable tab{s_q + (lane & (ROW_COPIES - 1))};
+    LegZero<DET> z;
+    int e0 = -1;
+    double4 f0 = make_double4(0., 0., 0., 0.);
+    int64_t off[L], el[L];
+    double amp = 0.0;
+    if (!MULTI) {
+#pragma unroll
+        for (int l = 0; l < L; ++l) { off[l] = insts[0].foff[l]; el[l] = off[l] / 3; }
+        amp = insts[0].amp_full;
+    }
+    int e0_next = r0 < r1 ? __ldg(c.row_e0 + r0) : 0;   // the next row's leg-0 element
+    int share = warp, used = 0;   // this warp's share, and how many rows it has taken from its stages
+    for (int r = r0;; ++r, ++used) {
+        while (r >= r1 && (share += n_warps) < shares) {   // fewer warps than shares: the next share
+            r = r0 = warp_row[w.share0 + share];
+            r1 = warp_row[w.share0 + share + 1];
+            if (lane == 0) fetch_first(used);
+            if (r < r1) e0_next = __ldg(c.row_e0 + r);
+        }
+        if (r >= r1) break;
+        const int s = used % ROW_STAGES;
+        const int e0_row = e0_next;
+        if (r + 1 < r1) e0_next = __ldg(c.row_e0 + r + 1);
+        if (!mbar_wait(&bar[s], uint32_t(used / ROW_STAGES) & 1u, wait_polls)) {
+            // record the failure and give the copies in flight a bounded
+            // chance to land before the block releases its shared memory
+            if (lane == 0) atomicExch(err_flag, 1);
+            for (int k = 0; k < ROW_STAGES && r + k < r1; ++k)
+                mbar_wait(&bar[(used + k) % ROW_STAGES], uint32_t((used + k) / ROW_STAGES) & 1u, 1 << 16);
+            break;
+        }
+        const unsigned char* b = stage + s * BYTES;
+        const RowMap<L> m(reinterpret_cast<const double*>(b) + lane);
+        const uint64_t mk = reinterpret_cast<const uint64_t*>(b + 256 * ND)[lane];
+        int e[L];
+        e[0] = e0_row;
+#pragma unroll
+        for (int l = 1; l < L; ++l) e[l] = reinterpret_cast<const int32_t*>(b + 256 * (ND + 1))[32 * (l - 1) + lane];
+        double tf = 1.0;
+        if (c.tamp && mk) tf = __ldg(c.tamp + __ldg(c.perm + int64_t(r) * 32 + lane));
+        const unsigned live = __ballot_sync(0xffffffffu, mk != 0ull);
+        if (!MULTI && e[0] != e0) {
+            if (e0 >= 0 && (!RATE || rate_leg <= 0)) z.flush(acc, off[0] + 3 * (int64_t)e0, fx);
+            e0 = e[0];
+            f0 = load_f4(f4 + el[0] + e0);
+        }
+        for (int k = 0; k < (MULTI ? n_insts : 1); ++k) {
+            if (MULTI) {
+                const InstDev& in = insts[k];
+                amp = in.amp_full;
+                if (amp == 0.0 || (ctl && ctl[in.run].done)) continue;
+#pragma unroll
+                for (int l = 0; l < L; ++l) { off[l] = in.foff[l]; el[l] = off[l] / 3; }
+                f0 = load_f4(f4 + el[0] + e[0]);
+            }
+            double4 f[L];
+            f[0] = f0;
+#pragma unroll
+            for (int l = 1; l < L; ++l) f[l] = load_f4(f4 + el[l] + e[l]);
+            RowOut<L> o;
+            const double wt = reinterpret_cast<const double*>(b)[32 * (ND - 1) + lane];
+            if (DET) row_tuple_listed<L, RATE>(c, m, mk, f, tab, wt, amp * tf, o);
+            else if (RATE) row_tuple_rate<L, DIRS>(c, m, mk, f, tab, wt * (amp * tf), o);
+            else row_tuple<L, DIRS>(c, m, mk, f, tab, wt * (amp * tf), o);
+            if (!RATE || rate_leg <= 0) {
+                z.add(o.v[0], fx);
+                if (MULTI) z.flush(acc, off[0] + 3 * (int64_t)e[0], fx);
+            }
+            if (DET) {
+#pragma unroll
+                for (int l = 1; l < L; ++l)
+                    if (mk && (!RATE || rate_leg < 0 || rate_leg == l))
+                        fx_add3(fx, off[l] + 3 * (int64_t)e[l], o.v[l][0], o.v[l][1], o.v[l][2]);
+            } else {
+                // entry 96 (l - 1) + 3 t + j: moment j of leg l of lane t's tuple
+                __syncwarp();
+#pragma unroll
+                for (int l = 1; l < L; ++l)
+#pragma unroll
+                    for (int j = 0; j < 3; ++j) s_v[96 * (l - 1) + 3 * lane + j] = o.v[l][j];
+                __syncwarp();
+#pragma unroll
+                for (int l = 1; l < L; ++l) {
+                    if (RATE && rate_leg >= 0 && rate_leg != l) continue;   // uniform
+#pragma unroll
+                    for (int p = 0; p < 3; ++p) {
+                        const int x = 32 * p + lane, t = x / 3;
+                        const int et = __shfl_sync(0xffffffffu, e[l], t);
+                        if ((live >> t) & 1u)
+                            atomicAdd(acc + off[l] + 3 * (int64_t)et + (x - 3 * t), s_v[96 * (l - 1) + x]);
+                    }
+                }
+            }
+        }
+        __syncwarp();   // every lane is done with the stage
+        if (lane == 0 && r + ROW_STAGES < r1) fetch(r + ROW_STAGES, s);
+    }
+    if (!MULTI && e0 >= 0 && (!RATE || rate_leg <= 0)) z.flush(acc, off[0] + 3 * (int64_t)e0, fx);
+    int bad = 0;
+    for (int i = tid; i < n_nf; i += blockDim.x) bad |= nf[i];
+    if (__syncthreads_or(bad))
+        spread_nonfinite<L>(c, insts, n_insts, w.t0, w.t1, f4, acc, ctl, RATE, rate_leg, fx);
+}
+
+static size_t rows_smem(int L, int nmc, int warps) {
+    return size_t(warps) * (ROW_STAGES * row_bytes(L) + 768 * size_t(L - 1)) +
+           sizeof(double) * size_t(nmc) * size_t(2 * (L - 2) + 1) * ROW_COPIES;
+}
+
+template <int L, int DIRS, bool RATE, bool DET, bool MULTI>
+static int launch_k_rows(const RowSet& rs, const ElemDev& ed, const double4* f4, const int* nf, double* acc,
+                         const DPCtl* ctl, cudaStream_t s, int rate_leg, const FxAcc& fx, const InstDev* one,
+                         int* err_flag, int polls) {
+    auto kern = k_rows<L, DIRS, RATE, DET, MULTI>;
+    // the shared-memory limit, set once on each device the kernel runs on
+    static std::atomic<unsigned long long> attr_devices{0};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev < 0 || dev >= 64 || !((attr_devices.load() >> dev) & 1ull)) {
+        TB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     int(rows_smem(L, 64, ROW_WARPS))));
+        if (dev >= 0 && dev < 64) attr_devices.fetch_or(1ull << dev);
+    }
+    const int warps = std::min(rs.shares, RowCap<RATE, DET>::W);
+    kern<<<unsigned(rs.nblocks), unsigned(32 * warps), rows_smem(L, rs.nmc_max, warps), s>>>(
+        rs.d_chan, rs.d_work, rs.d_warp_row, rs.shares, one, f4, nf, ed.nblk, acc, ctl, rate_leg, fx, err_flag, polls);
+    TB_CUDA(cudaGetLastError());
+    return TB_OK;
+}
+
+template <int L, int DIRS, bool RATE, bool DET>
+static int launch_rows_m(const RowSet& rs, const ElemDev& ed, const double4* f4, const int* nf, double* acc,
+                         const DPCtl* ctl, cudaStream_t s, int rate_leg, const FxAcc& fx, const InstDev* one,
+                         int* err_flag, int polls) {
+    if (rs.multi && !one)
+        return launch_k_rows<L, DIRS, RATE, DET, true>(rs, ed, f4, nf, acc, ctl, s, rate_leg, fx, one, err_flag, polls);
+    return launch_k_rows<L, DIRS, RATE, DET, false>(rs, ed, f4, nf, acc, ctl, s, rate_leg, fx, one, err_flag, polls);
+}
+
+// The directions of the channels that addScatteringChannelsWildcards builds in
+// the reference's examples ({in, in, out}, {in, out}) are compiled in; other
+// sets select the forms at run time.
+template <int L>
+static int launch_rows_l(const RowSet& rs, const ElemDev& ed, const double4* f4, const int* nf, double* acc,
+                         const DPCtl* ctl, cudaStream_t s, bool rate, int rate_leg, const FxAcc& fx,
+                         const InstDev* one, int* err_flag, int polls) {
+    constexpr int CANON = (1 << (L - 1)) - 1;   // every leg but the last ingoing
+#define TB_ROWS(DD, RR, XX) launch_rows_m<L, DD, RR, XX>(rs, ed, f4, nf, acc, ctl, s, rate_leg, fx, one, err_flag, polls)
+    if (fx.w) return rate ? TB_ROWS(-1, true, true) : TB_ROWS(-1, false, true);
+    if (rs.dirs == CANON) return rate ? TB_ROWS(CANON, true, false) : TB_ROWS(CANON, false, false);
+    return rate ? TB_ROWS(-1, true, false) : TB_ROWS(-1, false, false);
+#undef TB_ROWS
+}
+
+int launch_rows(const RowSet& rs, const ElemDev& ed, const double4* f4, const int* nf, double* acc, const DPCtl* ctl,
+                cudaStream_t s, bool rate, int rate_leg, const FxAcc& fx, int* err_flag, int polls,
+                const InstDev* one) {
+    if (rs.nblocks <= 0) return TB_OK;
+    if (rs.L == 2) return launch_rows_l<2>(rs, ed, f4, nf, acc, ctl, s, rate, rate_leg, fx, one, err_flag, polls);
+    if (rs.L == 3) return launch_rows_l<3>(rs, ed, f4, nf, acc, ctl, s, rate, rate_leg, fx, one, err_flag, polls);
+    set_error("rows hold two or three legs");
+    return TB_ERR_ARG;
+}
+
+int build_row_set(int L, int dirs, const std::vector<RowChan>& chan, const std::vector<const PointRows*>& rows,
+                  RowSet& out) {
+    out.release();
+    out.L = L;
+    out.dirs = dirs;
+    out.nmc_max = 0;
+    out.multi = false;
+    int64_t total = 0, nrows = 0;
+    for (size_t i = 0; i < chan.size(); ++i) {
+        total += rows[i]->cost.back();
+        nrows += rows[i]->nrows;
+        out.nmc_max = std::max(out.nmc_max, chan[i].nmc);
+        out.multi = out.multi || chan[i].n_insts > 1;
+    }
+    if (nrows <= 0) return TB_OK;
+    int dev = 0, nsm = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    // one block per SM; fewer warps in each where there are fewer rows than
+    // warps.  Every channel gets a block of its own at least, the others go one
+    // by one to the channel with the largest cost per block.
+    out.shares = int(std::min<int64_t>(ROW_WARPS, std::max<int64_t>(4, (nrows + nsm - 1) / nsm)));
+    std::vector<int64_t> nb(chan.size(), 1);
+    for (int64_t left = std::min<int64_t>(nsm, (nrows + out.shares - 1) / out.shares) - int64_t(chan.size()); left > 0;
+         --left) {
+        size_t best = 0;
+        for (size_t i = 1; i < chan.size(); ++i)
+            if (double(rows[i]->cost.back()) / double(nb[i]) > double(rows[best]->cost.back()) / double(nb[best])) best = i;
+        nb[best] += 1;
+    }
+    std::vector<RowWork> work;
+    std::vector<int32_t> warp_row;
+    for (size_t i = 0; i < chan.size(); ++i) {
+        const std::vector<int64_t>& cost = rows[i]->cost;
+        const int64_t parts = nb[i] * out.shares;
+        // rows up to the p-th share of the cost
+        auto bound = [&](int64_t p) {
+            return int32_t(std::lower_bound(cost.begin(), cost.end(), cost.back() * p / parts) - cost.begin());
+        };
+        for (int64_t b = 0; b < nb[i]; ++b) {
+            RowWork w{};
+            w.chan = int(i);
+            w.share0 = int(warp_row.size());
+            w.t0 = chan[i].n * b / nb[i];
+            w.t1 = chan[i].n * (b + 1) / nb[i];
+            work.push_back(w);
+            for (int64_t p = b * out.shares; p <= (b + 1) * out.shares; ++p) warp_row.push_back(bound(p));
+        }
+    }
+    if (cudaMalloc(&out.d_chan, sizeof(RowChan) * chan.size()) != cudaSuccess ||
+        cudaMalloc(&out.d_warp_row, sizeof(int32_t) * warp_row.size()) != cudaSuccess ||
+        cudaMalloc(&out.d_work, sizeof(RowWork) * work.size()) != cudaSuccess) {
+        cudaGetLastError();
+        out.release();
+        set_error("row set allocation failed");
+        return TB_ERR_OOM;
+    }
+    TB_CUDA(cudaMemcpy(out.d_chan, chan.data(), sizeof(RowChan) * chan.size(), cudaMemcpyHostToDevice));
+    TB_CUDA(cudaMemcpy(out.d_work, work.data(), sizeof(RowWork) * work.size(), cudaMemcpyHostToDevice));
+    TB_CUDA(cudaMemcpy(out.d_warp_row, warp_row.data(), sizeof(int32_t) * warp_row.size(), cudaMemcpyHostToDevice));
+    out.nblocks = int(work.size());
+    return TB_OK;
+}
+
+}  // namespace tb

@@ -1,0 +1,91 @@
+// tb_rows.cuh -- packed rows of tuples: the Monte-Carlo quadrature over the
+// points inside the simplices for channels with at most three legs.
+#pragma once
+
+#include <vector>
+
+#include "tb_kernels.cuh"
+#include "tb_theta.cuh"
+
+namespace tb {
+
+// The tuples of one channel that have a point inside the simplices, 32 to a
+// row; all tuples of a row share their leg-0 element (the last row of an
+// element is padded with tuples without points).  A row is one contiguous
+// block (row_bytes), each field 32 wide:
+//   double   a0[3], G[3][R]   the affine map of the constrained coordinates
+//   double   w                1 / (fact nmc |det|)
+//   uint64_t mask             the points inside
+//   int32_t  e[L - 1]         element ids of legs 1 .. L-1
+struct PointRows {
+    unsigned char* blk = nullptr;
+    int32_t* row_e0 = nullptr;      // [nrows]
+    int32_t* perm = nullptr;        // [nrows][32] index in the channel's list (padding: -1)
+    int64_t nrows = 0;
+    int64_t n = 0, points = 0;      // tuples and points inside
+    std::vector<int64_t> cost;      // [nrows + 1] running cost of the rows (host)
+    void release();
+};
+
+size_t row_bytes(int L);
+
+// Builds the rows from a ThetaList.  rows.blk stays null when there is no
+// room (the caller then keeps another path).
+int build_rows(const ChanDev& c, const ThetaList& th, PointRows& rows, cudaStream_t s);
+
+// What the kernel needs of one channel, in device memory.
+struct RowChan {
+    const unsigned char* blk;
+    const int32_t* row_e0;
+    const int32_t* perm;
+    const double* mc;
+    const double* tamp;             // functAmplitude per tuple, or null
+    const InstDev* insts;
+    int n_insts;
+    int nmc;
+    LegDev leg[3];
+    // the whole list, for states with non-finite coefficients
+    const int32_t* tup;
+    int64_t stride, n;
+};
+
+// One block's work: the rows of channel chan, in shares that the bounds
+// warp_row[share0 ..] delimit, and the part [t0, t1) of its whole list.
+struct RowWork {
+    int chan;
+    int share0;
+    int64_t t0, t1;
+};
+
+// A set of channels of equal leg count and directions that one launch
+// evaluates.
+struct RowSet {
+    int L = 0;
+    int dirs = 0;                   // bit l: leg l is ingoing
+    RowChan* d_chan = nullptr;
+    RowWork* d_work = nullptr;
+    int32_t* d_warp_row = nullptr;  // per block: the bounds of its shares
+    int nblocks = 0, shares = 0;
+    int nmc_max = 0;
+    bool multi = false;             // some channel has several instances
+    void release();
+};
+
+// Uploads the set for the given channels (rows of channel i in rows[i]);
+// blocks are dealt out by the rows' cost.
+int build_row_set(int L, int dirs, const std::vector<RowChan>& chan, const std::vector<const PointRows*>& rows,
+                  RowSet& out);
+
+// f4[e] = (f0, f1, f2, 0) of every element of the state; nf[b] != 0 marks an
+// element block that holds a non-finite coefficient.
+int launch_rows_prepare(const ElemDev& ed, const double* f, double4* f4, int* nf, const DPCtl* ctl, cudaStream_t s);
+
+// acc (or fx) += the collision terms of the set's channels; rate: the
+// scattering rate of leg rate_leg (of every leg when it is negative).
+// one non-null: that instance in place of the channels' instances.  err_flag
+// is set when a bounded wait (polls) for a staged row runs out.
+int launch_rows(const RowSet& rs, const ElemDev& ed, const double4* f4, const int* nf, double* acc, const DPCtl* ctl,
+                cudaStream_t s, bool rate, int rate_leg, const FxAcc& fx, int* err_flag, int polls,
+                const InstDev* one = nullptr);
+
+}  // namespace tb

@@ -41,6 +41,7 @@
 #include <tuple>
 #include <type_traits>
 
+#include "tb_bulk.cuh"
 #include "tb_dp45.cuh"
 #include "tb_geom.cuh"
 #include "tb_scatter.cuh"
@@ -227,39 +228,6 @@ __global__ void __launch_bounds__(256) k_build_moments(ChanDev c, const int32_t*
 }
 
 // ------------------------------------------------------------ contraction
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-__device__ __forceinline__ void mbar_init(uint64_t* bar, int count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));
-}
-
-__device__ __forceinline__ void mbar_expect_tx_arrive(uint64_t* bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes)
-                 : "memory");
-}
-
-// Bounded wait on an mbarrier phase; returns false when the spin limit is
-// reached (the caller records an error and abandons the tile).
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int limit = (1 << 22)) {
-    for (int it = 0; it < limit; ++it) {
-        uint32_t ok;
-        asm volatile(
-            "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-            : "=r"(ok)
-            : "r"(smem_u32(bar)), "r"(parity)
-            : "memory");
-        if (ok) return true;
-    }
-    return false;
-}
-
-__device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                     smem_u32(dst)),
-                 "l"(src), "r"(bytes), "r"(smem_u32(bar))
-                 : "memory");
-}
-
 // Moment j of this thread's tuple in a staged tile, as FP64.
 template <int KIND, int NMOM, int TT>
 __device__ __forceinline__ double tile_moment(const unsigned char* __restrict__ tile, int tid, int j) {
