@@ -371,7 +371,7 @@ int tb_read_scatt_indices(const char* path, int nlegs, const int32_t* nsplit, in
  * creation when the channel has at most 64 Monte-Carlo points; same sums as
  * the full quadrature for finite f), else 0 (every point of every tuple).
  * FP64 channels that TB_LAYOUT_AUTO resolved (2 or 3 legs, at most 64
- * points, shared by fewer than 16 runs) report TB_LAYOUT_T64 and stages 0,
+ * points; in the deterministic mode shared by fewer than 16 runs) report TB_LAYOUT_T64 and stages 0,
  * pair 6 too: they are evaluated over packed rows of the same tuples and
  * points, and their moment tensor is built only when a contraction schedule is
  * pinned, or by tb_options.autotune, which keeps the faster of the two.

@@ -72,19 +72,37 @@ def test_rhs_and_rates_match_the_oracle(gpu_lib, shape, deterministic):
         e.close()
 
 
-@pytest.mark.parametrize("runs", [2, 15])
-def test_shared_rows_of_a_small_batch(gpu_lib, runs):
-    mats = [_material(SHAPES["in_in_out"]["names"], [IN, IN, OUT], amp=0.5 + 0.1 * r) for r in range(runs)]
-    states = [W.initial_status(m, kT=0.05 + 0.01 * r, seed=r).vec for r, m in enumerate(mats)]
+@pytest.mark.parametrize("shape,runs", [("in_in_out", 2), ("in_in_out", 7), ("in_in_out", 8), ("in_out_out", 9),
+                                        ("in_in_out", 16), ("two_legs", 17), ("in_in_out", 33)])
+def test_shared_rows_of_a_batch(gpu_lib, shape, runs):
+    """One run after another below 8 runs, run-minor in groups of 8, 16 and 32 from there; beside them a run on
+    another mesh."""
+    kw = SHAPES[shape]
+    mats = [_material(amp=0.5 + 0.01 * r, **kw) for r in range(runs)] + [_material(**dict(kw, nsplit=(4, 5)))]
+    states = [W.initial_status(m, kT=0.05 + 0.005 * r, seed=r).vec for r, m in enumerate(mats)]
     be = E.BatchEngine(mats)
     try:
         be.set_amplitude(1, 0.0)   # a channel of the first run switched off
-        got = be.split(be.rhs(np.concatenate(states)))
-        rates = be.split(be.scattering_rates(np.concatenate(states)))
         mats[0].channels[1].amplitude = 0.0
-        for m, f, g, s in zip(mats, states, got, rates):
-            o = oracle.Oracle(m)
-            assert rel_l2(g, o.rhs(f)) < TOL and rel_l2(s, o.scattering_rates(f)) < TOL
+        refs = [oracle.Oracle(m) for m in mats]
+        f = np.concatenate(states)
+        for call in ("rhs", "scattering_rates", "rhs"):   # twice: what one evaluation leaves behind
+            for o, x, g in zip(refs, states, be.split(getattr(be, call)(f))):
+                assert rel_l2(g, getattr(o, call)(x)) < TOL
+        k = be.slices[runs - 1].start + 5   # a non-finite coefficient stays in its own run
+        f[k] = np.nan
+        bad = np.isfinite(be.rhs(f))
+        f[k] = 0.25
+        assert bad[:be.slices[runs - 1].start].all() and bad[be.slices[runs].start:].all() and not bad.all()
+        assert np.isfinite(be.rhs(f)).all()
+        if runs == 16:   # every run's integration, while others have ended
+            tf = np.linspace(0.05, 0.2, runs + 1)
+            got = be.dp45(np.concatenate(states), 0.0, tf, 0.05)
+            for m, x, g, t in zip(mats, states, got["runs"], tf):
+                one = E.Engine(m)
+                r = one.dp45(x, 0.0, t, 0.05)
+                one.close()
+                assert g["attempts"] == r["attempts"] and (len(r["dense"]) == 0 or rel_l2(g["dense"], r["dense"]) < 1e-11)
     finally:
         be.close()
 

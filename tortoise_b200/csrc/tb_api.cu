@@ -98,6 +98,8 @@ using namespace tb;
 namespace tb {
 int choose_layouts(tb_handle* h);
 int autotune(tb_handle* h);
+int build_run_states(tb_handle* h);
+void release_row_sets(tb_handle* h);
 }  // namespace tb
 
 namespace tb {
@@ -577,6 +579,7 @@ int build_runs(tb_handle* h, const tb_problem_desc* const* descs, int nruns) {
         h->dev_raw.push_back(p);
         h->d_nf = static_cast<int*>(p);
     }
+    TB_TRY(build_run_states(h));
     TB_TRY(refresh_row_sets(h));
     if (h->opts.autotune) {
         NvtxRange r("tb_create: autotune");
@@ -601,11 +604,12 @@ static int launch_group_mc(tb_handle* h, GroupChan& G, const InstDev* insts, int
                                148 * 32, rate_leg, nullptr, nullptr, h->fx);
 }
 
-static int row_dirs(const ChanDev& c) {
-    int d = 0;
-    for (int l = 0; l < c.L; ++l) d |= c.leg[l].dir > 0.0 ? 1 << l : 0;
-    return d;
-}
+// Channels shared by this many runs or more go over their rows run-minor, the
+// others one run after another (32x32 e-ph, us: 5 runs 257, 7 runs 344 one by
+// one; 8 runs 326 run-minor, where a group of 8 costs the same for 5).  Through
+// the moment tensor, the faster of its untuned schedules: 7 runs 822, 8 runs 884,
+// 16 runs 942, 48 runs 2221, against 344, 326, 536 and 1488 over rows.
+constexpr int ROWS_RUN_MINOR = 8;
 
 static RowChan row_chan(const GroupChan& G) {
     RowChan c{};
@@ -624,28 +628,121 @@ static RowChan row_chan(const GroupChan& G) {
     return c;
 }
 
-int refresh_row_sets(tb_handle* h) {
-    for (auto& rs : h->row_sets) rs.release();
-    h->row_sets.clear();
+// Sets of the channels that pass `take`, by legs, form and (run-minor)
+// lane group.
+template <class Take>
+static int make_row_sets(tb_handle* h, Take take, bool run_minor, std::vector<RowSet>& sets) {
     std::vector<bool> done(h->groups.size(), false);
     for (size_t a = 0; a < h->groups.size(); ++a) {
-        GroupChan& A = h->groups[a];
-        A.row_one.release();
-        if (!A.use_rows) continue;
-        TB_TRY(build_row_set(A.L, row_dirs(A.dev), {row_chan(A)}, {&A.rows}, A.row_one));
-        if (done[a]) continue;
+        const GroupChan& A = h->groups[a];
+        if (done[a] || !A.use_rows || !take(A)) continue;
+        const int S = run_minor ? rows_lane_group(int(A.insts.size())) : 0;
         std::vector<RowChan> chan;
         std::vector<const PointRows*> rows;
         for (size_t b = a; b < h->groups.size(); ++b) {
             const GroupChan& B = h->groups[b];
-            if (done[b] || !B.use_rows || B.L != A.L || row_dirs(B.dev) != row_dirs(A.dev)) continue;
+            if (done[b] || !B.use_rows || !take(B) || B.L != A.L || row_form(B.dev) != row_form(A.dev) ||
+                (run_minor && rows_lane_group(int(B.insts.size())) != S))
+                continue;
             chan.push_back(row_chan(B));
+            if (run_minor) {
+                RowChan& c = chan.back();
+                const RunState& st = h->run_states[size_t(B.run_state)];
+                const ChanInst& I = h->insts[B.insts[0]];
+                c.fT = st.fT;
+                c.accT = st.accT;
+                c.ndof = st.ndof;
+                for (int l = 0; l < B.L; ++l) c.loff[l] = I.dev.foff[l] - h->runs[size_t(I.run)].dof_off;
+            }
             rows.push_back(&B.rows);
             done[b] = true;
         }
-        h->row_sets.emplace_back();
-        TB_TRY(build_row_set(A.L, row_dirs(A.dev), chan, rows, h->row_sets.back()));
+        sets.emplace_back();
+        TB_TRY(build_row_set(A.L, row_form(A.dev), chan, rows, sets.back(), S));
     }
+    return TB_OK;
+}
+
+void release_row_sets(tb_handle* h) {
+    for (auto* sets : {&h->row_sets, &h->rate_sets, &h->run_sets}) {
+        for (auto& rs : *sets) rs.release();
+        sets->clear();
+    }
+    for (auto& G : h->groups) G.row_one.release();
+}
+
+int refresh_row_sets(tb_handle* h) {
+    release_row_sets(h);
+    for (auto& G : h->groups)
+        if (G.use_rows) TB_TRY(build_row_set(G.L, row_form(G.dev), {row_chan(G)}, {&G.rows}, G.row_one));
+    TB_TRY(make_row_sets(h, [](const GroupChan& G) { return G.run_state < 0; }, false, h->row_sets));
+    if (h->run_states.empty()) return TB_OK;
+    TB_TRY(make_row_sets(h, [](const GroupChan& G) { return G.run_state >= 0; }, false, h->rate_sets));
+    return make_row_sets(h, [](const GroupChan& G) { return G.run_state >= 0; }, true, h->run_sets);
+}
+
+// Run-minor states for the structures that ROWS_RUN_MINOR runs or more share
+// (each once, for all its channels over rows).  A structure that does not fit
+// stays with the rows one run after another.
+int build_run_states(tb_handle* h) {
+    if (h->opts.deterministic) return TB_OK;
+    int tiles = 0;
+    for (auto& G : h->groups) {
+        if (!G.use_rows || int(G.insts.size()) < ROWS_RUN_MINOR || G.run_state >= 0) continue;
+        std::vector<int> run;
+        std::vector<int64_t> off;
+        for (int id : G.insts) {
+            run.push_back(h->insts[id].run);
+            off.push_back(h->runs[size_t(run.back())].dof_off);
+        }
+        RunState st{};
+        st.n = int(run.size());
+        st.S = rows_lane_group(st.n);
+        st.np = (st.n + st.S - 1) / st.S * st.S;
+        st.ndof = h->runs[size_t(run[0])].ndofs;
+        const size_t bytes = sizeof(double) * size_t(st.ndof) * size_t(st.np);
+        void* p[4] = {nullptr, nullptr, nullptr, nullptr};
+        const size_t sz[4] = {bytes, bytes, sizeof(int64_t) * off.size(), sizeof(int) * run.size()};
+        bool ok = true;
+        for (int k = 0; k < 4 && ok; ++k) ok = cudaMalloc(&p[k], sz[k]) == cudaSuccess;
+        if (!ok) {
+            cudaGetLastError();
+            for (void* q : p) cudaFree(q);
+            continue;
+        }
+        for (void* q : p) h->run_allocs.push_back(q);
+        TB_CUDA(cudaMemset(p[0], 0, bytes));
+        TB_CUDA(cudaMemset(p[1], 0, bytes));
+        TB_CUDA(cudaMemcpy(p[2], off.data(), sz[2], cudaMemcpyHostToDevice));
+        TB_CUDA(cudaMemcpy(p[3], run.data(), sz[3], cudaMemcpyHostToDevice));
+        st.fT = static_cast<double*>(p[0]);
+        st.accT = static_cast<double*>(p[1]);
+        st.dof_off = static_cast<const int64_t*>(p[2]);
+        st.run = static_cast<const int*>(p[3]);
+        st.tiles_i = (st.np + 31) / 32;
+        st.tile0 = tiles;
+        tiles += int((st.ndof + 31) / 32) * st.tiles_i;
+        // every channel of the structure: the same runs
+        for (auto& H : h->groups)
+            if (H.use_rows && H.insts.size() == G.insts.size() && h->insts[H.insts[0]].run == run[0])
+                H.run_state = int(h->run_states.size());
+        h->run_states.push_back(st);
+    }
+    if (h->run_states.empty()) return TB_OK;
+    void *ds = nullptr, *dn = nullptr;
+    if (cudaMalloc(&ds, sizeof(RunState) * h->run_states.size()) != cudaSuccess ||
+        cudaMalloc(&dn, sizeof(int) * size_t(tiles)) != cudaSuccess) {
+        cudaGetLastError();
+        cudaFree(ds);
+        set_error("run state allocation failed");
+        return TB_ERR_OOM;
+    }
+    h->run_allocs.push_back(ds);
+    h->run_allocs.push_back(dn);
+    TB_CUDA(cudaMemcpy(ds, h->run_states.data(), sizeof(RunState) * h->run_states.size(), cudaMemcpyHostToDevice));
+    h->d_run_states = static_cast<RunState*>(ds);
+    h->d_run_nf = static_cast<int*>(dn);
+    h->n_run_tiles = tiles;
     return TB_OK;
 }
 
@@ -658,16 +755,22 @@ static int launch_row_sets(tb_handle* h, const double* d_in, double* d_acc, cons
         GroupChan& G = h->groups[I.group];
         if (!G.use_rows) return TB_OK;
         TB_TRY(launch_rows_prepare(h->ed, d_in, h->d_f4, h->d_nf, ctl, h->stream));
-        return launch_rows(G.row_one, h->ed, h->d_f4, h->d_nf, d_acc, ctl, h->stream, rate, rate_leg, h->fx,
+        return launch_rows(G.row_one, h->ed, d_in, h->d_f4, h->d_nf, d_acc, ctl, h->stream, rate, rate_leg, h->fx,
                            h->d_err, G.dev.wait_polls, I.d_single);
     }
-    if (h->row_sets.empty()) return TB_OK;
-    TB_TRY(launch_rows_prepare(h->ed, d_in, h->d_f4, h->d_nf, ctl, h->stream));
-    for (const RowSet& rs : h->row_sets)
-        if (rate_leg < rs.L)
-            TB_TRY(launch_rows(rs, h->ed, h->d_f4, h->d_nf, d_acc, ctl, h->stream, rate, rate_leg, h->fx, h->d_err,
-                               h->groups[0].dev.wait_polls));
-    return TB_OK;
+    const int polls = h->groups.empty() ? 0 : h->groups[0].dev.wait_polls;
+    const bool rates = rate && !h->rate_sets.empty();
+    if (!h->row_sets.empty() || rates) TB_TRY(launch_rows_prepare(h->ed, d_in, h->d_f4, h->d_nf, ctl, h->stream));
+    for (const auto* sets : {&h->row_sets, &h->rate_sets}) {
+        if (sets == &h->rate_sets && !rates) continue;
+        for (const RowSet& rs : *sets)
+            if (rate_leg < rs.L)
+                TB_TRY(launch_rows(rs, h->ed, d_in, h->d_f4, h->d_nf, d_acc, ctl, h->stream, rate, rate_leg, h->fx,
+                                   h->d_err, polls));
+    }
+    if (rate || h->run_sets.empty()) return TB_OK;
+    return launch_run_rows(h->run_sets, h->d_run_states, int(h->run_states.size()), h->n_run_tiles, d_in, h->d_run_nf,
+                           d_acc, ctl, h->stream, h->d_err, polls);
 }
 
 // A streamed group over this handle's work items.  Outside an integration
@@ -718,13 +821,6 @@ int run_rhs_acc(tb_handle* h, const double* d_in, double* d_acc, const DPCtl* ct
     return TB_OK;
 }
 
-// AUTO evaluates FP64 channels of at most three legs and 64 points over packed
-// rows, unless this many runs share one: there the contraction reads its f
-// run-minor.  Up to here the rows were faster at every size measured (12x12 to
-// 40x40: 1 run 36 against 56 and 119 against 443 us, 7 runs 70 against 116 and
-// 596 against 1513 us, 12 runs 100 against 150 and 1003 against 2412 us).
-constexpr int ROWS_MAX_INSTS = 16;
-
 // Times every contraction schedule of every moment-tensor group on a
 // representative state (all coefficients 0.25; the cost does not depend on
 // the values) and keeps the fastest (tune_tensor).  The accumulator is
@@ -738,12 +834,19 @@ static int tune_rows(tb_handle* h, GroupChan& G) {
     cudaEvent_t e0, e1;
     TB_CUDA(cudaEventCreate(&e0));
     TB_CUDA(cudaEventCreate(&e1));
-    TB_TRY(launch_rows_prepare(h->ed, h->d_f, h->d_f4, h->d_nf, nullptr, h->stream));
+    std::vector<RowSet> set;   // run-minor: this channel alone, its structure's state gathered and scattered
+    if (G.run_state >= 0) TB_TRY(make_row_sets(h, [&](const GroupChan& B) { return &B == &G; }, true, set));
     constexpr int REPS = 3;
     for (int r = 0; r <= REPS; ++r) {
         if (r == 1) cudaEventRecord(e0, h->stream);   // after a warm-up launch
-        TB_TRY(launch_rows(G.row_one, h->ed, h->d_f4, h->d_nf, h->d_acc, nullptr, h->stream, false, -1, h->fx, h->d_err,
-                           G.dev.wait_polls));
+        if (G.run_state >= 0) {
+            TB_TRY(launch_run_rows(set, h->d_run_states, int(h->run_states.size()), h->n_run_tiles, h->d_f,
+                                   h->d_run_nf, h->d_acc, nullptr, h->stream, h->d_err, G.dev.wait_polls));
+        } else {
+            TB_TRY(launch_rows_prepare(h->ed, h->d_f, h->d_f4, h->d_nf, nullptr, h->stream));
+            TB_TRY(launch_rows(G.row_one, h->ed, h->d_f, h->d_f4, h->d_nf, h->d_acc, nullptr, h->stream, false, -1,
+                               h->fx, h->d_err, G.dev.wait_polls));
+        }
     }
     cudaEventRecord(e1, h->stream);
     TB_CUDA(cudaEventSynchronize(e1));
@@ -751,6 +854,7 @@ static int tune_rows(tb_handle* h, GroupChan& G) {
     cudaEventElapsedTime(&ms, e0, e1);
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
+    for (auto& rs : set) rs.release();
     G.rows_seconds = 1e-3 * double(ms) / REPS;
     if (G.rows_seconds <= G.tensor.tuned_seconds) G.tensor.release();
     else G.use_rows = false;
@@ -789,6 +893,10 @@ int ensure_tensor(tb_handle* h, GroupChan& G) {
     return build_group_tensor(h, G, TK_F64);
 }
 
+// The deterministic mode has no run-minor rows: channels that this many runs
+// share stay with the run-minor contraction there.
+constexpr int ROWS_MAX_EXACT = 16;
+
 int choose_layouts(tb_handle* h) {
     size_t freeb = 0, totalb = 0;
     cudaMemGetInfo(&freeb, &totalb);
@@ -822,7 +930,8 @@ int choose_layouts(tb_handle* h) {
         if (want != TB_LAYOUT_MC64) {
             // AUTO's FP64 channels go over their packed rows; the tensor is
             // built when a contraction schedule is asked for
-            if (h->opts.layout == TB_LAYOUT_AUTO && want == TB_LAYOUT_T64 && int(G.insts.size()) < ROWS_MAX_INSTS) {
+            if (h->opts.layout == TB_LAYOUT_AUTO && want == TB_LAYOUT_T64  &&
+                !(h->opts.deterministic && int(G.insts.size()) >= ROWS_MAX_EXACT)) {
                 TB_TRY(build_theta_list(G.dev, G.tup, G.theta, h->stream));
                 if (G.theta.built) TB_TRY(build_rows(G.dev, G.theta, G.rows, h->stream));
                 G.use_rows = G.rows.blk != nullptr;
@@ -1028,10 +1137,10 @@ int tb_destroy(tb_handle* h) {
         G.tensor.release();
         G.theta.release();
         G.rows.release();
-        G.row_one.release();
         if (G.d_tamp) cudaFree(G.d_tamp);
     }
-    for (auto& rs : h->row_sets) rs.release();
+    release_row_sets(h);
+    for (void* p : h->run_allocs) cudaFree(p);
     for (double* p : h->dev_allocs) cudaFree(p);
     for (void* p : h->dev_raw) cudaFree(p);
     if (h->dp.dense) cudaFree(h->dp.dense);

@@ -38,6 +38,7 @@ struct GroupChan {
     // channels; row_one is the set of this channel only
     PointRows rows;
     bool use_rows = false;
+    int run_state = -1;           // the handle's run-minor state it is evaluated in, or -1
     double rows_seconds = 0.0;    // launch time the autotuner measured
     RowSet row_one;
     // streamed channel (TB_LAYOUT_STREAM): the candidate walk and this
@@ -91,9 +92,17 @@ struct tb_handle {
     double* d_out = nullptr;
     double* d_acc = nullptr;
     double* d_part = nullptr;
-    // channels evaluated over packed rows, by leg count and directions; the
+    // channels evaluated over packed rows, by leg count and form; the
     // state padded to four doubles an element, and its non-finite blocks
     std::vector<tb::RowSet> row_sets;
+    // those of them that many runs share, run-minor (propagation without the
+    // deterministic mode; the row sets hold the rest, the rate sets all)
+    std::vector<tb::RowSet> rate_sets, run_sets;
+    std::vector<tb::RunState> run_states;
+    std::vector<void*> run_allocs;
+    tb::RunState* d_run_states = nullptr;
+    int* d_run_nf = nullptr;
+    int n_run_tiles = 0;
     double4* d_f4 = nullptr;
     int* d_nf = nullptr;
     // deterministic mode: the exact accumulator behind d_acc (3 words per

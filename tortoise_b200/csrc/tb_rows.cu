@@ -54,8 +54,18 @@ constexpr int ROW_WARPS = 16;   // shares of rows that a block takes, one per wa
 // side: 421 us against 336), 12 hide less latency (350).  The rates of every
 // leg take 12 (184 us against 210 at 16, 40x24 with umklapp).
 template <bool RATE, bool DET> struct RowCap { static constexpr int W = RATE && !DET ? 12 : ROW_WARPS; };
+constexpr int RUN_WARPS = 16;   // the same, run-minor
 constexpr int ROW_STAGES = 2;    // rows of a warp in shared memory
 constexpr int ROW_COPIES = 16;   // copies of the point table, one per lane of a half warp
+
+// row_form of {fermion in, fermion out} and {fermion in, boson in, fermion out}
+constexpr int FORM_2 = 0x01, FORM_3 = 0x23;
+
+int row_form(const ChanDev& c) {
+    int d = 0;
+    for (int l = 0; l < c.L; ++l) d |= (c.leg[l].dir > 0.0 ? 1 << l : 0) | (c.leg[l].stat > 0.0 ? 16 << l : 0);
+    return d;
+}
 
 template <int L>
 struct RowDim {
@@ -75,6 +85,7 @@ void PointRows::release() {
     perm = nullptr;
     nrows = n = points = 0;
     cost.clear();
+    run_cost.clear();
 }
 
 void RowSet::release() {
@@ -131,7 +142,8 @@ __global__ void __launch_bounds__(256) k_rows_fill(ChanDev c, const int32_t* __r
 #pragma unroll
         for (int l = 1; l < L; ++l) ei[32 * (l - 1) + lane] = e[l];
         row_perm[row * 32 + lane] = perm[j];
-        atomicMax(row_pts + row, __popcll(mask[j]));
+        atomicMax(row_pts + 2 * row, __popcll(mask[j]));
+        atomicAdd(row_pts + 2 * row + 1, 7 + __popcll(mask[j]));
         if (lane == 0) row_e0[row] = e[0];
     }
 }
@@ -179,7 +191,7 @@ int build_rows(const ChanDev& c, const ThetaList& th, PointRows& rows, cudaStrea
         at += cnt[size_t(e)];
         nrows += (cnt[size_t(e)] + 31) / 32;
     }
-    int32_t* d_pts = static_cast<int32_t*>(tmp.get(sizeof(int32_t) * size_t(nrows)));
+    int32_t* d_pts = static_cast<int32_t*>(tmp.get(2 * sizeof(int32_t) * size_t(nrows)));
     const size_t bytes = row_bytes(c.L) * size_t(nrows);
     if (!d_pts || cudaMalloc(&rows.blk, bytes) != cudaSuccess ||
         cudaMalloc(&rows.row_e0, sizeof(int32_t) * size_t(nrows)) != cudaSuccess ||
@@ -190,7 +202,7 @@ int build_rows(const ChanDev& c, const ThetaList& th, PointRows& rows, cudaStrea
     }
     TB_CUDA(cudaMemsetAsync(rows.blk, 0, bytes, s));   // padding: no points, element 0
     TB_CUDA(cudaMemsetAsync(rows.perm, 0xff, sizeof(int32_t) * size_t(nrows) * 32, s));
-    TB_CUDA(cudaMemsetAsync(d_pts, 0, sizeof(int32_t) * size_t(nrows), s));
+    TB_CUDA(cudaMemsetAsync(d_pts, 0, 2 * sizeof(int32_t) * size_t(nrows), s));
     TB_CUDA(cudaMemcpyAsync(d_first, first.data(), sizeof(int64_t) * size_t(ne), cudaMemcpyHostToDevice, s));
     TB_CUDA(cudaMemcpyAsync(d_row0, row0.data(), sizeof(int64_t) * size_t(ne), cudaMemcpyHostToDevice, s));
     if (c.L == 2)
@@ -200,11 +212,17 @@ int build_rows(const ChanDev& c, const ThetaList& th, PointRows& rows, cudaStrea
         k_rows_fill<3><<<blocks, 256, 0, s>>>(c, th.ids, th.mask, th.perm, n, d_first, d_row0, rows.blk, rows.row_e0,
                                               rows.perm, d_pts);
     TB_CUDA(cudaGetLastError());
-    std::vector<int32_t> pts(size_t(nrows), 0);
-    TB_CUDA(cudaMemcpyAsync(pts.data(), d_pts, sizeof(int32_t) * size_t(nrows), cudaMemcpyDeviceToHost, s));
+    std::vector<int32_t> pts(2 * size_t(nrows), 0);
+    TB_CUDA(cudaMemcpyAsync(pts.data(), d_pts, sizeof(int32_t) * pts.size(), cudaMemcpyDeviceToHost, s));
     TB_CUDA(cudaStreamSynchronize(s));
+    // a row costs its longest lane beside a fixed part; run-minor, its tuples
+    // one after another
     rows.cost.assign(size_t(nrows) + 1, 0);
-    for (int64_t r = 0; r < nrows; ++r) rows.cost[size_t(r) + 1] = rows.cost[size_t(r)] + 6 + pts[size_t(r)];
+    rows.run_cost.assign(size_t(nrows) + 1, 0);
+    for (size_t r = 0; r < size_t(nrows); ++r) {
+        rows.cost[r + 1] = rows.cost[r] + 8 + pts[2 * r];
+        rows.run_cost[r + 1] = rows.run_cost[r] + pts[2 * r + 1];
+    }
     rows.nrows = nrows;
     rows.n = n;
     rows.points = th.points;
@@ -241,6 +259,12 @@ struct RowTable {
     __device__ __forceinline__ double operator()(int i) const { return q[i * ROW_COPIES]; }
 };
 
+// The same with one copy, for lanes that visit the same point.
+struct FlatTable {
+    const double* q;
+    __device__ __forceinline__ double operator()(int i) const { return q[i]; }
+};
+
 // One tuple's map, from this lane's column of the staged row.
 template <int L>
 struct RowMap {
@@ -258,6 +282,16 @@ struct RowMap {
     __device__ __forceinline__ double G(int k, int j) const { return G_[k][j]; }
 };
 
+// The same, read from the stage at each use: for lanes that share a tuple a
+// read is one broadcast, and the registers go to more warps.
+template <int L>
+struct StageMap {
+    static constexpr int R = RowDim<L>::R;
+    const double* d;
+    __device__ __forceinline__ double a0(int k) const { return d[32 * k]; }
+    __device__ __forceinline__ double G(int k, int j) const { return d[32 * (3 + k * R + j)]; }
+};
+
 // The padded coefficients of one element in one 32-byte load.
 __device__ __forceinline__ double4 load_f4(const double4* p) {
     double4 v;
@@ -272,11 +306,15 @@ struct RowOut {
     double v[L][3];
 };
 
-// Whether leg l is ingoing: from the template's direction mask, or (DIRS < 0)
-// from the channel.
-template <int DIRS>
+// Whether leg l is ingoing, and 1 + s t with its statistics s = +-1: from the
+// template's FORM (row_form), or (FORM < 0) from the channel.
+template <int FORM>
 __device__ __forceinline__ bool leg_in(const RowChan& c, int l) {
-    return DIRS >= 0 ? ((DIRS >> l) & 1) != 0 : c.leg[l].dir > 0.0;
+    return FORM >= 0 ? ((FORM >> l) & 1) != 0 : c.leg[l].dir > 0.0;
+}
+template <int FORM>
+__device__ __forceinline__ double leg_stat(const RowChan& c, int l) {
+    return FORM >= 0 ? (((FORM >> (4 + l)) & 1) ? 1.0 : -1.0) : c.leg[l].stat;
 }
 
 // The legs' linear forms as affine functions of q.  Free leg l < L - 2 lies
@@ -287,7 +325,8 @@ struct RowForms {
     static constexpr int R = RowDim<L>::R;
     double fr[L > 2 ? L - 2 : 1][3];   // free legs
     double p0, p[R], c0, c[R];
-    __device__ __forceinline__ void set(const RowMap<L>& m, const double4 (&f)[L]) {
+    template <class Map>
+    __device__ __forceinline__ void set(const Map& m, const double4 (&f)[L]) {
 #pragma unroll
         for (int l = 0; l < L - 2; ++l) { fr[l][0] = f[l].x; fr[l][1] = f[l].y; fr[l][2] = f[l].z; }
         const double4 P = f[L - 2], C = f[L - 1];
@@ -314,9 +353,9 @@ struct RowForms {
 // (ScatteringChannel.cpp:633-641) are t and 1 + s t (s the statistics), in
 // this order for an ingoing leg and swapped for an outgoing one; the loss
 // product carries leg 0's minus sign.
-template <int L, int DIRS>
-__device__ __forceinline__ void row_tuple(const RowChan& c, const RowMap<L>& m, uint64_t mk, const double4 (&f)[L],
-                                          const RowTable& tab, double scale, RowOut<L>& o) {
+template <int L, int FORM, class Map, class Table>
+__device__ __forceinline__ void row_tuple(const RowChan& c, const Map& m, uint64_t mk, const double4 (&f)[L],
+                                          const Table& tab, double scale, RowOut<L>& o) {
     constexpr int R = RowDim<L>::R;
     RowForms<L> F;
     F.set(m, f);
@@ -325,13 +364,13 @@ __device__ __forceinline__ void row_tuple(const RowChan& c, const RowMap<L>& m, 
     for (int j = 0; j < R; ++j) sq[j] = 0.0;
     double st[L];
 #pragma unroll
-    for (int l = 0; l < L; ++l) st[l] = c.leg[l].stat;
+    for (int l = 0; l < L; ++l) st[l] = leg_stat<FORM>(c, l);
     auto product = [&](const double (&t)[L]) {
         double pa = 1.0, pb = 1.0;
 #pragma unroll
         for (int l = 0; l < L; ++l) {
             const double u = fma(st[l], t[l], 1.0);
-            const bool in = leg_in<DIRS>(c, l);
+            const bool in = leg_in<FORM>(c, l);
             const double a = in ? t[l] : u, b = in ? u : t[l];
             pb = l ? pb * b : b;
             if (l < L - 1) pa = l ? pa * a : a;
@@ -362,7 +401,7 @@ __device__ __forceinline__ void row_tuple(const RowChan& c, const RowMap<L>& m, 
     }
 #pragma unroll
     for (int l = 0; l < L; ++l) {
-        const bool in = leg_in<DIRS>(c, l);
+        const bool in = leg_in<FORM>(c, l);
         const double x = l < L - 2 ? sq[l < L - 2 ? 2 * l : 0] : l == L - 2 ? sq[R - 1] : cx;
         const double z = l < L - 2 ? sq[l < L - 2 ? 2 * l + 1 : 0] : l == L - 2 ? y : cy;
         o.v[l][0] = in ? s0 : -s0;
@@ -373,7 +412,7 @@ __device__ __forceinline__ void row_tuple(const RowChan& c, const RowMap<L>& m, 
 
 // Scattering rates of one tuple: leg r's forms become the unit forms
 // (ScatteringChannel.cpp:562-564), for every leg r in one pass over the points.
-template <int L, int DIRS>
+template <int L, int FORM>
 __device__ __forceinline__ void row_tuple_rate(const RowChan& c, const RowMap<L>& m, uint64_t mk,
                                                const double4 (&f)[L], const RowTable& tab, double scale,
                                                RowOut<L>& o) {
@@ -389,7 +428,7 @@ __device__ __forceinline__ void row_tuple_rate(const RowChan& c, const RowMap<L>
     }
     double st[L];
 #pragma unroll
-    for (int l = 0; l < L; ++l) st[l] = c.leg[l].stat;
+    for (int l = 0; l < L; ++l) st[l] = leg_stat<FORM>(c, l);
     for (; mk; mk &= mk - 1) {
         const int i = (__ffsll((long long)mk) - 1) * R;
         double q[R], t[L], a[L], b[L];
@@ -399,13 +438,13 @@ __device__ __forceinline__ void row_tuple_rate(const RowChan& c, const RowMap<L>
 #pragma unroll
         for (int l = 0; l < L; ++l) {
             const double u = fma(st[l], t[l], 1.0);
-            const bool in = leg_in<DIRS>(c, l);
+            const bool in = leg_in<FORM>(c, l);
             a[l] = in ? t[l] : u;
             b[l] = in ? u : t[l];
         }
 #pragma unroll
         for (int r = 0; r < L; ++r) {
-            const bool in = leg_in<DIRS>(c, r);
+            const bool in = leg_in<FORM>(c, r);
             double pa = in ? -2.0 : -2.0 * st[r], pb = in ? 2.0 * st[r] : 2.0;
 #pragma unroll
             for (int l = 0; l < L; ++l)
@@ -433,7 +472,7 @@ __device__ __forceinline__ void row_tuple_rate(const RowChan& c, const RowMap<L>
                 z = fma(m.G(y, j), sq[r][j], z);
             }
         }
-        const double d = leg_in<DIRS>(c, r) ? -scale : scale;
+        const double d = leg_in<FORM>(c, r) ? -scale : scale;
         o.v[r][0] = d * s0[r];
         o.v[r][1] = d * x;
         o.v[r][2] = d * z;
@@ -571,7 +610,7 @@ struct LegZero<true> {
     }
 };
 
-__device__ __forceinline__ bool finite4(const double4& v) { return isfinite(v.x) && isfinite(v.y) && isfinite(v.z); }
+__device__ __forceinline__ bool finite3(const double* v) { return isfinite(v[0]) && isfinite(v[1]) && isfinite(v[2]); }
 
 // A state with non-finite coefficients: the full quadrature multiplies the
 // integrand of every tuple by its Theta, also by 0, so each tuple that touches
@@ -579,7 +618,7 @@ __device__ __forceinline__ bool finite4(const double4& v) { return isfinite(v.x)
 // [t0, t1) of the whole list.
 template <int L>
 __device__ __noinline__ void spread_nonfinite(const RowChan& c, const InstDev* insts, int n_insts, int64_t t0,
-                                              int64_t t1, const double4* f4, double* acc, const DPCtl* ctl, bool rate,
+                                              int64_t t1, const double* f, double* acc, const DPCtl* ctl, bool rate,
                                               int rate_leg, const FxAcc& fx) {
     const double nan = __longlong_as_double(0x7ff8000000000000ll);
     for (int64_t i = t0 + threadIdx.x; i < t1; i += blockDim.x) {
@@ -593,7 +632,7 @@ __device__ __noinline__ void spread_nonfinite(const RowChan& c, const InstDev* i
             int nbad = 0;
 #pragma unroll
             for (int l = 0; l < L; ++l) {
-                bad[l] = !finite4(f4[in.foff[l] / 3 + e[l]]);
+                bad[l] = !finite3(f + in.foff[l] + 3 * (int64_t)e[l]);
                 nbad += bad[l] ? 1 : 0;
             }
             if (nbad == 0) continue;
@@ -609,11 +648,12 @@ __device__ __noinline__ void spread_nonfinite(const RowChan& c, const InstDev* i
     }
 }
 
-template <int L, int DIRS, bool RATE, bool DET, bool MULTI>
+template <int L, int FORM, bool RATE, bool DET, bool MULTI>
 __global__ void __launch_bounds__(RowCap<RATE, DET>::W * 32, 1) k_rows(const RowChan* __restrict__ chans,
                                                             const RowWork* __restrict__ work,
                                                             const int32_t* __restrict__ warp_row, int shares,
                                                             const InstDev* __restrict__ one,
+                                                            const double* __restrict__ f,
                                                             const double4* __restrict__ f4,
                                                             const int* __restrict__ nf, int n_nf,
                                                             double* __restrict__ acc, const DPCtl* __restrict__ ctl,
@@ -722,8 +762,8 @@ __global__ void __launch_bounds__(RowCap<RATE, DET>::W * 32, 1) k_rows(const Row
             RowOut<L> o;
             const double wt = reinterpret_cast<const double*>(b)[32 * (ND - 1) + lane];
             if (DET) row_tuple_listed<L, RATE>(c, m, mk, f, tab, wt, amp * tf, o);
-            else if (RATE) row_tuple_rate<L, DIRS>(c, m, mk, f, tab, wt * (amp * tf), o);
-            else row_tuple<L, DIRS>(c, m, mk, f, tab, wt * (amp * tf), o);
+            else if (RATE) row_tuple_rate<L, FORM>(c, m, mk, f, tab, wt * (amp * tf), o);
+            else row_tuple<L, FORM>(c, m, mk, f, tab, wt * (amp * tf), o);
             if (!RATE || rate_leg <= 0) {
                 z.add(o.v[0], fx);
                 if (MULTI) z.flush(acc, off[0] + 3 * (int64_t)e[0], fx);
@@ -761,7 +801,7 @@ __global__ void __launch_bounds__(RowCap<RATE, DET>::W * 32, 1) k_rows(const Row
     int bad = 0;
     for (int i = tid; i < n_nf; i += blockDim.x) bad |= nf[i];
     if (__syncthreads_or(bad))
-        spread_nonfinite<L>(c, insts, n_insts, w.t0, w.t1, f4, acc, ctl, RATE, rate_leg, fx);
+        spread_nonfinite<L>(c, insts, n_insts, w.t0, w.t1, f, acc, ctl, RATE, rate_leg, fx);
 }
 
 static size_t rows_smem(int L, int nmc, int warps) {
@@ -769,11 +809,11 @@ static size_t rows_smem(int L, int nmc, int warps) {
            sizeof(double) * size_t(nmc) * size_t(2 * (L - 2) + 1) * ROW_COPIES;
 }
 
-template <int L, int DIRS, bool RATE, bool DET, bool MULTI>
-static int launch_k_rows(const RowSet& rs, const ElemDev& ed, const double4* f4, const int* nf, double* acc,
+template <int L, int FORM, bool RATE, bool DET, bool MULTI>
+static int launch_k_rows(const RowSet& rs, const ElemDev& ed, const double* f, const double4* f4, const int* nf, double* acc,
                          const DPCtl* ctl, cudaStream_t s, int rate_leg, const FxAcc& fx, const InstDev* one,
                          int* err_flag, int polls) {
-    auto kern = k_rows<L, DIRS, RATE, DET, MULTI>;
+    auto kern = k_rows<L, FORM, RATE, DET, MULTI>;
     // the shared-memory limit, set once on each device the kernel runs on
     static std::atomic<unsigned long long> attr_devices{0};
     int dev = 0;
@@ -785,56 +825,60 @@ static int launch_k_rows(const RowSet& rs, const ElemDev& ed, const double4* f4,
     }
     const int warps = std::min(rs.shares, RowCap<RATE, DET>::W);
     kern<<<unsigned(rs.nblocks), unsigned(32 * warps), rows_smem(L, rs.nmc_max, warps), s>>>(
-        rs.d_chan, rs.d_work, rs.d_warp_row, rs.shares, one, f4, nf, ed.nblk, acc, ctl, rate_leg, fx, err_flag, polls);
+        rs.d_chan, rs.d_work, rs.d_warp_row, rs.shares, one, f, f4, nf, ed.nblk, acc, ctl, rate_leg, fx, err_flag, polls);
     TB_CUDA(cudaGetLastError());
     return TB_OK;
 }
 
-template <int L, int DIRS, bool RATE, bool DET>
-static int launch_rows_m(const RowSet& rs, const ElemDev& ed, const double4* f4, const int* nf, double* acc,
+template <int L, int FORM, bool RATE, bool DET>
+static int launch_rows_m(const RowSet& rs, const ElemDev& ed, const double* f, const double4* f4, const int* nf, double* acc,
                          const DPCtl* ctl, cudaStream_t s, int rate_leg, const FxAcc& fx, const InstDev* one,
                          int* err_flag, int polls) {
     if (rs.multi && !one)
-        return launch_k_rows<L, DIRS, RATE, DET, true>(rs, ed, f4, nf, acc, ctl, s, rate_leg, fx, one, err_flag, polls);
-    return launch_k_rows<L, DIRS, RATE, DET, false>(rs, ed, f4, nf, acc, ctl, s, rate_leg, fx, one, err_flag, polls);
+        return launch_k_rows<L, FORM, RATE, DET, true>(rs, ed, f, f4, nf, acc, ctl, s, rate_leg, fx, one, err_flag, polls);
+    return launch_k_rows<L, FORM, RATE, DET, false>(rs, ed, f, f4, nf, acc, ctl, s, rate_leg, fx, one, err_flag, polls);
 }
 
-// The directions of the channels that addScatteringChannelsWildcards builds in
-// the reference's examples ({in, in, out}, {in, out}) are compiled in; other
-// sets select the forms at run time.
+// The channels that addScatteringChannelsWildcards builds in the reference's
+// examples are compiled in (FORM_2, FORM_3); others select their forms at run
+// time.
 template <int L>
-static int launch_rows_l(const RowSet& rs, const ElemDev& ed, const double4* f4, const int* nf, double* acc,
+static int launch_rows_l(const RowSet& rs, const ElemDev& ed, const double* f, const double4* f4, const int* nf, double* acc,
                          const DPCtl* ctl, cudaStream_t s, bool rate, int rate_leg, const FxAcc& fx,
                          const InstDev* one, int* err_flag, int polls) {
-    constexpr int CANON = (1 << (L - 1)) - 1;   // every leg but the last ingoing
-#define TB_ROWS(DD, RR, XX) launch_rows_m<L, DD, RR, XX>(rs, ed, f4, nf, acc, ctl, s, rate_leg, fx, one, err_flag, polls)
+    constexpr int CANON = L == 2 ? FORM_2 : FORM_3;
+#define TB_ROWS(DD, RR, XX) launch_rows_m<L, DD, RR, XX>(rs, ed, f, f4, nf, acc, ctl, s, rate_leg, fx, one, err_flag, polls)
     if (fx.w) return rate ? TB_ROWS(-1, true, true) : TB_ROWS(-1, false, true);
-    if (rs.dirs == CANON) return rate ? TB_ROWS(CANON, true, false) : TB_ROWS(CANON, false, false);
+    if (rs.form == CANON) return rate ? TB_ROWS(CANON, true, false) : TB_ROWS(CANON, false, false);
     return rate ? TB_ROWS(-1, true, false) : TB_ROWS(-1, false, false);
 #undef TB_ROWS
 }
 
-int launch_rows(const RowSet& rs, const ElemDev& ed, const double4* f4, const int* nf, double* acc, const DPCtl* ctl,
+int launch_rows(const RowSet& rs, const ElemDev& ed, const double* f, const double4* f4, const int* nf, double* acc, const DPCtl* ctl,
                 cudaStream_t s, bool rate, int rate_leg, const FxAcc& fx, int* err_flag, int polls,
                 const InstDev* one) {
     if (rs.nblocks <= 0) return TB_OK;
-    if (rs.L == 2) return launch_rows_l<2>(rs, ed, f4, nf, acc, ctl, s, rate, rate_leg, fx, one, err_flag, polls);
-    if (rs.L == 3) return launch_rows_l<3>(rs, ed, f4, nf, acc, ctl, s, rate, rate_leg, fx, one, err_flag, polls);
+    if (rs.L == 2) return launch_rows_l<2>(rs, ed, f, f4, nf, acc, ctl, s, rate, rate_leg, fx, one, err_flag, polls);
+    if (rs.L == 3) return launch_rows_l<3>(rs, ed, f, f4, nf, acc, ctl, s, rate, rate_leg, fx, one, err_flag, polls);
     set_error("rows hold two or three legs");
     return TB_ERR_ARG;
 }
 
-int build_row_set(int L, int dirs, const std::vector<RowChan>& chan, const std::vector<const PointRows*>& rows,
-                  RowSet& out) {
+int build_row_set(int L, int form, const std::vector<RowChan>& chan, const std::vector<const PointRows*>& rows,
+                  RowSet& out, int S) {
     out.release();
     out.L = L;
-    out.dirs = dirs;
+    out.form = form;
+    out.S = S;
     out.nmc_max = 0;
     out.multi = false;
-    int64_t total = 0, nrows = 0;
+    int64_t nrows = 0;
+    // what blocks are dealt out to: channels, run-minor each chunk of S runs
+    std::vector<std::pair<int, int>> item;   // (channel, chunk)
     for (size_t i = 0; i < chan.size(); ++i) {
-        total += rows[i]->cost.back();
-        nrows += rows[i]->nrows;
+        const int chunks = S ? (chan[i].n_insts + S - 1) / S : 1;
+        for (int k = 0; k < chunks; ++k) item.emplace_back(int(i), k);
+        nrows += rows[i]->nrows * chunks;
         out.nmc_max = std::max(out.nmc_max, chan[i].nmc);
         out.multi = out.multi || chan[i].n_insts > 1;
     }
@@ -843,21 +887,27 @@ int build_row_set(int L, int dirs, const std::vector<RowChan>& chan, const std::
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
     // one block per SM; fewer warps in each where there are fewer rows than
-    // warps.  Every channel gets a block of its own at least, the others go one
-    // by one to the channel with the largest cost per block.
-    out.shares = int(std::min<int64_t>(ROW_WARPS, std::max<int64_t>(4, (nrows + nsm - 1) / nsm)));
-    std::vector<int64_t> nb(chan.size(), 1);
-    for (int64_t left = std::min<int64_t>(nsm, (nrows + out.shares - 1) / out.shares) - int64_t(chan.size()); left > 0;
+    // warps.  Every item gets a block of its own at least, the others go one
+    // by one to the item with the largest cost per block.
+    out.shares = int(std::min<int64_t>(S ? RUN_WARPS : ROW_WARPS, std::max<int64_t>(4, (nrows + nsm - 1) / nsm)));
+    std::vector<int64_t> nb(item.size(), 1);
+    auto cost_of = [&](size_t i) -> const std::vector<int64_t>& {
+        const PointRows& r = *rows[size_t(item[i].first)];
+        return S ? r.run_cost : r.cost;
+    };
+    auto load = [&](size_t i) { return double(cost_of(i).back()) / double(nb[i]); };
+    for (int64_t left = std::min<int64_t>(nsm, (nrows + out.shares - 1) / out.shares) - int64_t(item.size()); left > 0;
          --left) {
         size_t best = 0;
-        for (size_t i = 1; i < chan.size(); ++i)
-            if (double(rows[i]->cost.back()) / double(nb[i]) > double(rows[best]->cost.back()) / double(nb[best])) best = i;
+        for (size_t i = 1; i < item.size(); ++i)
+            if (load(i) > load(best)) best = i;
         nb[best] += 1;
     }
     std::vector<RowWork> work;
     std::vector<int32_t> warp_row;
-    for (size_t i = 0; i < chan.size(); ++i) {
-        const std::vector<int64_t>& cost = rows[i]->cost;
+    for (size_t i = 0; i < item.size(); ++i) {
+        const RowChan& c = chan[size_t(item[i].first)];
+        const std::vector<int64_t>& cost = cost_of(i);
         const int64_t parts = nb[i] * out.shares;
         // rows up to the p-th share of the cost
         auto bound = [&](int64_t p) {
@@ -865,10 +915,11 @@ int build_row_set(int L, int dirs, const std::vector<RowChan>& chan, const std::
         };
         for (int64_t b = 0; b < nb[i]; ++b) {
             RowWork w{};
-            w.chan = int(i);
+            w.chan = item[i].first;
+            w.chunk = item[i].second;
             w.share0 = int(warp_row.size());
-            w.t0 = chan[i].n * b / nb[i];
-            w.t1 = chan[i].n * (b + 1) / nb[i];
+            w.t0 = c.n * b / nb[i];
+            w.t1 = c.n * (b + 1) / nb[i];
             work.push_back(w);
             for (int64_t p = b * out.shares; p <= (b + 1) * out.shares; ++p) warp_row.push_back(bound(p));
         }
@@ -885,6 +936,259 @@ int build_row_set(int L, int dirs, const std::vector<RowChan>& chan, const std::
     TB_CUDA(cudaMemcpy(out.d_work, work.data(), sizeof(RowWork) * work.size(), cudaMemcpyHostToDevice));
     TB_CUDA(cudaMemcpy(out.d_warp_row, warp_row.data(), sizeof(int32_t) * warp_row.size(), cudaMemcpyHostToDevice));
     out.nblocks = int(work.size());
+    return TB_OK;
+}
+
+// --------------------------------------------------------------- many runs
+int rows_lane_group(int n) {
+    int best = 32;
+    for (int S : {16, 8})
+        if ((n + S - 1) / S * S < (n + best - 1) / best * best) best = S;
+    return best;
+}
+
+__device__ __forceinline__ const RunState& tile_state(const RunState* st, int n_st, int tile) {
+    int k = 0;
+    while (k + 1 < n_st && tile >= st[k + 1].tile0) ++k;
+    return st[k];
+}
+
+__device__ __forceinline__ int64_t run_slot(const RunState& st, int64_t d, int i) {
+    return (int64_t(i / st.S) * st.ndof + d) * st.S + i % st.S;
+}
+
+// fT[i / S][d][i % S] = f[dof_off[i] + d], 32 dofs x 32 runs a tile
+__global__ void __launch_bounds__(256) k_runs_state_gather(const RunState* __restrict__ st, int n_st,
+                                                           const double* __restrict__ f, int* __restrict__ nf,
+                                                           const DPCtl* __restrict__ ctl) {
+    __shared__ double tile[32][33];
+    const RunState& S = tile_state(st, n_st, blockIdx.x);
+    const int k = blockIdx.x - S.tile0, tx = threadIdx.x, ty = threadIdx.y;
+    const int i0 = (k % S.tiles_i) * 32;
+    const int64_t d0 = int64_t(k / S.tiles_i) * 32;
+    bool bad = false;
+    for (int y = ty; y < 32; y += 8) {
+        const int i = i0 + y;
+        double v = 0.0;
+        if (i < S.n && d0 + tx < S.ndof && !(ctl && ctl[S.run[i]].done)) {
+            v = __ldg(f + S.dof_off[i] + d0 + tx);
+            bad = bad || !isfinite(v);
+        }
+        tile[y][tx] = v;
+    }
+    bad = __syncthreads_or(bad);
+    if (tx == 0 && ty == 0) nf[blockIdx.x] = bad ? 1 : 0;
+    for (int y = ty; y < 32; y += 8)
+        if (d0 + y < S.ndof && i0 + tx < S.np) S.fT[run_slot(S, d0 + y, i0 + tx)] = tile[tx][y];
+}
+
+// acc[dof_off[i] + d] += accT[i / S][d][i % S], which is cleared.  Every coefficient of
+// the state belongs to one run of one structure, so the adds need no atomics.
+__global__ void __launch_bounds__(256) k_runs_state_scatter(const RunState* __restrict__ st, int n_st,
+                                                            double* __restrict__ acc, const DPCtl* __restrict__ ctl) {
+    __shared__ double tile[32][33];
+    const RunState& S = tile_state(st, n_st, blockIdx.x);
+    const int k = blockIdx.x - S.tile0, tx = threadIdx.x, ty = threadIdx.y;
+    const int i0 = (k % S.tiles_i) * 32;
+    const int64_t d0 = int64_t(k / S.tiles_i) * 32;
+    for (int y = ty; y < 32; y += 8) {
+        double v = 0.0;
+        if (d0 + y < S.ndof && i0 + tx < S.np) {
+            double* p = S.accT + run_slot(S, d0 + y, i0 + tx);
+            v = *p;
+            *p = 0.0;
+        }
+        tile[y][tx] = v;
+    }
+    __syncthreads();
+    for (int y = ty; y < 32; y += 8) {
+        const int i = i0 + y;
+        if (i < S.n && d0 + tx < S.ndof && !(ctl && ctl[S.run[i]].done)) acc[S.dof_off[i] + d0 + tx] += tile[tx][y];
+    }
+}
+
+// The rows for S runs at a time: lane = (tuple of a group of 32 / S, run).  A
+// tuple's map, mask and points are the same for its S lanes (broadcast reads);
+// the legs' f and their adds are coalesced pieces of run-minor rows; leg 0's f
+// and sums stay in registers while the element does.  Per tuple and run it does
+// 19 FP64 instructions a point and 45 more, against 320 of the contraction over
+// 27 moments; it issues 46 % of the time, bound by fixed-latency dependencies.
+// 48 runs on three meshes (32x32, 24x24, 16x16) to t = 0.5: 152 ms against 334 ms
+// through k_collision_runs.  16 warps a block at 126 registers: 12 warps take
+// 182 ms, 20 (spilled) 165; two points a step 158.
+template <int L, int FORM, int S>
+__global__ void __launch_bounds__(RUN_WARPS * 32, 1) k_rows_runs(const RowChan* __restrict__ chans,
+                                                                 const RowWork* __restrict__ work,
+                                                                 const int32_t* __restrict__ warp_row, int shares,
+                                                                 const double* __restrict__ f,
+                                                                 const int* __restrict__ nf, int n_nf,
+                                                                 double* __restrict__ acc,
+                                                                 const DPCtl* __restrict__ ctl,
+                                                                 int* __restrict__ err_flag, int wait_polls) {
+    constexpr int R = RowDim<L>::R, ND = RowDim<L>::ND, G = 32 / S;
+    constexpr uint32_t BYTES = RowDim<L>::BYTES;
+    extern __shared__ __align__(128) unsigned char s_raw[];
+    __shared__ RowChan c;
+    __shared__ __align__(8) uint64_t s_bar[RUN_WARPS][ROW_STAGES];
+    const RowWork w = work[blockIdx.x];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, n_warps = blockDim.x >> 5;
+    for (int i = tid; i < int(sizeof(RowChan) / sizeof(int)); i += blockDim.x)
+        reinterpret_cast<int*>(&c)[i] = reinterpret_cast<const int*>(chans + w.chan)[i];
+    __syncthreads();
+    const int g = lane / S, run = w.chunk * S + lane % S;
+    double amp = 0.0;   // 0: padding, switched off or finished
+    if (run < c.n_insts) {
+        const InstDev& in = c.insts[run];
+        if (in.amp_full != 0.0 && !(ctl && ctl[in.run].done)) amp = in.amp_full;
+    }
+    if (__all_sync(0xffffffffu, amp == 0.0)) return;   // uniform in the block
+    const int r0 = warp_row[w.share0 + warp], r1 = warp_row[w.share0 + warp + 1];   // blockDim = 32 shares
+    unsigned char* const stage = s_raw + size_t(warp) * ROW_STAGES * BYTES;
+    uint64_t* const bar = s_bar[warp];
+    auto fetch = [&](int r, int s) {
+        mbar_expect_tx_arrive(&bar[s], BYTES);
+        bulk_g2s(stage + s * BYTES, c.blk + int64_t(r) * BYTES, BYTES, &bar[s]);
+    };
+    if (lane == 0) {
+        for (int s = 0; s < ROW_STAGES; ++s) mbar_init(&bar[s], 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        for (int s = 0; s < ROW_STAGES; ++s)
+            if (r0 + s < r1) fetch(r0 + s, s);
+    }
+    double* const s_q = reinterpret_cast<double*>(s_raw + size_t(n_warps) * ROW_STAGES * BYTES);
+    for (int i = tid; i < c.nmc * R; i += blockDim.x) s_q[i] = __ldg(c.mc + i);
+    __syncthreads();
+    const FlatTable tab{s_q};
+    // element e of leg l: coefficient j at [3 e S + j S]
+    const double* fl[L];
+    double* al[L];
+#pragma unroll
+    for (int l = 0; l < L; ++l) {
+        const int64_t o = (w.chunk * c.ndof + c.loff[l]) * S + lane % S;
+        fl[l] = c.fT + o;
+        al[l] = c.accT + o;
+    }
+    double z[3] = {0.0, 0.0, 0.0};
+    int e0 = -1;
+    double4 f0 = make_double4(0., 0., 0., 0.);
+    auto flush = [&]() {
+#pragma unroll
+        for (int o = S; o < 32; o *= 2)
+#pragma unroll
+            for (int j = 0; j < 3; ++j) z[j] += __shfl_xor_sync(0xffffffffu, z[j], o);
+        if (g == 0 && amp != 0.0) {
+            double* o = al[0] + 3 * S * e0;
+#pragma unroll
+            for (int j = 0; j < 3; ++j) atomicAdd(o + j * S, z[j]);
+        }
+        z[0] = z[1] = z[2] = 0.0;
+    };
+    for (int r = r0; r < r1; ++r) {
+        const int s = (r - r0) % ROW_STAGES;
+        const int e0_row = __ldg(c.row_e0 + r);
+        if (e0_row != e0) {
+            if (e0 >= 0) flush();
+            e0 = e0_row;
+            const double* p = fl[0] + 3 * S * e0;
+            f0 = make_double4(__ldg(p), __ldg(p + S), __ldg(p + 2 * S), 0.0);
+        }
+        if (!mbar_wait(&bar[s], uint32_t((r - r0) / ROW_STAGES) & 1u, wait_polls)) {
+            // record the failure and give the copies in flight a bounded
+            // chance to land before the block releases its shared memory
+            if (lane == 0) atomicExch(err_flag, 1);
+            for (int k = 0; k < ROW_STAGES && r + k < r1; ++k)
+                mbar_wait(&bar[(r + k - r0) % ROW_STAGES], uint32_t((r + k - r0) / ROW_STAGES) & 1u, 1 << 16);
+            break;
+        }
+        const unsigned char* b = stage + s * BYTES;
+#pragma unroll 1
+        for (int t0 = 0; t0 < 32; t0 += G) {
+            const int t = t0 + g;
+            const uint64_t mk = reinterpret_cast<const uint64_t*>(b + 256 * ND)[t];
+            if (__all_sync(0xffffffffu, mk == 0ull)) break;   // the padding of the element's last row
+            double4 fv[L];
+            double* o[L];
+            fv[0] = f0;
+#pragma unroll
+            for (int l = 1; l < L; ++l) {
+                const int k = 3 * S * reinterpret_cast<const int32_t*>(b + 256 * (ND + 1))[32 * (l - 1) + t];
+                const double* p = fl[l] + k;
+                o[l] = al[l] + k;
+                fv[l] = make_double4(__ldg(p), __ldg(p + S), __ldg(p + 2 * S), 0.0);
+            }
+            const StageMap<L> m{reinterpret_cast<const double*>(b) + t};
+            double scale = reinterpret_cast<const double*>(b)[32 * (ND - 1) + t] * amp;
+            if (c.tamp && mk) scale *= __ldg(c.tamp + __ldg(c.perm + int64_t(r) * 32 + t));
+            RowOut<L> v;
+            row_tuple<L, FORM>(c, m, mk, fv, tab, scale, v);
+#pragma unroll
+            for (int j = 0; j < 3; ++j) z[j] += v.v[0][j];
+            if (mk && amp != 0.0) {
+#pragma unroll
+                for (int l = 1; l < L; ++l)
+#pragma unroll
+                    for (int j = 0; j < 3; ++j) atomicAdd(o[l] + j * S, v.v[l][j]);
+            }
+        }
+        __syncwarp();   // every lane is done with the stage
+        if (lane == 0 && r + ROW_STAGES < r1) fetch(r + ROW_STAGES, s);
+    }
+    if (e0 >= 0) flush();
+    int bad = 0;
+    for (int i = tid; i < n_nf; i += blockDim.x) bad |= nf[i];
+    if (__syncthreads_or(bad)) {
+        const int i0 = w.chunk * S;
+        FxAcc none;
+        spread_nonfinite<L>(c, c.insts + i0, min(S, c.n_insts - i0), w.t0, w.t1, f, acc, ctl, false, -1, none);
+    }
+}
+
+template <int L, int FORM, int S>
+static int launch_k_rows_runs(const RowSet& rs, int n_tiles, const double* f, const int* nf, double* acc,
+                              const DPCtl* ctl, cudaStream_t s, int* err_flag, int polls) {
+    auto kern = k_rows_runs<L, FORM, S>;
+    auto bytes = [](int nmc, int warps) {
+        return size_t(warps) * ROW_STAGES * row_bytes(L) + sizeof(double) * size_t(nmc) * RowDim<L>::R;
+    };
+    static std::atomic<unsigned long long> attr_devices{0};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev < 0 || dev >= 64 || !((attr_devices.load() >> dev) & 1ull)) {
+        TB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes(64, RUN_WARPS))));
+        if (dev >= 0 && dev < 64) attr_devices.fetch_or(1ull << dev);
+    }
+    kern<<<unsigned(rs.nblocks), unsigned(32 * rs.shares), bytes(rs.nmc_max, rs.shares), s>>>(
+        rs.d_chan, rs.d_work, rs.d_warp_row, rs.shares, f, nf, n_tiles, acc, ctl, err_flag, polls);
+    TB_CUDA(cudaGetLastError());
+    return TB_OK;
+}
+
+template <int L, int FORM>
+static int launch_rows_runs_s(const RowSet& rs, int n_tiles, const double* f, const int* nf, double* acc,
+                              const DPCtl* ctl, cudaStream_t s, int* err_flag, int polls) {
+    if (rs.S == 8) return launch_k_rows_runs<L, FORM, 8>(rs, n_tiles, f, nf, acc, ctl, s, err_flag, polls);
+    if (rs.S == 16) return launch_k_rows_runs<L, FORM, 16>(rs, n_tiles, f, nf, acc, ctl, s, err_flag, polls);
+    return launch_k_rows_runs<L, FORM, 32>(rs, n_tiles, f, nf, acc, ctl, s, err_flag, polls);
+}
+
+int launch_run_rows(const std::vector<RowSet>& sets, const RunState* st, int n_st, int n_tiles, const double* f,
+                    int* nf, double* acc, const DPCtl* ctl, cudaStream_t s, int* err_flag, int polls) {
+    if (sets.empty()) return TB_OK;
+    k_runs_state_gather<<<unsigned(n_tiles), dim3(32, 8), 0, s>>>(st, n_st, f, nf, ctl);
+    TB_CUDA(cudaGetLastError());
+    for (const RowSet& rs : sets) {
+        if (rs.nblocks <= 0) continue;
+        int rc;
+        if (rs.L == 2)
+            rc = rs.form == FORM_2 ? launch_rows_runs_s<2, FORM_2>(rs, n_tiles, f, nf, acc, ctl, s, err_flag, polls)
+                              : launch_rows_runs_s<2, -1>(rs, n_tiles, f, nf, acc, ctl, s, err_flag, polls);
+        else
+            rc = rs.form == FORM_3 ? launch_rows_runs_s<3, FORM_3>(rs, n_tiles, f, nf, acc, ctl, s, err_flag, polls)
+                              : launch_rows_runs_s<3, -1>(rs, n_tiles, f, nf, acc, ctl, s, err_flag, polls);
+        TB_TRY(rc);
+    }
+    k_runs_state_scatter<<<unsigned(n_tiles), dim3(32, 8), 0, s>>>(st, n_st, acc, ctl);
+    TB_CUDA(cudaGetLastError());
     return TB_OK;
 }
 

@@ -24,10 +24,15 @@ struct PointRows {
     int64_t nrows = 0;
     int64_t n = 0, points = 0;      // tuples and points inside
     std::vector<int64_t> cost;      // [nrows + 1] running cost of the rows (host)
+    std::vector<int64_t> run_cost;  // the same, run-minor
     void release();
 };
 
 size_t row_bytes(int L);
+
+// Directions and statistics of a channel's legs: bit l: leg l is ingoing, bit
+// 4 + l: it is a boson.
+int row_form(const ChanDev& c);
 
 // Builds the rows from a ThetaList.  rows.blk stays null when there is no
 // room (the caller then keeps another path).
@@ -44,6 +49,12 @@ struct RowChan {
     int n_insts;
     int nmc;
     LegDev leg[3];
+    // shared by many runs: the structure's run-minor state and accumulator
+    // (RunState), the legs' band offsets within a run
+    const double* fT;
+    double* accT;
+    int64_t ndof;
+    int64_t loff[3];
     // the whole list, for states with non-finite coefficients
     const int32_t* tup;
     int64_t stride, n;
@@ -54,27 +65,46 @@ struct RowChan {
 struct RowWork {
     int chan;
     int share0;
+    int chunk;       // run-minor sets: which S runs
+    int pad;
     int64_t t0, t1;
 };
 
-// A set of channels of equal leg count and directions that one launch
+// A set of channels of equal leg count and form that one launch
 // evaluates.
 struct RowSet {
     int L = 0;
-    int dirs = 0;                   // bit l: leg l is ingoing
+    int form = 0;                   // row_form
     RowChan* d_chan = nullptr;
     RowWork* d_work = nullptr;
     int32_t* d_warp_row = nullptr;  // per block: the bounds of its shares
     int nblocks = 0, shares = 0;
     int nmc_max = 0;
     bool multi = false;             // some channel has several instances
+    int S = 0;                      // run-minor: runs per lane group (8, 16 or 32), else 0
     void release();
 };
 
+// A structure whose runs share its rows: the state of its n runs, run-minor
+// in groups of S ([i / S][dof][i % S]).
+// Run i of the structure starts at dof_off[i] of the handle's state.
+struct RunState {
+    double* fT;
+    double* accT;                   // all zero between evaluations
+    const int64_t* dof_off;         // [n]
+    const int* run;                 // [n] run numbers (DPCtl index)
+    int n, np, S;                   // np: n padded to whole groups
+    int64_t ndof;                   // dofs of one run
+    int tile0, tiles_i;             // first tile of the structure, tiles across runs
+};
+
+// Runs per lane group for n runs: the widest of 32, 16 and 8 that pads n least.
+int rows_lane_group(int n);
+
 // Uploads the set for the given channels (rows of channel i in rows[i]);
 // blocks are dealt out by the rows' cost.
-int build_row_set(int L, int dirs, const std::vector<RowChan>& chan, const std::vector<const PointRows*>& rows,
-                  RowSet& out);
+int build_row_set(int L, int form, const std::vector<RowChan>& chan, const std::vector<const PointRows*>& rows,
+                  RowSet& out, int S = 0);
 
 // f4[e] = (f0, f1, f2, 0) of every element of the state; nf[b] != 0 marks an
 // element block that holds a non-finite coefficient.
@@ -84,8 +114,14 @@ int launch_rows_prepare(const ElemDev& ed, const double* f, double4* f4, int* nf
 // scattering rate of leg rate_leg (of every leg when it is negative).
 // one non-null: that instance in place of the channels' instances.  err_flag
 // is set when a bounded wait (polls) for a staged row runs out.
-int launch_rows(const RowSet& rs, const ElemDev& ed, const double4* f4, const int* nf, double* acc, const DPCtl* ctl,
+int launch_rows(const RowSet& rs, const ElemDev& ed, const double* f, const double4* f4, const int* nf, double* acc, const DPCtl* ctl,
                 cudaStream_t s, bool rate, int rate_leg, const FxAcc& fx, int* err_flag, int polls,
                 const InstDev* one = nullptr);
+
+// The run-minor sets: the structures' states gathered, each set evaluated,
+// their accumulators added to acc and cleared.  st: device copy of the n_st
+// structures (n_tiles tiles in all); nf as above, one flag per tile.
+int launch_run_rows(const std::vector<RowSet>& sets, const RunState* st, int n_st, int n_tiles, const double* f,
+                    int* nf, double* acc, const DPCtl* ctl, cudaStream_t s, int* err_flag, int polls);
 
 }  // namespace tb
