@@ -99,6 +99,7 @@ namespace tb {
 int choose_layouts(tb_handle* h);
 int autotune(tb_handle* h);
 int build_run_states(tb_handle* h);
+int64_t rows_room();
 void release_row_sets(tb_handle* h);
 }  // namespace tb
 
@@ -565,7 +566,7 @@ int build_runs(tb_handle* h, const tb_problem_desc* const* descs, int nruns) {
         for (auto& G : h->groups)
             if (G.layout == TB_LAYOUT_MC64) {
                 TB_TRY(build_theta_list(G.dev, G.tup, G.theta, h->stream));
-                if (G.theta.built) TB_TRY(build_rows(G.dev, G.theta, G.rows, h->stream));
+                if (G.theta.built) TB_TRY(build_rows(G.dev, G.theta, G.rows, rows_room(), h->stream));
                 G.use_rows = G.rows.blk != nullptr;
             }
     }
@@ -604,6 +605,13 @@ static int launch_group_mc(tb_handle* h, GroupChan& G, const InstDev* insts, int
                                148 * 32, rate_leg, nullptr, nullptr, h->fx);
 }
 
+// The most that the rows of one channel may take: what moment tensors may.
+int64_t rows_room() {
+    size_t freeb = 0, totalb = 0;
+    cudaMemGetInfo(&freeb, &totalb);
+    return int64_t(double(freeb) * 0.6);
+}
+
 // Channels shared by this many runs or more go over their rows run-minor, the
 // others one run after another (32x32 e-ph, us: 5 runs 257, 7 runs 344 one by
 // one; 8 runs 326 run-minor, where a group of 8 costs the same for 5).  Through
@@ -622,9 +630,11 @@ static RowChan row_chan(const GroupChan& G) {
     c.n_insts = int(G.insts.size());
     c.nmc = G.dev.nmc;
     for (int l = 0; l < G.L; ++l) c.leg[l] = G.dev.leg[l];
+    // the Monte-Carlo layout visits the tuples with points inside only, also
+    // for states with non-finite coefficients; a contraction visits every tuple
     c.tup = G.tup.d;
     c.stride = G.tup.cap;
-    c.n = G.tup.n;
+    c.n = G.layout == TB_LAYOUT_MC64 ? 0 : G.tup.n;
     return c;
 }
 
@@ -658,7 +668,7 @@ static int make_row_sets(tb_handle* h, Take take, bool run_minor, std::vector<Ro
             done[b] = true;
         }
         sets.emplace_back();
-        TB_TRY(build_row_set(A.L, row_form(A.dev), chan, rows, sets.back(), S));
+        TB_TRY(build_row_set(A.L, row_form(A.dev), chan, rows, h->ndofs, sets.back(), S));
     }
     return TB_OK;
 }
@@ -674,11 +684,31 @@ void release_row_sets(tb_handle* h) {
 int refresh_row_sets(tb_handle* h) {
     release_row_sets(h);
     for (auto& G : h->groups)
-        if (G.use_rows) TB_TRY(build_row_set(G.L, row_form(G.dev), {row_chan(G)}, {&G.rows}, G.row_one));
+        if (G.use_rows) TB_TRY(build_row_set(G.L, row_form(G.dev), {row_chan(G)}, {&G.rows}, h->ndofs, G.row_one));
     TB_TRY(make_row_sets(h, [](const GroupChan& G) { return G.run_state < 0; }, false, h->row_sets));
-    if (h->run_states.empty()) return TB_OK;
-    TB_TRY(make_row_sets(h, [](const GroupChan& G) { return G.run_state >= 0; }, false, h->rate_sets));
-    return make_row_sets(h, [](const GroupChan& G) { return G.run_state >= 0; }, true, h->run_sets);
+    if (!h->run_states.empty()) {
+        TB_TRY(make_row_sets(h, [](const GroupChan& G) { return G.run_state >= 0; }, false, h->rate_sets));
+        TB_TRY(make_row_sets(h, [](const GroupChan& G) { return G.run_state >= 0; }, true, h->run_sets));
+    }
+    // the further accumulators (not in the deterministic mode, whose adds are
+    // exact); without room the blocks share one
+    int copies = 1;
+    for (const auto* sets : {&h->row_sets, &h->rate_sets})
+        for (const RowSet& rs : *sets) copies = std::max(copies, rs.copies);
+    for (const auto& G : h->groups) copies = std::max(copies, G.row_one.copies);
+    if (copies - 1 > h->n_accr && !h->opts.deterministic) {
+        if (h->d_accr) cudaFree(h->d_accr);
+        h->n_accr = 0;
+        const size_t bytes = sizeof(double) * size_t(copies - 1) * size_t(h->ndofs);
+        if (cudaMalloc(&h->d_accr, bytes) != cudaSuccess) {
+            cudaGetLastError();
+            h->d_accr = nullptr;
+            return TB_OK;
+        }
+        TB_CUDA(cudaMemset(h->d_accr, 0, bytes));
+        h->n_accr = copies - 1;
+    }
+    return TB_OK;
 }
 
 // Run-minor states for the structures that ROWS_RUN_MINOR runs or more share
@@ -756,7 +786,7 @@ static int launch_row_sets(tb_handle* h, const double* d_in, double* d_acc, cons
         if (!G.use_rows) return TB_OK;
         TB_TRY(launch_rows_prepare(h->ed, d_in, h->d_f4, h->d_nf, ctl, h->stream));
         return launch_rows(G.row_one, h->ed, d_in, h->d_f4, h->d_nf, d_acc, ctl, h->stream, rate, rate_leg, h->fx,
-                           h->d_err, G.dev.wait_polls, I.d_single);
+                           h->d_err, G.dev.wait_polls, h->d_accr, I.d_single);
     }
     const int polls = h->groups.empty() ? 0 : h->groups[0].dev.wait_polls;
     const bool rates = rate && !h->rate_sets.empty();
@@ -766,7 +796,7 @@ static int launch_row_sets(tb_handle* h, const double* d_in, double* d_acc, cons
         for (const RowSet& rs : *sets)
             if (rate_leg < rs.L)
                 TB_TRY(launch_rows(rs, h->ed, d_in, h->d_f4, h->d_nf, d_acc, ctl, h->stream, rate, rate_leg, h->fx,
-                                   h->d_err, polls));
+                                   h->d_err, polls, h->d_accr));
     }
     if (rate || h->run_sets.empty()) return TB_OK;
     return launch_run_rows(h->run_sets, h->d_run_states, int(h->run_states.size()), h->n_run_tiles, d_in, h->d_run_nf,
@@ -845,7 +875,7 @@ static int tune_rows(tb_handle* h, GroupChan& G) {
         } else {
             TB_TRY(launch_rows_prepare(h->ed, h->d_f, h->d_f4, h->d_nf, nullptr, h->stream));
             TB_TRY(launch_rows(G.row_one, h->ed, h->d_f, h->d_f4, h->d_nf, h->d_acc, nullptr, h->stream, false, -1,
-                               h->fx, h->d_err, G.dev.wait_polls));
+                               h->fx, h->d_err, G.dev.wait_polls, h->d_accr));
         }
     }
     cudaEventRecord(e1, h->stream);
@@ -933,7 +963,7 @@ int choose_layouts(tb_handle* h) {
             if (h->opts.layout == TB_LAYOUT_AUTO && want == TB_LAYOUT_T64  &&
                 !(h->opts.deterministic && int(G.insts.size()) >= ROWS_MAX_EXACT)) {
                 TB_TRY(build_theta_list(G.dev, G.tup, G.theta, h->stream));
-                if (G.theta.built) TB_TRY(build_rows(G.dev, G.theta, G.rows, h->stream));
+                if (G.theta.built) TB_TRY(build_rows(G.dev, G.theta, G.rows, rows_room(), h->stream));
                 G.use_rows = G.rows.blk != nullptr;
                 if (G.use_rows) continue;
                 G.theta.release();
@@ -1141,6 +1171,7 @@ int tb_destroy(tb_handle* h) {
     }
     release_row_sets(h);
     for (void* p : h->run_allocs) cudaFree(p);
+    if (h->d_accr) cudaFree(h->d_accr);
     for (double* p : h->dev_allocs) cudaFree(p);
     for (void* p : h->dev_raw) cudaFree(p);
     if (h->dp.dense) cudaFree(h->dp.dense);

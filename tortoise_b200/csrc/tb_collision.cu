@@ -15,6 +15,8 @@
 //     go to the exact fixed-point accumulator instead (tb_exact.cuh), one
 //     lane at a time.
 // The kernel is FP64-FMA bound (about 55 FP64 operations per MC point for L=4).
+// Channels with at most 64 points go over packed rows instead (tb_rows.cu) where
+// those fit the device memory.
 // LIST: the same quadrature over a ThetaList (tb_theta.cu): the tuples with at
 // least one point inside the simplices, each visiting only those points (set
 // bits of its mask, in increasing order), i.e. the dense sums without their

@@ -33,7 +33,7 @@ struct GroupChan {
     int layout = TB_LAYOUT_MC64;
     MomentTensor tensor;
     ThetaList theta;              // tuples with points inside the simplices, and which (Monte-Carlo layout, rows)
-    // packed rows of those tuples (at most three legs; tb_rows.cuh): use_rows
+    // packed rows of those tuples (tb_rows.cuh): use_rows
     // evaluates the channel over them, alone or with the handle's other such
     // channels; row_one is the set of this channel only
     PointRows rows;
@@ -103,6 +103,8 @@ struct tb_handle {
     tb::RunState* d_run_states = nullptr;
     int* d_run_nf = nullptr;
     int n_run_tiles = 0;
+    double* d_accr = nullptr;    // further accumulators of the row sets, n_accr of ndofs
+    int n_accr = 0;
     double4* d_f4 = nullptr;
     int* d_nf = nullptr;
     // deterministic mode: the exact accumulator behind d_acc (3 words per

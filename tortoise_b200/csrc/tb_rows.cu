@@ -5,8 +5,8 @@
 // simplices only (tb_theta.cu), and everything but the legs' f is fixed for the
 // life of a handle.  A row keeps, for 32 tuples that share their leg-0 element,
 // the affine map of the constrained coordinates, the weight and the mask of
-// points inside, so an evaluation reads 120 bytes per three-leg tuple, in whole
-// lines, instead of the 864 bytes of its moments or the element tables of
+// points inside, so an evaluation reads 120 bytes per three-leg tuple (172 with
+// four legs), in whole lines, instead of the 864 bytes of its moments or the element tables of
 // three legs.
 //
 //   * One warp takes consecutive rows, one lane per tuple.  Rows of one leg-0
@@ -30,7 +30,10 @@
 // Measured (64x64 two-band e-ph, 8.7 M tuples, 50 M points, whole right-hand
 // side): 333 us against 1589 us through the FP64 moment tensor; three bands and
 // two phonons at 72x56: 689 against 3283 us; the rates of every leg at 40x24
-// with umklapp: 203 against 1797 us.  The kernel reads 3.4 TB/s and issues half
+// with umklapp: 203 against 1797 us; 16x16 e-e (40.8 M tuples of 172 bytes, 156 M
+// points): 1.58 ms against 3.58 ms of the list kernel (k_collision_mc), of which
+// the adds take 0.2 and the reads could take 1.07 at the copy rate; an 8x8 e-e
+// integration 21 against 32 ms.  The 64x64 kernel reads 3.4 TB/s and issues half
 // of the time, with 27 % of the FP64 pipe: fixed-latency dependencies of the
 // 16 warps on an SM bound it, then the shared-memory pipe (65 %).
 //
@@ -48,18 +51,22 @@
 
 namespace tb {
 
-constexpr int ROW_WARPS = 16;   // shares of rows that a block takes, one per warp
-// Warps of a block.  16 warps leave 128 registers a thread, which the
-// propagation and the exact variant fit; 20 spill (a 64x64 e-ph right-hand
-// side: 421 us against 336), 12 hide less latency (350).  The rates of every
-// leg take 12 (184 us against 210 at 16, 40x24 with umklapp).
-template <bool RATE, bool DET> struct RowCap { static constexpr int W = RATE && !DET ? 12 : ROW_WARPS; };
-constexpr int RUN_WARPS = 16;   // the same, run-minor
+// Shares of rows that a block takes, one per warp.  16 warps leave 128 registers
+// a thread, which the three-leg propagation and its exact variant fit; 20 spill
+// (a 64x64 e-ph right-hand side: 421 us against 336), 12 hide less latency
+// (350).  Four legs need 168 registers and 11 KB of stages a warp: 12 warps.
+__host__ __device__ constexpr int row_shares(int L) { return L == 4 ? 12 : 16; }
+// Warps of a block: the rates of every leg take fewer (184 us against 210 with
+// 16 at 40x24 e-ph with umklapp).
+template <int L, bool RATE, bool DET> struct RowCap {
+    static constexpr int W = RATE ? (L == 4 ? 8 : DET ? 16 : 12) : row_shares(L);
+};
 constexpr int ROW_STAGES = 2;    // rows of a warp in shared memory
 constexpr int ROW_COPIES = 16;   // copies of the point table, one per lane of a half warp
 
-// row_form of {fermion in, fermion out} and {fermion in, boson in, fermion out}
-constexpr int FORM_2 = 0x01, FORM_3 = 0x23;
+// row_form of {fermion in, fermion out}, {fermion in, boson in, fermion out} and
+// {two fermions in, two fermions out}
+constexpr int FORM_2 = 0x01, FORM_3 = 0x23, FORM_4 = 0x03;
 
 int row_form(const ChanDev& c) {
     int d = 0;
@@ -74,7 +81,7 @@ struct RowDim {
     static constexpr int BYTES = 32 * (8 * ND + 8 + 4 * (L - 1));
 };
 
-size_t row_bytes(int L) { return L == 2 ? RowDim<2>::BYTES : RowDim<3>::BYTES; }
+size_t row_bytes(int L) { return L == 2 ? RowDim<2>::BYTES : L == 3 ? RowDim<3>::BYTES : RowDim<4>::BYTES; }
 
 void PointRows::release() {
     if (blk) cudaFree(blk);
@@ -102,6 +109,21 @@ void RowSet::release() {
 __global__ void k_rows_count(const int32_t* __restrict__ e0, int64_t n, int32_t* __restrict__ count) {
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
         atomicAdd(count + e0[i], 1);
+}
+
+// The lanes of an element's last row that hold no tuple: no points, element 0.
+template <int L>
+__global__ void __launch_bounds__(256) k_rows_pad(const int32_t* __restrict__ count, const int64_t* __restrict__ row0,
+                                                  int ne, unsigned char* __restrict__ blk, int32_t* __restrict__ perm) {
+    constexpr int ND = RowDim<L>::ND;
+    const int e = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (e >= ne || count[e] % 32 == 0 || lane < count[e] % 32) return;
+    const int64_t row = row0[e] + count[e] / 32;
+    unsigned char* b = blk + row * RowDim<L>::BYTES;
+    for (int k = 0; k < ND; ++k) reinterpret_cast<double*>(b)[32 * k + lane] = 0.0;
+    reinterpret_cast<uint64_t*>(b + 256 * ND)[lane] = 0ull;
+    for (int l = 1; l < L; ++l) reinterpret_cast<int32_t*>(b + 256 * (ND + 1))[32 * (l - 1) + lane] = 0;
+    perm[row * 32 + lane] = -1;
 }
 
 // Tuple j of the sorted list goes to lane (j - first[e0]) % 32 of row
@@ -166,10 +188,10 @@ struct Tmp {
 };
 }  // namespace
 
-int build_rows(const ChanDev& c, const ThetaList& th, PointRows& rows, cudaStream_t s) {
+int build_rows(const ChanDev& c, const ThetaList& th, PointRows& rows, int64_t max_bytes, cudaStream_t s) {
     rows.release();
     const int64_t n = th.n;
-    if (n <= 0 || c.L > 3) return TB_OK;
+    if (n <= 0) return TB_OK;
     const int ne = c.leg[0].ne;
     Tmp tmp;
     int32_t* d_cnt = static_cast<int32_t*>(tmp.get(sizeof(int32_t) * size_t(ne)));
@@ -193,24 +215,26 @@ int build_rows(const ChanDev& c, const ThetaList& th, PointRows& rows, cudaStrea
     }
     int32_t* d_pts = static_cast<int32_t*>(tmp.get(2 * sizeof(int32_t) * size_t(nrows)));
     const size_t bytes = row_bytes(c.L) * size_t(nrows);
-    if (!d_pts || cudaMalloc(&rows.blk, bytes) != cudaSuccess ||
+    if (int64_t(bytes) > max_bytes || !d_pts || cudaMalloc(&rows.blk, bytes) != cudaSuccess ||
         cudaMalloc(&rows.row_e0, sizeof(int32_t) * size_t(nrows)) != cudaSuccess ||
         cudaMalloc(&rows.perm, sizeof(int32_t) * size_t(nrows) * 32) != cudaSuccess) {
         cudaGetLastError();
         rows.release();
         return TB_OK;
     }
-    TB_CUDA(cudaMemsetAsync(rows.blk, 0, bytes, s));   // padding: no points, element 0
-    TB_CUDA(cudaMemsetAsync(rows.perm, 0xff, sizeof(int32_t) * size_t(nrows) * 32, s));
     TB_CUDA(cudaMemsetAsync(d_pts, 0, 2 * sizeof(int32_t) * size_t(nrows), s));
     TB_CUDA(cudaMemcpyAsync(d_first, first.data(), sizeof(int64_t) * size_t(ne), cudaMemcpyHostToDevice, s));
     TB_CUDA(cudaMemcpyAsync(d_row0, row0.data(), sizeof(int64_t) * size_t(ne), cudaMemcpyHostToDevice, s));
-    if (c.L == 2)
-        k_rows_fill<2><<<blocks, 256, 0, s>>>(c, th.ids, th.mask, th.perm, n, d_first, d_row0, rows.blk, rows.row_e0,
-                                              rows.perm, d_pts);
-    else
-        k_rows_fill<3><<<blocks, 256, 0, s>>>(c, th.ids, th.mask, th.perm, n, d_first, d_row0, rows.blk, rows.row_e0,
-                                              rows.perm, d_pts);
+#define TB_FILL(LL)                                                                                                    \
+    k_rows_pad<LL><<<unsigned((int64_t(ne) * 32 + 255) / 256), 256, 0, s>>>(d_cnt, d_row0, ne, rows.blk, rows.perm);   \
+    k_rows_fill<LL><<<blocks, 256, 0, s>>>(c, th.ids, th.mask, th.perm, n, d_first, d_row0, rows.blk, rows.row_e0,     \
+                                           rows.perm, d_pts)
+    switch (c.L) {
+        case 2: TB_FILL(2); break;
+        case 3: TB_FILL(3); break;
+        default: TB_FILL(4); break;
+    }
+#undef TB_FILL
     TB_CUDA(cudaGetLastError());
     std::vector<int32_t> pts(2 * size_t(nrows), 0);
     TB_CUDA(cudaMemcpyAsync(pts.data(), d_pts, sizeof(int32_t) * pts.size(), cudaMemcpyDeviceToHost, s));
@@ -649,23 +673,25 @@ __device__ __noinline__ void spread_nonfinite(const RowChan& c, const InstDev* i
 }
 
 template <int L, int FORM, bool RATE, bool DET, bool MULTI>
-__global__ void __launch_bounds__(RowCap<RATE, DET>::W * 32, 1) k_rows(const RowChan* __restrict__ chans,
+__global__ void __launch_bounds__(RowCap<L, RATE, DET>::W * 32, 1) k_rows(const RowChan* __restrict__ chans,
                                                             const RowWork* __restrict__ work,
                                                             const int32_t* __restrict__ warp_row, int shares,
                                                             const InstDev* __restrict__ one,
                                                             const double* __restrict__ f,
                                                             const double4* __restrict__ f4,
                                                             const int* __restrict__ nf, int n_nf,
-                                                            double* __restrict__ acc, const DPCtl* __restrict__ ctl,
+                                                            double* __restrict__ acc, double* __restrict__ accr,
+                                                            int copies, int64_t ndofs, const DPCtl* __restrict__ ctl,
                                                             int rate_leg, FxAcc fx, int* __restrict__ err_flag,
                                                             int wait_polls) {
     constexpr int R = RowDim<L>::R, ND = RowDim<L>::ND;
     constexpr uint32_t BYTES = RowDim<L>::BYTES;
     extern __shared__ __align__(128) unsigned char s_raw[];
     __shared__ RowChan c;
-    __shared__ __align__(8) uint64_t s_bar[RowCap<RATE, DET>::W][ROW_STAGES];
+    __shared__ __align__(8) uint64_t s_bar[RowCap<L, RATE, DET>::W][ROW_STAGES];
     const RowWork w = work[blockIdx.x];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, n_warps = blockDim.x >> 5;
+    if (accr && blockIdx.x % copies) acc = accr + int64_t(blockIdx.x % copies - 1) * ndofs;
     for (int i = tid; i < int(sizeof(RowChan) / sizeof(int)); i += blockDim.x)
         reinterpret_cast<int*>(&c)[i] = reinterpret_cast<const int*>(chans + w.chan)[i];
     __syncthreads();
@@ -804,6 +830,38 @@ __global__ void __launch_bounds__(RowCap<RATE, DET>::W * 32, 1) k_rows(const Row
         spread_nonfinite<L>(c, insts, n_insts, w.t0, w.t1, f, acc, ctl, RATE, rate_leg, fx);
 }
 
+// acc += the further accumulators, which are cleared.
+__global__ void __launch_bounds__(256) k_rows_fold(double* __restrict__ acc, double* __restrict__ accr, int n,
+                                                   int64_t ndofs) {
+    __shared__ double s[8][32];
+    const int64_t d = int64_t(blockIdx.x) * 32 + threadIdx.x;
+    double v = 0.0;
+    if (d < ndofs)
+        for (int k = threadIdx.y; k < n; k += 8) {
+            double* p = accr + k * ndofs + d;
+            v += *p;
+            *p = 0.0;
+        }
+    s[threadIdx.y][threadIdx.x] = v;
+    __syncthreads();
+    if (threadIdx.y || d >= ndofs) return;
+    for (int k = 1; k < 8; ++k) v += s[k][threadIdx.x];
+    acc[d] += v;
+}
+
+// Accumulators for a set of nblocks blocks: the adds of small meshes fall on so
+// few sectors that the L2 serialises them.  Where an element takes more than
+// ROW_ADDS of them every block has its own copy, within ROW_COPY_BYTES for all.
+// Measured: 16x16 e-e (239,000 adds an element) 6.6 ms with one copy, 1.79 with
+// 32, 1.71 with 64, 1.58 with 148; an 8x8 e-e integration (29,000) 165 ms with
+// one, 54 with 4, 29 with 16, 23 with 64 and with 148; 64x64 e-ph (900) 324 us
+// with one, 335 with 2, 340 with 8.
+constexpr int64_t ROW_ADDS = 2000, ROW_COPY_BYTES = int64_t(64) << 20;
+static int row_copies(int64_t adds_per_element, int nblocks, int64_t ndofs) {
+    if (adds_per_element <= ROW_ADDS) return 1;
+    return int(std::max<int64_t>(1, std::min<int64_t>(nblocks, ROW_COPY_BYTES / (8 * std::max<int64_t>(ndofs, 1)))));
+}
+
 static size_t rows_smem(int L, int nmc, int warps) {
     return size_t(warps) * (ROW_STAGES * row_bytes(L) + 768 * size_t(L - 1)) +
            sizeof(double) * size_t(nmc) * size_t(2 * (L - 2) + 1) * ROW_COPIES;
@@ -812,7 +870,7 @@ static size_t rows_smem(int L, int nmc, int warps) {
 template <int L, int FORM, bool RATE, bool DET, bool MULTI>
 static int launch_k_rows(const RowSet& rs, const ElemDev& ed, const double* f, const double4* f4, const int* nf, double* acc,
                          const DPCtl* ctl, cudaStream_t s, int rate_leg, const FxAcc& fx, const InstDev* one,
-                         int* err_flag, int polls) {
+                         int* err_flag, int polls, double* accr) {
     auto kern = k_rows<L, FORM, RATE, DET, MULTI>;
     // the shared-memory limit, set once on each device the kernel runs on
     static std::atomic<unsigned long long> attr_devices{0};
@@ -820,12 +878,17 @@ static int launch_k_rows(const RowSet& rs, const ElemDev& ed, const double* f, c
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64 || !((attr_devices.load() >> dev) & 1ull)) {
         TB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     int(rows_smem(L, 64, ROW_WARPS))));
+                                     int(rows_smem(L, 64, RowCap<L, RATE, DET>::W))));
         if (dev >= 0 && dev < 64) attr_devices.fetch_or(1ull << dev);
     }
-    const int warps = std::min(rs.shares, RowCap<RATE, DET>::W);
+    const int warps = std::min(rs.shares, RowCap<L, RATE, DET>::W);
     kern<<<unsigned(rs.nblocks), unsigned(32 * warps), rows_smem(L, rs.nmc_max, warps), s>>>(
-        rs.d_chan, rs.d_work, rs.d_warp_row, rs.shares, one, f, f4, nf, ed.nblk, acc, ctl, rate_leg, fx, err_flag, polls);
+        rs.d_chan, rs.d_work, rs.d_warp_row, rs.shares, one, f, f4, nf, ed.nblk, acc, accr, rs.copies,
+        ed.ndofs, ctl, rate_leg, fx, err_flag, polls);
+    if (accr && rs.copies > 1) {
+        TB_CUDA(cudaGetLastError());
+        k_rows_fold<<<unsigned((ed.ndofs + 31) / 32), dim3(32, 8), 0, s>>>(acc, accr, rs.copies - 1, ed.ndofs);
+    }
     TB_CUDA(cudaGetLastError());
     return TB_OK;
 }
@@ -833,21 +896,21 @@ static int launch_k_rows(const RowSet& rs, const ElemDev& ed, const double* f, c
 template <int L, int FORM, bool RATE, bool DET>
 static int launch_rows_m(const RowSet& rs, const ElemDev& ed, const double* f, const double4* f4, const int* nf, double* acc,
                          const DPCtl* ctl, cudaStream_t s, int rate_leg, const FxAcc& fx, const InstDev* one,
-                         int* err_flag, int polls) {
+                         int* err_flag, int polls, double* accr) {
     if (rs.multi && !one)
-        return launch_k_rows<L, FORM, RATE, DET, true>(rs, ed, f, f4, nf, acc, ctl, s, rate_leg, fx, one, err_flag, polls);
-    return launch_k_rows<L, FORM, RATE, DET, false>(rs, ed, f, f4, nf, acc, ctl, s, rate_leg, fx, one, err_flag, polls);
+        return launch_k_rows<L, FORM, RATE, DET, true>(rs, ed, f, f4, nf, acc, ctl, s, rate_leg, fx, one, err_flag, polls, accr);
+    return launch_k_rows<L, FORM, RATE, DET, false>(rs, ed, f, f4, nf, acc, ctl, s, rate_leg, fx, one, err_flag, polls, accr);
 }
 
 // The channels that addScatteringChannelsWildcards builds in the reference's
-// examples are compiled in (FORM_2, FORM_3); others select their forms at run
+// examples are compiled in (FORM_2, FORM_3, FORM_4); others select their forms at run
 // time.
 template <int L>
 static int launch_rows_l(const RowSet& rs, const ElemDev& ed, const double* f, const double4* f4, const int* nf, double* acc,
                          const DPCtl* ctl, cudaStream_t s, bool rate, int rate_leg, const FxAcc& fx,
-                         const InstDev* one, int* err_flag, int polls) {
-    constexpr int CANON = L == 2 ? FORM_2 : FORM_3;
-#define TB_ROWS(DD, RR, XX) launch_rows_m<L, DD, RR, XX>(rs, ed, f, f4, nf, acc, ctl, s, rate_leg, fx, one, err_flag, polls)
+                         const InstDev* one, int* err_flag, int polls, double* accr) {
+    constexpr int CANON = L == 2 ? FORM_2 : L == 3 ? FORM_3 : FORM_4;
+#define TB_ROWS(DD, RR, XX) launch_rows_m<L, DD, RR, XX>(rs, ed, f, f4, nf, acc, ctl, s, rate_leg, fx, one, err_flag, polls, accr)
     if (fx.w) return rate ? TB_ROWS(-1, true, true) : TB_ROWS(-1, false, true);
     if (rs.form == CANON) return rate ? TB_ROWS(CANON, true, false) : TB_ROWS(CANON, false, false);
     return rate ? TB_ROWS(-1, true, false) : TB_ROWS(-1, false, false);
@@ -856,16 +919,15 @@ static int launch_rows_l(const RowSet& rs, const ElemDev& ed, const double* f, c
 
 int launch_rows(const RowSet& rs, const ElemDev& ed, const double* f, const double4* f4, const int* nf, double* acc, const DPCtl* ctl,
                 cudaStream_t s, bool rate, int rate_leg, const FxAcc& fx, int* err_flag, int polls,
-                const InstDev* one) {
+                double* accr, const InstDev* one) {
     if (rs.nblocks <= 0) return TB_OK;
-    if (rs.L == 2) return launch_rows_l<2>(rs, ed, f, f4, nf, acc, ctl, s, rate, rate_leg, fx, one, err_flag, polls);
-    if (rs.L == 3) return launch_rows_l<3>(rs, ed, f, f4, nf, acc, ctl, s, rate, rate_leg, fx, one, err_flag, polls);
-    set_error("rows hold two or three legs");
-    return TB_ERR_ARG;
+    if (rs.L == 2) return launch_rows_l<2>(rs, ed, f, f4, nf, acc, ctl, s, rate, rate_leg, fx, one, err_flag, polls, accr);
+    if (rs.L == 3) return launch_rows_l<3>(rs, ed, f, f4, nf, acc, ctl, s, rate, rate_leg, fx, one, err_flag, polls, accr);
+    return launch_rows_l<4>(rs, ed, f, f4, nf, acc, ctl, s, rate, rate_leg, fx, one, err_flag, polls, accr);
 }
 
 int build_row_set(int L, int form, const std::vector<RowChan>& chan, const std::vector<const PointRows*>& rows,
-                  RowSet& out, int S) {
+                  int64_t ndofs, RowSet& out, int S) {
     out.release();
     out.L = L;
     out.form = form;
@@ -889,7 +951,7 @@ int build_row_set(int L, int form, const std::vector<RowChan>& chan, const std::
     // one block per SM; fewer warps in each where there are fewer rows than
     // warps.  Every item gets a block of its own at least, the others go one
     // by one to the item with the largest cost per block.
-    out.shares = int(std::min<int64_t>(S ? RUN_WARPS : ROW_WARPS, std::max<int64_t>(4, (nrows + nsm - 1) / nsm)));
+    out.shares = int(std::min<int64_t>(row_shares(L), std::max<int64_t>(4, (nrows + nsm - 1) / nsm)));
     std::vector<int64_t> nb(item.size(), 1);
     auto cost_of = [&](size_t i) -> const std::vector<int64_t>& {
         const PointRows& r = *rows[size_t(item[i].first)];
@@ -936,6 +998,13 @@ int build_row_set(int L, int form, const std::vector<RowChan>& chan, const std::
     TB_CUDA(cudaMemcpy(out.d_work, work.data(), sizeof(RowWork) * work.size(), cudaMemcpyHostToDevice));
     TB_CUDA(cudaMemcpy(out.d_warp_row, warp_row.data(), sizeof(int32_t) * warp_row.size(), cudaMemcpyHostToDevice));
     out.nblocks = int(work.size());
+    int64_t adds = 0;   // of the channel whose smallest band takes the most for each element
+    for (size_t i = 0; i < chan.size(); ++i) {
+        int64_t ne = chan[i].leg[1].ne;
+        for (int l = 2; l < L; ++l) ne = std::min<int64_t>(ne, chan[i].leg[l].ne);
+        adds = std::max(adds, rows[i]->n * (L - 1) / std::max<int64_t>(ne, 1));
+    }
+    out.copies = S ? 1 : row_copies(adds, out.nblocks, ndofs);
     return TB_OK;
 }
 
@@ -1017,7 +1086,7 @@ __global__ void __launch_bounds__(256) k_runs_state_scatter(const RunState* __re
 // through k_collision_runs.  16 warps a block at 126 registers: 12 warps take
 // 182 ms, 20 (spilled) 165; two points a step 158.
 template <int L, int FORM, int S>
-__global__ void __launch_bounds__(RUN_WARPS * 32, 1) k_rows_runs(const RowChan* __restrict__ chans,
+__global__ void __launch_bounds__(row_shares(L) * 32, 1) k_rows_runs(const RowChan* __restrict__ chans,
                                                                  const RowWork* __restrict__ work,
                                                                  const int32_t* __restrict__ warp_row, int shares,
                                                                  const double* __restrict__ f,
@@ -1029,7 +1098,7 @@ __global__ void __launch_bounds__(RUN_WARPS * 32, 1) k_rows_runs(const RowChan* 
     constexpr uint32_t BYTES = RowDim<L>::BYTES;
     extern __shared__ __align__(128) unsigned char s_raw[];
     __shared__ RowChan c;
-    __shared__ __align__(8) uint64_t s_bar[RUN_WARPS][ROW_STAGES];
+    __shared__ __align__(8) uint64_t s_bar[row_shares(L)][ROW_STAGES];
     const RowWork w = work[blockIdx.x];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, n_warps = blockDim.x >> 5;
     for (int i = tid; i < int(sizeof(RowChan) / sizeof(int)); i += blockDim.x)
@@ -1154,7 +1223,7 @@ static int launch_k_rows_runs(const RowSet& rs, int n_tiles, const double* f, co
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64 || !((attr_devices.load() >> dev) & 1ull)) {
-        TB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes(64, RUN_WARPS))));
+        TB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes(64, row_shares(L)))));
         if (dev >= 0 && dev < 64) attr_devices.fetch_or(1ull << dev);
     }
     kern<<<unsigned(rs.nblocks), unsigned(32 * rs.shares), bytes(rs.nmc_max, rs.shares), s>>>(
@@ -1182,6 +1251,9 @@ int launch_run_rows(const std::vector<RowSet>& sets, const RunState* st, int n_s
         if (rs.L == 2)
             rc = rs.form == FORM_2 ? launch_rows_runs_s<2, FORM_2>(rs, n_tiles, f, nf, acc, ctl, s, err_flag, polls)
                               : launch_rows_runs_s<2, -1>(rs, n_tiles, f, nf, acc, ctl, s, err_flag, polls);
+        else if (rs.L == 4)
+            rc = rs.form == FORM_4 ? launch_rows_runs_s<4, FORM_4>(rs, n_tiles, f, nf, acc, ctl, s, err_flag, polls)
+                                   : launch_rows_runs_s<4, -1>(rs, n_tiles, f, nf, acc, ctl, s, err_flag, polls);
         else
             rc = rs.form == FORM_3 ? launch_rows_runs_s<3, FORM_3>(rs, n_tiles, f, nf, acc, ctl, s, err_flag, polls)
                               : launch_rows_runs_s<3, -1>(rs, n_tiles, f, nf, acc, ctl, s, err_flag, polls);

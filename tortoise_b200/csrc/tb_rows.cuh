@@ -1,5 +1,5 @@
 // tb_rows.cuh -- packed rows of tuples: the Monte-Carlo quadrature over the
-// points inside the simplices for channels with at most three legs.
+// points inside the simplices.
 #pragma once
 
 #include <vector>
@@ -34,9 +34,9 @@ size_t row_bytes(int L);
 // 4 + l: it is a boson.
 int row_form(const ChanDev& c);
 
-// Builds the rows from a ThetaList.  rows.blk stays null when there is no
-// room (the caller then keeps another path).
-int build_rows(const ChanDev& c, const ThetaList& th, PointRows& rows, cudaStream_t s);
+// Builds the rows from a ThetaList.  rows.blk stays null when they would take
+// more than max_bytes (the caller then keeps another path).
+int build_rows(const ChanDev& c, const ThetaList& th, PointRows& rows, int64_t max_bytes, cudaStream_t s);
 
 // What the kernel needs of one channel, in device memory.
 struct RowChan {
@@ -48,13 +48,13 @@ struct RowChan {
     const InstDev* insts;
     int n_insts;
     int nmc;
-    LegDev leg[3];
+    LegDev leg[4];
     // shared by many runs: the structure's run-minor state and accumulator
     // (RunState), the legs' band offsets within a run
     const double* fT;
     double* accT;
     int64_t ndof;
-    int64_t loff[3];
+    int64_t loff[4];
     // the whole list, for states with non-finite coefficients
     const int32_t* tup;
     int64_t stride, n;
@@ -80,6 +80,7 @@ struct RowSet {
     int32_t* d_warp_row = nullptr;  // per block: the bounds of its shares
     int nblocks = 0, shares = 0;
     int nmc_max = 0;
+    int copies = 1;                 // accumulators that its blocks share out (row_copies)
     bool multi = false;             // some channel has several instances
     int S = 0;                      // run-minor: runs per lane group (8, 16 or 32), else 0
     void release();
@@ -101,10 +102,11 @@ struct RunState {
 // Runs per lane group for n runs: the widest of 32, 16 and 8 that pads n least.
 int rows_lane_group(int n);
 
-// Uploads the set for the given channels (rows of channel i in rows[i]);
+// Uploads the set for the given channels (rows of channel i in rows[i]) of a
+// handle with ndofs coefficients;
 // blocks are dealt out by the rows' cost.
 int build_row_set(int L, int form, const std::vector<RowChan>& chan, const std::vector<const PointRows*>& rows,
-                  RowSet& out, int S = 0);
+                  int64_t ndofs, RowSet& out, int S = 0);
 
 // f4[e] = (f0, f1, f2, 0) of every element of the state; nf[b] != 0 marks an
 // element block that holds a non-finite coefficient.
@@ -113,10 +115,12 @@ int launch_rows_prepare(const ElemDev& ed, const double* f, double4* f4, int* nf
 // acc (or fx) += the collision terms of the set's channels; rate: the
 // scattering rate of leg rate_leg (of every leg when it is negative).
 // one non-null: that instance in place of the channels' instances.  err_flag
-// is set when a bounded wait (polls) for a staged row runs out.
+// is set when a bounded wait (polls) for a staged row runs out.  accr: the
+// rs.copies - 1 further accumulators of ed.ndofs doubles, all zero between
+// launches (null: one accumulator for all blocks).
 int launch_rows(const RowSet& rs, const ElemDev& ed, const double* f, const double4* f4, const int* nf, double* acc, const DPCtl* ctl,
                 cudaStream_t s, bool rate, int rate_leg, const FxAcc& fx, int* err_flag, int polls,
-                const InstDev* one = nullptr);
+                double* accr, const InstDev* one = nullptr);
 
 // The run-minor sets: the structures' states gathered, each set evaluated,
 // their accumulators added to acc and cleared.  st: device copy of the n_st
