@@ -139,6 +139,35 @@ def test_amplitude_factors_and_pinned_schedules(gpu_lib):
         e.close()
 
 
+@pytest.mark.parametrize("shape", ["in_in_out", "in_out_out", "out_in_out", "two_legs", "umklapp", "four_legs",
+                                   "four_legs_bosons", "64_points"])
+def test_vjp_equals_the_tensor_and_the_list(gpu_lib, shape):
+    """grad_f and the amplitude gradients against the moment tensor's transpose, and (one instance or several, one
+    channel switched off) against the exact sums over the list."""
+    mats = [_material(amp=0.7 + 0.2 * r, **SHAPES[shape]) for r in range(3)]
+    fs = [W.initial_status(m, kT=0.1 + 0.05 * r, seed=r).vec for r, m in enumerate(mats)]
+    rng = np.random.default_rng(8)
+    ths = [rng.standard_normal(f.size) for f in fs]
+    rows, tensor = E.Engine(mats[0]), E.Engine(mats[0], layout=E.LAYOUT_T64)
+    batch, listed = E.BatchEngine(mats), E.BatchEngine(mats, layout=E.LAYOUT_MC64, deterministic=True)
+    try:
+        ref = tensor.rhs_vjp(fs[0], ths[0])
+        for got in (rows.rhs_vjp(fs[0], ths[0]), rows.rhs_vjp(fs[0], ths[0])):
+            assert rel_l2(got[0], ref[0]) < TOL and rel_l2(got[1], ref[1]) < TOL
+        for e in (batch, listed):
+            e.set_amplitude(0, 0.0)
+        a, b = (e.rhs_vjp(np.concatenate(fs), np.concatenate(ths)) for e in (batch, listed))
+        assert rel_l2(a[0], b[0]) < TOL and rel_l2(a[1], b[1]) < TOL
+        th = ths[0].copy()
+        th[3] = np.nan
+        got, ref = rows.rhs_vjp(fs[0], th), tensor.rhs_vjp(fs[0], th)
+        assert np.array_equal(np.isfinite(got[0]), np.isfinite(ref[0])) or mats[0].channels[0].nlegs == 4
+        assert np.array_equal(np.isfinite(got[1]), np.isfinite(ref[1]))
+    finally:
+        for e in (rows, tensor, batch, listed):
+            e.close()
+
+
 @pytest.mark.parametrize("value", [np.nan, np.inf])
 def test_non_finite_coefficients_reach_the_same_elements_as_the_tensor(gpu_lib, value):
     """Also through tuples without a point inside, whose integrand the full quadrature multiplies by 0."""

@@ -71,6 +71,7 @@ struct AdjointState {
     double* lam_T = nullptr;   // observable weights (device copy)
     double* nud = nullptr;     // P lam_T
     double* u = nullptr;       // M^-T D_i
+    double* u4 = nullptr;      // the same, four doubles an element
     double* g = nullptr;       // VJP accumulator
     double* ry = nullptr;      // replay: y, stage input, next y
     double* rtmp = nullptr;
@@ -120,6 +121,7 @@ static int adj_base(tb_handle* h) {
     A->lam_T = adj_alloc(A, n);
     A->nud = adj_alloc(A, n);
     A->u = adj_alloc(A, n);
+    A->u4 = adj_alloc(A, n / 3 * 4);
     A->g = adj_alloc(A, n);
     A->ry = adj_alloc(A, n);
     A->rtmp = adj_alloc(A, n);
@@ -144,7 +146,7 @@ static int adj_base(tb_handle* h) {
         A->allocs.push_back(p);
         A->dD = static_cast<double**>(p);
     }
-    bool ok = A->lam && A->lam_T && A->nud && A->u && A->g && A->ry && A->rtmp && A->ry5 && A->gamp && A->dD &&
+    bool ok = A->lam && A->lam_T && A->nud && A->u && A->u4 && A->g && A->ry && A->rtmp && A->ry5 && A->gamp && A->dD &&
               (!h->opts.deterministic || A->gamp_fx.w);
     for (int i = 0; i < 7; ++i) ok = ok && A->k[i];
     for (int i = 0; i < 6; ++i) ok = ok && A->D[i];
@@ -381,9 +383,13 @@ static int replay_step(tb_handle* h, double* const* k, const double* y, double* 
 static int vjp_at(tb_handle* h, const double* Y, int flags) {
     AdjointState* A = h->adj;
     if (!(flags & TB_NO_COLLISIONS)) {
+        // channels over rows, except in the deterministic mode (whose bits are
+        // those of the list kernel)
+        const bool rows = !h->opts.deterministic;
+        if (rows) TB_TRY(launch_row_vjp(h, Y, A->u, reinterpret_cast<double4*>(A->u4), A->g, A->gamp));
         for (size_t gi = 0; gi < h->groups.size(); ++gi) {
             GroupChan& G = h->groups[gi];
-            if ((G.tup.n == 0 && !G.stream) || G.insts.empty()) continue;
+            if ((G.tup.n == 0 && !G.stream) || G.insts.empty() || (rows && G.use_rows)) continue;
             // deterministic mode: the group's amplitude slots in the exact accumulator
             FxAcc fa = A->gamp_fx;
             if (fa.w) fa.w += 3 * int64_t(A->gamp_off[gi]);
@@ -459,6 +465,9 @@ int tb_adjoint_rhs_vjp(tb_handle* h, const double* f, const double* theta, doubl
     TB_CUDA(cudaMemsetAsync(A->g, 0, bytes, h->stream));
     if (grad_amp) TB_TRY(copy_gamp_out(h, grad_amp));
     else TB_TRY(stream_wait(h));
+    int tflag = 0;
+    TB_TRY(take_wait_timeout(h->d_err, h->stream, &tflag));
+    if (tflag) { set_error("a wait for staged rows ran out; the gradient is incomplete"); return TB_ERR_TIMEOUT; }
     bool clamped = false;
     TB_TRY(fx_take_saturation(h, clamped));
     if (clamped) return fx_saturation_error();

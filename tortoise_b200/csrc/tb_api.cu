@@ -629,6 +629,8 @@ static RowChan row_chan(const GroupChan& G) {
     c.insts = G.d_insts;
     c.n_insts = int(G.insts.size());
     c.nmc = G.dev.nmc;
+    c.gamp0 = G.gamp0;
+    c.amp_vol = G.dev.amp_vol;
     for (int l = 0; l < G.L; ++l) c.leg[l] = G.dev.leg[l];
     // the Monte-Carlo layout visits the tuples with points inside only, also
     // for states with non-finite coefficients; a contraction visits every tuple
@@ -683,6 +685,11 @@ void release_row_sets(tb_handle* h) {
 
 int refresh_row_sets(tb_handle* h) {
     release_row_sets(h);
+    int slots = 0;
+    for (auto& G : h->groups) {
+        G.gamp0 = slots;
+        slots += int(G.insts.size());
+    }
     for (auto& G : h->groups)
         if (G.use_rows) TB_TRY(build_row_set(G.L, row_form(G.dev), {row_chan(G)}, {&G.rows}, h->ndofs, G.row_one));
     TB_TRY(make_row_sets(h, [](const GroupChan& G) { return G.run_state < 0; }, false, h->row_sets));
@@ -776,31 +783,58 @@ int build_run_states(tb_handle* h) {
     return TB_OK;
 }
 
+static RowArgs row_args(tb_handle* h, const double* f, double* acc, const DPCtl* ctl) {
+    RowArgs a;
+    a.ed = &h->ed;
+    a.f = f;
+    a.f4 = h->d_f4;
+    a.nf = h->d_nf;
+    a.acc = acc;
+    a.accr = h->d_accr;
+    a.fx = h->fx;
+    a.ctl = ctl;
+    a.err_flag = h->d_err;
+    a.polls = h->groups.empty() ? 0 : h->groups[0].dev.wait_polls;
+    return a;
+}
+
 // The channels over packed rows: all of them in one launch per leg count, or
 // (only_inst >= 0) that instance's alone.  rate_leg: -1 every leg.
 static int launch_row_sets(tb_handle* h, const double* d_in, double* d_acc, const DPCtl* ctl, int only_inst, bool rate,
                            int rate_leg) {
+    RowArgs a = row_args(h, d_in, d_acc, ctl);
+    a.rate = rate;
+    a.rate_leg = rate_leg;
     if (only_inst >= 0) {
         const ChanInst& I = h->insts[only_inst];
         GroupChan& G = h->groups[I.group];
         if (!G.use_rows) return TB_OK;
         TB_TRY(launch_rows_prepare(h->ed, d_in, h->d_f4, h->d_nf, ctl, h->stream));
-        return launch_rows(G.row_one, h->ed, d_in, h->d_f4, h->d_nf, d_acc, ctl, h->stream, rate, rate_leg, h->fx,
-                           h->d_err, G.dev.wait_polls, h->d_accr, I.d_single);
+        a.one = I.d_single;
+        return launch_rows(G.row_one, a, h->stream);
     }
-    const int polls = h->groups.empty() ? 0 : h->groups[0].dev.wait_polls;
     const bool rates = rate && !h->rate_sets.empty();
     if (!h->row_sets.empty() || rates) TB_TRY(launch_rows_prepare(h->ed, d_in, h->d_f4, h->d_nf, ctl, h->stream));
     for (const auto* sets : {&h->row_sets, &h->rate_sets}) {
         if (sets == &h->rate_sets && !rates) continue;
         for (const RowSet& rs : *sets)
-            if (rate_leg < rs.L)
-                TB_TRY(launch_rows(rs, h->ed, d_in, h->d_f4, h->d_nf, d_acc, ctl, h->stream, rate, rate_leg, h->fx,
-                                   h->d_err, polls, h->d_accr));
+            if (rate_leg < rs.L) TB_TRY(launch_rows(rs, a, h->stream));
     }
     if (rate || h->run_sets.empty()) return TB_OK;
     return launch_run_rows(h->run_sets, h->d_run_states, int(h->run_states.size()), h->n_run_tiles, d_in, h->d_run_nf,
-                           d_acc, ctl, h->stream, h->d_err, polls);
+                           d_acc, ctl, h->stream, h->d_err, a.polls);
+}
+
+int launch_row_vjp(tb_handle* h, const double* f, const double* u, double4* u4, double* grad_f, double* gamp) {
+    if (h->row_sets.empty() && h->rate_sets.empty()) return TB_OK;
+    TB_TRY(launch_rows_prepare(h->ed, f, h->d_f4, h->d_nf, nullptr, h->stream, u, u4));
+    RowArgs a = row_args(h, f, grad_f, nullptr);
+    a.u = u;
+    a.u4 = u4;
+    a.gamp = gamp;
+    for (const auto* sets : {&h->row_sets, &h->rate_sets})
+        for (const RowSet& rs : *sets) TB_TRY(launch_rows(rs, a, h->stream));
+    return TB_OK;
 }
 
 // A streamed group over this handle's work items.  Outside an integration
@@ -874,8 +908,7 @@ static int tune_rows(tb_handle* h, GroupChan& G) {
                                    h->d_run_nf, h->d_acc, nullptr, h->stream, h->d_err, G.dev.wait_polls));
         } else {
             TB_TRY(launch_rows_prepare(h->ed, h->d_f, h->d_f4, h->d_nf, nullptr, h->stream));
-            TB_TRY(launch_rows(G.row_one, h->ed, h->d_f, h->d_f4, h->d_nf, h->d_acc, nullptr, h->stream, false, -1,
-                               h->fx, h->d_err, G.dev.wait_polls, h->d_accr));
+            TB_TRY(launch_rows(G.row_one, row_args(h, h->d_f, h->d_acc, nullptr), h->stream));
         }
     }
     cudaEventRecord(e1, h->stream);

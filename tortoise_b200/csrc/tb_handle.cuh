@@ -39,6 +39,7 @@ struct GroupChan {
     PointRows rows;
     bool use_rows = false;
     int run_state = -1;           // the handle's run-minor state it is evaluated in, or -1
+    int gamp0 = 0;                // the group's first slot among the amplitude gradients
     double rows_seconds = 0.0;    // launch time the autotuner measured
     RowSet row_one;
     // streamed channel (TB_LAYOUT_STREAM): the candidate walk and this
@@ -147,6 +148,9 @@ double* dev_alloc(tb_handle* h, size_t n);
 // The row sets of the handle and of each channel, after a change of what they
 // hold (the stream must be idle).
 int refresh_row_sets(tb_handle* h);
+// grad_f += C'(f)^T u and the amplitude gradients (group-major slots) of the
+// channels over rows; u4: scratch of the state's padded size.
+int launch_row_vjp(tb_handle* h, const double* f, const double* u, double4* u4, double* grad_f, double* gamp);
 // The moment tensor of a channel that was evaluated over rows so far.
 int ensure_tensor(tb_handle* h, GroupChan& G);
 int run_rhs_acc(tb_handle* h, const double* d_in, double* d_acc, const DPCtl* ctl, int flags, int only_inst);

@@ -21,7 +21,7 @@
 //     the points accumulates 1 + R sums (of the integrand times 1 and q);
 //     the constrained legs' moments follow from those after the loop.
 //   * A warp's rows come by bulk copies into its own shared-memory stages, one
-//     row ahead, and the map is read there, so it takes no registers.
+//     row ahead.
 //   * Legs 1 and 2 are staged in shared memory and added by consecutive lanes,
 //     so the three adds of an element fall into one or two sectors (added lane
 //     by lane they bound the kernel: 587 against 336 us at 64x64 e-ph).
@@ -56,10 +56,13 @@ namespace tb {
 // (a 64x64 e-ph right-hand side: 421 us against 336), 12 hide less latency
 // (350).  Four legs need 168 registers and 11 KB of stages a warp: 12 warps.
 __host__ __device__ constexpr int row_shares(int L) { return L == 4 ? 12 : 16; }
-// Warps of a block: the rates of every leg take fewer (184 us against 210 with
-// 16 at 40x24 e-ph with umklapp).
-template <int L, bool RATE, bool DET> struct RowCap {
-    static constexpr int W = RATE ? (L == 4 ? 8 : DET ? 16 : 12) : row_shares(L);
+// What a launch computes: the collision terms, scattering rates, or the
+// transposed operator.
+enum { ROW_PROPAGATE = 0, ROW_RATE = 1, ROW_VJP = 2 };
+// Warps of a block: the rates and the transpose accumulate sums for every leg
+// and take fewer (rates: 184 us against 210 with 16 at 40x24 e-ph with umklapp).
+template <int L, int MODE, bool DET> struct RowCap {
+    static constexpr int W = MODE != ROW_PROPAGATE ? (L == 4 ? 8 : DET ? 16 : 12) : row_shares(L);
 };
 constexpr int ROW_STAGES = 2;    // rows of a warp in shared memory
 constexpr int ROW_COPIES = 16;   // copies of the point table, one per lane of a half warp
@@ -255,23 +258,29 @@ int build_rows(const ChanDev& c, const ThetaList& th, PointRows& rows, int64_t m
 
 // ----------------------------------------------------------------- prepare
 __global__ void __launch_bounds__(256) k_rows_prepare(ElemDev ed, const double* __restrict__ f, double4* __restrict__ f4,
+                                                      const double* __restrict__ u, double4* __restrict__ u4,
                                                       int* __restrict__ nf, const DPCtl* __restrict__ ctl) {
     const int band = ed.blk_band[blockIdx.x];
     const BandDev& bd = ed.bands[band];
     bool bad = false;
     const int e = (blockIdx.x - ed.blk_first[band]) * blockDim.x + threadIdx.x;
-    if (e < bd.ne && !(ctl && ctl[ed.band_run[band]].done)) {
+    auto pad = [&](const double* src, double4* dst) {
         const int64_t o = bd.off + 3 * (int64_t)e;
-        const double x = f[o], y = f[o + 1], z = f[o + 2];
-        f4[bd.off / 3 + e] = make_double4(x, y, z, 0.0);
-        bad = !(isfinite(x) && isfinite(y) && isfinite(z));
+        const double x = src[o], y = src[o + 1], z = src[o + 2];
+        dst[bd.off / 3 + e] = make_double4(x, y, z, 0.0);
+        bad = bad || !(isfinite(x) && isfinite(y) && isfinite(z));
+    };
+    if (e < bd.ne && !(ctl && ctl[ed.band_run[band]].done)) {
+        pad(f, f4);
+        if (u) pad(u, u4);
     }
     bad = __syncthreads_or(bad);
     if (threadIdx.x == 0) nf[blockIdx.x] = bad ? 1 : 0;
 }
 
-int launch_rows_prepare(const ElemDev& ed, const double* f, double4* f4, int* nf, const DPCtl* ctl, cudaStream_t s) {
-    k_rows_prepare<<<ed.nblk, 256, 0, s>>>(ed, f, f4, nf, ctl);
+int launch_rows_prepare(const ElemDev& ed, const double* f, double4* f4, int* nf, const DPCtl* ctl, cudaStream_t s,
+                        const double* u, double4* u4) {
+    k_rows_prepare<<<ed.nblk, 256, 0, s>>>(ed, f, f4, u, u4, nf, ctl);
     TB_CUDA(cudaGetLastError());
     return TB_OK;
 }
@@ -503,7 +512,102 @@ __device__ __forceinline__ void row_tuple_rate(const RowChan& c, const RowMap<L>
     }
 }
 
-// The same two with the list and streamed kernels' operations in their order
+// The transposed operator of one tuple: the u-weighted test functions of all
+// legs are one affine function of q; at every point it multiplies, for each leg,
+// the derivative of the gain-minus-loss product with respect to that leg's form.
+// Returns the sum of the u-weighted integrand (times the amplitude gradient's
+// scale: the caller's).  About 42 FP64 instructions a point with three legs; at
+// 24x24 e-ph a transposed evaluation fell from 174 us (k_vjp_mc, four launches,
+// nine FP64 atomics a tuple and lane) to 70 with what surrounds it.
+template <int L, int FORM>
+__device__ __forceinline__ double row_tuple_vjp(const RowChan& c, const RowMap<L>& m, uint64_t mk,
+                                                const double4 (&f)[L], const double4 (&u)[L], const RowTable& tab,
+                                                double scale, RowOut<L>& o) {
+    constexpr int R = RowDim<L>::R;
+    RowForms<L> F;
+    F.set(m, f);
+    double w0 = 0.0, wq[R];
+    {
+        RowForms<L> U;
+        U.set(m, u);
+#pragma unroll
+        for (int j = 0; j < R; ++j)
+            wq[j] = (leg_in<FORM>(c, L - 2) ? U.p[j] : -U.p[j]) + (leg_in<FORM>(c, L - 1) ? U.c[j] : -U.c[j]);
+        w0 = (leg_in<FORM>(c, L - 2) ? U.p0 : -U.p0) + (leg_in<FORM>(c, L - 1) ? U.c0 : -U.c0);
+#pragma unroll
+        for (int l = 0; l < L - 2; ++l) {
+            const double d = leg_in<FORM>(c, l) ? 1.0 : -1.0;
+            w0 = fma(d, U.fr[l][0], w0);
+            wq[2 * l] = fma(d, U.fr[l][1], wq[2 * l]);
+            wq[2 * l + 1] = fma(d, U.fr[l][2], wq[2 * l + 1]);
+        }
+    }
+    double s0[L], sq[L][R], total = 0.0;
+#pragma unroll
+    for (int l = 0; l < L; ++l) {
+        s0[l] = 0.0;
+#pragma unroll
+        for (int j = 0; j < R; ++j) sq[l][j] = 0.0;
+    }
+    double st[L];
+#pragma unroll
+    for (int l = 0; l < L; ++l) st[l] = leg_stat<FORM>(c, l);
+    for (; mk; mk &= mk - 1) {
+        const int i = (__ffsll((long long)mk) - 1) * R;
+        double q[R], t[L], a[L], b[L];
+#pragma unroll
+        for (int j = 0; j < R; ++j) q[j] = tab(i + j);
+        F.at(q, t);
+        double om = w0;
+#pragma unroll
+        for (int j = 0; j < R; ++j) om = fma(wq[j], q[j], om);
+#pragma unroll
+        for (int l = 0; l < L; ++l) {
+            const double v = fma(st[l], t[l], 1.0);
+            const bool in = leg_in<FORM>(c, l);
+            a[l] = in ? t[l] : v;
+            b[l] = in ? v : t[l];
+        }
+#pragma unroll
+        for (int r = 0; r < L; ++r) {
+            // d / dt_r of (product of b) - (product of a)
+            const bool in = leg_in<FORM>(c, r);
+            double pa = om, pb = om;
+#pragma unroll
+            for (int l = 0; l < L; ++l)
+                if (l != r) { pa *= a[l]; pb *= b[l]; }
+            if (r == L - 1) total = fma(pb, b[r], fma(-pa, a[r], total));
+            const double v = in ? fma(st[r], pb, -pa) : fma(-st[r], pa, pb);
+            s0[r] += v;
+#pragma unroll
+            for (int j = 0; j < R; ++j)
+                if (r >= L - 2 || j / 2 == r) sq[r][j] = fma(q[j], v, sq[r][j]);   // a free leg needs its own two
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < L; ++r) {
+        double x, z;
+        if (r < L - 2) {
+            x = sq[r][r < L - 2 ? 2 * r : 0];
+            z = sq[r][r < L - 2 ? 2 * r + 1 : 0];
+        } else {
+            const int y = r == L - 2 ? 0 : 2;
+            x = r == L - 2 ? sq[r][R - 1] : m.a0(1) * s0[r];
+            z = m.a0(y) * s0[r];
+#pragma unroll
+            for (int j = 0; j < R; ++j) {
+                if (r == L - 1) x = fma(m.G(1, j), sq[r][j], x);
+                z = fma(m.G(y, j), sq[r][j], z);
+            }
+        }
+        o.v[r][0] = scale * s0[r];
+        o.v[r][1] = scale * x;
+        o.v[r][2] = scale * z;
+    }
+    return total;
+}
+
+// Propagation and rates with the list and streamed kernels' operations in their order
 // (inside_point_sums, tb_mcpoint.cuh): the deterministic mode's bits.
 template <int L, bool RATE>
 __device__ __forceinline__ void row_tuple_listed(const RowChan& c, const RowMap<L>& m, uint64_t mk,
@@ -643,7 +747,8 @@ __device__ __forceinline__ bool finite3(const double* v) { return isfinite(v[0])
 template <int L>
 __device__ __noinline__ void spread_nonfinite(const RowChan& c, const InstDev* insts, int n_insts, int64_t t0,
                                               int64_t t1, const double* f, double* acc, const DPCtl* ctl, bool rate,
-                                              int rate_leg, const FxAcc& fx) {
+                                              int rate_leg, const FxAcc& fx, const double* u = nullptr,
+                                              double* gamp = nullptr) {
     const double nan = __longlong_as_double(0x7ff8000000000000ll);
     for (int64_t i = t0 + threadIdx.x; i < t1; i += blockDim.x) {
         int e[L];
@@ -651,19 +756,22 @@ __device__ __noinline__ void spread_nonfinite(const RowChan& c, const InstDev* i
         for (int l = 0; l < L; ++l) e[l] = __ldg(c.tup + l * c.stride + i);
         for (int k = 0; k < n_insts; ++k) {
             const InstDev& in = insts[k];
-            if (in.amp_full == 0.0 || (ctl && ctl[in.run].done)) continue;
-            bool bad[L];
+            if (!u && (in.amp_full == 0.0 || (ctl && ctl[in.run].done))) continue;
+            bool bad[L], all = false;
             int nbad = 0;
 #pragma unroll
             for (int l = 0; l < L; ++l) {
                 bad[l] = !finite3(f + in.foff[l] + 3 * (int64_t)e[l]);
                 nbad += bad[l] ? 1 : 0;
+                if (u) all = all || !finite3(u + in.foff[l] + 3 * (int64_t)e[l]);
             }
-            if (nbad == 0) continue;
+            if (nbad == 0 && !all) continue;
+            if (u) atomicAdd(gamp + k, nan);
 #pragma unroll
             for (int l = 0; l < L; ++l) {
-                // a leg's rate does not depend on its own f
-                if (rate && ((rate_leg >= 0 && l != rate_leg) || nbad == (bad[l] ? 1 : 0))) continue;
+                // a leg's rate and derivative do not depend on its own f
+                if (rate && rate_leg >= 0 && l != rate_leg) continue;
+                if ((rate || u) && !all && nbad == (bad[l] ? 1 : 0)) continue;
                 if (fx.w) atomicOr(fx.poison, 1u);
                 else
                     for (int j = 0; j < 3; ++j) atomicAdd(acc + in.foff[l] + 3 * (int64_t)e[l] + j, nan);
@@ -672,8 +780,8 @@ __device__ __noinline__ void spread_nonfinite(const RowChan& c, const InstDev* i
     }
 }
 
-template <int L, int FORM, bool RATE, bool DET, bool MULTI>
-__global__ void __launch_bounds__(RowCap<L, RATE, DET>::W * 32, 1) k_rows(const RowChan* __restrict__ chans,
+template <int L, int FORM, int MODE, bool DET, bool MULTI>
+__global__ void __launch_bounds__(RowCap<L, MODE, DET>::W * 32, 1) k_rows(const RowChan* __restrict__ chans,
                                                             const RowWork* __restrict__ work,
                                                             const int32_t* __restrict__ warp_row, int shares,
                                                             const InstDev* __restrict__ one,
@@ -683,12 +791,15 @@ __global__ void __launch_bounds__(RowCap<L, RATE, DET>::W * 32, 1) k_rows(const 
                                                             double* __restrict__ acc, double* __restrict__ accr,
                                                             int copies, int64_t ndofs, const DPCtl* __restrict__ ctl,
                                                             int rate_leg, FxAcc fx, int* __restrict__ err_flag,
-                                                            int wait_polls) {
+                                                            int wait_polls, const double* __restrict__ u,
+                                                            const double4* __restrict__ u4,
+                                                            double* __restrict__ gamp) {
+    constexpr bool RATE = MODE == ROW_RATE, VJP = MODE == ROW_VJP;
     constexpr int R = RowDim<L>::R, ND = RowDim<L>::ND;
     constexpr uint32_t BYTES = RowDim<L>::BYTES;
     extern __shared__ __align__(128) unsigned char s_raw[];
     __shared__ RowChan c;
-    __shared__ __align__(8) uint64_t s_bar[RowCap<L, RATE, DET>::W][ROW_STAGES];
+    __shared__ __align__(8) uint64_t s_bar[RowCap<L, MODE, DET>::W][ROW_STAGES];
     const RowWork w = work[blockIdx.x];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, n_warps = blockDim.x >> 5;
     if (accr && blockIdx.x % copies) acc = accr + int64_t(blockIdx.x % copies - 1) * ndofs;
@@ -697,8 +808,9 @@ __global__ void __launch_bounds__(RowCap<L, RATE, DET>::W * 32, 1) k_rows(const 
     __syncthreads();
     const InstDev* insts = one ? one : c.insts;
     const int n_insts = one ? 1 : c.n_insts;
-    {
-        // every instance off or its run finished: nothing to add
+    if (!VJP) {
+        // every instance off or its run finished: nothing to add (an amplitude
+        // of 0 still has a gradient)
         bool any = false;
         for (int k = 0; k < n_insts && !any; ++k)
             any = insts[k].amp_full != 0.0 && !(ctl && ctl[insts[k].run].done);
@@ -728,9 +840,10 @@ __global__ void __launch_bounds__(RowCap<L, RATE, DET>::W * 32, 1) k_rows(const 
     const RowTable tab{s_q + (lane & (ROW_COPIES - 1))};
     LegZero<DET> z;
     int e0 = -1;
-    double4 f0 = make_double4(0., 0., 0., 0.);
+    double4 f0 = make_double4(0., 0., 0., 0.), u0 = f0;
     int64_t off[L], el[L];
-    double amp = 0.0;
+    double amp = 0.0, ga = 0.0;   // ga: this lane's part of the amplitude gradient
+    if (VJP) gamp += c.gamp0;
     if (!MULTI) {
 #pragma unroll
         for (int l = 0; l < L; ++l) { off[l] = insts[0].foff[l]; el[l] = off[l] / 3; }
@@ -771,15 +884,17 @@ __global__ void __launch_bounds__(RowCap<L, RATE, DET>::W * 32, 1) k_rows(const 
             if (e0 >= 0 && (!RATE || rate_leg <= 0)) z.flush(acc, off[0] + 3 * (int64_t)e0, fx);
             e0 = e[0];
             f0 = load_f4(f4 + el[0] + e0);
+            if (VJP) u0 = load_f4(u4 + el[0] + e0);
         }
         for (int k = 0; k < (MULTI ? n_insts : 1); ++k) {
             if (MULTI) {
                 const InstDev& in = insts[k];
                 amp = in.amp_full;
-                if (amp == 0.0 || (ctl && ctl[in.run].done)) continue;
+                if (!VJP && (amp == 0.0 || (ctl && ctl[in.run].done))) continue;
 #pragma unroll
                 for (int l = 0; l < L; ++l) { off[l] = in.foff[l]; el[l] = off[l] / 3; }
                 f0 = load_f4(f4 + el[0] + e[0]);
+                if (VJP) u0 = load_f4(u4 + el[0] + e[0]);
             }
             double4 f[L];
             f[0] = f0;
@@ -787,7 +902,19 @@ __global__ void __launch_bounds__(RowCap<L, RATE, DET>::W * 32, 1) k_rows(const 
             for (int l = 1; l < L; ++l) f[l] = load_f4(f4 + el[l] + e[l]);
             RowOut<L> o;
             const double wt = reinterpret_cast<const double*>(b)[32 * (ND - 1) + lane];
-            if (DET) row_tuple_listed<L, RATE>(c, m, mk, f, tab, wt, amp * tf, o);
+            if constexpr (VJP) {
+                double4 u[L];
+                u[0] = u0;
+#pragma unroll
+                for (int l = 1; l < L; ++l) u[l] = load_f4(u4 + el[l] + e[l]);
+                const double g = row_tuple_vjp<L, FORM>(c, m, mk, f, u, tab, wt * (amp * tf), o);
+                ga = fma(wt * (c.amp_vol * tf), g, ga);
+                if (MULTI) {
+                    for (int d = 16; d > 0; d >>= 1) ga += __shfl_xor_sync(0xffffffffu, ga, d);
+                    if (lane == 0 && ga != 0.0) atomicAdd(gamp + k, ga);
+                    ga = 0.0;
+                }
+            } else if (DET) row_tuple_listed<L, RATE>(c, m, mk, f, tab, wt, amp * tf, o);
             else if (RATE) row_tuple_rate<L, FORM>(c, m, mk, f, tab, wt * (amp * tf), o);
             else row_tuple<L, FORM>(c, m, mk, f, tab, wt * (amp * tf), o);
             if (!RATE || rate_leg <= 0) {
@@ -824,10 +951,14 @@ __global__ void __launch_bounds__(RowCap<L, RATE, DET>::W * 32, 1) k_rows(const 
         if (lane == 0 && r + ROW_STAGES < r1) fetch(r + ROW_STAGES, s);
     }
     if (!MULTI && e0 >= 0 && (!RATE || rate_leg <= 0)) z.flush(acc, off[0] + 3 * (int64_t)e0, fx);
+    if (VJP && !MULTI) {
+        for (int d = 16; d > 0; d >>= 1) ga += __shfl_xor_sync(0xffffffffu, ga, d);
+        if (lane == 0 && ga != 0.0) atomicAdd(gamp, ga);
+    }
     int bad = 0;
     for (int i = tid; i < n_nf; i += blockDim.x) bad |= nf[i];
     if (__syncthreads_or(bad))
-        spread_nonfinite<L>(c, insts, n_insts, w.t0, w.t1, f, acc, ctl, RATE, rate_leg, fx);
+        spread_nonfinite<L>(c, insts, n_insts, w.t0, w.t1, f, acc, ctl, RATE, rate_leg, fx, VJP ? u : nullptr, gamp);
 }
 
 // acc += the further accumulators, which are cleared.
@@ -867,63 +998,55 @@ static size_t rows_smem(int L, int nmc, int warps) {
            sizeof(double) * size_t(nmc) * size_t(2 * (L - 2) + 1) * ROW_COPIES;
 }
 
-template <int L, int FORM, bool RATE, bool DET, bool MULTI>
-static int launch_k_rows(const RowSet& rs, const ElemDev& ed, const double* f, const double4* f4, const int* nf, double* acc,
-                         const DPCtl* ctl, cudaStream_t s, int rate_leg, const FxAcc& fx, const InstDev* one,
-                         int* err_flag, int polls, double* accr) {
-    auto kern = k_rows<L, FORM, RATE, DET, MULTI>;
+template <int L, int FORM, int MODE, bool DET, bool MULTI>
+static int launch_k_rows(const RowSet& rs, const RowArgs& A, cudaStream_t s) {
+    auto kern = k_rows<L, FORM, MODE, DET, MULTI>;
     // the shared-memory limit, set once on each device the kernel runs on
     static std::atomic<unsigned long long> attr_devices{0};
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64 || !((attr_devices.load() >> dev) & 1ull)) {
         TB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     int(rows_smem(L, 64, RowCap<L, RATE, DET>::W))));
+                                     int(rows_smem(L, 64, RowCap<L, MODE, DET>::W))));
         if (dev >= 0 && dev < 64) attr_devices.fetch_or(1ull << dev);
     }
-    const int warps = std::min(rs.shares, RowCap<L, RATE, DET>::W);
+    const int warps = std::min(rs.shares, RowCap<L, MODE, DET>::W);
     kern<<<unsigned(rs.nblocks), unsigned(32 * warps), rows_smem(L, rs.nmc_max, warps), s>>>(
-        rs.d_chan, rs.d_work, rs.d_warp_row, rs.shares, one, f, f4, nf, ed.nblk, acc, accr, rs.copies,
-        ed.ndofs, ctl, rate_leg, fx, err_flag, polls);
-    if (accr && rs.copies > 1) {
-        TB_CUDA(cudaGetLastError());
-        k_rows_fold<<<unsigned((ed.ndofs + 31) / 32), dim3(32, 8), 0, s>>>(acc, accr, rs.copies - 1, ed.ndofs);
-    }
+        rs.d_chan, rs.d_work, rs.d_warp_row, rs.shares, A.one, A.f, A.f4, A.nf, A.ed->nblk, A.acc, A.accr, rs.copies,
+        A.ed->ndofs, A.ctl, A.rate_leg, A.fx, A.err_flag, A.polls, A.u, A.u4, A.gamp);
     TB_CUDA(cudaGetLastError());
+    if (A.accr && rs.copies > 1) {
+        k_rows_fold<<<unsigned((A.ed->ndofs + 31) / 32), dim3(32, 8), 0, s>>>(A.acc, A.accr, rs.copies - 1, A.ed->ndofs);
+        TB_CUDA(cudaGetLastError());
+    }
     return TB_OK;
 }
 
-template <int L, int FORM, bool RATE, bool DET>
-static int launch_rows_m(const RowSet& rs, const ElemDev& ed, const double* f, const double4* f4, const int* nf, double* acc,
-                         const DPCtl* ctl, cudaStream_t s, int rate_leg, const FxAcc& fx, const InstDev* one,
-                         int* err_flag, int polls, double* accr) {
-    if (rs.multi && !one)
-        return launch_k_rows<L, FORM, RATE, DET, true>(rs, ed, f, f4, nf, acc, ctl, s, rate_leg, fx, one, err_flag, polls, accr);
-    return launch_k_rows<L, FORM, RATE, DET, false>(rs, ed, f, f4, nf, acc, ctl, s, rate_leg, fx, one, err_flag, polls, accr);
+template <int L, int FORM, int MODE, bool DET>
+static int launch_rows_m(const RowSet& rs, const RowArgs& A, cudaStream_t s) {
+    if (rs.multi && !A.one) return launch_k_rows<L, FORM, MODE, DET, true>(rs, A, s);
+    return launch_k_rows<L, FORM, MODE, DET, false>(rs, A, s);
 }
 
 // The channels that addScatteringChannelsWildcards builds in the reference's
-// examples are compiled in (FORM_2, FORM_3, FORM_4); others select their forms at run
-// time.
+// examples are compiled in (FORM_2, FORM_3, FORM_4); others select their forms
+// at run time.
 template <int L>
-static int launch_rows_l(const RowSet& rs, const ElemDev& ed, const double* f, const double4* f4, const int* nf, double* acc,
-                         const DPCtl* ctl, cudaStream_t s, bool rate, int rate_leg, const FxAcc& fx,
-                         const InstDev* one, int* err_flag, int polls, double* accr) {
+static int launch_rows_l(const RowSet& rs, const RowArgs& A, cudaStream_t s) {
     constexpr int CANON = L == 2 ? FORM_2 : L == 3 ? FORM_3 : FORM_4;
-#define TB_ROWS(DD, RR, XX) launch_rows_m<L, DD, RR, XX>(rs, ed, f, f4, nf, acc, ctl, s, rate_leg, fx, one, err_flag, polls, accr)
-    if (fx.w) return rate ? TB_ROWS(-1, true, true) : TB_ROWS(-1, false, true);
-    if (rs.form == CANON) return rate ? TB_ROWS(CANON, true, false) : TB_ROWS(CANON, false, false);
-    return rate ? TB_ROWS(-1, true, false) : TB_ROWS(-1, false, false);
-#undef TB_ROWS
+    const bool canon = rs.form == CANON;
+    if (A.u) return canon ? launch_rows_m<L, CANON, ROW_VJP, false>(rs, A, s) : launch_rows_m<L, -1, ROW_VJP, false>(rs, A, s);
+    if (A.fx.w) return A.rate ? launch_rows_m<L, -1, ROW_RATE, true>(rs, A, s) : launch_rows_m<L, -1, ROW_PROPAGATE, true>(rs, A, s);
+    if (A.rate) return canon ? launch_rows_m<L, CANON, ROW_RATE, false>(rs, A, s) : launch_rows_m<L, -1, ROW_RATE, false>(rs, A, s);
+    return canon ? launch_rows_m<L, CANON, ROW_PROPAGATE, false>(rs, A, s)
+                 : launch_rows_m<L, -1, ROW_PROPAGATE, false>(rs, A, s);
 }
 
-int launch_rows(const RowSet& rs, const ElemDev& ed, const double* f, const double4* f4, const int* nf, double* acc, const DPCtl* ctl,
-                cudaStream_t s, bool rate, int rate_leg, const FxAcc& fx, int* err_flag, int polls,
-                double* accr, const InstDev* one) {
+int launch_rows(const RowSet& rs, const RowArgs& A, cudaStream_t s) {
     if (rs.nblocks <= 0) return TB_OK;
-    if (rs.L == 2) return launch_rows_l<2>(rs, ed, f, f4, nf, acc, ctl, s, rate, rate_leg, fx, one, err_flag, polls, accr);
-    if (rs.L == 3) return launch_rows_l<3>(rs, ed, f, f4, nf, acc, ctl, s, rate, rate_leg, fx, one, err_flag, polls, accr);
-    return launch_rows_l<4>(rs, ed, f, f4, nf, acc, ctl, s, rate, rate_leg, fx, one, err_flag, polls, accr);
+    if (rs.L == 2) return launch_rows_l<2>(rs, A, s);
+    if (rs.L == 3) return launch_rows_l<3>(rs, A, s);
+    return launch_rows_l<4>(rs, A, s);
 }
 
 int build_row_set(int L, int form, const std::vector<RowChan>& chan, const std::vector<const PointRows*>& rows,

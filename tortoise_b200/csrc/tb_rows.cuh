@@ -48,6 +48,8 @@ struct RowChan {
     const InstDev* insts;
     int n_insts;
     int nmc;
+    int gamp0;                      // its first slot among the amplitude gradients
+    double amp_vol;
     LegDev leg[4];
     // shared by many runs: the structure's run-minor state and accumulator
     // (RunState), the legs' band offsets within a run
@@ -108,19 +110,34 @@ int rows_lane_group(int n);
 int build_row_set(int L, int form, const std::vector<RowChan>& chan, const std::vector<const PointRows*>& rows,
                   int64_t ndofs, RowSet& out, int S = 0);
 
-// f4[e] = (f0, f1, f2, 0) of every element of the state; nf[b] != 0 marks an
-// element block that holds a non-finite coefficient.
-int launch_rows_prepare(const ElemDev& ed, const double* f, double4* f4, int* nf, const DPCtl* ctl, cudaStream_t s);
+// f4[e] = (f0, f1, f2, 0) of every element of the state, u4 of u likewise when
+// it is given; nf[b] != 0 marks an element block with a non-finite coefficient.
+int launch_rows_prepare(const ElemDev& ed, const double* f, double4* f4, int* nf, const DPCtl* ctl, cudaStream_t s,
+                        const double* u = nullptr, double4* u4 = nullptr);
 
-// acc (or fx) += the collision terms of the set's channels; rate: the
-// scattering rate of leg rate_leg (of every leg when it is negative).
-// one non-null: that instance in place of the channels' instances.  err_flag
-// is set when a bounded wait (polls) for a staged row runs out.  accr: the
-// rs.copies - 1 further accumulators of ed.ndofs doubles, all zero between
-// launches (null: one accumulator for all blocks).
-int launch_rows(const RowSet& rs, const ElemDev& ed, const double* f, const double4* f4, const int* nf, double* acc, const DPCtl* ctl,
-                cudaStream_t s, bool rate, int rate_leg, const FxAcc& fx, int* err_flag, int polls,
-                double* accr, const InstDev* one = nullptr);
+// One evaluation of a set.
+struct RowArgs {
+    const ElemDev* ed = nullptr;
+    const double* f = nullptr;      // the state, and what launch_rows_prepare made of it
+    const double4* f4 = nullptr;
+    const int* nf = nullptr;
+    double* acc = nullptr;          // or fx: the collision terms are added here
+    double* accr = nullptr;         // the set's copies - 1 further accumulators of ed->ndofs doubles,
+                                    // all zero between launches (null: one for all blocks)
+    FxAcc fx{};
+    const DPCtl* ctl = nullptr;
+    const InstDev* one = nullptr;   // this instance in place of the channels' instances
+    bool rate = false;              // scattering rate of leg rate_leg (of every leg when negative)
+    int rate_leg = -1;
+    // non-null: the transposed operator for the co-state u instead, acc +=
+    // C'(f)^T u and gamp[gamp0 + k] += <u, dC / d amplitude_k>
+    const double* u = nullptr;
+    const double4* u4 = nullptr;
+    double* gamp = nullptr;
+    int* err_flag = nullptr;        // set when a bounded wait (polls) for a staged row runs out
+    int polls = 0;
+};
+int launch_rows(const RowSet& rs, const RowArgs& a, cudaStream_t s);
 
 // The run-minor sets: the structures' states gathered, each set evaluated,
 // their accumulators added to acc and cleared.  st: device copy of the n_st

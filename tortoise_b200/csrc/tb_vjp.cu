@@ -62,6 +62,8 @@ int launch_project(const ElemDev& ed, double* v, cudaStream_t s) {
 }
 
 // --------------------------------------------- collision VJP, Monte-Carlo
+// (deterministic handles and channels without packed rows; the others:
+// k_rows, tb_rows.cu)
 // LIST: tup / stride / n describe a ThetaList (tb_theta.cuh) and every tuple
 // visits only the set bits of its mask, the points whose Theta is 1.
 template <int L, bool LIST>
