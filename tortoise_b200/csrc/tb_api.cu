@@ -690,8 +690,6 @@ int refresh_row_sets(tb_handle* h) {
         G.gamp0 = slots;
         slots += int(G.insts.size());
     }
-    for (auto& G : h->groups)
-        if (G.use_rows) TB_TRY(build_row_set(G.L, row_form(G.dev), {row_chan(G)}, {&G.rows}, h->ndofs, G.row_one));
     TB_TRY(make_row_sets(h, [](const GroupChan& G) { return G.run_state < 0; }, false, h->row_sets));
     if (!h->run_states.empty()) {
         TB_TRY(make_row_sets(h, [](const GroupChan& G) { return G.run_state >= 0; }, false, h->rate_sets));
@@ -702,7 +700,6 @@ int refresh_row_sets(tb_handle* h) {
     int copies = 1;
     for (const auto* sets : {&h->row_sets, &h->rate_sets})
         for (const RowSet& rs : *sets) copies = std::max(copies, rs.copies);
-    for (const auto& G : h->groups) copies = std::max(copies, G.row_one.copies);
     if (copies - 1 > h->n_accr && !h->opts.deterministic) {
         if (h->d_accr) cudaFree(h->d_accr);
         h->n_accr = 0;
@@ -783,6 +780,15 @@ int build_run_states(tb_handle* h) {
     return TB_OK;
 }
 
+// The set of G alone, made when it is first asked for.  (Its blocks may share
+// fewer accumulators than it would take alone: those of the handle's sets.)
+static int row_one(tb_handle* h, GroupChan& G) {
+    if (G.row_one.nblocks > 0) return TB_OK;
+    TB_TRY(build_row_set(G.L, row_form(G.dev), {row_chan(G)}, {&G.rows}, h->ndofs, G.row_one));
+    G.row_one.copies = std::min(G.row_one.copies, h->n_accr + 1);
+    return TB_OK;
+}
+
 static RowArgs row_args(tb_handle* h, const double* f, double* acc, const DPCtl* ctl) {
     RowArgs a;
     a.ed = &h->ed;
@@ -811,6 +817,7 @@ static int launch_row_sets(tb_handle* h, const double* d_in, double* d_acc, cons
         if (!G.use_rows) return TB_OK;
         TB_TRY(launch_rows_prepare(h->ed, d_in, h->d_f4, h->d_nf, ctl, h->stream));
         a.one = I.d_single;
+        TB_TRY(row_one(h, G));
         return launch_rows(G.row_one, a, h->stream);
     }
     const bool rates = rate && !h->rate_sets.empty();
@@ -898,6 +905,7 @@ static int tune_rows(tb_handle* h, GroupChan& G) {
     cudaEvent_t e0, e1;
     TB_CUDA(cudaEventCreate(&e0));
     TB_CUDA(cudaEventCreate(&e1));
+    if (G.run_state < 0) TB_TRY(row_one(h, G));
     std::vector<RowSet> set;   // run-minor: this channel alone, its structure's state gathered and scattered
     if (G.run_state >= 0) TB_TRY(make_row_sets(h, [&](const GroupChan& B) { return &B == &G; }, true, set));
     constexpr int REPS = 3;

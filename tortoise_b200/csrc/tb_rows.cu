@@ -43,6 +43,9 @@
 #include <algorithm>
 #include <atomic>
 #include <cmath>
+#include <cstring>
+#include <memory>
+#include <utility>
 
 #include "tb_bulk.cuh"
 #include "tb_dp45.cuh"
@@ -87,9 +90,7 @@ struct RowDim {
 size_t row_bytes(int L) { return L == 2 ? RowDim<2>::BYTES : L == 3 ? RowDim<3>::BYTES : RowDim<4>::BYTES; }
 
 void PointRows::release() {
-    if (blk) cudaFree(blk);
-    if (row_e0) cudaFree(row_e0);
-    if (perm) cudaFree(perm);
+    if (blk) cudaFree(blk);   // the allocation's base: rows, perm, row_e0
     blk = nullptr;
     row_e0 = nullptr;
     perm = nullptr;
@@ -99,29 +100,37 @@ void PointRows::release() {
 }
 
 void RowSet::release() {
-    if (d_chan) cudaFree(d_chan);
-    if (d_work) cudaFree(d_work);
+    if (d_chan) cudaFree(d_chan);   // the allocation's base: channels, work, bounds
     d_chan = nullptr;
     d_work = nullptr;
-    if (d_warp_row) cudaFree(d_warp_row);
     d_warp_row = nullptr;
     nblocks = 0;
 }
 
 // ------------------------------------------------------------------ build
-__global__ void k_rows_count(const int32_t* __restrict__ e0, int64_t n, int32_t* __restrict__ count) {
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        atomicAdd(count + e0[i], 1);
+// first[e] = the first tuple whose leg-0 element is e or above (e0 ascending)
+__global__ void k_rows_first(const int32_t* __restrict__ e0, int64_t n, int ne, int64_t* __restrict__ first) {
+    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e > ne) return;
+    int64_t lo = 0, hi = n;
+    while (lo < hi) {
+        const int64_t m = (lo + hi) / 2;
+        if (e0[m] < e) lo = m + 1;
+        else hi = m;
+    }
+    first[e] = lo;
 }
 
 // The lanes of an element's last row that hold no tuple: no points, element 0.
 template <int L>
-__global__ void __launch_bounds__(256) k_rows_pad(const int32_t* __restrict__ count, const int64_t* __restrict__ row0,
+__global__ void __launch_bounds__(256) k_rows_pad(const int64_t* __restrict__ first, const int64_t* __restrict__ row0,
                                                   int ne, unsigned char* __restrict__ blk, int32_t* __restrict__ perm) {
     constexpr int ND = RowDim<L>::ND;
     const int e = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (e >= ne || count[e] % 32 == 0 || lane < count[e] % 32) return;
-    const int64_t row = row0[e] + count[e] / 32;
+    if (e >= ne) return;
+    const int64_t count = first[e + 1] - first[e];
+    if (count % 32 == 0 || lane < count % 32) return;
+    const int64_t row = row0[e] + count / 32;
     unsigned char* b = blk + row * RowDim<L>::BYTES;
     for (int k = 0; k < ND; ++k) reinterpret_cast<double*>(b)[32 * k + lane] = 0.0;
     reinterpret_cast<uint64_t*>(b + 256 * ND)[lane] = 0ull;
@@ -173,63 +182,43 @@ __global__ void __launch_bounds__(256) k_rows_fill(ChanDev c, const int32_t* __r
     }
 }
 
-namespace {
-struct Tmp {
-    std::vector<void*> p;
-    void* get(size_t bytes) {
-        void* q = nullptr;
-        if (cudaMalloc(&q, bytes + 16) != cudaSuccess) {
-            cudaGetLastError();
-            return nullptr;
-        }
-        p.push_back(q);
-        return q;
-    }
-    ~Tmp() {
-        for (void* q : p) cudaFree(q);
-    }
-};
-}  // namespace
-
 int build_rows(const ChanDev& c, const ThetaList& th, PointRows& rows, int64_t max_bytes, cudaStream_t s) {
     rows.release();
     const int64_t n = th.n;
     if (n <= 0) return TB_OK;
     const int ne = c.leg[0].ne;
-    Tmp tmp;
-    int32_t* d_cnt = static_cast<int32_t*>(tmp.get(sizeof(int32_t) * size_t(ne)));
-    int64_t* d_first = static_cast<int64_t*>(tmp.get(sizeof(int64_t) * size_t(ne)));
-    int64_t* d_row0 = static_cast<int64_t*>(tmp.get(sizeof(int64_t) * size_t(ne)));
-    if (!d_cnt || !d_first || !d_row0) return TB_OK;
-    TB_CUDA(cudaMemsetAsync(d_cnt, 0, sizeof(int32_t) * size_t(ne), s));
-    const unsigned blocks = unsigned(std::min<int64_t>((n + 255) / 256, 148 * 16));
-    k_rows_count<<<blocks, 256, 0, s>>>(th.ids, n, d_cnt);
-    TB_CUDA(cudaGetLastError());
-    std::vector<int32_t> cnt(size_t(ne), 0);
-    TB_CUDA(cudaMemcpyAsync(cnt.data(), d_cnt, sizeof(int32_t) * size_t(ne), cudaMemcpyDeviceToHost, s));
-    TB_CUDA(cudaStreamSynchronize(s));
-    std::vector<int64_t> first(size_t(ne), 0), row0(size_t(ne), 0);
-    int64_t at = 0, nrows = 0;
-    for (int e = 0; e < ne; ++e) {
-        first[size_t(e)] = at;
-        row0[size_t(e)] = nrows;
-        at += cnt[size_t(e)];
-        nrows += (cnt[size_t(e)] + 31) / 32;
-    }
-    int32_t* d_pts = static_cast<int32_t*>(tmp.get(2 * sizeof(int32_t) * size_t(nrows)));
-    const size_t bytes = row_bytes(c.L) * size_t(nrows);
-    if (int64_t(bytes) > max_bytes || !d_pts || cudaMalloc(&rows.blk, bytes) != cudaSuccess ||
-        cudaMalloc(&rows.row_e0, sizeof(int32_t) * size_t(nrows)) != cudaSuccess ||
-        cudaMalloc(&rows.perm, sizeof(int32_t) * size_t(nrows) * 32) != cudaSuccess) {
+    // an element's tuples fill (count + 31) / 32 rows
+    const int64_t most = n / 32 + ne + 1;
+    const size_t elem = sizeof(int64_t) * size_t(ne + 1);
+    char* base = nullptr;
+    if (cudaMalloc(&base, 2 * elem + 2 * sizeof(int32_t) * size_t(most)) != cudaSuccess) {
         cudaGetLastError();
-        rows.release();
         return TB_OK;
     }
+    std::unique_ptr<char, cudaError_t (*)(char*)> tmp(base, [](char* p) { return cudaFree(p); });
+    int64_t* d_first = reinterpret_cast<int64_t*>(base);
+    int64_t* d_row0 = reinterpret_cast<int64_t*>(base + elem);
+    int32_t* d_pts = reinterpret_cast<int32_t*>(base + 2 * elem);
+    const unsigned blocks = unsigned(std::min<int64_t>((n + 255) / 256, 148 * 16));
+    k_rows_first<<<unsigned(ne / 256 + 1), 256, 0, s>>>(th.ids, n, ne, d_first);
+    TB_CUDA(cudaGetLastError());
+    std::vector<int64_t> first(size_t(ne) + 1, 0), row0(size_t(ne) + 1, 0);
+    TB_CUDA(cudaMemcpyAsync(first.data(), d_first, elem, cudaMemcpyDeviceToHost, s));
+    TB_CUDA(cudaStreamSynchronize(s));
+    for (size_t e = 0; e < size_t(ne); ++e) row0[e + 1] = row0[e] + (first[e + 1] - first[e] + 31) / 32;
+    const int64_t nrows = row0[size_t(ne)];
+    const size_t bytes = row_bytes(c.L) * size_t(nrows), words = 33 * sizeof(int32_t) * size_t(nrows);
+    if (int64_t(bytes + words) > max_bytes || cudaMalloc(&rows.blk, bytes + words) != cudaSuccess) {
+        cudaGetLastError();
+        rows.blk = nullptr;
+        return TB_OK;
+    }
+    rows.perm = reinterpret_cast<int32_t*>(rows.blk + bytes);
+    rows.row_e0 = rows.perm + 32 * nrows;
     TB_CUDA(cudaMemsetAsync(d_pts, 0, 2 * sizeof(int32_t) * size_t(nrows), s));
-    TB_CUDA(cudaMemcpyAsync(d_first, first.data(), sizeof(int64_t) * size_t(ne), cudaMemcpyHostToDevice, s));
-    TB_CUDA(cudaMemcpyAsync(d_row0, row0.data(), sizeof(int64_t) * size_t(ne), cudaMemcpyHostToDevice, s));
+    TB_CUDA(cudaMemcpyAsync(d_row0, row0.data(), elem, cudaMemcpyHostToDevice, s));
 #define TB_FILL(LL)                                                                                                    \
-    k_rows_pad<LL><<<unsigned((int64_t(ne) * 32 + 255) / 256), 256, 0, s>>>(d_cnt, d_row0, ne, rows.blk, rows.perm);   \
+    k_rows_pad<LL><<<unsigned((int64_t(ne) * 32 + 255) / 256), 256, 0, s>>>(d_first, d_row0, ne, rows.blk, rows.perm); \
     k_rows_fill<LL><<<blocks, 256, 0, s>>>(c, th.ids, th.mask, th.perm, n, d_first, d_row0, rows.blk, rows.row_e0,     \
                                            rows.perm, d_pts)
     switch (c.L) {
@@ -1109,17 +1098,21 @@ int build_row_set(int L, int form, const std::vector<RowChan>& chan, const std::
             for (int64_t p = b * out.shares; p <= (b + 1) * out.shares; ++p) warp_row.push_back(bound(p));
         }
     }
-    if (cudaMalloc(&out.d_chan, sizeof(RowChan) * chan.size()) != cudaSuccess ||
-        cudaMalloc(&out.d_warp_row, sizeof(int32_t) * warp_row.size()) != cudaSuccess ||
-        cudaMalloc(&out.d_work, sizeof(RowWork) * work.size()) != cudaSuccess) {
+    const size_t cb = (sizeof(RowChan) * chan.size() + 255) / 256 * 256, wb = (sizeof(RowWork) * work.size() + 255) / 256 * 256;
+    std::vector<char> all(cb + wb + sizeof(int32_t) * warp_row.size());
+    std::memcpy(all.data(), chan.data(), sizeof(RowChan) * chan.size());
+    std::memcpy(all.data() + cb, work.data(), sizeof(RowWork) * work.size());
+    std::memcpy(all.data() + cb + wb, warp_row.data(), sizeof(int32_t) * warp_row.size());
+    char* base = nullptr;
+    if (cudaMalloc(&base, all.size()) != cudaSuccess) {
         cudaGetLastError();
-        out.release();
         set_error("row set allocation failed");
         return TB_ERR_OOM;
     }
-    TB_CUDA(cudaMemcpy(out.d_chan, chan.data(), sizeof(RowChan) * chan.size(), cudaMemcpyHostToDevice));
-    TB_CUDA(cudaMemcpy(out.d_work, work.data(), sizeof(RowWork) * work.size(), cudaMemcpyHostToDevice));
-    TB_CUDA(cudaMemcpy(out.d_warp_row, warp_row.data(), sizeof(int32_t) * warp_row.size(), cudaMemcpyHostToDevice));
+    out.d_chan = reinterpret_cast<RowChan*>(base);
+    out.d_work = reinterpret_cast<RowWork*>(base + cb);
+    out.d_warp_row = reinterpret_cast<int32_t*>(base + cb + wb);
+    TB_CUDA(cudaMemcpy(base, all.data(), all.size(), cudaMemcpyHostToDevice));
     out.nblocks = int(work.size());
     int64_t adds = 0;   // of the channel whose smallest band takes the most for each element
     for (size_t i = 0; i < chan.size(); ++i) {

@@ -23,6 +23,7 @@
 #include <cub/cub.cuh>
 
 #include <algorithm>
+#include <memory>
 
 #include "tb_geom.cuh"
 #include "tb_theta.cuh"
@@ -30,9 +31,7 @@
 namespace tb {
 
 void ThetaList::release() {
-    if (ids) cudaFree(ids);
-    if (mask) cudaFree(mask);
-    if (perm) cudaFree(perm);
+    if (mask) cudaFree(mask);   // the allocation's base: masks, ids, perm
     ids = nullptr;
     mask = nullptr;
     perm = nullptr;
@@ -97,28 +96,6 @@ __global__ void k_theta_gather(const int32_t* __restrict__ tup, int64_t stride, 
     }
 }
 
-namespace {
-
-// Temporaries of one build, freed on every return path.
-struct Scratch {
-    std::vector<void*> p;
-    template <class T>
-    T* get(size_t n) {
-        void* q = nullptr;
-        if (cudaMalloc(&q, n * sizeof(T) + 16) != cudaSuccess) {
-            cudaGetLastError();
-            return nullptr;
-        }
-        p.push_back(q);
-        return static_cast<T*>(q);
-    }
-    ~Scratch() {
-        for (void* q : p) cudaFree(q);
-    }
-};
-
-}  // namespace
-
 int build_theta_list(const ChanDev& c, const DeviceTuples& tup, ThetaList& out, cudaStream_t stream) {
     out.release();
     const int64_t n = tup.n;
@@ -126,12 +103,25 @@ int build_theta_list(const ChanDev& c, const DeviceTuples& tup, ThetaList& out, 
     // point count, below the 0xffffffff of tuples without a point (so the
     // element must fit 25 bits); cub sorts int-sized inputs
     if (n <= 0 || c.nmc < 1 || c.nmc > 64 || c.leg[0].ne >= (1 << 25) || n > int64_t(0x7fffffff)) return TB_OK;
-    Scratch tmp;
-    uint64_t* mask = tmp.get<uint64_t>(size_t(n));
-    uint32_t* key[2] = {tmp.get<uint32_t>(size_t(n)), tmp.get<uint32_t>(size_t(n))};
-    int32_t* idx[2] = {tmp.get<int32_t>(size_t(n)), tmp.get<int32_t>(size_t(n))};
-    unsigned long long* counts = tmp.get<unsigned long long>(2);
-    if (!mask || !key[0] || !key[1] || !idx[0] || !idx[1] || !counts) return TB_OK;   // no room: full quadrature
+    // the temporaries in one allocation, freed on every return path
+    size_t tbytes = 0;
+    {
+        cub::DoubleBuffer<uint32_t> k0(nullptr, nullptr);
+        cub::DoubleBuffer<int32_t> v0(nullptr, nullptr);
+        TB_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tbytes, k0, v0, int(n), 0, 32, stream));
+    }
+    const size_t wide = (sizeof(uint64_t) * size_t(n) + 255) / 256 * 256, word = (sizeof(int32_t) * size_t(n) + 255) / 256 * 256;
+    char* base = nullptr;
+    if (cudaMalloc(&base, wide + 4 * word + 256 + tbytes) != cudaSuccess) {
+        cudaGetLastError();
+        return TB_OK;   // no room: full quadrature
+    }
+    std::unique_ptr<char, cudaError_t (*)(char*)> tmp(base, [](char* p) { return cudaFree(p); });
+    uint64_t* mask = reinterpret_cast<uint64_t*>(base);
+    uint32_t* key[2] = {reinterpret_cast<uint32_t*>(base + wide), reinterpret_cast<uint32_t*>(base + wide + word)};
+    int32_t* idx[2] = {reinterpret_cast<int32_t*>(base + wide + 2 * word), reinterpret_cast<int32_t*>(base + wide + 3 * word)};
+    unsigned long long* counts = reinterpret_cast<unsigned long long*>(base + wide + 4 * word);
+    void* d_tmp = base + wide + 4 * word + 256;
     TB_CUDA(cudaMemsetAsync(counts, 0, 2 * sizeof(unsigned long long), stream));
     const int threads = 256;
     const int64_t blocks = std::min<int64_t>((n + threads - 1) / threads, 148 * 16);
@@ -145,23 +135,20 @@ int build_theta_list(const ChanDev& c, const DeviceTuples& tup, ThetaList& out, 
     TB_CUDA(cudaGetLastError());
     cub::DoubleBuffer<uint32_t> kb(key[0], key[1]);
     cub::DoubleBuffer<int32_t> vb(idx[0], idx[1]);
-    size_t tbytes = 0;
-    TB_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tbytes, kb, vb, int(n), 0, 32, stream));
-    void* d_tmp = tmp.get<char>(tbytes);
-    if (!d_tmp) return TB_OK;
     TB_CUDA(cub::DeviceRadixSort::SortPairs(d_tmp, tbytes, kb, vb, int(n), 0, 32, stream));   // stable
     unsigned long long h_counts[2] = {0, 0};
     TB_CUDA(cudaMemcpyAsync(h_counts, counts, sizeof(h_counts), cudaMemcpyDeviceToHost, stream));
     TB_CUDA(cudaStreamSynchronize(stream));
     const int64_t nl = int64_t(h_counts[0]);
     if (nl > 0) {
-        if (cudaMalloc(&out.ids, sizeof(int32_t) * size_t(c.L + 1) * size_t(nl)) != cudaSuccess ||
-            cudaMalloc(&out.mask, sizeof(uint64_t) * size_t(nl)) != cudaSuccess ||
-            cudaMalloc(&out.perm, sizeof(int32_t) * size_t(nl)) != cudaSuccess) {
+        const size_t nn = size_t(nl);
+        if (cudaMalloc(&out.mask, sizeof(uint64_t) * nn + sizeof(int32_t) * size_t(c.L + 2) * nn) != cudaSuccess) {
             cudaGetLastError();
-            out.release();
+            out.mask = nullptr;
             return TB_OK;
         }
+        out.ids = reinterpret_cast<int32_t*>(out.mask + nn);
+        out.perm = out.ids + size_t(c.L + 1) * nn;
         const int64_t gb = std::min<int64_t>((nl + threads - 1) / threads, 148 * 16);
         k_theta_gather<<<unsigned(gb), threads, 0, stream>>>(tup.d, tup.cap, c.L, vb.Current(), mask, nl, out.ids,
                                                              out.mask, out.perm);
