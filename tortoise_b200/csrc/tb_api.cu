@@ -805,9 +805,12 @@ static RowArgs row_args(tb_handle* h, const double* f, double* acc, const DPCtl*
 }
 
 // The channels over packed rows: all of them in one launch per leg count, or
-// (only_inst >= 0) that instance's alone.  rate_leg: -1 every leg.
+// (only_inst >= 0) that instance's alone.  rate_leg: -1 every leg.  drift: in:
+// add the drift term as well if that takes no launch of its own; out: it did.
 static int launch_row_sets(tb_handle* h, const double* d_in, double* d_acc, const DPCtl* ctl, int only_inst, bool rate,
-                           int rate_leg) {
+                           int rate_leg, bool& drift) {
+    const bool want_drift = drift;
+    drift = false;
     RowArgs a = row_args(h, d_in, d_acc, ctl);
     a.rate = rate;
     a.rate_leg = rate_leg;
@@ -821,7 +824,11 @@ static int launch_row_sets(tb_handle* h, const double* d_in, double* d_acc, cons
         return launch_rows(G.row_one, a, h->stream);
     }
     const bool rates = rate && !h->rate_sets.empty();
-    if (!h->row_sets.empty() || rates) TB_TRY(launch_rows_prepare(h->ed, d_in, h->d_f4, h->d_nf, ctl, h->stream));
+    if (!h->row_sets.empty() || rates) {
+        drift = want_drift;
+        TB_TRY(launch_rows_prepare(h->ed, d_in, h->d_f4, h->d_nf, ctl, h->stream, nullptr, nullptr,
+                                   drift ? d_acc : nullptr));
+    }
     for (const auto* sets : {&h->row_sets, &h->rate_sets}) {
         if (sets == &h->rate_sets && !rates) continue;
         for (const RowSet& rs : *sets)
@@ -857,8 +864,12 @@ static int launch_group_stream(tb_handle* h, GroupChan& G, const InstDev* insts,
 }
 
 int run_rhs_acc(tb_handle* h, const double* d_in, double* d_acc, const DPCtl* ctl, int flags, int only_inst) {
+    bool drift = !(flags & TB_NO_DRIFT) && only_inst < 0 && h->any_drift;
     if (!(flags & TB_NO_COLLISIONS)) {
-        TB_TRY(launch_row_sets(h, d_in, d_acc, ctl, only_inst, false, -1));
+        // sharded: the drift is replicated, so it follows the all-reduce
+        bool with_rows = drift && h->opts.shard_count <= 1 && !h->comm;
+        TB_TRY(launch_row_sets(h, d_in, d_acc, ctl, only_inst, false, -1, with_rows));
+        if (with_rows) drift = false;
         for (size_t gi = 0; gi < h->groups.size(); ++gi) {
             GroupChan& G = h->groups[gi];
             if ((G.tup.n == 0 && !G.stream) || G.use_rows) continue;
@@ -888,7 +899,7 @@ int run_rhs_acc(tb_handle* h, const double* d_in, double* d_acc, const DPCtl* ct
         // (replicated) drift term
         TB_TRY(shard_allreduce(h, d_acc, size_t(h->ndofs)));
     }
-    if (!(flags & TB_NO_DRIFT) && only_inst < 0 && h->any_drift) TB_TRY(launch_drift(h->ed, d_in, d_acc, ctl, h->stream));
+    if (drift) TB_TRY(launch_drift(h->ed, d_in, d_acc, ctl, h->stream));
     return TB_OK;
 }
 
@@ -1598,7 +1609,8 @@ int tb_scattering_rates(tb_handle* h, int ch, int leg, const double* f, double* 
         d_res = h->d_out;
     }
     TB_CUDA(cudaMemsetAsync(h->d_acc, 0, bytes, h->stream));
-    TB_TRY(launch_row_sets(h, d_in, h->d_acc, nullptr, ch, true, leg));
+    bool no_drift = false;
+    TB_TRY(launch_row_sets(h, d_in, h->d_acc, nullptr, ch, true, leg, no_drift));
     for (size_t gi = 0; gi < h->groups.size(); ++gi) {
         GroupChan& G = h->groups[gi];
         if ((G.tup.n == 0 && !G.stream) || G.use_rows) continue;

@@ -49,6 +49,7 @@
 
 #include "tb_bulk.cuh"
 #include "tb_dp45.cuh"
+#include "tb_drift.cuh"
 #include "tb_geom.cuh"
 #include "tb_rows.cuh"
 
@@ -64,8 +65,10 @@ __host__ __device__ constexpr int row_shares(int L) { return L == 4 ? 12 : 16; }
 enum { ROW_PROPAGATE = 0, ROW_RATE = 1, ROW_VJP = 2 };
 // Warps of a block: the rates and the transpose accumulate sums for every leg
 // and take fewer (rates: 184 us against 210 with 16 at 40x24 e-ph with umklapp).
-template <int L, int MODE, bool DET> struct RowCap {
-    static constexpr int W = MODE != ROW_PROPAGATE ? (L == 4 ? 8 : DET ? 16 : 12) : row_shares(L);
+__host__ __device__ constexpr int row_shares_few(int L) { return L == 4 ? 8 : 12; }
+template <int L, int MODE> struct RowCap {
+    static constexpr bool FEW = MODE != ROW_PROPAGATE;
+    static constexpr int W = FEW ? row_shares_few(L) : row_shares(L);
 };
 constexpr int ROW_STAGES = 2;    // rows of a warp in shared memory
 constexpr int ROW_COPIES = 16;   // copies of the point table, one per lane of a half warp
@@ -103,7 +106,7 @@ void RowSet::release() {
     if (d_chan) cudaFree(d_chan);   // the allocation's base: channels, work, bounds
     d_chan = nullptr;
     d_work = nullptr;
-    d_warp_row = nullptr;
+    d_bounds[0] = d_bounds[1] = nullptr;
     nblocks = 0;
 }
 
@@ -248,7 +251,8 @@ int build_rows(const ChanDev& c, const ThetaList& th, PointRows& rows, int64_t m
 // ----------------------------------------------------------------- prepare
 __global__ void __launch_bounds__(256) k_rows_prepare(ElemDev ed, const double* __restrict__ f, double4* __restrict__ f4,
                                                       const double* __restrict__ u, double4* __restrict__ u4,
-                                                      int* __restrict__ nf, const DPCtl* __restrict__ ctl) {
+                                                      int* __restrict__ nf, double* __restrict__ drift_acc,
+                                                      const DPCtl* __restrict__ ctl) {
     const int band = ed.blk_band[blockIdx.x];
     const BandDev& bd = ed.bands[band];
     bool bad = false;
@@ -262,14 +266,15 @@ __global__ void __launch_bounds__(256) k_rows_prepare(ElemDev ed, const double* 
     if (e < bd.ne && !(ctl && ctl[ed.band_run[band]].done)) {
         pad(f, f4);
         if (u) pad(u, u4);
+        if (drift_acc && (bd.vel[0] != 0.0 || bd.vel[1] != 0.0)) drift_element(bd, f, e, drift_acc);
     }
     bad = __syncthreads_or(bad);
     if (threadIdx.x == 0) nf[blockIdx.x] = bad ? 1 : 0;
 }
 
 int launch_rows_prepare(const ElemDev& ed, const double* f, double4* f4, int* nf, const DPCtl* ctl, cudaStream_t s,
-                        const double* u, double4* u4) {
-    k_rows_prepare<<<ed.nblk, 256, 0, s>>>(ed, f, f4, u, u4, nf, ctl);
+                        const double* u, double4* u4, double* drift_acc) {
+    k_rows_prepare<<<ed.nblk, 256, 0, s>>>(ed, f, f4, u, u4, nf, drift_acc, ctl);
     TB_CUDA(cudaGetLastError());
     return TB_OK;
 }
@@ -770,9 +775,9 @@ __device__ __noinline__ void spread_nonfinite(const RowChan& c, const InstDev* i
 }
 
 template <int L, int FORM, int MODE, bool DET, bool MULTI>
-__global__ void __launch_bounds__(RowCap<L, MODE, DET>::W * 32, 1) k_rows(const RowChan* __restrict__ chans,
+__global__ void __launch_bounds__(RowCap<L, MODE>::W * 32, 1) k_rows(const RowChan* __restrict__ chans,
                                                             const RowWork* __restrict__ work,
-                                                            const int32_t* __restrict__ warp_row, int shares,
+                                                            const int32_t* __restrict__ bounds,
                                                             const InstDev* __restrict__ one,
                                                             const double* __restrict__ f,
                                                             const double4* __restrict__ f4,
@@ -788,7 +793,7 @@ __global__ void __launch_bounds__(RowCap<L, MODE, DET>::W * 32, 1) k_rows(const 
     constexpr uint32_t BYTES = RowDim<L>::BYTES;
     extern __shared__ __align__(128) unsigned char s_raw[];
     __shared__ RowChan c;
-    __shared__ __align__(8) uint64_t s_bar[RowCap<L, MODE, DET>::W][ROW_STAGES];
+    __shared__ __align__(8) uint64_t s_bar[RowCap<L, MODE>::W][ROW_STAGES];
     const RowWork w = work[blockIdx.x];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, n_warps = blockDim.x >> 5;
     if (accr && blockIdx.x % copies) acc = accr + int64_t(blockIdx.x % copies - 1) * ndofs;
@@ -806,21 +811,19 @@ __global__ void __launch_bounds__(RowCap<L, MODE, DET>::W * 32, 1) k_rows(const 
         if (!any) return;
     }
     // this warp's rows, and the copies of its first ones
-    int r0 = warp_row[w.share0 + warp], r1 = warp_row[w.share0 + warp + 1];
+    bounds += blockIdx.x * (n_warps + 1) + warp;   // one share a warp
+    const int r0 = bounds[0], r1 = bounds[1];
     unsigned char* const stage = s_raw + size_t(warp) * ROW_STAGES * BYTES;
     uint64_t* const bar = s_bar[warp];
     auto fetch = [&](int r, int s) {
         mbar_expect_tx_arrive(&bar[s], BYTES);
         bulk_g2s(stage + s * BYTES, c.blk + int64_t(r) * BYTES, BYTES, &bar[s]);
     };
-    auto fetch_first = [&](int used) {
-        for (int k = 0; k < ROW_STAGES; ++k)
-            if (r0 + k < r1) fetch(r0 + k, (used + k) % ROW_STAGES);
-    };
     if (lane == 0) {
         for (int s = 0; s < ROW_STAGES; ++s) mbar_init(&bar[s], 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        fetch_first(0);
+        for (int s = 0; s < ROW_STAGES; ++s)
+            if (r0 + s < r1) fetch(r0 + s, s);
     }
     double* const s_v = reinterpret_cast<double*>(s_raw + size_t(n_warps) * ROW_STAGES * BYTES) + warp * 96 * (L - 1);
     double* const s_q = reinterpret_cast<double*>(s_raw + size_t(n_warps) * (ROW_STAGES * BYTES + 768 * (L - 1)));
@@ -839,15 +842,8 @@ __global__ void __launch_bounds__(RowCap<L, MODE, DET>::W * 32, 1) k_rows(const 
         amp = insts[0].amp_full;
     }
     int e0_next = r0 < r1 ? __ldg(c.row_e0 + r0) : 0;   // the next row's leg-0 element
-    int share = warp, used = 0;   // this warp's share, and how many rows it has taken from its stages
-    for (int r = r0;; ++r, ++used) {
-        while (r >= r1 && (share += n_warps) < shares) {   // fewer warps than shares: the next share
-            r = r0 = warp_row[w.share0 + share];
-            r1 = warp_row[w.share0 + share + 1];
-            if (lane == 0) fetch_first(used);
-            if (r < r1) e0_next = __ldg(c.row_e0 + r);
-        }
-        if (r >= r1) break;
+    for (int r = r0; r < r1; ++r) {
+        const int used = r - r0;
         const int s = used % ROW_STAGES;
         const int e0_row = e0_next;
         if (r + 1 < r1) e0_next = __ldg(c.row_e0 + r + 1);
@@ -996,12 +992,12 @@ static int launch_k_rows(const RowSet& rs, const RowArgs& A, cudaStream_t s) {
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64 || !((attr_devices.load() >> dev) & 1ull)) {
         TB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     int(rows_smem(L, 64, RowCap<L, MODE, DET>::W))));
+                                     int(rows_smem(L, 64, RowCap<L, MODE>::W))));
         if (dev >= 0 && dev < 64) attr_devices.fetch_or(1ull << dev);
     }
-    const int warps = std::min(rs.shares, RowCap<L, MODE, DET>::W);
+    const int warps = rs.shares[RowCap<L, MODE>::FEW];
     kern<<<unsigned(rs.nblocks), unsigned(32 * warps), rows_smem(L, rs.nmc_max, warps), s>>>(
-        rs.d_chan, rs.d_work, rs.d_warp_row, rs.shares, A.one, A.f, A.f4, A.nf, A.ed->nblk, A.acc, A.accr, rs.copies,
+        rs.d_chan, rs.d_work, rs.d_bounds[RowCap<L, MODE>::FEW], A.one, A.f, A.f4, A.nf, A.ed->nblk, A.acc, A.accr, rs.copies,
         A.ed->ndofs, A.ctl, A.rate_leg, A.fx, A.err_flag, A.polls, A.u, A.u4, A.gamp);
     TB_CUDA(cudaGetLastError());
     if (A.accr && rs.copies > 1) {
@@ -1063,14 +1059,16 @@ int build_row_set(int L, int form, const std::vector<RowChan>& chan, const std::
     // one block per SM; fewer warps in each where there are fewer rows than
     // warps.  Every item gets a block of its own at least, the others go one
     // by one to the item with the largest cost per block.
-    out.shares = int(std::min<int64_t>(row_shares(L), std::max<int64_t>(4, (nrows + nsm - 1) / nsm)));
+    const int64_t per_sm = std::max<int64_t>(4, (nrows + nsm - 1) / nsm);
+    out.shares[0] = int(std::min<int64_t>(row_shares(L), per_sm));
+    out.shares[1] = int(std::min<int64_t>(row_shares_few(L), per_sm));
     std::vector<int64_t> nb(item.size(), 1);
     auto cost_of = [&](size_t i) -> const std::vector<int64_t>& {
         const PointRows& r = *rows[size_t(item[i].first)];
         return S ? r.run_cost : r.cost;
     };
     auto load = [&](size_t i) { return double(cost_of(i).back()) / double(nb[i]); };
-    for (int64_t left = std::min<int64_t>(nsm, (nrows + out.shares - 1) / out.shares) - int64_t(item.size()); left > 0;
+    for (int64_t left = std::min<int64_t>(nsm, (nrows + out.shares[0] - 1) / out.shares[0]) - int64_t(item.size()); left > 0;
          --left) {
         size_t best = 0;
         for (size_t i = 1; i < item.size(); ++i)
@@ -1078,31 +1076,31 @@ int build_row_set(int L, int form, const std::vector<RowChan>& chan, const std::
         nb[best] += 1;
     }
     std::vector<RowWork> work;
-    std::vector<int32_t> warp_row;
+    std::vector<int32_t> bounds[2];
     for (size_t i = 0; i < item.size(); ++i) {
         const RowChan& c = chan[size_t(item[i].first)];
         const std::vector<int64_t>& cost = cost_of(i);
-        const int64_t parts = nb[i] * out.shares;
-        // rows up to the p-th share of the cost
-        auto bound = [&](int64_t p) {
-            return int32_t(std::lower_bound(cost.begin(), cost.end(), cost.back() * p / parts) - cost.begin());
-        };
         for (int64_t b = 0; b < nb[i]; ++b) {
             RowWork w{};
             w.chan = item[i].first;
             w.chunk = item[i].second;
-            w.share0 = int(warp_row.size());
             w.t0 = c.n * b / nb[i];
             w.t1 = c.n * (b + 1) / nb[i];
             work.push_back(w);
-            for (int64_t p = b * out.shares; p <= (b + 1) * out.shares; ++p) warp_row.push_back(bound(p));
+            for (int k = 0; k < 2; ++k)
+                for (int64_t p = b * out.shares[k]; p <= (b + 1) * out.shares[k]; ++p)   // rows up to the p-th share
+                    bounds[k].push_back(int32_t(std::lower_bound(cost.begin(), cost.end(),
+                                                                 cost.back() * p / (nb[i] * out.shares[k])) -
+                                                cost.begin()));
         }
     }
     const size_t cb = (sizeof(RowChan) * chan.size() + 255) / 256 * 256, wb = (sizeof(RowWork) * work.size() + 255) / 256 * 256;
-    std::vector<char> all(cb + wb + sizeof(int32_t) * warp_row.size());
+    const size_t bb = sizeof(int32_t) * bounds[0].size();
+    std::vector<char> all(cb + wb + bb + sizeof(int32_t) * bounds[1].size());
     std::memcpy(all.data(), chan.data(), sizeof(RowChan) * chan.size());
     std::memcpy(all.data() + cb, work.data(), sizeof(RowWork) * work.size());
-    std::memcpy(all.data() + cb + wb, warp_row.data(), sizeof(int32_t) * warp_row.size());
+    std::memcpy(all.data() + cb + wb, bounds[0].data(), bb);
+    std::memcpy(all.data() + cb + wb + bb, bounds[1].data(), sizeof(int32_t) * bounds[1].size());
     char* base = nullptr;
     if (cudaMalloc(&base, all.size()) != cudaSuccess) {
         cudaGetLastError();
@@ -1111,7 +1109,8 @@ int build_row_set(int L, int form, const std::vector<RowChan>& chan, const std::
     }
     out.d_chan = reinterpret_cast<RowChan*>(base);
     out.d_work = reinterpret_cast<RowWork*>(base + cb);
-    out.d_warp_row = reinterpret_cast<int32_t*>(base + cb + wb);
+    out.d_bounds[0] = reinterpret_cast<int32_t*>(base + cb + wb);
+    out.d_bounds[1] = reinterpret_cast<int32_t*>(base + cb + wb + bb);
     TB_CUDA(cudaMemcpy(base, all.data(), all.size(), cudaMemcpyHostToDevice));
     out.nblocks = int(work.size());
     int64_t adds = 0;   // of the channel whose smallest band takes the most for each element
@@ -1204,7 +1203,7 @@ __global__ void __launch_bounds__(256) k_runs_state_scatter(const RunState* __re
 template <int L, int FORM, int S>
 __global__ void __launch_bounds__(row_shares(L) * 32, 1) k_rows_runs(const RowChan* __restrict__ chans,
                                                                  const RowWork* __restrict__ work,
-                                                                 const int32_t* __restrict__ warp_row, int shares,
+                                                                 const int32_t* __restrict__ bounds,
                                                                  const double* __restrict__ f,
                                                                  const int* __restrict__ nf, int n_nf,
                                                                  double* __restrict__ acc,
@@ -1227,7 +1226,8 @@ __global__ void __launch_bounds__(row_shares(L) * 32, 1) k_rows_runs(const RowCh
         if (in.amp_full != 0.0 && !(ctl && ctl[in.run].done)) amp = in.amp_full;
     }
     if (__all_sync(0xffffffffu, amp == 0.0)) return;   // uniform in the block
-    const int r0 = warp_row[w.share0 + warp], r1 = warp_row[w.share0 + warp + 1];   // blockDim = 32 shares
+    bounds += blockIdx.x * (n_warps + 1) + warp;   // one share a warp
+    const int r0 = bounds[0], r1 = bounds[1];
     unsigned char* const stage = s_raw + size_t(warp) * ROW_STAGES * BYTES;
     uint64_t* const bar = s_bar[warp];
     auto fetch = [&](int r, int s) {
@@ -1342,8 +1342,8 @@ static int launch_k_rows_runs(const RowSet& rs, int n_tiles, const double* f, co
         TB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes(64, row_shares(L)))));
         if (dev >= 0 && dev < 64) attr_devices.fetch_or(1ull << dev);
     }
-    kern<<<unsigned(rs.nblocks), unsigned(32 * rs.shares), bytes(rs.nmc_max, rs.shares), s>>>(
-        rs.d_chan, rs.d_work, rs.d_warp_row, rs.shares, f, nf, n_tiles, acc, ctl, err_flag, polls);
+    kern<<<unsigned(rs.nblocks), unsigned(32 * rs.shares[0]), bytes(rs.nmc_max, rs.shares[0]), s>>>(
+        rs.d_chan, rs.d_work, rs.d_bounds[0], f, nf, n_tiles, acc, ctl, err_flag, polls);
     TB_CUDA(cudaGetLastError());
     return TB_OK;
 }

@@ -62,13 +62,11 @@ struct RowChan {
     int64_t stride, n;
 };
 
-// One block's work: the rows of channel chan, in shares that the bounds
-// warp_row[share0 ..] delimit, and the part [t0, t1) of its whole list.
+// One block's work: rows of channel chan, in shares that RowSet's bounds
+// delimit, and the part [t0, t1) of its whole list.
 struct RowWork {
     int chan;
-    int share0;
     int chunk;       // run-minor sets: which S runs
-    int pad;
     int64_t t0, t1;
 };
 
@@ -79,8 +77,11 @@ struct RowSet {
     int form = 0;                   // row_form
     RowChan* d_chan = nullptr;
     RowWork* d_work = nullptr;
-    int32_t* d_warp_row = nullptr;  // per block: the bounds of its shares
-    int nblocks = 0, shares = 0;
+    // per block the bounds of its shares (shares + 1), one share a warp: for
+    // propagation, and for the kernels that take fewer warps
+    int32_t* d_bounds[2] = {nullptr, nullptr};
+    int shares[2] = {0, 0};
+    int nblocks = 0;
     int nmc_max = 0;
     int copies = 1;                 // accumulators that its blocks share out (row_copies)
     bool multi = false;             // some channel has several instances
@@ -112,8 +113,10 @@ int build_row_set(int L, int form, const std::vector<RowChan>& chan, const std::
 
 // f4[e] = (f0, f1, f2, 0) of every element of the state, u4 of u likewise when
 // it is given; nf[b] != 0 marks an element block with a non-finite coefficient.
+// drift_acc non-null: the drift term is added there too (launch_drift's; the
+// same pass over the elements saves its launch, 5 us).
 int launch_rows_prepare(const ElemDev& ed, const double* f, double4* f4, int* nf, const DPCtl* ctl, cudaStream_t s,
-                        const double* u = nullptr, double4* u4 = nullptr);
+                        const double* u = nullptr, double4* u4 = nullptr, double* drift_acc = nullptr);
 
 // One evaluation of a set.
 struct RowArgs {
