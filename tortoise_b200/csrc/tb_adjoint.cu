@@ -110,6 +110,7 @@ void adjoint_release(tb_handle* h) {
 
 // Buffers independent of the step budget (replay tool, reverse sweep).
 static int adj_base(tb_handle* h) {
+    h->acc_clean = false;
     if (!h->adj) h->adj = new AdjointState();
     AdjointState* A = h->adj;
     if (A->lam) return TB_OK;
@@ -464,14 +465,7 @@ int tb_adjoint_rhs_vjp(tb_handle* h, const double* f, const double* theta, doubl
     else TB_CUDA(cudaMemcpyAsync(grad_f, A->g, bytes, cudaMemcpyDeviceToDevice, h->stream));
     TB_CUDA(cudaMemsetAsync(A->g, 0, bytes, h->stream));
     if (grad_amp) TB_TRY(copy_gamp_out(h, grad_amp));
-    else TB_TRY(stream_wait(h));
-    int tflag = 0;
-    TB_TRY(take_wait_timeout(h->d_err, h->stream, &tflag));
-    if (tflag) { set_error("a wait for staged rows ran out; the gradient is incomplete"); return TB_ERR_TIMEOUT; }
-    bool clamped = false;
-    TB_TRY(fx_take_saturation(h, clamped));
-    if (clamped) return fx_saturation_error();
-    return TB_OK;
+    return check_status(h);
 }
 
 int tb_dp45_replay(tb_handle* h, const double* f0, const double* dts, int64_t n_steps, double dense_s, double* f_out,
@@ -603,6 +597,7 @@ int tb_adjoint_backward(tb_handle* h, const double* lambda_T, double* grad_f0, d
     if (!h->adj || !h->adj->have_forward) { set_error("tb_adjoint_forward was not called"); return TB_ERR_ARG; }
     TB_CUDA(cudaSetDevice(h->device));
     AdjointState* A = h->adj;
+    h->acc_clean = false;
     const int rflags = A->flags;
     const size_t n = size_t(h->ndofs);
     const size_t bytes = sizeof(double) * n;
@@ -668,13 +663,7 @@ int tb_adjoint_backward(tb_handle* h, const double* lambda_T, double* grad_f0, d
         if (flags & TB_PTR_HOST) TB_CUDA(cudaMemcpyAsync(grad_f0, out, bytes, cudaMemcpyDeviceToHost, h->stream));
     }
     if (grad_amp) TB_TRY(copy_gamp_out(h, grad_amp));
-    TB_TRY(stream_wait(h));
-    int tflag = 0;
-    TB_TRY(take_wait_timeout(h->d_err, h->stream, &tflag));
-    if (tflag) { set_error("moment-tensor copy wait ran out"); return TB_ERR_TIMEOUT; }
-    bool clamped = false;
-    TB_TRY(fx_take_saturation(h, clamped));
-    if (clamped) return fx_saturation_error();
+    TB_TRY(check_status(h));
     if (st) {
         std::memset(st, 0, sizeof(*st));
         st->t_obs = A->t_obs;

@@ -105,6 +105,12 @@ void release_row_sets(tb_handle* h);
 
 namespace tb {
 
+// Results up to this size come through a buffer of the handle in host-pointer
+// calls: one copy brings the result and the status words, where the flag took a
+// copy and a wait of its own (with the accumulator's two memsets gone, an 8x8
+// e-ph right-hand side 75 -> 52 us); larger ones go to the caller's memory.
+constexpr size_t HOST_IO_MAX = size_t(256) << 10;
+
 double* dev_alloc(tb_handle* h, size_t n) {
     double* p = nullptr;
     if (cudaMalloc(&p, sizeof(double) * (n ? n : 1)) != cudaSuccess) return nullptr;
@@ -385,18 +391,19 @@ int build_runs(tb_handle* h, const tb_problem_desc* const* descs, int nruns) {
     }
     // state scratch
     h->d_f = dev_alloc(h, size_t(h->ndofs));
-    h->d_out = dev_alloc(h, size_t(h->ndofs));
+    h->d_out = dev_alloc(h, size_t(h->ndofs) + 1);   // and the status words
     h->d_acc = dev_alloc(h, size_t(h->ndofs));
     h->d_part = dev_alloc(h, size_t(2 * h->ed.nblk + 8));
     if (!h->d_f || !h->d_out || !h->d_acc || !h->d_part) { set_error("state allocation failed"); return TB_ERR_OOM; }
     TB_CUDA(cudaMemsetAsync(h->d_acc, 0, sizeof(double) * size_t(h->ndofs), h->stream));
     if (h->opts.deterministic) TB_TRY(fx_alloc(h, h->ndofs, h->fx));
+    h->d_err = reinterpret_cast<int*>(h->d_out + h->ndofs);
+    TB_CUDA(cudaMemset(h->d_err, 0, 2 * sizeof(int)));
+    if (h->opts.deterministic) h->fx.sat = reinterpret_cast<unsigned int*>(h->d_err + 1);
     {
-        void* p = nullptr;
-        if (cudaMalloc(&p, sizeof(int)) != cudaSuccess) { set_error("flag allocation failed"); return TB_ERR_OOM; }
-        h->dev_raw.push_back(p);
-        h->d_err = static_cast<int*>(p);
-        TB_CUDA(cudaMemset(h->d_err, 0, sizeof(int)));
+        const size_t io = sizeof(double) * size_t(h->ndofs) <= HOST_IO_MAX ? size_t(h->ndofs) : 0;
+        h->h_io.resize(io + 1);
+        h->h_status = reinterpret_cast<int*>(h->h_io.data() + io);
     }
     // channel groups and instances
     std::vector<int> group_chan0(group_first_run.size(), -1);
@@ -1047,7 +1054,7 @@ int dp_alloc(tb_handle* h, int64_t max_dense) {
         if (cudaMalloc(&c, sizeof(DPCtl) * nruns) != cudaSuccess) { set_error("controller allocation failed"); return TB_ERR_OOM; }
         B.ctl = c;
         h->dev_raw.push_back(c);
-        if (cudaMallocHost(&h->h_ctl, sizeof(DPCtl) * nruns) != cudaSuccess) {
+        if (cudaMallocHost(&h->h_ctl, sizeof(DPCtl) * nruns + sizeof(double)) != cudaSuccess) {
             set_error("pinned allocation failed");
             return TB_ERR_OOM;
         }
@@ -1134,26 +1141,69 @@ void fill_stats(const DPCtl& c, tb_dp45_stats* st) {
     st->done = c.done;
 }
 
-// Deterministic mode: was a contribution clamped to the exact accumulator's
-// range since the flag was last cleared?  Reading clears it.
-int fx_take_saturation(tb_handle* h, bool& clamped) {
-    clamped = false;
-    if (!h->fx.sat) return TB_OK;
-    unsigned int v = 0;
-    TB_CUDA(cudaMemcpyAsync(&v, h->fx.sat, sizeof(v), cudaMemcpyDeviceToHost, h->stream));
-    TB_CUDA(cudaStreamSynchronize(h->stream));
-    if (v) {
-        clamped = true;
-        TB_CUDA(cudaMemsetAsync(h->fx.sat, 0, sizeof(v), h->stream));
-    }
-    return TB_OK;
-}
-
 int fx_saturation_error() {
     set_error("deterministic mode: a contribution of magnitude 2^64 or more was clamped to the exact accumulator's "
               "range; the result is unreliable");
     return TB_ERR_NONFINITE;
 }
+}  // namespace tb
+
+namespace tb {
+
+// TB_ERR_TIMEOUT when a bounded wait for staged data ran out since the last
+// check (the kernels that gave up left their part of the sum out).  The words
+// are in h_status.
+static int status_error(tb_handle* h) {
+    if (h->h_status[0]) {
+        TB_CUDA(cudaMemsetAsync(h->d_err, 0, sizeof(int), h->stream));
+        set_error("a moment-tensor contraction gave up waiting for its staged tiles; the result is incomplete");
+        return TB_ERR_TIMEOUT;
+    }
+    if (h->fx.sat && h->h_status[1]) {
+        TB_CUDA(cudaMemsetAsync(h->fx.sat, 0, sizeof(int), h->stream));
+        return fx_saturation_error();
+    }
+    return TB_OK;
+}
+
+int check_status(tb_handle* h) {
+    TB_TRY(stream_wait(h));
+    TB_CUDA(cudaMemcpyAsync(h->h_status, h->d_err, 2 * sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+    TB_CUDA(cudaStreamSynchronize(h->stream));
+    return status_error(h);
+}
+
+// The input of an operator call on the device and a clean accumulator; with
+// host pointers the result goes to d_out.
+static int host_in(tb_handle* h, const double* f, int flags, const double*& d_in, double*& d_res) {
+    const size_t bytes = sizeof(double) * size_t(h->ndofs);
+    if (flags & TB_PTR_HOST) {
+        TB_CUDA(cudaMemcpyAsync(h->d_f, f, bytes, cudaMemcpyHostToDevice, h->stream));
+        d_in = h->d_f;
+        d_res = h->d_out;
+    }
+    if (!h->acc_clean) TB_CUDA(cudaMemsetAsync(h->d_acc, 0, bytes, h->stream));
+    h->acc_clean = false;   // until the call has read and cleared it
+    return TB_OK;
+}
+
+// With host pointers: the result to the caller, and what the kernels flagged.
+static int host_out(tb_handle* h, double* out, int flags) {
+    if (!(flags & TB_PTR_HOST)) return TB_OK;
+    const size_t bytes = sizeof(double) * size_t(h->ndofs);
+    if (h->comm) TB_TRY(stream_wait(h));   // bounded, unlike the copies below
+    if (h->h_io.size() > 1) {
+        TB_CUDA(cudaMemcpyAsync(h->h_io.data(), h->d_out, bytes + 2 * sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+        TB_TRY(stream_wait(h));
+        std::memcpy(out, h->h_io.data(), bytes);
+    } else {
+        TB_CUDA(cudaMemcpyAsync(out, h->d_out, bytes, cudaMemcpyDeviceToHost, h->stream));
+        TB_CUDA(cudaMemcpyAsync(h->h_status, h->d_err, 2 * sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+        TB_TRY(stream_wait(h));
+    }
+    return status_error(h);
+}
+
 }  // namespace tb
 
 // ====================================================================== C API
@@ -1548,42 +1598,16 @@ int tb_set_amplitude(tb_handle* h, int ch, double amplitude) {
     return TB_OK;
 }
 
-// TB_ERR_TIMEOUT when a contraction's bounded wait ran out since the last
-// check (the kernels that gave up left their part of the sum out).
-static int check_wait_timeout(tb_handle* h) {
-    int tflag = 0;
-    TB_TRY(take_wait_timeout(h->d_err, h->stream, &tflag));
-    if (tflag) {
-        set_error("a moment-tensor contraction gave up waiting for its staged tiles; the result is incomplete");
-        return TB_ERR_TIMEOUT;
-    }
-    bool clamped = false;
-    TB_TRY(tb::fx_take_saturation(h, clamped));
-    if (clamped) return tb::fx_saturation_error();
-    return TB_OK;
-}
-
 static int rhs_common(tb_handle* h, const double* f, double* out, int flags, int only_inst) {
     if (!h || !f || !out) { set_error("null argument"); return TB_ERR_ARG; }
     TB_CUDA(cudaSetDevice(h->device));
-    const size_t bytes = sizeof(double) * size_t(h->ndofs);
     const double* d_in = f;
     double* d_res = out;
-    if (flags & TB_PTR_HOST) {
-        TB_CUDA(cudaMemcpyAsync(h->d_f, f, bytes, cudaMemcpyHostToDevice, h->stream));
-        d_in = h->d_f;
-        d_res = h->d_out;
-    }
-    TB_CUDA(cudaMemsetAsync(h->d_acc, 0, bytes, h->stream));
+    TB_TRY(host_in(h, f, flags, d_in, d_res));
     TB_TRY(run_rhs_acc(h, d_in, h->d_acc, nullptr, flags, only_inst));
-    TB_TRY(launch_inverse_mass(h->ed, h->d_acc, d_res, h->stream));
-    TB_CUDA(cudaMemsetAsync(h->d_acc, 0, bytes, h->stream));
-    if (flags & TB_PTR_HOST) {
-        TB_CUDA(cudaMemcpyAsync(out, h->d_out, bytes, cudaMemcpyDeviceToHost, h->stream));
-        TB_TRY(stream_wait(h));
-        TB_TRY(check_wait_timeout(h));
-    }
-    return TB_OK;
+    TB_TRY(launch_inverse_mass(h->ed, h->d_acc, d_res, true, h->stream));
+    h->acc_clean = true;
+    return host_out(h, out, flags);
 }
 
 int tb_rhs(tb_handle* h, const double* f, double* dfdt, int flags) {
@@ -1600,15 +1624,9 @@ int tb_scattering_rates(tb_handle* h, int ch, int leg, const double* f, double* 
         return TB_ERR_ARG;
     }
     TB_CUDA(cudaSetDevice(h->device));
-    const size_t bytes = sizeof(double) * size_t(h->ndofs);
     const double* d_in = f;
     double* d_res = rates;
-    if (flags & TB_PTR_HOST) {
-        TB_CUDA(cudaMemcpyAsync(h->d_f, f, bytes, cudaMemcpyHostToDevice, h->stream));
-        d_in = h->d_f;
-        d_res = h->d_out;
-    }
-    TB_CUDA(cudaMemsetAsync(h->d_acc, 0, bytes, h->stream));
+    TB_TRY(host_in(h, f, flags, d_in, d_res));
     bool no_drift = false;
     TB_TRY(launch_row_sets(h, d_in, h->d_acc, nullptr, ch, true, leg, no_drift));
     for (size_t gi = 0; gi < h->groups.size(); ++gi) {
@@ -1634,14 +1652,9 @@ int tb_scattering_rates(tb_handle* h, int ch, int leg, const double* f, double* 
     }
     TB_TRY(launch_fx_flush(h->fx, h->d_acc, h->ndofs, h->stream));
     TB_TRY(shard_allreduce(h, h->d_acc, size_t(h->ndofs)));
-    TB_TRY(launch_inverse_mass(h->ed, h->d_acc, d_res, h->stream));
-    TB_CUDA(cudaMemsetAsync(h->d_acc, 0, bytes, h->stream));
-    if (flags & TB_PTR_HOST) {
-        TB_CUDA(cudaMemcpyAsync(rates, h->d_out, bytes, cudaMemcpyDeviceToHost, h->stream));
-        TB_TRY(stream_wait(h));
-        TB_TRY(check_wait_timeout(h));
-    }
-    return TB_OK;
+    TB_TRY(launch_inverse_mass(h->ed, h->d_acc, d_res, true, h->stream));
+    h->acc_clean = true;
+    return host_out(h, rates, flags);
 }
 
 int tb_channel_propagate(tb_handle* h, int ch, const double* f, double* out, int flags) {
@@ -1714,6 +1727,7 @@ int dp_begin(tb_handle* h, const double* f0, const double* t0, const double* t_f
         if (!(dense_step[r] > 0.0)) { set_error("dense_step must be > 0"); return TB_ERR_ARG; }
     TB_CUDA(cudaSetDevice(h->device));
     TB_TRY(dp_alloc(h, max_dense));
+    h->acc_clean = false;
     const int rflags = flags & (TB_NO_DRIFT | TB_NO_COLLISIONS);
     h->dp_flags = flags;
     h->wait_timed_out = false;
@@ -1796,9 +1810,11 @@ static int poll_all(tb_handle* h) {
     if (!h || !h->dp_ready) { set_error("tb_dp45_begin was not called"); return TB_ERR_ARG; }
     TB_CUDA(cudaSetDevice(h->device));
     TB_CUDA(cudaMemcpyAsync(h->h_ctl, h->dp.ctl, sizeof(DPCtl) * h->runs.size(), cudaMemcpyDeviceToHost, h->stream));
+    int* status = reinterpret_cast<int*>(h->h_ctl + h->runs.size());
+    TB_CUDA(cudaMemcpyAsync(status, h->d_err, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
     TB_TRY(stream_wait(h));
-    int tflag = 0;
-    TB_TRY(take_wait_timeout(h->d_err, h->stream, &tflag));
+    const bool tflag = status[0] != 0;
+    if (tflag) TB_CUDA(cudaMemsetAsync(h->d_err, 0, sizeof(int), h->stream));
     if (tflag) h->wait_timed_out = true;   // sticky for this integration: its state is unreliable
     if (h->wait_timed_out)
         for (size_t r = 0; r < h->runs.size(); ++r) { h->h_ctl[r].status = TB_ERR_TIMEOUT; h->h_ctl[r].done = 1; }
@@ -1870,9 +1886,7 @@ int tb_dp45_integrate(tb_handle* h, double* f_inout, double t0, double t_final, 
 
 int tb_synchronize(tb_handle* h) {
     if (!h) return TB_ERR_ARG;
-    TB_TRY(stream_wait(h));
-    TB_TRY(check_wait_timeout(h));
-    return TB_OK;
+    return check_status(h);
 }
 
 int tb_set_copy_wait_limit(tb_handle* h, int64_t polls) {

@@ -277,20 +277,22 @@ int launch_collision_mc(const ChanDev& c, const InstDev* insts, int n_insts, con
 }
 
 // ------------------------------------------------------------ inverse mass
-__global__ void k_inverse_mass(ElemDev ed, const double* __restrict__ acc, double* __restrict__ out) {
+// clear: acc is zeroed once read (acc and out are different arrays)
+__global__ void k_inverse_mass(ElemDev ed, double* __restrict__ acc, double* __restrict__ out, bool clear) {
     const int band = ed.blk_band[blockIdx.x];
     const BandDev& bd = ed.bands[band];
     const int e = (blockIdx.x - ed.blk_first[band]) * blockDim.x + threadIdx.x;
     if (e >= bd.ne) return;
-    const double* a = acc + bd.off + 3 * (int64_t)e;
+    double* a = acc + bd.off + 3 * (int64_t)e;
     double* o = out + bd.off + 3 * (int64_t)e;
     const double x = a[0], y = a[1], z = a[2];
+    if (clear) { a[0] = 0.0; a[1] = 0.0; a[2] = 0.0; }
 #pragma unroll
     for (int j = 0; j < 3; ++j) o[j] = x * bd.mesh.Minv[0][j] + y * bd.mesh.Minv[1][j] + z * bd.mesh.Minv[2][j];
 }
 
-int launch_inverse_mass(const ElemDev& ed, const double* acc, double* out, cudaStream_t s) {
-    k_inverse_mass<<<ed.nblk, 256, 0, s>>>(ed, acc, out);
+int launch_inverse_mass(const ElemDev& ed, double* acc, double* out, bool clear, cudaStream_t s) {
+    k_inverse_mass<<<ed.nblk, 256, 0, s>>>(ed, acc, out, clear);
     TB_CUDA(cudaGetLastError());
     return TB_OK;
 }

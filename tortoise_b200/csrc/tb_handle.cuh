@@ -114,6 +114,12 @@ struct tb_handle {
     // set by a contraction kernel whose bounded wait for a staged tile ran
     // out; read and cleared by the synchronising calls (TB_ERR_TIMEOUT)
     int* d_err = nullptr;
+    // where a host-pointer call's result lands (nothing beyond HOST_IO_MAX),
+    // and behind it the two status words that follow d_out on the device:
+    // d_err and the deterministic mode's clamp flag
+    std::vector<double> h_io;
+    int* h_status = nullptr;
+    bool acc_clean = false;        // d_acc is all zero
     bool wait_timed_out = false;   // the current integration met a timed-out wait
     // DP45
     tb::DPBufs dp{};
@@ -123,7 +129,7 @@ struct tb_handle {
     std::vector<tb::RunDev> hruns;
     cudaGraphExec_t graph = nullptr;
     int graph_flags = -1;
-    tb::DPCtl* h_ctl = nullptr;   // pinned host mirror [nruns]
+    tb::DPCtl* h_ctl = nullptr;   // pinned host mirror [nruns], then the status words
     int dp_flags = 0;
     // adjoint (tb_adjoint.cu)
     tb::AdjointState* adj = nullptr;
@@ -163,8 +169,10 @@ void adjoint_release(tb_handle* h);
 // A zeroed exact accumulator of n slots (3 words each) plus its poison word,
 // owned by the handle (deterministic mode).
 int fx_alloc(tb_handle* h, int64_t n, FxAcc& out);
-// deterministic mode's clamp flag: read (and clear) it; the error it reports
-int fx_take_saturation(tb_handle* h, bool& clamped);
+// Reads the status words (waits for the stream); clears what is set and returns
+// the error it stands for.
+int check_status(tb_handle* h);
+// the error that the deterministic mode's clamp flag reports
 int fx_saturation_error();
 
 // tb_shard.cu

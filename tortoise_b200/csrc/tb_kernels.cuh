@@ -55,7 +55,7 @@ int launch_fx_flush(const FxAcc& fx, double* acc, int64_t n, cudaStream_t s);
 // with a nonzero drift velocity, added into acc.
 int launch_drift(const ElemDev& ed, const double* f, double* acc, const DPCtl* ctl, cudaStream_t s);
 
-// out = acc * M^-1 per element (Function::applyInverseMass).
-int launch_inverse_mass(const ElemDev& ed, const double* acc, double* out, cudaStream_t s);
+// out = acc * M^-1 per element (Function::applyInverseMass); clear: acc = 0.
+int launch_inverse_mass(const ElemDev& ed, double* acc, double* out, bool clear, cudaStream_t s);
 
 }  // namespace tb

@@ -1162,13 +1162,4 @@ int tune_tensor(const ChanDev& c, const InstDev* insts, int n_insts, MomentTenso
     return TB_OK;
 }
 
-int take_wait_timeout(int* flag, cudaStream_t s, int* value) {
-    *value = 0;
-    if (!flag) return TB_OK;
-    TB_CUDA(cudaMemcpyAsync(value, flag, sizeof(int), cudaMemcpyDeviceToHost, s));
-    TB_CUDA(cudaStreamSynchronize(s));
-    if (*value) TB_CUDA(cudaMemsetAsync(flag, 0, sizeof(int), s));
-    return TB_OK;
-}
-
 }  // namespace tb

@@ -64,9 +64,4 @@ int prepare_runs(const ChanDev& c, int n_insts, bool distinct_runs, MomentTensor
 int tune_tensor(const ChanDev& c, const InstDev* insts, int n_insts, MomentTensor& T, const int32_t* tup,
                 int64_t stride, int64_t n, const double* f, double* acc, cudaStream_t s);
 
-// *value = 1 when a bounded wait of a contraction kernel ran out since the
-// last call (the handle's flag, ChanDev::err_flag; then TB_ERR_TIMEOUT), and
-// the flag is cleared.  Waits for s (the stream the kernels ran on).
-int take_wait_timeout(int* flag, cudaStream_t s, int* value);
-
 }  // namespace tb
