@@ -531,7 +531,7 @@ int build_runs(tb_handle* h, const tb_problem_desc* const* descs, int nruns) {
                         maxs[l] = d_maxE[legband[l]];
                     }
                     NvtxRange enum_range("tb_create: enumerate tuples");
-                    TB_TRY(enumerate_channel(c, h->meshes.data(), h->bands.data(), legband, G.d_mc_pre, mins, maxs,
+                    TB_TRY(enumerate_channel(c, h->meshes.data(), h->bands.data(), legband, pre, G.d_mc_pre, mins, maxs,
                                              h->stream, G.tup, G.diag));
                 }
             }

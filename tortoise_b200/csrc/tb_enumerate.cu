@@ -17,10 +17,25 @@
 // element id (which is the reference's MeshSubsetElementIterator order).  A
 // count pass, an exclusive scan and a write pass then emit the surviving
 // tuples in exactly the reference's order, deterministically, with no sort.
+//
+// Two count passes.  k_enumerate scans an item per thread and evaluates every
+// point of a candidate in the reference's order, and the write pass does all of
+// it again.  k_enum_walk is the streamed operator's walk (tb_walk.cuh): it
+// gathers the candidates of each stage into full warps, drops those whose domain
+// excludes every point, decides points on the fused map where the rounding bound
+// allows (the same decisions), and leaves one bit per surviving candidate of an
+// item, so that k_enum_write has no test to repeat.  It takes tables of at most
+// 64 points inside the reference domain, and boxes of at most 64 candidates;
+// a channel that does not fit goes through k_enumerate.  Measured, whole
+// tb_create: 64x64 two-band e-ph 97 -> 45 ms (enumeration 72 -> 17), 16x16 e-e 410 -> 135
+// ms (367 -> 91).
 #include <cub/cub.cuh>
+
+#include <algorithm>
 
 #include "tb_enumerate.cuh"
 #include "tb_geom.cuh"
+#include "tb_walk.cuh"
 
 namespace tb {
 
@@ -194,10 +209,225 @@ __global__ void __launch_bounds__(256) k_enumerate(EnumArgs a, int64_t item0, in
     }
 }
 
+constexpr int EW_WARPS = 8;
+
+// bits[item - item0]: bit k set when candidate k of the item's box survives;
+// diag += candidates inside the energy window, with a valid determinant;
+// *overflow is set when a box holds more than 64 candidates.
+template <int L>
+__global__ void __launch_bounds__(EW_WARPS * 32, 2) k_enum_walk(ChanDev c, StreamDev sd, int64_t item0, int64_t count,
+                                                                unsigned long long* __restrict__ bits,
+                                                                unsigned long long* __restrict__ diag,
+                                                                int* __restrict__ overflow) {
+    constexpr int R = 2 * (L - 2) + 1;
+    extern __shared__ double s_pre[];
+    // per-warp queues: [0] inside the energy window, [1] past the determinant
+    // filter and the domain test.  Row L: the umklapp column, row L + 1: the
+    // item (relative) and the candidate's bit
+    __shared__ int32_t s_q[2][EW_WARPS][L + 2][ST_QUEUE];
+    __shared__ double s_cnt[65];   // prodc added k times to 0.0, in sequence
+    for (int i = threadIdx.x; i < c.nmc * R; i += blockDim.x) s_pre[i] = sd.mc_pre[i];
+    if (threadIdx.x == 0) {
+        const double sqrt2 = 1.4142135623730951;   // sqrt(2.0) correctly rounded
+        double prodc = 1.0, t = 0.0;
+        for (int l = 0; l < L; ++l) prodc *= sqrt2;
+        s_cnt[0] = t;
+        for (int k = 1; k <= 64; ++k) s_cnt[k] = (t += prodc);
+    }
+    __syncthreads();
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    unsigned long long n_pre = 0, n_det = 0;
+    int q1n = 0;   // candidates in queue 1 (warp-uniform)
+
+    auto take = [&](int q, int first, int n, int (&e)[L], int& u, int& code) {
+        const bool valid = lane < n;
+#pragma unroll
+        for (int l = 0; l < L; ++l) e[l] = valid ? s_q[q][warp][l][first + lane] : 0;
+        u = valid ? s_q[q][warp][L][first + lane] : 0;
+        code = valid ? s_q[q][warp][L + 1][first + lane] : 0;
+        return valid;
+    };
+    auto filter = [&](int first, int n) {
+        int e[L], u, code;
+        const bool valid = take(0, first, n, e, u, code);
+        TupleGeom<L> g;
+        tuple_geometry<L>(c, e, u, g);
+        bool ok = valid && (fabs(g.det) >= c.min_det);
+        n_pre += valid ? 1 : 0;
+        n_det += ok ? 1 : 0;
+        if (ok && c.threshold >= 0.0) {
+            double Ci[3][3];
+            dc_inverse<L>(g, Ci);
+            AlphaMap<L> am;
+            alpha_map<L>(g, Ci, am);
+            ok = !domain_excludes<L>(am);
+        }
+        const unsigned bal = __ballot_sync(full, ok);
+        if (ok) {
+            const int pos = q1n + __popc(bal & ((1u << lane) - 1u));
+#pragma unroll
+            for (int l = 0; l < L; ++l) s_q[1][warp][l][pos] = e[l];
+            s_q[1][warp][L][pos] = u;
+            s_q[1][warp][L + 1][pos] = code;
+        }
+        q1n += __popc(bal);
+        __syncwarp();
+    };
+    auto survive = [&](int first, int n) {
+        int e[L], u, code;
+        const bool valid = take(1, first, n, e, u, code);
+        TupleGeom<L> g;
+        tuple_geometry<L>(c, e, u, g);
+        const double adet = fabs(g.det);
+        double Ci[3][3];
+        dc_inverse<L>(g, Ci);
+        AlphaMap<L> am;
+        alpha_map<L>(g, Ci, am);
+        double T[2];
+        outside_thresholds<L>(am, T);
+        int cnt = 0;
+        for (int m = 0; m < c.nmc; ++m) cnt += theta_decide_t<L>(g, Ci, am, T, s_pre + m * R) ? 1 : 0;
+        double res = (1.0 / (c.fact * double(c.nmc) * adet)) * s_cnt[cnt];
+        res *= c.amp_vol;
+        if (valid && (adet >= c.min_det) && (fabs(res) > c.threshold)) atomicOr(bits + (code >> 6), 1ull << (code & 63));
+        __syncwarp();
+    };
+
+    int qn = 0;   // queued candidates (warp-uniform)
+    const int64_t n_warps = int64_t(gridDim.x) * EW_WARPS;
+    const int64_t run = int64_t(ST_SPAN) * 32;
+    const WalkLeg& ml = sd.leg[L - 1];
+    const int64_t it1 = item0 + count;
+    for (int64_t rb = item0 + (int64_t(blockIdx.x) * EW_WARPS + warp) * run; rb < it1; rb += n_warps * run) {
+        WalkPos<L> p;
+        walk_decode<L>(sd, rb + lane, p);
+        WalkFront fr;
+        bool front_ok = false;
+        for (int st = 0; st < ST_SPAN; ++st) {
+            const int64_t base = rb + int64_t(st) * 32;
+            if (base >= it1) break;
+            const int64_t item = base + lane;
+            int e[L];
+            int lo[2] = {0, 0}, hi[2] = {0, 0};
+            double pmn = 0.0, pmx = 0.0;
+            int ncand = 0;
+            if (item < it1) {
+                walk_at<L>(c, sd, p, fr, front_ok, e, lo, hi, pmn, pmx);
+                if (lo[0] != hi[0] && lo[1] != hi[1]) ncand = 2 * (hi[0] - lo[0]) * (hi[1] - lo[1]);
+            }
+            if (ncand > 64) {
+                *overflow = 1;
+                ncand = 0;
+            }
+            const int maxc = __reduce_max_sync(full, unsigned(ncand));
+            int cx = lo[0], cy = lo[1];
+            for (int k = 0; k < maxc; ++k) {
+                const int ie = k & 1;
+                bool pass = false;
+                int el = 0;
+                if (k < ncand) {
+                    el = 2 * (cx + cy * ml.nx) + ie;
+                    const double emin = __ldg(ml.minE + el), emax = __ldg(ml.maxE + el);
+                    const double minE = pmn + ((c.leg[L - 1].dir > 0) ? emin : -emax);
+                    const double maxE = pmx + ((c.leg[L - 1].dir > 0) ? emax : -emin);
+                    pass = (minE <= 0.0) && (maxE >= 0.0);
+                }
+                if (ie && ++cx == hi[0]) { cx = lo[0]; ++cy; }
+                const unsigned bal = __ballot_sync(full, pass);
+                if (pass) {
+                    const int pos = qn + __popc(bal & ((1u << lane) - 1u));
+#pragma unroll
+                    for (int l = 0; l < L - 1; ++l) s_q[0][warp][l][pos] = e[l];
+                    s_q[0][warp][L - 1][pos] = el;
+                    s_q[0][warp][L][pos] = p.u;
+                    s_q[0][warp][L + 1][pos] = int32_t(item - item0) << 6 | k;
+                }
+                qn += __popc(bal);
+                __syncwarp();
+                if (qn >= 32) {
+                    filter(qn - 32, 32);
+                    qn -= 32;
+                    if (q1n >= 32) {
+                        survive(q1n - 32, 32);
+                        q1n -= 32;
+                    }
+                    __syncwarp();   // the slots are reused
+                }
+            }
+            if (walk_advance<L>(sd, p)) front_ok = false;
+        }
+    }
+    if (qn > 0) filter(0, qn);
+    while (q1n > 0) {
+        const int t = min(q1n, 32);
+        survive(q1n - t, t);
+        q1n -= t;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        n_pre += __shfl_down_sync(full, n_pre, o);
+        n_det += __shfl_down_sync(full, n_det, o);
+    }
+    if (lane == 0 && (n_pre | n_det)) {
+        atomicAdd(diag + 0, n_pre);
+        atomicAdd(diag + 1, n_det);
+    }
+}
+
+// The surviving candidates of each item at base + offsets[item - item0] on.
+template <int L>
+__global__ void __launch_bounds__(256) k_enum_write(ChanDev c, StreamDev sd, int64_t item0, int64_t count,
+                                                    const unsigned long long* __restrict__ bits,
+                                                    const uint32_t* __restrict__ offsets, int32_t* __restrict__ out,
+                                                    int64_t stride, int64_t base) {
+    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    unsigned long long b = t < count ? bits[t] : 0ull;
+    if (!b) return;
+    WalkPos<L> p;
+    walk_decode<L>(sd, item0 + t, p);
+    WalkFront fr;
+    bool front_ok = false;
+    int e[L], lo[2], hi[2];
+    double pmn, pmx;
+    walk_at<L>(c, sd, p, fr, front_ok, e, lo, hi, pmn, pmx);
+    const int nbx = hi[0] - lo[0];
+    for (int64_t pos = base + offsets[t]; b; b &= b - 1, ++pos) {
+        const int k = __ffsll((long long)b) - 1, cell = k >> 1;
+        e[L - 1] = 2 * (lo[0] + cell % nbx + (lo[1] + cell / nbx) * sd.leg[L - 1].nx) + (k & 1);
+#pragma unroll
+        for (int l = 0; l < L; ++l) out[l * stride + pos] = e[l];
+        out[L * stride + pos] = p.u;
+    }
+}
+
+struct BitCount {
+    __host__ __device__ uint32_t operator()(unsigned long long b) const {
+#ifdef __CUDA_ARCH__
+        return uint32_t(__popcll((long long)b));
+#else
+        return uint32_t(__builtin_popcountll(b));
+#endif
+    }
+};
+
+// Free points in the reference triangle, the last coordinate in [0, 1]: what
+// domain_excludes and outside_thresholds assume of a table.
+static bool in_domain(const double* q, int nmc, int L) {
+    const int R = 2 * (L - 2) + 1;
+    for (int m = 0; m < nmc; ++m) {
+        const double* p = q + size_t(m) * R;
+        for (int b = 0; b < L - 2; ++b)
+            if (!(p[2 * b] >= 0.0 && p[2 * b + 1] >= 0.0 && p[2 * b] + p[2 * b + 1] <= 1.0)) return false;
+        if (!(p[R - 1] >= 0.0 && p[R - 1] <= 1.0)) return false;
+    }
+    return true;
+}
+
 // Host driver: chunked count / scan / write.  Output is SoA with L+1 rows
 // (L element-id rows, then the umklapp row) of length `cap`.
 int enumerate_channel(const ChanDev& c, const HostMesh* meshes, const HostBand* bands, const int* leg_band,
-                      const double* d_mc_pre, const double* const* d_minE, const double* const* d_maxE,
+                      const double* h_mc_pre, const double* d_mc_pre, const double* const* d_minE, const double* const* d_maxE,
                       cudaStream_t stream, DeviceTuples& outT, int64_t diag[3]) {
     const int L = c.L;
     EnumArgs a;
@@ -245,7 +475,91 @@ int enumerate_channel(const ChanDev& c, const HostMesh* meshes, const HostBand* 
     const size_t smem = sizeof(double) * size_t(c.nmc) * c.R;
     int64_t n = 0;
     if (outT.cap == 0 && rc == TB_OK) rc = outT.reserve(L, int64_t(1) << 20, stream);
-    for (int64_t s = 0; s < total && rc == TB_OK; s += chunk) {
+    // room for `add` more tuples behind the first n
+    auto room = [&](uint64_t add) {
+        int64_t want = outT.cap;
+        while (want < n + int64_t(add)) want *= 2;
+        return want > outT.cap ? outT.grow(L, want, n, stream) : int(TB_OK);
+    };
+    bool walked = false;
+    if (rc == TB_OK && c.nmc <= 64 && in_domain(h_mc_pre, c.nmc, L)) {
+        StreamDev sd{};
+        for (int l = 0; l < L; ++l) {
+            const EnumLeg& el = a.leg[l];
+            WalkLeg& w = sd.leg[l];
+            w.minE = el.minE;
+            w.maxE = el.maxE;
+            w.nx = el.nx;
+            w.ny = el.ny;
+            for (int i = 0; i < 2; ++i) {
+                w.origin[i] = el.origin[i];
+                for (int j = 0; j < 2; ++j) { w.dG[i][j] = el.dG[i][j]; w.invdG[i][j] = el.invdG[i][j]; }
+            }
+        }
+        for (int l = 0; l < TB_MAX_LEGS; ++l) sd.nsec[l] = a.nsec[l];
+        sd.n_items = total;
+        sd.mc_pre = d_mc_pre;
+        // one bit per candidate of an item, the overflow flag behind them
+        unsigned long long* bits = nullptr;
+        int overflow = 0;
+        walked = cudaMalloc(&bits, sizeof(unsigned long long) * size_t(chunk + 1)) == cudaSuccess;
+        if (!walked) cudaGetLastError();   // no room: the other pass
+        cub::TransformInputIterator<uint32_t, BitCount, const unsigned long long*> pops(bits, BitCount{});
+        void* d_tmp2 = nullptr;
+        size_t tmp2 = 0;
+        if (walked) {
+            cub::DeviceScan::ExclusiveSum(nullptr, tmp2, pops, d_offsets, int(chunk), stream);
+            if (cudaMalloc(&d_tmp2, tmp2) != cudaSuccess) fail(TB_ERR_OOM, "scan scratch allocation failed");
+            cudaMemsetAsync(bits + chunk, 0, sizeof(unsigned long long), stream);
+        }
+        int* d_over = reinterpret_cast<int*>(bits + chunk);
+        for (int64_t s = 0; s < total && walked && rc == TB_OK && !overflow; s += chunk) {
+            const int64_t cnt = (total - s) < chunk ? (total - s) : chunk;
+            const int64_t runs = (cnt + ST_SPAN * 32 - 1) / (ST_SPAN * 32);
+            const unsigned grid = unsigned(std::min<int64_t>((runs + EW_WARPS - 1) / EW_WARPS, 148 * 2 * 8));
+            const unsigned wgrid = unsigned((cnt + 255) / 256);
+            cudaMemsetAsync(bits, 0, sizeof(unsigned long long) * size_t(cnt), stream);
+            switch (L) {
+                case 2: k_enum_walk<2><<<grid, EW_WARPS * 32, smem, stream>>>(c, sd, s, cnt, bits, d_diag, d_over); break;
+                case 3: k_enum_walk<3><<<grid, EW_WARPS * 32, smem, stream>>>(c, sd, s, cnt, bits, d_diag, d_over); break;
+                default: k_enum_walk<4><<<grid, EW_WARPS * 32, smem, stream>>>(c, sd, s, cnt, bits, d_diag, d_over); break;
+            }
+            if (cudaGetLastError() != cudaSuccess) { fail(TB_ERR_CUDA, "walk launch failed"); break; }
+            cub::DeviceScan::ExclusiveSum(d_tmp2, tmp2, pops, d_offsets, int(cnt), stream);
+            uint32_t last = 0;
+            unsigned long long last_bits = 0;
+            cudaMemcpyAsync(&last, d_offsets + cnt - 1, sizeof(last), cudaMemcpyDeviceToHost, stream);
+            cudaMemcpyAsync(&last_bits, bits + cnt - 1, sizeof(last_bits), cudaMemcpyDeviceToHost, stream);
+            cudaMemcpyAsync(&overflow, d_over, sizeof(overflow), cudaMemcpyDeviceToHost, stream);
+            if (cudaStreamSynchronize(stream) != cudaSuccess) { fail(TB_ERR_CUDA, "count pass failed"); break; }
+            const uint64_t add = uint64_t(last) + BitCount{}(last_bits);
+            if (overflow || add == 0) continue;
+            if (add >= (uint64_t(1) << 31)) { fail(TB_ERR_CAPACITY, "more than 2^31 survivors in one chunk"); break; }
+            rc = room(add);
+            if (rc != TB_OK) break;
+            switch (L) {
+                case 2: k_enum_write<2><<<wgrid, 256, 0, stream>>>(c, sd, s, cnt, bits, d_offsets, outT.d, outT.cap, n); break;
+                case 3: k_enum_write<3><<<wgrid, 256, 0, stream>>>(c, sd, s, cnt, bits, d_offsets, outT.d, outT.cap, n); break;
+                default: k_enum_write<4><<<wgrid, 256, 0, stream>>>(c, sd, s, cnt, bits, d_offsets, outT.d, outT.cap, n); break;
+            }
+            if (cudaGetLastError() != cudaSuccess) { fail(TB_ERR_CUDA, "write launch failed"); break; }
+            n += int64_t(add);
+        }
+        if (rc == TB_OK && walked && cudaStreamSynchronize(stream) != cudaSuccess) fail(TB_ERR_CUDA, "write pass failed");
+        cudaFree(bits);
+        cudaFree(d_tmp2);
+        if (overflow && rc == TB_OK) {   // a box beyond the bits: from the start with the other pass
+            walked = false;
+            n = 0;
+            cudaMemsetAsync(d_diag, 0, sizeof(unsigned long long) * 3, stream);
+        }
+        if (rc == TB_OK && walked) {
+            const unsigned long long ns = (unsigned long long)n;
+            cudaMemcpyAsync(d_diag + 2, &ns, sizeof(ns), cudaMemcpyHostToDevice, stream);
+            cudaStreamSynchronize(stream);
+        }
+    }
+    for (int64_t s = 0; s < total && rc == TB_OK && !walked; s += chunk) {
         const int64_t cnt = (total - s) < chunk ? (total - s) : chunk;
         const unsigned grid = unsigned((cnt + 255) / 256);
         switch (L) {
@@ -262,12 +576,8 @@ int enumerate_channel(const ChanDev& c, const HostMesh* meshes, const HostBand* 
         const uint64_t add = uint64_t(last[0]) + uint64_t(last[1]);
         if (add >= (uint64_t(1) << 31)) { fail(TB_ERR_CAPACITY, "more than 2^31 survivors in one chunk"); break; }
         if (add == 0) continue;
-        if (n + int64_t(add) > outT.cap) {
-            int64_t want = outT.cap;
-            while (want < n + int64_t(add)) want *= 2;
-            rc = outT.grow(L, want, n, stream);
-            if (rc != TB_OK) break;
-        }
+        rc = room(add);
+        if (rc != TB_OK) break;
         switch (L) {
             case 2: k_enumerate<2><<<grid, 256, smem, stream>>>(a, s, cnt, nullptr, d_offsets, outT.d, outT.cap, n, nullptr); break;
             case 3: k_enumerate<3><<<grid, 256, smem, stream>>>(a, s, cnt, nullptr, d_offsets, outT.d, outT.cap, n, nullptr); break;

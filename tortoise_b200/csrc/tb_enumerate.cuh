@@ -16,8 +16,9 @@ struct DeviceTuples {
     void release();
 };
 
+// h_mc_pre: the survival table d_mc_pre on the host.
 int enumerate_channel(const ChanDev& c, const HostMesh* meshes, const HostBand* bands, const int* leg_band,
-                      const double* d_mc_pre, const double* const* d_minE, const double* const* d_maxE,
+                      const double* h_mc_pre, const double* d_mc_pre, const double* const* d_minE, const double* const* d_maxE,
                       cudaStream_t stream, DeviceTuples& out, int64_t diag[3]);
 
 }  // namespace tb
