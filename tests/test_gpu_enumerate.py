@@ -26,6 +26,13 @@ def _outside_points():
     return mat
 
 
+def _threshold(t):
+    mat = W.parabolic_ee(4, mesh_nsplit=(4, 3))
+    for c in mat.channels:
+        c.scattElemeThreshold = t
+    return mat
+
+
 def _fine_last_leg():
     """The last leg on a mesh so much finer than the others' that its boxes hold more than 64 candidates."""
     region = Region((-1.0, -1.0), ((2.0, 0.0), (0.0, 2.0)))
@@ -49,6 +56,10 @@ CASES = {
     "outside_points": _outside_points,
     "fine_last_leg": _fine_last_leg,
     "four_legs": lambda: W.parabolic_ee(5, mesh_nsplit=(5, 4)),
+    "one_point": lambda: _eph(n_mc=1),
+    "33_points": lambda: _eph(n_mc=33),
+    "high_threshold": lambda: _threshold(2e-6),    # more than one point inside needed
+    "negative_threshold": lambda: _threshold(-1.0),   # none needed
 }
 
 
@@ -67,3 +78,22 @@ def test_tuples_equal_the_oracle(gpu_lib, name):
         assert total > 0
     finally:
         e.close()
+
+
+@pytest.mark.parametrize("name", ["walk", "one_point", "33_points", "64_points", "four_legs", "high_threshold",
+                                  "negative_threshold"])
+def test_streamed_walk_equals_the_stored_list(gpu_lib, name):
+    """The streamed operator takes the same decisions: the same bits in the deterministic mode."""
+    mat = CASES[name]()
+    f = W.initial_status(mat, kT=0.15, seed=6).vec
+    stored = E.Engine(mat, layout=E.LAYOUT_MC64, deterministic=True)
+    streamed = E.Engine(mat, deterministic=True, stream_legs=2)
+    try:
+        assert np.array_equal(stored.rhs(f), streamed.rhs(f))
+        for ch in range(len(mat.channels)):
+            assert streamed.channel_info(ch)["n_tuples"] == stored.channel_info(ch)["n_tuples"]
+            if stored.channel_info(ch)["n_tuples"]:
+                assert streamed.points_inside(ch) == stored.points_inside(ch)
+    finally:
+        stored.close()
+        streamed.close()

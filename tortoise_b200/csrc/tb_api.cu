@@ -303,7 +303,7 @@ int build_runs(tb_handle* h, const tb_problem_desc* const* descs, int nruns) {
     // per-band device tables (every band its own; equal-structure runs read
     // their group's first-run tables inside the channel kernels)
     const int nb = int(h->bands.size());
-    std::vector<const double*> d_disp(nb), d_kx(nb), d_ky(nb), d_minE(nb), d_maxE(nb);
+    std::vector<const double*> d_table(nb), d_minE(nb), d_maxE(nb);
     h->banddev.resize(nb);
     for (int b = 0; b < nb; ++b) {
         HostBand& B = h->bands[b];
@@ -321,12 +321,16 @@ int build_runs(tb_handle* h, const tb_problem_desc* const* descs, int nruns) {
                 B.minE[e] = std::min(n0, std::min(n1, n2));
                 B.maxE[e] = std::max(n0, std::max(n1, n2));
             }
-            d_disp[b] = dev_upload(h, B.disp);
-            d_kx[b] = dev_upload(h, B.kx);
-            d_ky[b] = dev_upload(h, B.ky);
+            std::vector<double> table(size_t(m.ne) * 12, 0.0);
+            for (int e = 0; e < m.ne; ++e) {
+                const double *x = &B.kx[size_t(3) * e], *y = &B.ky[size_t(3) * e], *z = &B.disp[size_t(3) * e];
+                const double row[9] = {x[0], y[0], z[0], x[1], y[1], z[1], x[2], y[2], z[2]};
+                std::copy(row, row + 9, &table[size_t(12) * e]);
+            }
+            d_table[b] = dev_upload(h, table);
             d_minE[b] = dev_upload(h, B.minE);
             d_maxE[b] = dev_upload(h, B.maxE);
-            if (!d_disp[b] || !d_kx[b] || !d_ky[b] || !d_minE[b] || !d_maxE[b]) {
+            if (!d_table[b] || !d_minE[b] || !d_maxE[b]) {
                 set_error("band table allocation failed");
                 return TB_ERR_OOM;
             }
@@ -428,9 +432,7 @@ int build_runs(tb_handle* h, const tb_problem_desc* const* descs, int nruns) {
                     const int gb = ri.band0 + cd.band[l];
                     const HostBand& B = h->bands[gb];
                     LegDev& lg = c.leg[l];
-                    lg.disp = d_disp[gb];
-                    lg.kx = d_kx[gb];
-                    lg.ky = d_ky[gb];
+                    lg.table = reinterpret_cast<const double4*>(d_table[gb]);
                     lg.foff = B.off;
                     lg.dir = double(cd.dir[l]);
                     lg.stat = B.stat;

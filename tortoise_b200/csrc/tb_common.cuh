@@ -74,9 +74,10 @@ struct HostBand {
 // ---------------------------------------------------- device-side records
 // Everything a kernel needs about one leg of a channel.
 struct LegDev {
-    const double* disp;   // [ne*3]
-    const double* kx;     // [ne*3]
-    const double* ky;     // [ne*3]
+    // per element the P1 coefficients of kx, ky and E in three 32-byte pieces,
+    // (kx0 ky0 E0 kx1) (ky1 E1 kx2 ky2) (E2 . . .): the lanes of a warp gather
+    // different elements, and a load costs a cache lookup a lane
+    const double4* table;
     int64_t foff;         // band offset in the status vector
     double dir;           // +1 in, -1 out
     double stat;          // -1 fermion, +1 boson

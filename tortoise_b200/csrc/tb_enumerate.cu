@@ -21,14 +21,14 @@
 // Two count passes.  k_enumerate scans an item per thread and evaluates every
 // point of a candidate in the reference's order, and the write pass does all of
 // it again.  k_enum_walk is the streamed operator's walk (tb_walk.cuh): it
-// gathers the candidates of each stage into full warps, drops those whose domain
-// excludes every point, decides points on the fused map where the rounding bound
-// allows (the same decisions), and leaves one bit per surviving candidate of an
+// gathers the candidates of each stage into full warps, drops those that FP32
+// places outside at every point, decides the others on the fused map where the
+// rounding bound allows (the same decisions), and leaves one bit per surviving candidate of an
 // item, so that k_enum_write has no test to repeat.  It takes tables of at most
 // 64 points inside the reference domain, and boxes of at most 64 candidates;
 // a channel that does not fit goes through k_enumerate.  Measured, whole
-// tb_create: 64x64 two-band e-ph 97 -> 45 ms (enumeration 72 -> 17), 16x16 e-e 410 -> 135
-// ms (367 -> 91).
+// tb_create: 64x64 two-band e-ph 97 -> 43 ms (enumeration 72 -> 14), 16x16 e-e
+// 410 -> 105 ms (367 -> 64).
 #include <cub/cub.cuh>
 
 #include <algorithm>
@@ -220,13 +220,18 @@ __global__ void __launch_bounds__(EW_WARPS * 32, 2) k_enum_walk(ChanDev c, Strea
                                                                 unsigned long long* __restrict__ diag,
                                                                 int* __restrict__ overflow) {
     constexpr int R = 2 * (L - 2) + 1;
-    extern __shared__ double s_pre[];
-    // per-warp queues: [0] inside the energy window, [1] past the determinant
-    // filter and the domain test.  Row L: the umklapp column, row L + 1: the
+    extern __shared__ __align__(16) double s_pre[];   // the table, then its FP32 copy
+    // per-warp queues: [0] inside the energy window, [1] with a
+    // valid determinant and points that may be inside.  Row L: the umklapp column, row L + 1: the
     // item (relative) and the candidate's bit
     __shared__ int32_t s_q[2][EW_WARPS][L + 2][ST_QUEUE];
+    __shared__ uint64_t s_may[EW_WARPS][ST_QUEUE];   // queue 1: points that may be inside
     __shared__ double s_cnt[65];   // prodc added k times to 0.0, in sequence
-    for (int i = threadIdx.x; i < c.nmc * R; i += blockDim.x) s_pre[i] = sd.mc_pre[i];
+    float* s_fl = reinterpret_cast<float*>(s_pre + (c.nmc * R + 1) / 2 * 2);
+    for (int i = threadIdx.x; i < c.nmc * R; i += blockDim.x) {
+        s_pre[i] = sd.mc_pre[i];
+        s_fl[i / R * FloatTable<L>::FT + i % R] = float(sd.mc_pre[i]);
+    }
     if (threadIdx.x == 0) {
         const double sqrt2 = 1.4142135623730951;   // sqrt(2.0) correctly rounded
         double prodc = 1.0, t = 0.0;
@@ -256,12 +261,16 @@ __global__ void __launch_bounds__(EW_WARPS * 32, 2) k_enum_walk(ChanDev c, Strea
         bool ok = valid && (fabs(g.det) >= c.min_det);
         n_pre += valid ? 1 : 0;
         n_det += ok ? 1 : 0;
-        if (ok && c.threshold >= 0.0) {
+        uint64_t may = 0;
+        if (ok) {
             double Ci[3][3];
             dc_inverse<L>(g, Ci);
             AlphaMap<L> am;
             alpha_map<L>(g, Ci, am);
-            ok = !domain_excludes<L>(am);
+            double T[2];
+            outside_thresholds<L>(am, T);
+            may = maybe_inside<L>(am, T, s_fl, c.nmc);
+            ok = may != 0ull || c.threshold < 0.0;
         }
         const unsigned bal = __ballot_sync(full, ok);
         if (ok) {
@@ -270,6 +279,7 @@ __global__ void __launch_bounds__(EW_WARPS * 32, 2) k_enum_walk(ChanDev c, Strea
             for (int l = 0; l < L; ++l) s_q[1][warp][l][pos] = e[l];
             s_q[1][warp][L][pos] = u;
             s_q[1][warp][L + 1][pos] = code;
+            s_may[warp][pos] = may;
         }
         q1n += __popc(bal);
         __syncwarp();
@@ -286,9 +296,16 @@ __global__ void __launch_bounds__(EW_WARPS * 32, 2) k_enum_walk(ChanDev c, Strea
         alpha_map<L>(g, Ci, am);
         double T[2];
         outside_thresholds<L>(am, T);
+        const double per = 1.0 / (c.fact * double(c.nmc) * adet);
+        // res grows with the count: where one point inside is enough, the first one ends the search
+        const bool one = fabs(per * s_cnt[1] * c.amp_vol) > c.threshold;
         int cnt = 0;
-        for (int m = 0; m < c.nmc; ++m) cnt += theta_decide_t<L>(g, Ci, am, T, s_pre + m * R) ? 1 : 0;
-        double res = (1.0 / (c.fact * double(c.nmc) * adet)) * s_cnt[cnt];
+        for (uint64_t mk = valid ? s_may[warp][first + lane] : 0ull; mk; mk &= mk - 1)
+            if (theta_decide_t<L>(g, Ci, am, T, s_pre + (__ffsll((long long)mk) - 1) * R)) {
+                ++cnt;
+                if (one) break;
+            }
+        double res = per * s_cnt[cnt];
         res *= c.amp_vol;
         if (valid && (adet >= c.min_det) && (fabs(res) > c.threshold)) atomicOr(bits + (code >> 6), 1ull << (code & 63));
         __syncwarp();
@@ -412,7 +429,7 @@ struct BitCount {
 };
 
 // Free points in the reference triangle, the last coordinate in [0, 1]: what
-// domain_excludes and outside_thresholds assume of a table.
+// outside_thresholds and maybe_inside assume of a table.
 static bool in_domain(const double* q, int nmc, int L) {
     const int R = 2 * (L - 2) + 1;
     for (int m = 0; m < nmc; ++m) {
@@ -518,11 +535,12 @@ int enumerate_channel(const ChanDev& c, const HostMesh* meshes, const HostBand* 
             const int64_t runs = (cnt + ST_SPAN * 32 - 1) / (ST_SPAN * 32);
             const unsigned grid = unsigned(std::min<int64_t>((runs + EW_WARPS - 1) / EW_WARPS, 148 * 2 * 8));
             const unsigned wgrid = unsigned((cnt + 255) / 256);
+            const size_t wsmem = smem + 16 + sizeof(float) * 8 * size_t(c.nmc);
             cudaMemsetAsync(bits, 0, sizeof(unsigned long long) * size_t(cnt), stream);
             switch (L) {
-                case 2: k_enum_walk<2><<<grid, EW_WARPS * 32, smem, stream>>>(c, sd, s, cnt, bits, d_diag, d_over); break;
-                case 3: k_enum_walk<3><<<grid, EW_WARPS * 32, smem, stream>>>(c, sd, s, cnt, bits, d_diag, d_over); break;
-                default: k_enum_walk<4><<<grid, EW_WARPS * 32, smem, stream>>>(c, sd, s, cnt, bits, d_diag, d_over); break;
+                case 2: k_enum_walk<2><<<grid, EW_WARPS * 32, wsmem, stream>>>(c, sd, s, cnt, bits, d_diag, d_over); break;
+                case 3: k_enum_walk<3><<<grid, EW_WARPS * 32, wsmem, stream>>>(c, sd, s, cnt, bits, d_diag, d_over); break;
+                default: k_enum_walk<4><<<grid, EW_WARPS * 32, wsmem, stream>>>(c, sd, s, cnt, bits, d_diag, d_over); break;
             }
             if (cudaGetLastError() != cudaSuccess) { fail(TB_ERR_CUDA, "walk launch failed"); break; }
             cub::DeviceScan::ExclusiveSum(d_tmp2, tmp2, pops, d_offsets, int(cnt), stream);

@@ -21,6 +21,13 @@ __device__ __forceinline__ double xm(double a, double b) { return __dmul_rn(a, b
 __device__ __forceinline__ double xa(double a, double b) { return __dadd_rn(a, b); }
 __device__ __forceinline__ double xs(double a, double b) { return __dsub_rn(a, b); }
 
+// One 32-byte load.
+__device__ __forceinline__ double4 load_32(const double4* p) {
+    double4 v;
+    asm("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(v.w) : "l"(p));
+    return v;
+}
+
 template <int L>
 struct TupleGeom {
     double D[3][2 * L];
@@ -30,26 +37,19 @@ struct TupleGeom {
 
 template <int L>
 __device__ __forceinline__ void tuple_geometry(const ChanDev& c, const int (&e)[L], int umk, TupleGeom<L>& g) {
-#pragma unroll
-    for (int l = 0; l < L; ++l) {
-        const double d = c.leg[l].dir;
-        const double* kx = c.leg[l].kx + 3 * (int64_t)e[l];
-        const double* ky = c.leg[l].ky + 3 * (int64_t)e[l];
-        const double* en = c.leg[l].disp + 3 * (int64_t)e[l];
-#pragma unroll
-        for (int j = 0; j < 2; ++j) {
-            g.D[0][2 * l + j] = d * __ldg(kx + 1 + j);
-            g.D[1][2 * l + j] = d * __ldg(ky + 1 + j);
-            g.D[2][2 * l + j] = d * __ldg(en + 1 + j);
-        }
-    }
     g.N[0] = 0.0; g.N[1] = 0.0; g.N[2] = 0.0;
 #pragma unroll
     for (int l = 0; l < L; ++l) {
         const double d = c.leg[l].dir;
-        g.N[0] = xs(g.N[0], xm(d, __ldg(c.leg[l].kx + 3 * (int64_t)e[l])));
-        g.N[1] = xs(g.N[1], xm(d, __ldg(c.leg[l].ky + 3 * (int64_t)e[l])));
-        g.N[2] = xs(g.N[2], xm(d, __ldg(c.leg[l].disp + 3 * (int64_t)e[l])));
+        const double4* t = c.leg[l].table + 3 * (int64_t)e[l];
+        const double4 x = load_32(t), y = load_32(t + 1), z = load_32(t + 2);
+        // (kx0 ky0 E0 kx1) (ky1 E1 kx2 ky2) (E2 . . .)
+        g.D[0][2 * l] = d * x.w; g.D[0][2 * l + 1] = d * y.z;
+        g.D[1][2 * l] = d * y.x; g.D[1][2 * l + 1] = d * y.w;
+        g.D[2][2 * l] = d * y.y; g.D[2][2 * l + 1] = d * z.x;
+        g.N[0] = xs(g.N[0], xm(d, x.x));
+        g.N[1] = xs(g.N[1], xm(d, x.y));
+        g.N[2] = xs(g.N[2], xm(d, x.z));
     }
     const double u0 = c.umk[2 * umk], u1 = c.umk[2 * umk + 1];
 #pragma unroll

@@ -319,13 +319,6 @@ struct StageMap {
     __device__ __forceinline__ double G(int k, int j) const { return d[32 * (3 + k * R + j)]; }
 };
 
-// The padded coefficients of one element in one 32-byte load.
-__device__ __forceinline__ double4 load_f4(const double4* p) {
-    double4 v;
-    asm("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(v.w) : "l"(p));
-    return v;
-}
-
 // The values a tuple adds to its legs' elements: v[l] = (1, x_l, y_l)
 // moments of the integrand, scaled.
 template <int L>
@@ -868,8 +861,8 @@ __global__ void __launch_bounds__(RowCap<L, MODE>::W * 32, 1) k_rows(const RowCh
         if (!MULTI && e[0] != e0) {
             if (e0 >= 0 && (!RATE || rate_leg <= 0)) z.flush(acc, off[0] + 3 * (int64_t)e0, fx);
             e0 = e[0];
-            f0 = load_f4(f4 + el[0] + e0);
-            if (VJP) u0 = load_f4(u4 + el[0] + e0);
+            f0 = load_32(f4 + el[0] + e0);
+            if (VJP) u0 = load_32(u4 + el[0] + e0);
         }
         for (int k = 0; k < (MULTI ? n_insts : 1); ++k) {
             if (MULTI) {
@@ -878,20 +871,20 @@ __global__ void __launch_bounds__(RowCap<L, MODE>::W * 32, 1) k_rows(const RowCh
                 if (!VJP && (amp == 0.0 || (ctl && ctl[in.run].done))) continue;
 #pragma unroll
                 for (int l = 0; l < L; ++l) { off[l] = in.foff[l]; el[l] = off[l] / 3; }
-                f0 = load_f4(f4 + el[0] + e[0]);
-                if (VJP) u0 = load_f4(u4 + el[0] + e[0]);
+                f0 = load_32(f4 + el[0] + e[0]);
+                if (VJP) u0 = load_32(u4 + el[0] + e[0]);
             }
             double4 f[L];
             f[0] = f0;
 #pragma unroll
-            for (int l = 1; l < L; ++l) f[l] = load_f4(f4 + el[l] + e[l]);
+            for (int l = 1; l < L; ++l) f[l] = load_32(f4 + el[l] + e[l]);
             RowOut<L> o;
             const double wt = reinterpret_cast<const double*>(b)[32 * (ND - 1) + lane];
             if constexpr (VJP) {
                 double4 u[L];
                 u[0] = u0;
 #pragma unroll
-                for (int l = 1; l < L; ++l) u[l] = load_f4(u4 + el[l] + e[l]);
+                for (int l = 1; l < L; ++l) u[l] = load_32(u4 + el[l] + e[l]);
                 const double g = row_tuple_vjp<L, FORM>(c, m, mk, f, u, tab, wt * (amp * tf), o);
                 ga = fma(wt * (c.amp_vol * tf), g, ga);
                 if (MULTI) {

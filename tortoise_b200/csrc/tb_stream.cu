@@ -26,8 +26,9 @@
 // time (one per lane); the lanes step through their boxes in lock step and
 // push the candidates that pass the energy window into a per-warp queue in
 // shared memory.  Three stages drain the queues, each on 32 entries at a
-// time, one per lane: determinant filter and domain test (queue 0 -> 1), the
-// survival test (queue 1 -> 2), then the points inside, the sums and the
+// time, one per lane: the determinant filter and an FP32 pass over the survival
+// points, which ends most candidates (queue 0 -> 1); the FP64 survival test at
+// the points it left (queue 1 -> 2); then the points inside, the sums and the
 // scatter for the surviving tuples.  So every stage runs on full warps
 // whatever the box sizes and the pass rate of the stage before.
 #include "tb_dp45.cuh"
@@ -67,15 +68,20 @@ __global__ void __launch_bounds__(ST_WARPS * 32, TB_STREAM_MIN_BLOCKS)
         if (!any) return;
     }
     constexpr int R = 2 * (L - 2) + 1;
-    extern __shared__ double s_tab[];   // [nmc R] quadrature table, then [nmc R] survival table
+    extern __shared__ __align__(16) double s_tab[];   // [nmc R] quadrature table, then [nmc R] survival table
     // per-warp candidate queues: [0] inside the energy window, [1] past the
-    // determinant filter and the domain test, [2] surviving tuples
+    // determinant filter and with points that may be inside, [2] surviving tuples
     __shared__ int32_t s_q[3][ST_WARPS][L + 1][ST_QUEUE];
+    __shared__ uint64_t s_may[ST_WARPS][ST_QUEUE];   // queue 1: survival points that may be inside
     double* s_mc = s_tab;
     double* s_pre = s_tab + c.nmc * R;
+    float* s_fmc = reinterpret_cast<float*>(s_tab + (2 * c.nmc * R + 1) / 2 * 2);   // their FP32 copies
+    float* s_fpre = s_fmc + c.nmc * FloatTable<L>::FT;
     for (int i = threadIdx.x; i < c.nmc * R; i += blockDim.x) {
         s_mc[i] = c.mc[i];
         s_pre[i] = sd.mc_pre[i];
+        s_fmc[i / R * FloatTable<L>::FT + i % R] = float(c.mc[i]);
+        s_fpre[i / R * FloatTable<L>::FT + i % R] = float(sd.mc_pre[i]);
     }
     __syncthreads();
     const unsigned full = 0xffffffffu;
@@ -99,10 +105,9 @@ __global__ void __launch_bounds__(ST_WARPS * 32, TB_STREAM_MIN_BLOCKS)
     int q3n = 0;   // surviving tuples in queue 2 (warp-uniform)
 
     // Stage 1 for `take` candidates of queue 0 from slot `first` on, one per
-    // lane: the determinant filter, then the domain test; the candidates that
-    // may have a point inside go to queue 1.  Cheap next to stage 2 (about
-    // 150 operations against 2 x NMC simplex tests), and most candidates of
-    // the energy window end here.
+    // lane: the determinant filter, then the points of the survival table that
+    // FP32 cannot place outside; the candidates with such a point go to queue 1.
+    // Most candidates of the energy window end here.
     auto stage1 = [&](int first, int take) {
         const bool valid = lane < take;
         int e[L];
@@ -115,18 +120,23 @@ __global__ void __launch_bounds__(ST_WARPS * 32, TB_STREAM_MIN_BLOCKS)
         bool ok = valid && (fabs(g.det) >= c.min_det);
         n_pre += valid ? 1 : 0;
         n_det += ok ? 1 : 0;
-        if (ok && c.threshold >= 0.0) {
+        uint64_t may = 0;
+        if (ok) {
             double Ci[3][3];
             dc_inverse<L>(g, Ci);
             AlphaMap<L> am;
             alpha_map<L>(g, Ci, am);
-            ok = !domain_excludes<L>(am);
+            double T[2];
+            outside_thresholds<L>(am, T);
+            may = maybe_inside<L>(am, T, s_fpre, c.nmc);
+            ok = may != 0ull || c.threshold < 0.0;
         }
         const unsigned bal = __ballot_sync(full, ok);
         if (ok) {
             const int pos = q2n + __popc(bal & ((1u << lane) - 1u));
 #pragma unroll
             for (int l = 0; l <= L; ++l) s_q[1][warp][l][pos] = l < L ? e[l] : u;
+            s_may[warp][pos] = may;
         }
         q2n += __popc(bal);
         __syncwarp();
@@ -158,9 +168,16 @@ __global__ void __launch_bounds__(ST_WARPS * 32, TB_STREAM_MIN_BLOCKS)
         // such terms is s_cnt[cnt], the same additions in the same order)
         double T[2];
         outside_thresholds<L>(am, T);
+        const double per = 1.0 / (c.fact * double(c.nmc) * adet);
+        // res grows with the count: where one point inside is enough, the first one ends the search
+        const bool one = fabs(per * s_cnt[1] * c.amp_vol) > c.threshold;
         int cnt = 0;
-        for (int m = 0; m < c.nmc; ++m) cnt += theta_decide_t<L>(g, Ci, am, T, s_pre + m * R) ? 1 : 0;
-        double res = (1.0 / (c.fact * double(c.nmc) * adet)) * s_cnt[cnt];
+        for (uint64_t mk = valid ? s_may[warp][first + lane] : 0ull; mk; mk &= mk - 1)
+            if (theta_decide_t<L>(g, Ci, am, T, s_pre + (__ffsll((long long)mk) - 1) * R)) {
+                ++cnt;
+                if (one) break;
+            }
+        double res = per * s_cnt[cnt];
         res *= c.amp_vol;
         ok = ok && (fabs(res) > c.threshold);
         n_surv += ok ? 1 : 0;
@@ -197,8 +214,10 @@ __global__ void __launch_bounds__(ST_WARPS * 32, TB_STREAM_MIN_BLOCKS)
         if (valid) {
             double T[2];
             outside_thresholds<L>(am, T);
-            for (int m = 0; m < c.nmc; ++m)
+            for (uint64_t w = maybe_inside<L>(am, T, s_fmc, c.nmc); w; w &= w - 1) {
+                const int m = __ffsll((long long)w) - 1;
                 if (theta_decide_t<L>(g, Ci, am, T, s_mc + m * R)) mk |= 1ull << m;
+            }
         }
         n_pts += __popcll(mk);
         n_tin += mk ? 1 : 0;
@@ -375,7 +394,7 @@ static int launch_stream(const ChanDev& c, const StreamDev& sd, int64_t it0, int
                          const FxAcc& fx_amp = FxAcc{}) {
     auto kern = k_collision_stream<L, MODE>;
     const int threads = ST_WARPS * 32;
-    const size_t smem = 2 * sizeof(double) * size_t(c.nmc) * c.R;
+    const size_t smem = 2 * sizeof(double) * size_t(c.nmc) * c.R + 16 + 2 * sizeof(float) * size_t(c.nmc) * FloatTable<L>::FT;
     int dev = 0, nsm = 148, per_sm = 1;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);

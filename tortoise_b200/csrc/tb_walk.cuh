@@ -163,42 +163,6 @@ __device__ __forceinline__ void walk_at(const ChanDev& c, const StreamDev& sd, c
     }
 }
 
-// True when no point of the Monte-Carlo domain -- every free leg's point in
-// its reference triangle, the partially constrained leg's coordinate in
-// [0, 1] -- can pass the simplex tests ThetapC * ThetaFC
-// (IntegratorCore.hpp:318-320), whatever the order the constrained
-// coordinates are evaluated in: over the whole domain one of al0, al1, al2
-// stays below 0, or kp0 + al0 or al1 + al2 stays above 1, by more than four
-// times the rounding bound am.mg (which already covers the distance between
-// the fused map and the reference-order evaluation).  Then neither table has
-// a point inside: the survival sum is 0 and the tuple does not survive.
-template <int L>
-__device__ __forceinline__ bool domain_excludes(const AlphaMap<L>& am) {
-    constexpr int R = AlphaMap<L>::R;
-    const double eps = 2.220446049250313e-16;
-    double hi[3];
-    double plo = am.a0[0];                 // min of kp0 + al0
-    double slo = am.a0[1] + am.a0[2];      // min of al1 + al2
-#pragma unroll
-    for (int r = 0; r < 3; ++r) hi[r] = am.a0[r];
-#pragma unroll
-    for (int b = 0; b < L - 2; ++b) {      // free legs: vertices (0,0), (1,0), (0,1)
-#pragma unroll
-        for (int r = 0; r < 3; ++r) hi[r] += fmax(0.0, fmax(am.G[r][2 * b], am.G[r][2 * b + 1]));
-        plo += fmin(0.0, fmin(am.G[0][2 * b], am.G[0][2 * b + 1]));
-        slo += fmin(0.0, fmin(am.G[1][2 * b] + am.G[2][2 * b], am.G[1][2 * b + 1] + am.G[2][2 * b + 1]));
-    }
-#pragma unroll
-    for (int r = 0; r < 3; ++r) hi[r] += fmax(0.0, am.G[r][R - 1]);   // kp0 in [0, 1]
-    plo += fmin(0.0, am.G[0][R - 1] + 1.0);
-    slo += fmin(0.0, am.G[1][R - 1] + am.G[2][R - 1]);
-    const double m0 = 4.0 * am.mg[0], m1 = 4.0 * am.mg[1], m2 = 4.0 * am.mg[2];
-    if (hi[0] < -m0 || hi[1] < -m1 || hi[2] < -m2) return true;
-    if (plo - m0 > 1.0 + 8.0 * eps * (1.0 + fabs(plo))) return true;
-    if (slo - (m1 + m2) > 1.0 + 8.0 * eps * (1.0 + fabs(slo))) return true;
-    return false;
-}
-
 // Per-tuple thresholds of a cheaper "clearly outside" test than
 // theta_decide's: T[0] for kp0 + al0, T[1] for al1 + al2.  Over the whole
 // Monte-Carlo domain (every coordinate of q in [0, 1]) the fused
@@ -242,6 +206,69 @@ __device__ __forceinline__ bool theta_decide_t(const TupleGeom<L>& g, const doub
                      (__dadd_rn(kp0, al[0]) > T[0]) || (__dadd_rn(al[1], al[2]) > T[1]);
     if (out) return false;
     return alpha_theta<L>(g, Ci, am, qv, al);
+}
+
+// The Monte-Carlo table in FP32, FT floats a point (built by the block).
+template <int L>
+struct FloatTable {
+    static constexpr int R = 2 * (L - 2) + 1;
+    static constexpr int FT = R <= 1 ? 1 : R <= 4 ? 4 : 8;
+};
+
+// The points that FP32 arithmetic cannot place clearly outside: bit m is clear
+// only where theta_decide is false.  Most points of most tuples are far outside,
+// and FP32 runs beside the FP64 pipe at twice its rate, so the FP64 decisions
+// are left to the set bits (12x10 e-e, streamed: 13.0 -> 10.3 ms; enumeration of
+// 16x16 e-e: 91 -> 62 ms).  With u = 2^-24, B_r = |a0_r| + sum_j |G_rj| and q in
+// [0, 1], the FP32 value of alpha_r (operands rounded to FP32, at most R + 1 fused
+// steps) is within (R + 4) u B_r of the real map, R <= 5, and so within E_r =
+// 16 u B_r: a value below -(E_r + 4 mg_r) leaves the FP64 one below -mg_r, and
+// kp0 + alpha_0 or alpha_1 + alpha_2 above their threshold T (outside_thresholds)
+// by those E and 16 u of the operands leaves the FP64 sum above T.  Comparisons
+// with NaN are false, and an infinite bound keeps every point.
+template <int L>
+__device__ __forceinline__ uint64_t maybe_inside(const AlphaMap<L>& am, const double (&T)[2], const float* tab, int nmc) {
+    constexpr int R = AlphaMap<L>::R, FT = FloatTable<L>::FT;
+    const double u = 5.9604644775390625e-8;
+    float a[3], G[3][R], lo[3], B[3];
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+        double b = fabs(am.a0[r]);
+        a[r] = float(am.a0[r]);
+#pragma unroll
+        for (int j = 0; j < R; ++j) {
+            b += fabs(am.G[r][j]);
+            G[r][j] = float(am.G[r][j]);
+        }
+        B[r] = __double2float_ru(16.0 * u * b);
+        lo[r] = -__double2float_ru(16.0 * u * b + 4.0 * am.mg[r]);
+    }
+    const float hi0 = __double2float_ru(T[0] + 32.0 * u) + 2.0f * B[0];
+    const float hi1 = __double2float_ru(T[1] + 32.0 * u) + 2.0f * (B[1] + B[2]);
+    uint32_t word[2] = {0u, 0u};
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const int m0 = 32 * h, m1 = min(nmc, m0 + 32);
+        uint32_t bit = 1u;
+#pragma unroll 1   // more points a step cost registers (a 12x10 e-e evaluation: 2 11.2 ms, 4 12.2, against 10.3)
+        for (int m = m0; m < m1; ++m, bit += bit) {
+            float q[R];
+#pragma unroll
+            for (int j = 0; j < R; ++j) q[j] = tab[m * FT + j];
+            float al[3];
+#pragma unroll
+            for (int r = 0; r < 3; ++r) {
+                al[r] = a[r];
+#pragma unroll
+                for (int j = 0; j < R; ++j) al[r] = fmaf(G[r][j], q[j], al[r]);
+            }
+            const bool out = (al[0] < lo[0]) || (al[1] < lo[1]) || (al[2] < lo[2]) || (q[R - 1] + al[0] > hi0) ||
+                             (al[1] + al[2] > hi1);
+            word[h] |= out ? 0u : bit;
+        }
+    }
+    const uint64_t mask = uint64_t(word[1]) << 32 | word[0];
+    return mask;
 }
 
 }  // namespace tb
