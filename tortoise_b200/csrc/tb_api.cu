@@ -99,7 +99,6 @@ namespace tb {
 int choose_layouts(tb_handle* h);
 int autotune(tb_handle* h);
 int build_run_states(tb_handle* h);
-int64_t rows_room();
 void release_row_sets(tb_handle* h);
 }  // namespace tb
 
@@ -572,10 +571,13 @@ int build_runs(tb_handle* h, const tb_problem_desc* const* descs, int nruns) {
     }
     {
         NvtxRange r("tb_create: points inside the simplices");
+        size_t freeb = 0, totalb = 0;
+        cudaMemGetInfo(&freeb, &totalb);
+        const int64_t room = int64_t(double(freeb) * 0.6);   // the most that a channel's rows may take, as for tensors
         for (auto& G : h->groups)
             if (G.layout == TB_LAYOUT_MC64) {
                 TB_TRY(build_theta_list(G.dev, G.tup, G.theta, h->stream));
-                if (G.theta.built) TB_TRY(build_rows(G.dev, G.theta, G.rows, rows_room(), h->stream));
+                if (G.theta.built) TB_TRY(build_rows(G.dev, G.theta, G.rows, room, h->stream));
                 G.use_rows = G.rows.blk != nullptr;
             }
     }
@@ -612,13 +614,6 @@ static int launch_group_mc(tb_handle* h, GroupChan& G, const InstDev* insts, int
                                    h->stream, 148 * 32, rate_leg, G.theta.mask, G.theta.perm, h->fx);
     return launch_collision_mc(G.dev, insts, n_insts, G.tup.d, G.tup.cap, G.tup.n, d_in, d_acc, ctl, h->stream,
                                148 * 32, rate_leg, nullptr, nullptr, h->fx);
-}
-
-// The most that the rows of one channel may take: what moment tensors may.
-int64_t rows_room() {
-    size_t freeb = 0, totalb = 0;
-    cudaMemGetInfo(&freeb, &totalb);
-    return int64_t(double(freeb) * 0.6);
 }
 
 // Channels shared by this many runs or more go over their rows run-minor, the
@@ -1019,12 +1014,13 @@ int choose_layouts(tb_handle* h) {
         }
         G.layout = want;
         if (want != TB_LAYOUT_MC64) {
+            const int64_t room = int64_t(double(freeb) * 0.6);   // as for a tensor
             // AUTO's FP64 channels go over their packed rows; the tensor is
             // built when a contraction schedule is asked for
             if (h->opts.layout == TB_LAYOUT_AUTO && want == TB_LAYOUT_T64  &&
                 !(h->opts.deterministic && int(G.insts.size()) >= ROWS_MAX_EXACT)) {
                 TB_TRY(build_theta_list(G.dev, G.tup, G.theta, h->stream));
-                if (G.theta.built) TB_TRY(build_rows(G.dev, G.theta, G.rows, rows_room(), h->stream));
+                if (G.theta.built) TB_TRY(build_rows(G.dev, G.theta, G.rows, room, h->stream));
                 G.use_rows = G.rows.blk != nullptr;
                 if (G.use_rows) continue;
                 G.theta.release();

@@ -215,7 +215,7 @@ constexpr int EW_WARPS = 8;
 // diag += candidates inside the energy window, with a valid determinant;
 // *overflow is set when a box holds more than 64 candidates.
 template <int L>
-__global__ void __launch_bounds__(EW_WARPS * 32, 2) k_enum_walk(ChanDev c, StreamDev sd, int64_t item0, int64_t count,
+__global__ void __launch_bounds__(EW_WARPS * 32, 2) k_enum_walk(ChanDev c, StreamDev sd, int64_t item0, int64_t count, int span,
                                                                 unsigned long long* __restrict__ bits,
                                                                 unsigned long long* __restrict__ diag,
                                                                 int* __restrict__ overflow) {
@@ -313,7 +313,7 @@ __global__ void __launch_bounds__(EW_WARPS * 32, 2) k_enum_walk(ChanDev c, Strea
 
     int qn = 0;   // queued candidates (warp-uniform)
     const int64_t n_warps = int64_t(gridDim.x) * EW_WARPS;
-    const int64_t run = int64_t(ST_SPAN) * 32;
+    const int64_t run = int64_t(span) * 32;
     const WalkLeg& ml = sd.leg[L - 1];
     const int64_t it1 = item0 + count;
     for (int64_t rb = item0 + (int64_t(blockIdx.x) * EW_WARPS + warp) * run; rb < it1; rb += n_warps * run) {
@@ -321,7 +321,7 @@ __global__ void __launch_bounds__(EW_WARPS * 32, 2) k_enum_walk(ChanDev c, Strea
         walk_decode<L>(sd, rb + lane, p);
         WalkFront fr;
         bool front_ok = false;
-        for (int st = 0; st < ST_SPAN; ++st) {
+        for (int st = 0; st < span; ++st) {
             const int64_t base = rb + int64_t(st) * 32;
             if (base >= it1) break;
             const int64_t item = base + lane;
@@ -471,22 +471,34 @@ int enumerate_channel(const ChanDev& c, const HostMesh* meshes, const HostBand* 
     const int64_t CH = int64_t(1) << 24;
     const int64_t chunk = total < CH ? total : CH;
     uint32_t *d_counts = nullptr, *d_offsets = nullptr;
-    unsigned long long* d_diag = nullptr;
+    unsigned long long *d_diag = nullptr, *bits = nullptr;
     void* d_tmp = nullptr;
-    size_t tmp_bytes = 0;
+    char* base = nullptr;
+    size_t tmp_bytes = 0, scan_bytes = 0;
     int rc = TB_OK;
     auto fail = [&](int code, const char* what) {
         set_error(std::string("enumerate: ") + what);
         rc = code;
     };
-    if (cudaMalloc(&d_counts, sizeof(uint32_t) * (chunk > 0 ? chunk : 1)) != cudaSuccess ||
-        cudaMalloc(&d_offsets, sizeof(uint32_t) * (chunk > 0 ? chunk : 1)) != cudaSuccess ||
-        cudaMalloc(&d_diag, sizeof(unsigned long long) * 3) != cudaSuccess) {
-        fail(TB_ERR_OOM, "counts allocation failed");
+    // one allocation: a 64-bit word per item (the walk's bits; the other pass
+    // keeps its counts there), the walk's overflow flag, the totals, the offsets
+    // and the scan's scratch
+    const size_t items = size_t(chunk > 0 ? chunk : 1);
+    cub::DeviceScan::ExclusiveSum(nullptr, tmp_bytes, d_counts, d_offsets, int(items), stream);
+    {
+        cub::TransformInputIterator<uint32_t, BitCount, const unsigned long long*> p0(bits, BitCount{});
+        cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, p0, d_offsets, int(items), stream);
     }
-    if (rc == TB_OK) {
-        cub::DeviceScan::ExclusiveSum(nullptr, tmp_bytes, d_counts, d_offsets, int(chunk > 0 ? chunk : 1), stream);
-        if (cudaMalloc(&d_tmp, tmp_bytes) != cudaSuccess) fail(TB_ERR_OOM, "scan scratch allocation failed");
+    tmp_bytes = std::max(tmp_bytes, scan_bytes);
+    const size_t offs = sizeof(unsigned long long) * (items + 4), tmps = (offs + sizeof(uint32_t) * items + 255) / 256 * 256;
+    if (cudaMalloc(&base, tmps + tmp_bytes) != cudaSuccess) {
+        fail(TB_ERR_OOM, "scratch allocation failed");
+    } else {
+        bits = reinterpret_cast<unsigned long long*>(base);
+        d_counts = reinterpret_cast<uint32_t*>(base);
+        d_diag = bits + items + 1;
+        d_offsets = reinterpret_cast<uint32_t*>(base + offs);
+        d_tmp = base + tmps;
     }
     if (rc == TB_OK) cudaMemsetAsync(d_diag, 0, sizeof(unsigned long long) * 3, stream);
     const size_t smem = sizeof(double) * size_t(c.nmc) * c.R;
@@ -516,34 +528,27 @@ int enumerate_channel(const ChanDev& c, const HostMesh* meshes, const HostBand* 
         for (int l = 0; l < TB_MAX_LEGS; ++l) sd.nsec[l] = a.nsec[l];
         sd.n_items = total;
         sd.mc_pre = d_mc_pre;
-        // one bit per candidate of an item, the overflow flag behind them
-        unsigned long long* bits = nullptr;
         int overflow = 0;
-        walked = cudaMalloc(&bits, sizeof(unsigned long long) * size_t(chunk + 1)) == cudaSuccess;
-        if (!walked) cudaGetLastError();   // no room: the other pass
+        walked = true;
         cub::TransformInputIterator<uint32_t, BitCount, const unsigned long long*> pops(bits, BitCount{});
-        void* d_tmp2 = nullptr;
-        size_t tmp2 = 0;
-        if (walked) {
-            cub::DeviceScan::ExclusiveSum(nullptr, tmp2, pops, d_offsets, int(chunk), stream);
-            if (cudaMalloc(&d_tmp2, tmp2) != cudaSuccess) fail(TB_ERR_OOM, "scan scratch allocation failed");
-            cudaMemsetAsync(bits + chunk, 0, sizeof(unsigned long long), stream);
-        }
-        int* d_over = reinterpret_cast<int*>(bits + chunk);
+        cudaMemsetAsync(bits + items, 0, sizeof(unsigned long long), stream);
+        int* d_over = reinterpret_cast<int*>(bits + items);
         for (int64_t s = 0; s < total && walked && rc == TB_OK && !overflow; s += chunk) {
             const int64_t cnt = (total - s) < chunk ? (total - s) : chunk;
-            const int64_t runs = (cnt + ST_SPAN * 32 - 1) / (ST_SPAN * 32);
+            // shorter runs of items where there are few: a warp's run is serial (8x8 e-ph: 170 us a channel at 16)
+            const int span = int(std::max<int64_t>(1, std::min<int64_t>(ST_SPAN, cnt / (32 * 148 * 2 * EW_WARPS))));
+            const int64_t runs = (cnt + span * 32 - 1) / (span * 32);
             const unsigned grid = unsigned(std::min<int64_t>((runs + EW_WARPS - 1) / EW_WARPS, 148 * 2 * 8));
             const unsigned wgrid = unsigned((cnt + 255) / 256);
             const size_t wsmem = smem + 16 + sizeof(float) * 8 * size_t(c.nmc);
             cudaMemsetAsync(bits, 0, sizeof(unsigned long long) * size_t(cnt), stream);
             switch (L) {
-                case 2: k_enum_walk<2><<<grid, EW_WARPS * 32, wsmem, stream>>>(c, sd, s, cnt, bits, d_diag, d_over); break;
-                case 3: k_enum_walk<3><<<grid, EW_WARPS * 32, wsmem, stream>>>(c, sd, s, cnt, bits, d_diag, d_over); break;
-                default: k_enum_walk<4><<<grid, EW_WARPS * 32, wsmem, stream>>>(c, sd, s, cnt, bits, d_diag, d_over); break;
+                case 2: k_enum_walk<2><<<grid, EW_WARPS * 32, wsmem, stream>>>(c, sd, s, cnt, span, bits, d_diag, d_over); break;
+                case 3: k_enum_walk<3><<<grid, EW_WARPS * 32, wsmem, stream>>>(c, sd, s, cnt, span, bits, d_diag, d_over); break;
+                default: k_enum_walk<4><<<grid, EW_WARPS * 32, wsmem, stream>>>(c, sd, s, cnt, span, bits, d_diag, d_over); break;
             }
             if (cudaGetLastError() != cudaSuccess) { fail(TB_ERR_CUDA, "walk launch failed"); break; }
-            cub::DeviceScan::ExclusiveSum(d_tmp2, tmp2, pops, d_offsets, int(cnt), stream);
+            cub::DeviceScan::ExclusiveSum(d_tmp, tmp_bytes, pops, d_offsets, int(cnt), stream);
             uint32_t last = 0;
             unsigned long long last_bits = 0;
             cudaMemcpyAsync(&last, d_offsets + cnt - 1, sizeof(last), cudaMemcpyDeviceToHost, stream);
@@ -564,8 +569,6 @@ int enumerate_channel(const ChanDev& c, const HostMesh* meshes, const HostBand* 
             n += int64_t(add);
         }
         if (rc == TB_OK && walked && cudaStreamSynchronize(stream) != cudaSuccess) fail(TB_ERR_CUDA, "write pass failed");
-        cudaFree(bits);
-        cudaFree(d_tmp2);
         if (overflow && rc == TB_OK) {   // a box beyond the bits: from the start with the other pass
             walked = false;
             n = 0;
@@ -611,10 +614,7 @@ int enumerate_channel(const ChanDev& c, const HostMesh* meshes, const HostBand* 
         diag[0] = int64_t(h[0]); diag[1] = int64_t(h[1]); diag[2] = int64_t(h[2]);
         outT.n = n;
     }
-    cudaFree(d_counts);
-    cudaFree(d_offsets);
-    cudaFree(d_diag);
-    cudaFree(d_tmp);
+    cudaFree(base);
     return rc;
 }
 
