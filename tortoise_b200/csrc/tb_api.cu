@@ -688,6 +688,8 @@ void release_row_sets(tb_handle* h) {
 }
 
 int refresh_row_sets(tb_handle* h) {
+    // a captured attempt holds the sets' addresses
+    if (h->graph) { cudaGraphExecDestroy(h->graph); h->graph = nullptr; }
     release_row_sets(h);
     int slots = 0;
     for (auto& G : h->groups) {
@@ -788,9 +790,13 @@ int build_run_states(tb_handle* h) {
 // fewer accumulators than it would take alone: those of the handle's sets.)
 static int row_one(tb_handle* h, GroupChan& G) {
     if (G.row_one.nblocks > 0) return TB_OK;
-    TB_TRY(build_row_set(G.L, row_form(G.dev), {row_chan(G)}, {&G.rows}, h->ndofs, G.row_one));
+    // the caller may be capturing the handle's stream; the copy is on another
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    TB_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
+    const int rc = build_row_set(G.L, row_form(G.dev), {row_chan(G)}, {&G.rows}, h->ndofs, G.row_one);
+    TB_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
     G.row_one.copies = std::min(G.row_one.copies, h->n_accr + 1);
-    return TB_OK;
+    return rc;
 }
 
 static RowArgs row_args(tb_handle* h, const double* f, double* acc, const DPCtl* ctl) {
