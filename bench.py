@@ -218,6 +218,38 @@ def moment_bytes(L, layout):
             "t48": 4 * (nm + (nm + 1) // 2)}.get(layout, 0)
 
 
+def over_rows(eng, ch):
+    """Whether a stored channel is evaluated over packed rows of the tuples
+    with points inside the simplices (tb_channel_schedule: pair 6)."""
+    sc = eng.schedule(ch)
+    return bool(sc.get("inside_only")) and not sc.get("streamed")
+
+
+def row_bytes(L):
+    """Bytes of one tuple in a packed row (tb_rows.cu): the affine map of the
+    three constrained coordinates, the weight, the mask of points inside and
+    the element ids of all legs but the first."""
+    R = 2 * (L - 2) + 1
+    return 8 * (3 * (R + 1) + 2) + 4 * (L - 1)
+
+
+def channel_bytes(eng, ch, L, info):
+    """Algorithmic bytes of one channel's collision evaluation."""
+    if over_rows(eng, ch):
+        return eng.points_inside(ch)[0] * row_bytes(L)
+    return info["n_tuples"] * (moment_bytes(L, info["layout"]) + 4 * (L + 1))
+
+
+def row_fp64_instructions(L, tuples, points):
+    """FP64-pipe instructions of an evaluation over rows (row_tuple,
+    tb_rows.cu): per point the legs' forms as affine functions of the point
+    (2 (L - 2) + 2 R), 1 + s t (L), the two products and their difference
+    (2 L - 2) and the sums (1 + R); per tuple the forms' coefficients
+    (3 R + 3) and the moments (4 R + 8)."""
+    R = 2 * (L - 2) + 1
+    return points * (2 * (L - 2) + 2 * R + L + 2 * L - 2 + 1 + R) + tuples * (7 * R + 11)
+
+
 def mixed_flag(args):
     return {None: 0, "t32": 1, "t40": 2, "t48": 3}[args.mixed]
 
@@ -261,10 +293,8 @@ def ours(args, world, rank, local, pg):
     ev1.synchronize()
     t_coll = ev0.elapsed_time(ev1) * 1e-3 / reps
     bytes_coll = 0
-    for c, inf in zip(mat.channels, infos):
-        L, n = c.nlegs, inf["n_tuples"]
-        bytes_coll += n * moment_bytes(L, inf["layout"])
-        bytes_coll += n * 4 * (L + 1)
+    for ch, (c, inf) in enumerate(zip(mat.channels, infos)):
+        bytes_coll += channel_bytes(eng, ch, c.nlegs, inf)
     bytes_coll += eng.ndofs * 8 * 3   # f read once, accumulator read + written once
     hbm, peak_kind = peaks()
     achieved = bytes_coll / t_coll / 1e9
@@ -289,8 +319,11 @@ def ours(args, world, rank, local, pg):
     t_max = reduce_max(pg, t_dev, dev)
     value = args.steps / t_max if args.shard else aggregate_rate(world, args.steps, t_max)
     drift_launch = 1 if any(b.drift_velocity != (0.0, 0.0) for b in mat.bands) else 0
-    active = sum(1 for c, i in zip(mat.channels, infos) if c.amplitude != 0 and i["n_tuples"] > 0)
-    launches = args.steps * (7 + 6 * (active + drift_launch) + 3)
+    on = [ch for ch, (c, i) in enumerate(zip(mat.channels, infos)) if c.amplitude != 0 and i["n_tuples"] > 0]
+    rows = [ch for ch in on if over_rows(eng, ch)]
+    # all channels over rows: one launch, after one that pads the state and adds the drift
+    per_rhs = len(on) - len(rows) + (2 if rows else 0) + (0 if rows and not args.shard else drift_launch)
+    launches = args.steps * (7 + 6 * per_rhs + 3)
 
     # ---- end to end through the C ABI with host buffers ------------------
     # tb_dp45_integrate from host memory to host memory (k1 evaluation, graph
@@ -330,7 +363,7 @@ def ours(args, world, rank, local, pg):
     if os.path.exists(tp):
         d = json.load(open(tp))
         key = infos[0]["layout"]
-        if key in d and d[key].get("bytes_per_tuple"):
+        if not rows and key in d and d[key].get("bytes_per_tuple"):
             traffic = d[key]["bytes_per_tuple"] * ntup
     line = {"metric": METRIC, "value": value, "unit": "DP45 steps/s", "n_gpus": world, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": 1e3 * t_max / args.steps, "higher_is_better": True,
@@ -343,10 +376,11 @@ def ours(args, world, rank, local, pg):
                               if args.shard else {})),
             "kernels": {"layouts": [i["layout"] for i in infos],
                         "schedules": [eng.schedule(c) for c in range(nch)],
-                        "l2": "moment tensors (%.1f GB) exceed L2; no flush" % (bytes_coll / 1e9)},
+                        "l2": "packed rows / moment tensors (%.1f GB) exceed L2; no flush" % (bytes_coll / 1e9)},
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s",
                          "frac": achieved / hbm, "traffic": traffic,
-                         "kernel": "collision contraction, all channels, per RHS evaluation",
+                         "kernel": ("collision over packed rows" if rows else "collision contraction")
+                                   + ", all channels, per RHS evaluation",
                          "algorithmic_bytes": bytes_coll, "seconds_per_launch": t_coll,
                          "peak_source": peak_kind},
             "cpu_baseline": cpu,
@@ -491,18 +525,19 @@ def batched_measure(n_runs, steps, warmup, mixed, layout_name="auto", tune=True)
     ndofs = be.ndofs
     # FP64 roofline of the collision: every (tuple, run) pair of a shared
     # group is one contraction of FP64_INSTR[L] FP64-pipe instructions
-    run_tuples = {}
+    run_tuples, instr = {}, 0
     for r, m in enumerate(mats):
         for k, ch in enumerate(m.channels):
             if ch.amplitude != 0:
-                L = ch.nlegs
-                run_tuples[L] = run_tuples.get(L, 0) + be.channel_info(be.chan0[r] + k)["n_tuples"]
+                L, c = ch.nlegs, be.chan0[r] + k
+                n = be.channel_info(c)["n_tuples"]
+                run_tuples[L] = run_tuples.get(L, 0) + n
+                instr += row_fp64_instructions(L, *be.points_inside(c)) if over_rows(be, c) else n * FP64_INSTR[L]
     be.close()
-    instr = sum(n * FP64_INSTR[L] for L, n in run_tuples.items())
     fma_rate = E.fp64_fma_rate(0)
     roof64 = {"bound": "fp64", "achieved": instr / t_coll / 1e12, "peak": fma_rate / 1e12,
               "unit": "T FP64-pipe instructions/s", "frac": instr / t_coll / fma_rate,
-              "run_tuples": run_tuples, "instructions_per_run_tuple": {L: FP64_INSTR[L] for L in run_tuples},
+              "run_tuples": run_tuples, "instructions": instr,
               "peak_source": "measured in this run: tb_fp64_fma_rate (register-resident DFMA chains on every SM, "
                              "CUDA events)",
               "floor_ms": 1e3 * instr / fma_rate}
@@ -660,8 +695,8 @@ def mixed_measure(eng64, mat, f0, steps, warmup, dev):
     ev1.record(stream)
     ev1.synchronize()
     t_coll = ev0.elapsed_time(ev1) * 1e-3 / 20
-    bytes_coll = sum(i["n_tuples"] * (moment_bytes(c.nlegs, i["layout"]) + 4 * (c.nlegs + 1))
-                     for c, i in zip(mat.channels, infos)) + eng.ndofs * 8 * 3
+    bytes_coll = sum(channel_bytes(eng, ch, c.nlegs, i)
+                     for ch, (c, i) in enumerate(zip(mat.channels, infos))) + eng.ndofs * 8 * 3
     eng.dp45_begin(f0, 0.0, 1.0e9, DENSE, 0)
     eng.dp45_advance(warmup)
     eng.synchronize()
