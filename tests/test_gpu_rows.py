@@ -111,6 +111,26 @@ def test_shared_rows_of_a_batch(gpu_lib, shape, runs):
         be.close()
 
 
+@pytest.mark.parametrize("runs", [7, 9, 47, 48, 65])
+def test_three_and_four_legs_of_a_batch_choose_by_themselves(gpu_lib, runs):
+    """Three legs go run-minor from 8 runs, four legs (small channels) from 48: none, one and both kinds."""
+    def make(r):
+        m = _material(amp=0.5 + 0.01 * r, **dict(SHAPES["in_in_out"], nsplit=(3, 2)))
+        for c in m.addScatteringChannelsWildcards(["el:P"] * 4, [IN, IN, OUT, OUT], 0):
+            c.amplitude = 0.3 + 0.01 * r
+        return m
+    mats = [make(r) for r in range(runs)]
+    states = [W.initial_status(m, kT=0.05 + 0.005 * r, seed=r).vec for r, m in enumerate(mats)]
+    be = E.BatchEngine(mats)
+    try:
+        f = np.concatenate(states)
+        for call in ("rhs", "scattering_rates", "rhs"):
+            for m, x, g in zip(mats, states, be.split(getattr(be, call)(f))):
+                assert rel_l2(g, getattr(oracle.Oracle(m), call)(x)) < TOL
+    finally:
+        be.close()
+
+
 def test_amplitude_factors_and_pinned_schedules(gpu_lib):
     """functAmplitude through the rows; then a contraction schedule, whose tensor is built on request, and back."""
     mat = _material(**SHAPES["in_in_out"])

@@ -131,7 +131,7 @@ static int adj_base(tb_handle* h) {
     for (size_t gi = 0; gi < h->groups.size(); ++gi)
         A->gamp_off[gi + 1] = A->gamp_off[gi] + int(h->groups[gi].insts.size());
     A->n_slots = A->gamp_off.back();
-    A->gamp = adj_alloc(A, size_t(std::max(A->n_slots, 1)));
+    A->gamp = adj_alloc(A, size_t(A->n_slots + 1));   // and the status words, to leave in one copy
     if (h->opts.deterministic) {
         // 3 words per slot and the poison word, in double-sized units
         double* p3 = adj_alloc(A, size_t(3 * std::max(A->n_slots, 1) + 1));
@@ -419,19 +419,22 @@ static int vjp_at(tb_handle* h, const double* Y, int flags) {
     return TB_OK;
 }
 
+// The amplitude gradients, and what the kernels flagged, in one copy.
 static int copy_gamp_out(tb_handle* h, double* grad_amp) {
     AdjointState* A = h->adj;
     TB_TRY(launch_fx_flush(A->gamp_fx, A->gamp, A->n_slots, h->stream));   // deterministic mode
     TB_TRY(shard_allreduce(h, A->gamp, size_t(A->n_slots)));   // sharded: all ranks' partial sums
-    std::vector<double> slots(size_t(std::max(A->n_slots, 1)));
-    TB_CUDA(cudaMemcpyAsync(slots.data(), A->gamp, sizeof(double) * size_t(A->n_slots), cudaMemcpyDeviceToHost,
-                            h->stream));
+    if (h->comm) TB_TRY(stream_wait(h));   // bounded, unlike the copy below
+    std::vector<double> slots(size_t(A->n_slots + 1));
+    TB_CUDA(cudaMemcpyAsync(A->gamp + A->n_slots, h->d_err, sizeof(double), cudaMemcpyDeviceToDevice, h->stream));
+    TB_CUDA(cudaMemcpyAsync(slots.data(), A->gamp, sizeof(double) * slots.size(), cudaMemcpyDeviceToHost, h->stream));
     TB_TRY(stream_wait(h));
+    std::memcpy(h->h_status, &slots[size_t(A->n_slots)], 2 * sizeof(int));
     for (size_t c = 0; c < h->insts.size(); ++c) {
         const ChanInst& I = h->insts[c];
         grad_amp[c] = slots[size_t(A->gamp_off[I.group] + I.slot)];
     }
-    return TB_OK;
+    return status_error(h);
 }
 
 }  // namespace tb
@@ -464,8 +467,7 @@ int tb_adjoint_rhs_vjp(tb_handle* h, const double* f, const double* theta, doubl
     if (flags & TB_PTR_HOST) TB_CUDA(cudaMemcpyAsync(grad_f, A->g, bytes, cudaMemcpyDeviceToHost, h->stream));
     else TB_CUDA(cudaMemcpyAsync(grad_f, A->g, bytes, cudaMemcpyDeviceToDevice, h->stream));
     TB_CUDA(cudaMemsetAsync(A->g, 0, bytes, h->stream));
-    if (grad_amp) TB_TRY(copy_gamp_out(h, grad_amp));
-    return check_status(h);
+    return grad_amp ? copy_gamp_out(h, grad_amp) : check_status(h);
 }
 
 int tb_dp45_replay(tb_handle* h, const double* f0, const double* dts, int64_t n_steps, double dense_s, double* f_out,
@@ -662,8 +664,7 @@ int tb_adjoint_backward(tb_handle* h, const double* lambda_T, double* grad_f0, d
         TB_CUDA(cudaGetLastError());
         if (flags & TB_PTR_HOST) TB_CUDA(cudaMemcpyAsync(grad_f0, out, bytes, cudaMemcpyDeviceToHost, h->stream));
     }
-    if (grad_amp) TB_TRY(copy_gamp_out(h, grad_amp));
-    TB_TRY(check_status(h));
+    TB_TRY(grad_amp ? copy_gamp_out(h, grad_amp) : check_status(h));
     if (st) {
         std::memset(st, 0, sizeof(*st));
         st->t_obs = A->t_obs;

@@ -623,6 +623,21 @@ static int launch_group_mc(tb_handle* h, GroupChan& G, const InstDev* insts, int
 // 16 runs 942, 48 runs 2221, against 344, 326, 536 and 1488 over rows.
 constexpr int ROWS_RUN_MINOR = 8;
 
+// Four legs spread more adds over fewer rows, so run-minor groups pay off later
+// (e-e, us, one by one / run-minor: 6x6 16 runs 248 / 382, 40 runs 612 / 764,
+// 48 runs 748 / 605; 8x8 16 runs 825 / 1296, 32 runs 1661 / 1885, 48 runs 2488 /
+// 2092; 9x9, 2.2 million tuples, 24 runs 2170 / 2844, 32 runs 2898 / 1933; 12x12
+// 16 runs 5900 / 6936, 32 runs 12078 / 8131).
+constexpr int ROWS_RUN_MINOR_4 = 48;
+constexpr int ROWS_RUN_MINOR_4_LARGE = 32;
+constexpr int64_t ROWS_LARGE_4 = 2000000;
+
+static bool rows_run_minor(const GroupChan& G) {
+    const int n = int(G.insts.size());
+    if (!G.use_rows || G.L <= 3) return G.use_rows && n >= ROWS_RUN_MINOR;
+    return n >= (G.rows.n >= ROWS_LARGE_4 ? ROWS_RUN_MINOR_4_LARGE : ROWS_RUN_MINOR_4);
+}
+
 static RowChan row_chan(const GroupChan& G) {
     RowChan c{};
     c.blk = G.rows.blk;
@@ -721,14 +736,14 @@ int refresh_row_sets(tb_handle* h) {
     return TB_OK;
 }
 
-// Run-minor states for the structures that ROWS_RUN_MINOR runs or more share
-// (each once, for all its channels over rows).  A structure that does not fit
+// Run-minor states for the structures with channels that enough runs share
+// (each once, for all its channels that go run-minor).  A structure that does not fit
 // stays with the rows one run after another.
 int build_run_states(tb_handle* h) {
     if (h->opts.deterministic) return TB_OK;
     int tiles = 0;
     for (auto& G : h->groups) {
-        if (!G.use_rows || int(G.insts.size()) < ROWS_RUN_MINOR || G.run_state >= 0) continue;
+        if (!rows_run_minor(G) || G.run_state >= 0) continue;
         std::vector<int> run;
         std::vector<int64_t> off;
         for (int id : G.insts) {
@@ -764,7 +779,7 @@ int build_run_states(tb_handle* h) {
         tiles += int((st.ndof + 31) / 32) * st.tiles_i;
         // every channel of the structure: the same runs
         for (auto& H : h->groups)
-            if (H.use_rows && H.insts.size() == G.insts.size() && h->insts[H.insts[0]].run == run[0])
+            if (rows_run_minor(H) && H.insts.size() == G.insts.size() && h->insts[H.insts[0]].run == run[0])
                 H.run_state = int(h->run_states.size());
         h->run_states.push_back(st);
     }
@@ -1157,7 +1172,7 @@ namespace tb {
 // TB_ERR_TIMEOUT when a bounded wait for staged data ran out since the last
 // check (the kernels that gave up left their part of the sum out).  The words
 // are in h_status.
-static int status_error(tb_handle* h) {
+int status_error(tb_handle* h) {
     if (h->h_status[0]) {
         TB_CUDA(cudaMemsetAsync(h->d_err, 0, sizeof(int), h->stream));
         set_error("a moment-tensor contraction gave up waiting for its staged tiles; the result is incomplete");
@@ -1171,9 +1186,9 @@ static int status_error(tb_handle* h) {
 }
 
 int check_status(tb_handle* h) {
-    TB_TRY(stream_wait(h));
+    if (h->comm) TB_TRY(stream_wait(h));   // bounded, unlike the copy below
     TB_CUDA(cudaMemcpyAsync(h->h_status, h->d_err, 2 * sizeof(int), cudaMemcpyDeviceToHost, h->stream));
-    TB_CUDA(cudaStreamSynchronize(h->stream));
+    TB_TRY(stream_wait(h));
     return status_error(h);
 }
 

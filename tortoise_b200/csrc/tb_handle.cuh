@@ -171,6 +171,7 @@ void adjoint_release(tb_handle* h);
 int fx_alloc(tb_handle* h, int64_t n, FxAcc& out);
 // Reads the status words (waits for the stream); clears what is set and returns
 // the error it stands for.
+int status_error(tb_handle* h);   // of the words in h_status
 int check_status(tb_handle* h);
 // the error that the deterministic mode's clamp flag reports
 int fx_saturation_error();
