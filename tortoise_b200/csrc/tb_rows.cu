@@ -6,8 +6,8 @@
 // life of a handle.  A row keeps, for 32 tuples that share their leg-0 element,
 // the affine map of the constrained coordinates, the weight and the mask of
 // points inside, so an evaluation reads 120 bytes per three-leg tuple (172 with
-// four legs), in whole lines, instead of the 864 bytes of its moments or the element tables of
-// three legs.
+// four legs), in whole lines, instead of the 864 bytes of its moments or the
+// element tables of three legs.
 //
 //   * One warp takes consecutive rows, one lane per tuple.  Rows of one leg-0
 //     element follow one another and their tuples are sorted by point count,
@@ -28,10 +28,10 @@
 //   * All channels of a handle run in one launch; blocks are dealt out by cost.
 //
 // Measured (64x64 two-band e-ph, 8.7 M tuples, 50 M points, whole right-hand
-// side): 333 us against 1589 us through the FP64 moment tensor; three bands and
-// two phonons at 72x56: 689 against 3283 us; the rates of every leg at 40x24
-// with umklapp: 203 against 1797 us; 16x16 e-e (40.8 M tuples of 172 bytes, 156 M
-// points): 1.58 ms against 3.58 ms of the list kernel (k_collision_mc), of which
+// side): 306-328 us against 1516-1596 us through the FP64 moment tensor; three bands and
+// two phonons at 72x56: 640 against 3128 us; the rates of every leg at 40x24
+// with umklapp: 178 against 1792 us; 16x16 e-e (40.8 M tuples of 172 bytes, 156 M
+// points): 1.56 ms against 3.58 ms of the list kernel (k_collision_mc), of which
 // the adds take 0.2 and the reads could take 1.07 at the copy rate; an 8x8 e-e
 // integration 21 against 32 ms.  The 64x64 kernel reads 3.4 TB/s and issues half
 // of the time, with 27 % of the FP64 pipe: fixed-latency dependencies of the
