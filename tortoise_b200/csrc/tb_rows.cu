@@ -942,7 +942,8 @@ __global__ void __launch_bounds__(RowCap<L, MODE>::W * 32, 1) k_rows(const RowCh
 // acc += the further accumulators, which are cleared.  A latency chain on the
 // small meshes that have them: FOLD_LOADS loads of a thread are in flight before
 // the first is cleared, and a block's 32 warps cover up to 160 accumulators at
-// once (147 of 96 dofs: 7.9 us with 8 warps and one load at a time, 4.4 now).
+// once (147 of 96 dofs: 7.9 us with 8 warps and one load at a time, 4.4 now; a
+// 5x5 e-e right-hand side 32.8 us and 28.7, an 8x8 integration 21.0 ms and 20.6).
 constexpr int FOLD_LOADS = 5;
 __global__ void __launch_bounds__(1024) k_rows_fold(double* __restrict__ acc, double* __restrict__ accr, int n,
                                                     int64_t ndofs) {
