@@ -981,6 +981,9 @@ int autotune(tb_handle* h) {
         TB_TRY(tune_tensor(G.dev, G.d_insts, int(G.insts.size()), G.tensor, G.tup.d, G.tup.cap, G.tup.n, h->d_f,
                            h->d_acc, h->stream));
     }
+    // what the timed launches added, also to the deterministic mode's exact sums
+    TB_TRY(launch_fx_flush(h->fx, h->d_acc, h->ndofs, h->stream));
+    if (h->fx.sat) TB_CUDA(cudaMemsetAsync(h->fx.sat, 0, sizeof(unsigned int), h->stream));
     TB_CUDA(cudaMemsetAsync(h->d_acc, 0, sizeof(double) * n, h->stream));
     TB_CUDA(cudaStreamSynchronize(h->stream));
     return refresh_row_sets(h);
