@@ -158,7 +158,11 @@ typedef struct tb_options {
                                      atomics) that are rounded to FP64 once per evaluation,
                                      instead of FP64 atomics, so a result depends on the
                                      per-tuple values only -- not on thread arrival order,
-                                     launch geometry or the contraction schedule.  Slower;
+                                     launch geometry, the number of runs in the handle,
+                                     autotune or the contraction schedule.  (Packed rows and
+                                     a moment tensor round a tuple's value differently: a
+                                     channel moved from one to the other by
+                                     tb_set_channel_schedule changes in the last bits.)  Slower;
                                      24 more bytes of device memory per dof (and per slot of
                                      a run-minor group's accumulator).  A non-finite
                                      contribution makes the whole evaluation NaN; a finite one
@@ -371,10 +375,10 @@ int tb_read_scatt_indices(const char* path, int nlegs, const int32_t* nsplit, in
  * creation when the channel has at most 64 Monte-Carlo points; same sums as
  * the full quadrature for finite f), else 0 (every point of every tuple).
  * FP64 channels that TB_LAYOUT_AUTO resolved (2 or 3 legs, at most 64
- * points; in the deterministic mode shared by fewer than 16 runs) report TB_LAYOUT_T64 and stages 0,
- * pair 6 too: they are evaluated over packed rows of the same tuples and
- * points, and their moment tensor is built only when a contraction schedule is
- * pinned, or by tb_options.autotune, which keeps the faster of the two.
+ * points) report TB_LAYOUT_T64 and stages 0, pair 6 too: they are evaluated
+ * over packed rows of the same tuples and points, and their moment tensor is
+ * built only when a contraction schedule is pinned, or by tb_options.autotune,
+ * which keeps the faster of the two (the rows in the deterministic mode).
  * No counterpart in the reference. */
 int tb_channel_schedule(const tb_handle* h, int ch, int32_t* stages, int32_t* pair, double* seconds);
 

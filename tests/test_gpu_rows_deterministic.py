@@ -3,6 +3,7 @@ could change what a call returns."""
 import numpy as np
 import pytest
 
+import oracle
 from conftest import rel_l2
 from tortoise_b200 import engine as E
 from tortoise_b200 import workloads as W
@@ -29,3 +30,34 @@ def test_autotuned_handle_starts_from_empty_sums(gpu_lib, runs, call):
         finally:
             e.close()
     assert rel_l2(got[1], got[0]) < TOL
+
+
+@pytest.mark.parametrize("runs", [2, 15, 16, 40])
+def test_a_run_has_the_same_bits_alone_and_in_a_batch(gpu_lib, runs):
+    """AUTO's arithmetic depends neither on the number of runs nor on what autotune timed."""
+    mats, f = _runs(runs, Ns=(4, 5))
+    th = np.random.default_rng(5).standard_normal(f.size)
+
+    def calls(e, f, th):
+        d = e.dp45(f, 0.0, 0.1, 0.05)
+        return e.rhs(f), e.scattering_rates(f), e.rhs_vjp(f, th)[0], d["y"]
+
+    be = E.BatchEngine(mats, deterministic=True)
+    tuned = E.BatchEngine(mats, deterministic=True, autotune=True)
+    try:
+        got = calls(be, f, th)
+        for a, b in zip(got, calls(tuned, f, th)):
+            assert np.array_equal(a, b)
+        for r in (0, 1, runs - 1):
+            s = be.slices[r]
+            for tune in (False, True):
+                one = E.Engine(mats[r], deterministic=True, autotune=tune)
+                try:
+                    for a, b in zip(got, calls(one, f[s], th[s])):
+                        assert np.array_equal(a[s], b)
+                finally:
+                    one.close()
+            assert rel_l2(got[0][s], oracle.Oracle(mats[r]).rhs(f[s])) < TOL
+    finally:
+        be.close()
+        tuned.close()

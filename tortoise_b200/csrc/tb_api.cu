@@ -933,11 +933,17 @@ int run_rhs_acc(tb_handle* h, const double* d_in, double* d_acc, const DPCtl* ct
 // the values) and keeps the fastest (tune_tensor).  The accumulator is
 // cleared afterwards.
 static int tune_rows(tb_handle* h, GroupChan& G) {
-    const int rc = ensure_tensor(h, G);
-    if (rc == TB_ERR_OOM) return TB_OK;   // no room for the tensor: the rows stay
-    TB_TRY(rc);
-    TB_TRY(tune_tensor(G.dev, G.d_insts, int(G.insts.size()), G.tensor, G.tup.d, G.tup.cap, G.tup.n, h->d_f, h->d_acc,
-                       h->stream));
+    // the deterministic mode's bits must not depend on a timing: its channels
+    // stay with the rows (their quadrature and the moments' contraction round
+    // differently), whose time is only recorded
+    const bool choose = !h->opts.deterministic;
+    if (choose) {
+        const int rc = ensure_tensor(h, G);
+        if (rc == TB_ERR_OOM) return TB_OK;   // no room for the tensor: the rows stay
+        TB_TRY(rc);
+        TB_TRY(tune_tensor(G.dev, G.d_insts, int(G.insts.size()), G.tensor, G.tup.d, G.tup.cap, G.tup.n, h->d_f,
+                           h->d_acc, h->stream));
+    }
     cudaEvent_t e0, e1;
     TB_CUDA(cudaEventCreate(&e0));
     TB_CUDA(cudaEventCreate(&e1));
@@ -963,6 +969,7 @@ static int tune_rows(tb_handle* h, GroupChan& G) {
     cudaEventDestroy(e1);
     for (auto& rs : set) rs.release();
     G.rows_seconds = 1e-3 * double(ms) / REPS;
+    if (!choose) return TB_OK;
     if (G.rows_seconds <= G.tensor.tuned_seconds) G.tensor.release();
     else G.use_rows = false;
     return TB_OK;
@@ -1003,10 +1010,6 @@ int ensure_tensor(tb_handle* h, GroupChan& G) {
     return build_group_tensor(h, G, TK_F64);
 }
 
-// The deterministic mode has no run-minor rows: channels that this many runs
-// share stay with the run-minor contraction there.
-constexpr int ROWS_MAX_EXACT = 16;
-
 int choose_layouts(tb_handle* h) {
     size_t freeb = 0, totalb = 0;
     cudaMemGetInfo(&freeb, &totalb);
@@ -1041,8 +1044,7 @@ int choose_layouts(tb_handle* h) {
             const int64_t room = int64_t(double(freeb) * 0.6);   // as for a tensor
             // AUTO's FP64 channels go over their packed rows; the tensor is
             // built when a contraction schedule is asked for
-            if (h->opts.layout == TB_LAYOUT_AUTO && want == TB_LAYOUT_T64  &&
-                !(h->opts.deterministic && int(G.insts.size()) >= ROWS_MAX_EXACT)) {
+            if (h->opts.layout == TB_LAYOUT_AUTO && want == TB_LAYOUT_T64) {
                 TB_TRY(build_theta_list(G.dev, G.tup, G.theta, h->stream));
                 if (G.theta.built) TB_TRY(build_rows(G.dev, G.theta, G.rows, room, h->stream));
                 G.use_rows = G.rows.blk != nullptr;
