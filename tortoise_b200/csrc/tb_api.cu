@@ -808,7 +808,7 @@ static int row_one(tb_handle* h, GroupChan& G) {
     // the caller may be capturing the handle's stream; the copy is on another
     cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
     TB_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
-    const int rc = build_row_set(G.L, row_form(G.dev), {row_chan(G)}, {&G.rows}, h->ndofs, G.row_one);
+    const int rc = build_row_set(G.L, row_form(G.dev), {row_chan(G)}, {&G.rows}, h->ndofs, G.row_one, 0, true);
     TB_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
     G.row_one.copies = std::min(G.row_one.copies, h->n_accr + 1);
     return rc;
@@ -947,9 +947,9 @@ static int tune_rows(tb_handle* h, GroupChan& G) {
     cudaEvent_t e0, e1;
     TB_CUDA(cudaEventCreate(&e0));
     TB_CUDA(cudaEventCreate(&e1));
-    if (G.run_state < 0) TB_TRY(row_one(h, G));
-    std::vector<RowSet> set;   // run-minor: this channel alone, its structure's state gathered and scattered
-    if (G.run_state >= 0) TB_TRY(make_row_sets(h, [&](const GroupChan& B) { return &B == &G; }, true, set));
+    std::vector<RowSet> set;   // this channel alone (run-minor: its structure's state gathered and scattered)
+    TB_TRY(make_row_sets(h, [&](const GroupChan& B) { return &B == &G; }, G.run_state >= 0, set));
+    for (auto& rs : set) rs.copies = std::min(rs.copies, h->n_accr + 1);
     constexpr int REPS = 3;
     for (int r = 0; r <= REPS; ++r) {
         if (r == 1) cudaEventRecord(e0, h->stream);   // after a warm-up launch
@@ -958,7 +958,7 @@ static int tune_rows(tb_handle* h, GroupChan& G) {
                                    h->d_run_nf, h->d_acc, nullptr, h->stream, h->d_err, G.dev.wait_polls));
         } else {
             TB_TRY(launch_rows_prepare(h->ed, h->d_f, h->d_f4, h->d_nf, nullptr, h->stream));
-            TB_TRY(launch_rows(G.row_one, row_args(h, h->d_f, h->d_acc, nullptr), h->stream));
+            for (const RowSet& rs : set) TB_TRY(launch_rows(rs, row_args(h, h->d_f, h->d_acc, nullptr), h->stream));
         }
     }
     cudaEventRecord(e1, h->stream);

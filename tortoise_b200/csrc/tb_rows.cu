@@ -793,8 +793,8 @@ __global__ void __launch_bounds__(RowCap<L, MODE>::W * 32, 1) k_rows(const RowCh
     for (int i = tid; i < int(sizeof(RowChan) / sizeof(int)); i += blockDim.x)
         reinterpret_cast<int*>(&c)[i] = reinterpret_cast<const int*>(chans + w.chan)[i];
     __syncthreads();
-    const InstDev* insts = one ? one : c.insts;
-    const int n_insts = one ? 1 : c.n_insts;
+    const InstDev* insts = one ? one : c.insts + w.i0;
+    const int n_insts = one ? 1 : w.i1 - w.i0;
     if (!VJP) {
         // every instance off or its run finished: nothing to add (an amplitude
         // of 0 still has a gradient)
@@ -828,7 +828,7 @@ __global__ void __launch_bounds__(RowCap<L, MODE>::W * 32, 1) k_rows(const RowCh
     double4 f0 = make_double4(0., 0., 0., 0.), u0 = f0;
     int64_t off[L], el[L];
     double amp = 0.0, ga = 0.0;   // ga: this lane's part of the amplitude gradient
-    if (VJP) gamp += c.gamp0;
+    if (VJP) gamp += c.gamp0 + w.i0;
     if (!MULTI) {
 #pragma unroll
         for (int l = 0; l < L; ++l) { off[l] = insts[0].foff[l]; el[l] = off[l] / 3; }
@@ -1039,27 +1039,39 @@ int launch_rows(const RowSet& rs, const RowArgs& A, cudaStream_t s) {
 }
 
 int build_row_set(int L, int form, const std::vector<RowChan>& chan, const std::vector<const PointRows*>& rows,
-                  int64_t ndofs, RowSet& out, int S) {
+                  int64_t ndofs, RowSet& out, int S, bool whole) {
     out.release();
     out.L = L;
     out.form = form;
     out.S = S;
     out.nmc_max = 0;
     out.multi = false;
-    int64_t nrows = 0;
-    // what blocks are dealt out to: channels, run-minor each chunk of S runs
-    std::vector<std::pair<int, int>> item;   // (channel, chunk)
-    for (size_t i = 0; i < chan.size(); ++i) {
-        const int chunks = S ? (chan[i].n_insts + S - 1) / S : 1;
-        for (int k = 0; k < chunks; ++k) item.emplace_back(int(i), k);
-        nrows += rows[i]->nrows * chunks;
-        out.nmc_max = std::max(out.nmc_max, chan[i].nmc);
-        out.multi = out.multi || chan[i].n_insts > 1;
-    }
-    if (nrows <= 0) return TB_OK;
     int dev = 0, nsm = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    int64_t nrows = 0;
+    for (const PointRows* r : rows) nrows += r->nrows;
+    if (nrows <= 0) return TB_OK;
+    // a warp takes the instances of a row one after another; where the rows do
+    // not fill the chip's warps, parts of the instances go to blocks of their
+    // own.  Deterministic 8x8 e-ph right-hand sides, us, without and with: 16 runs
+    // 361 / 160, 48 runs 1037 / 368, 128 runs 2732 / 953 (the run-minor
+    // contraction of exact sums took 243, 587 and 1370); FP64 atomics, 7 runs
+    // 55 / 35; from 16x16 on the rows fill the chip.
+    const int64_t parts = whole ? 1 : std::max<int64_t>(1, int64_t(nsm) * row_shares(L) / nrows);
+    nrows = 0;
+    // what blocks are dealt out to: (channel, part of its instances)
+    struct Item { int chan, chunk, i0, i1; };
+    std::vector<Item> item;
+    for (size_t i = 0; i < chan.size(); ++i) {
+        const int n = chan[i].n_insts;
+        const int chunks = S ? (n + S - 1) / S : int(std::min<int64_t>(n, parts));
+        for (int k = 0; k < chunks; ++k)
+            item.push_back({int(i), k, int(int64_t(n) * k / chunks), int(int64_t(n) * (k + 1) / chunks)});
+        nrows += rows[i]->nrows * chunks;
+        out.nmc_max = std::max(out.nmc_max, chan[i].nmc);
+        out.multi = out.multi || n > 1;
+    }
     // one block per SM; fewer warps in each where there are fewer rows than
     // warps.  Every item gets a block of its own at least, the others go one
     // by one to the item with the largest cost per block.
@@ -1068,10 +1080,12 @@ int build_row_set(int L, int form, const std::vector<RowChan>& chan, const std::
     out.shares[1] = int(std::min<int64_t>(row_shares_few(L), per_sm));
     std::vector<int64_t> nb(item.size(), 1);
     auto cost_of = [&](size_t i) -> const std::vector<int64_t>& {
-        const PointRows& r = *rows[size_t(item[i].first)];
+        const PointRows& r = *rows[size_t(item[i].chan)];
         return S ? r.run_cost : r.cost;
     };
-    auto load = [&](size_t i) { return double(cost_of(i).back()) / double(nb[i]); };
+    auto load = [&](size_t i) {
+        return double(cost_of(i).back()) * (S ? 1 : item[i].i1 - item[i].i0) / double(nb[i]);
+    };
     for (int64_t left = std::min<int64_t>(nsm, (nrows + out.shares[0] - 1) / out.shares[0]) - int64_t(item.size()); left > 0;
          --left) {
         size_t best = 0;
@@ -1082,12 +1096,14 @@ int build_row_set(int L, int form, const std::vector<RowChan>& chan, const std::
     std::vector<RowWork> work;
     std::vector<int32_t> bounds[2];
     for (size_t i = 0; i < item.size(); ++i) {
-        const RowChan& c = chan[size_t(item[i].first)];
+        const RowChan& c = chan[size_t(item[i].chan)];
         const std::vector<int64_t>& cost = cost_of(i);
         for (int64_t b = 0; b < nb[i]; ++b) {
             RowWork w{};
-            w.chan = item[i].first;
-            w.chunk = item[i].second;
+            w.chan = item[i].chan;
+            w.chunk = item[i].chunk;
+            w.i0 = item[i].i0;
+            w.i1 = item[i].i1;
             w.t0 = c.n * b / nb[i];
             w.t1 = c.n * (b + 1) / nb[i];
             work.push_back(w);

@@ -67,6 +67,7 @@ struct RowChan {
 struct RowWork {
     int chan;
     int chunk;       // run-minor sets: which S runs
+    int i0, i1;      // other sets: instances [i0, i1) of the channel
     int64_t t0, t1;
 };
 
@@ -107,9 +108,10 @@ int rows_lane_group(int n);
 
 // Uploads the set for the given channels (rows of channel i in rows[i]) of a
 // handle with ndofs coefficients;
-// blocks are dealt out by the rows' cost.
+// blocks are dealt out by the rows' cost.  whole: every block takes all
+// instances of its channel (a set that is also launched for one instance).
 int build_row_set(int L, int form, const std::vector<RowChan>& chan, const std::vector<const PointRows*>& rows,
-                  int64_t ndofs, RowSet& out, int S = 0);
+                  int64_t ndofs, RowSet& out, int S = 0, bool whole = false);
 
 // f4[e] = (f0, f1, f2, 0) of every element of the state, u4 of u likewise when
 // it is given; nf[b] != 0 marks an element block with a non-finite coefficient.
