@@ -61,3 +61,28 @@ def test_a_run_has_the_same_bits_alone_and_in_a_batch(gpu_lib, runs):
     finally:
         be.close()
         tuned.close()
+
+
+@pytest.mark.parametrize("where", ["state", "co-state"])
+def test_vjp_non_finite_values_reach_tuples_without_a_point_inside(gpu_lib, where):
+    """A non-finite coefficient of an element that is in no tuple with a point inside: the moments' contraction
+    multiplies its tuples' zero moments by it, and a poisoned exact sum reads NaN everywhere."""
+    mat = W.build_material(5, ("P", "D"), (0.2,), ee=False, eph=True, n_mc=1)
+    f = W.initial_status(mat, seed=2).vec
+    th = np.random.default_rng(3).standard_normal(f.size)
+    rows, tensor = E.Engine(mat, deterministic=True), E.Engine(mat, layout=E.LAYOUT_T64, deterministic=True)
+    try:
+        assert any(rows.schedule(c).get("inside_only") for c in range(len(mat.channels)))
+        some = 0
+        for k in range(1, f.size, 3):
+            a, b = f.copy(), th.copy()
+            (a if where == "state" else b)[k] = np.nan
+            got, ref = rows.rhs_vjp(a, b), tensor.rhs_vjp(a, b)
+            for x, y in zip(got, ref):
+                assert np.array_equal(np.isnan(x), np.isnan(y)), k
+            some += np.isnan(ref[0]).all()
+        assert some
+        assert np.isfinite(rows.rhs_vjp(f, th)[0]).all()   # the poison is gone
+    finally:
+        rows.close()
+        tensor.close()

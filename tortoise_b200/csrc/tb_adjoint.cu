@@ -385,9 +385,10 @@ static int vjp_at(tb_handle* h, const double* Y, int flags) {
     AdjointState* A = h->adj;
     if (!(flags & TB_NO_COLLISIONS)) {
         // channels over rows, except in the deterministic mode (whose bits are
-        // those of the list kernel)
+        // those of the list kernel), where the list leaves out the tuples that
+        // only non-finite coefficients reach
         const bool rows = !h->opts.deterministic;
-        if (rows) TB_TRY(launch_row_vjp(h, Y, A->u, reinterpret_cast<double4*>(A->u4), A->g, A->gamp));
+        TB_TRY(launch_row_vjp(h, Y, A->u, reinterpret_cast<double4*>(A->u4), A->g, A->gamp, A->gamp_fx));
         for (size_t gi = 0; gi < h->groups.size(); ++gi) {
             GroupChan& G = h->groups[gi];
             if ((G.tup.n == 0 && !G.stream) || G.insts.empty() || (rows && G.use_rows)) continue;

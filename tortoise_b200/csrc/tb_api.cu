@@ -864,7 +864,8 @@ static int launch_row_sets(tb_handle* h, const double* d_in, double* d_acc, cons
                            d_acc, ctl, h->stream, h->d_err, a.polls);
 }
 
-int launch_row_vjp(tb_handle* h, const double* f, const double* u, double4* u4, double* grad_f, double* gamp) {
+int launch_row_vjp(tb_handle* h, const double* f, const double* u, double4* u4, double* grad_f, double* gamp,
+                   const FxAcc& gamp_fx) {
     if (h->row_sets.empty() && h->rate_sets.empty()) return TB_OK;
     TB_TRY(launch_rows_prepare(h->ed, f, h->d_f4, h->d_nf, nullptr, h->stream, u, u4));
     RowArgs a = row_args(h, f, grad_f, nullptr);
@@ -872,7 +873,8 @@ int launch_row_vjp(tb_handle* h, const double* f, const double* u, double4* u4, 
     a.u4 = u4;
     a.gamp = gamp;
     for (const auto* sets : {&h->row_sets, &h->rate_sets})
-        for (const RowSet& rs : *sets) TB_TRY(launch_rows(rs, a, h->stream));
+        for (const RowSet& rs : *sets)
+            TB_TRY(h->opts.deterministic ? launch_rows_spread(rs, a, gamp_fx, h->stream) : launch_rows(rs, a, h->stream));
     return TB_OK;
 }
 

@@ -155,8 +155,11 @@ double* dev_alloc(tb_handle* h, size_t n);
 // hold (the stream must be idle).
 int refresh_row_sets(tb_handle* h);
 // grad_f += C'(f)^T u and the amplitude gradients (group-major slots) of the
-// channels over rows; u4: scratch of the state's padded size.
-int launch_row_vjp(tb_handle* h, const double* f, const double* u, double4* u4, double* grad_f, double* gamp);
+// channels over rows; u4: scratch of the state's padded size.  Deterministic
+// handles, whose channels go over the point lists instead (to h->fx and gamp_fx):
+// the part of non-finite coefficients only.
+int launch_row_vjp(tb_handle* h, const double* f, const double* u, double4* u4, double* grad_f, double* gamp,
+                   const FxAcc& gamp_fx);
 // The moment tensor of a channel that was evaluated over rows so far.
 int ensure_tensor(tb_handle* h, GroupChan& G);
 int run_rhs_acc(tb_handle* h, const double* d_in, double* d_acc, const DPCtl* ctl, int flags, int only_inst);

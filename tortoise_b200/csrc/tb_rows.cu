@@ -735,7 +735,7 @@ template <int L>
 __device__ __noinline__ void spread_nonfinite(const RowChan& c, const InstDev* insts, int n_insts, int64_t t0,
                                               int64_t t1, const double* f, double* acc, const DPCtl* ctl, bool rate,
                                               int rate_leg, const FxAcc& fx, const double* u = nullptr,
-                                              double* gamp = nullptr) {
+                                              double* gamp = nullptr, const FxAcc& fx_amp = FxAcc{}) {
     const double nan = __longlong_as_double(0x7ff8000000000000ll);
     for (int64_t i = t0 + threadIdx.x; i < t1; i += blockDim.x) {
         int e[L];
@@ -753,7 +753,8 @@ __device__ __noinline__ void spread_nonfinite(const RowChan& c, const InstDev* i
                 if (u) all = all || !finite3(u + in.foff[l] + 3 * (int64_t)e[l]);
             }
             if (nbad == 0 && !all) continue;
-            if (u) atomicAdd(gamp + k, nan);
+            if (u && fx_amp.w) atomicOr(fx_amp.poison, 1u);
+            else if (u) atomicAdd(gamp + k, nan);
 #pragma unroll
             for (int l = 0; l < L; ++l) {
                 // a leg's rate and derivative do not depend on its own f
@@ -939,6 +940,21 @@ __global__ void __launch_bounds__(RowCap<L, MODE>::W * 32, 1) k_rows(const RowCh
         spread_nonfinite<L>(c, insts, n_insts, w.t0, w.t1, f, acc, ctl, RATE, rate_leg, fx, VJP ? u : nullptr, gamp);
 }
 
+// spread_nonfinite of a transposed evaluation alone, for handles whose
+// transpose is evaluated by another kernel.
+template <int L>
+__global__ void __launch_bounds__(256) k_rows_spread(const RowChan* __restrict__ chans, const RowWork* __restrict__ work,
+                                                     const double* __restrict__ f, const int* __restrict__ nf, int n_nf,
+                                                     FxAcc fx, const double* __restrict__ u, FxAcc fx_amp) {
+    int bad = 0;
+    for (int i = threadIdx.x; i < n_nf; i += blockDim.x) bad |= nf[i];
+    if (!__syncthreads_or(bad)) return;
+    const RowWork w = work[blockIdx.x];
+    const RowChan& c = chans[w.chan];
+    spread_nonfinite<L>(c, c.insts + w.i0, w.i1 - w.i0, w.t0, w.t1, f, nullptr, nullptr, false, -1, fx, u, nullptr,
+                        fx_amp);
+}
+
 // acc += the further accumulators, which are cleared.  A latency chain on the
 // small meshes that have them: FOLD_LOADS loads of a thread are in flight before
 // the first is cleared, and a block's 32 warps cover up to 160 accumulators at
@@ -1036,6 +1052,14 @@ int launch_rows(const RowSet& rs, const RowArgs& A, cudaStream_t s) {
     if (rs.L == 2) return launch_rows_l<2>(rs, A, s);
     if (rs.L == 3) return launch_rows_l<3>(rs, A, s);
     return launch_rows_l<4>(rs, A, s);
+}
+
+int launch_rows_spread(const RowSet& rs, const RowArgs& A, const FxAcc& fx_amp, cudaStream_t s) {
+    if (rs.nblocks <= 0) return TB_OK;
+    auto kern = rs.L == 2 ? k_rows_spread<2> : rs.L == 3 ? k_rows_spread<3> : k_rows_spread<4>;
+    kern<<<unsigned(rs.nblocks), 256, 0, s>>>(rs.d_chan, rs.d_work, A.f, A.nf, A.ed->nblk, A.fx, A.u, fx_amp);
+    TB_CUDA(cudaGetLastError());
+    return TB_OK;
 }
 
 int build_row_set(int L, int form, const std::vector<RowChan>& chan, const std::vector<const PointRows*>& rows,

@@ -144,6 +144,10 @@ struct RowArgs {
 };
 int launch_rows(const RowSet& rs, const RowArgs& a, cudaStream_t s);
 
+// What the tuples without a point inside add to the exact sums of a transposed
+// evaluation (a.u) when a.nf marks non-finite coefficients.
+int launch_rows_spread(const RowSet& rs, const RowArgs& a, const FxAcc& fx_amp, cudaStream_t s);
+
 // The run-minor sets: the structures' states gathered, each set evaluated,
 // their accumulators added to acc and cleared.  st: device copy of the n_st
 // structures (n_tiles tiles in all); nf as above, one flag per tile.
