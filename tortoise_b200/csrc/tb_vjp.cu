@@ -10,6 +10,8 @@
 // Each leg factor of a tuple is affine in its element's 3 coefficients of f
 // (ScatteringChannel.cpp:633-641), so the derivative of the product of L
 // factors is the sum over legs of (other legs' factors) x (that leg's slope).
+#include <algorithm>
+
 #include "tb_dp45.cuh"
 #include "tb_geom.cuh"
 #include "tb_mcpoint.cuh"
@@ -65,7 +67,11 @@ int launch_project(const ElemDev& ed, double* v, cudaStream_t s) {
 // (deterministic handles and channels without packed rows; the others:
 // k_rows, tb_rows.cu)
 // LIST: tup / stride / n describe a ThetaList (tb_theta.cuh) and every tuple
-// visits only the set bits of its mask, the points whose Theta is 1.
+// visits only the set bits of its mask, the points whose Theta is 1.  The
+// grid's y dimension shares out the instances: one after another they are a
+// serial chain where the tuples are few (deterministic gradient of e-ph batches,
+// us: 8x8, 16 runs 945 -> 326; 16x16, 15 runs 1685 -> 1204, through the moment
+// tensor 1525; 32x32, 16 runs 7860 -> 7583).
 template <int L, bool LIST>
 __global__ void __launch_bounds__(128) k_vjp_mc(ChanDev c, const InstDev* __restrict__ insts, int n_insts,
                                                 const int32_t* __restrict__ tup, int64_t stride, int64_t n,
@@ -93,7 +99,7 @@ __global__ void __launch_bounds__(128) k_vjp_mc(ChanDev c, const InstDev* __rest
         // functAmplitude of the tuple
         const double tf = (c.tamp && valid) ? __ldg(c.tamp + (LIST ? int64_t(__ldg(perm + i)) : i)) : 1.0;
         const uint64_t mk0 = (LIST && valid) ? __ldg(reinterpret_cast<const unsigned long long*>(mask) + i) : 0ull;
-        for (int k = 0; k < n_insts; ++k) {
+        for (int k = blockIdx.y; k < n_insts; k += gridDim.y) {
             const InstDev in = insts[k];
             double gA[L][3], gB[L][3], gamp, sa[L], sb[L];
             vjp_point_sums<L, LIST>(c, in, f, u, e, g, Ci, s_mc, mk0, valid, gA, gB, gamp, sa, sb);
@@ -276,7 +282,8 @@ int launch_collision_vjp(const ChanDev& c, const InstDev* insts, int n_insts, in
     if (blocks > 148 * 64) blocks = 148 * 64;
     if (layout == TB_LAYOUT_MC64) {
         const size_t smem = sizeof(double) * size_t(c.nmc) * c.R;
-#define TB_VJP_MC(LL, LS) k_vjp_mc<LL, LS><<<unsigned(blocks), threads, smem, s>>>(c, insts, n_insts, tup, stride, n, \
+        const dim3 grid(unsigned(blocks), unsigned(std::max<int64_t>(1, std::min<int64_t>(n_insts, 148 * 32 / blocks))));
+#define TB_VJP_MC(LL, LS) k_vjp_mc<LL, LS><<<grid, threads, smem, s>>>(c, insts, n_insts, tup, stride, n, \
                                                                                  mask, perm, f, u, grad_f, grad_amp, \
                                                                                  fx, fx_amp)
         const bool list = mask != nullptr;
