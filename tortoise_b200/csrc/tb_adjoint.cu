@@ -136,7 +136,7 @@ static int adj_base(tb_handle* h) {
         // 3 words per slot and the poison word, in double-sized units
         double* p3 = adj_alloc(A, size_t(3 * std::max(A->n_slots, 1) + 1));
         if (p3) {
-            TB_CUDA(cudaMemset(p3, 0, sizeof(double) * size_t(3 * std::max(A->n_slots, 1) + 1)));
+            TB_CUDA(cudaMemsetAsync(p3, 0, sizeof(double) * size_t(3 * std::max(A->n_slots, 1) + 1), h->stream));
             A->gamp_fx.w = reinterpret_cast<unsigned long long*>(p3);
             A->gamp_fx.poison = reinterpret_cast<unsigned int*>(A->gamp_fx.w + 3 * std::max(A->n_slots, 1));
             A->gamp_fx.sat = h->fx.sat;   // one sticky flag per handle
@@ -156,8 +156,8 @@ static int adj_base(tb_handle* h) {
         set_error("adjoint allocation failed");
         return TB_ERR_OOM;
     }
-    TB_CUDA(cudaMemset(A->g, 0, sizeof(double) * n));
-    TB_CUDA(cudaMemcpy(A->dD, A->D, sizeof(double*) * 6, cudaMemcpyHostToDevice));
+    TB_CUDA(cudaMemsetAsync(A->g, 0, sizeof(double) * n, h->stream));
+    TB_CUDA(cudaMemcpyAsync(A->dD, A->D, sizeof(double*) * 6, cudaMemcpyHostToDevice, h->stream));
     return TB_OK;
 }
 

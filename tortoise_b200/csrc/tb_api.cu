@@ -110,6 +110,10 @@ namespace tb {
 // e-ph right-hand side 75 -> 52 us); larger ones go to the caller's memory.
 constexpr size_t HOST_IO_MAX = size_t(256) << 10;
 
+// The handle's stream does not wait for the default stream: device memory is
+// written in the handle's stream order (pageable host memory has been read when
+// such a copy returns).
+
 double* dev_alloc(tb_handle* h, size_t n) {
     double* p = nullptr;
     if (cudaMalloc(&p, sizeof(double) * (n ? n : 1)) != cudaSuccess) return nullptr;
@@ -126,7 +130,7 @@ int fx_alloc(tb_handle* h, int64_t n, FxAcc& out) {
         return TB_ERR_OOM;
     }
     h->dev_raw.push_back(p);
-    TB_CUDA(cudaMemset(p, 0, bytes));
+    TB_CUDA(cudaMemsetAsync(p, 0, bytes, h->stream));
     out.w = static_cast<unsigned long long*>(p);
     // the last word: the poison flag (cleared by every flush), then the
     // sticky saturation flag (cleared by the host when it reports it)
@@ -140,13 +144,13 @@ T* dev_upload_raw(tb_handle* h, const T* src, size_t n) {
     void* p = nullptr;
     if (cudaMalloc(&p, sizeof(T) * (n ? n : 1)) != cudaSuccess) return nullptr;
     h->dev_raw.push_back(p);
-    if (n) cudaMemcpy(p, src, sizeof(T) * n, cudaMemcpyHostToDevice);
+    if (n) cudaMemcpyAsync(p, src, sizeof(T) * n, cudaMemcpyHostToDevice, h->stream);
     return static_cast<T*>(p);
 }
 
 double* dev_upload(tb_handle* h, const std::vector<double>& v) {
     double* p = dev_alloc(h, v.size());
-    if (p && !v.empty()) cudaMemcpy(p, v.data(), sizeof(double) * v.size(), cudaMemcpyHostToDevice);
+    if (p && !v.empty()) cudaMemcpyAsync(p, v.data(), sizeof(double) * v.size(), cudaMemcpyHostToDevice, h->stream);
     return p;
 }
 
@@ -401,7 +405,7 @@ int build_runs(tb_handle* h, const tb_problem_desc* const* descs, int nruns) {
     TB_CUDA(cudaMemsetAsync(h->d_acc, 0, sizeof(double) * size_t(h->ndofs), h->stream));
     if (h->opts.deterministic) TB_TRY(fx_alloc(h, h->ndofs, h->fx));
     h->d_err = reinterpret_cast<int*>(h->d_out + h->ndofs);
-    TB_CUDA(cudaMemset(h->d_err, 0, 2 * sizeof(int)));
+    TB_CUDA(cudaMemsetAsync(h->d_err, 0, 2 * sizeof(int), h->stream));
     if (h->opts.deterministic) h->fx.sat = reinterpret_cast<unsigned int*>(h->d_err + 1);
     {
         const size_t io = sizeof(double) * size_t(h->ndofs) <= HOST_IO_MAX ? size_t(h->ndofs) : 0;
@@ -481,7 +485,8 @@ int build_runs(tb_handle* h, const tb_problem_desc* const* descs, int nruns) {
                         for (int l = 0; l < G.L; ++l) soa[size_t(l) * cd.n_tuples + i] = cd.tuples[i * G.L + l];
                         soa[size_t(G.L) * cd.n_tuples + i] = cd.tuple_umklapp[i];
                     }
-                    TB_CUDA(cudaMemcpy(G.tup.d, soa.data(), sizeof(int32_t) * soa.size(), cudaMemcpyHostToDevice));
+                    TB_CUDA(cudaMemcpyAsync(G.tup.d, soa.data(), sizeof(int32_t) * soa.size(), cudaMemcpyHostToDevice,
+                                            h->stream));
                     G.tup.n = cd.n_tuples;
                     G.diag[0] = G.diag[1] = G.diag[2] = -1;
                 } else if (h->opts.stream_legs >= 2 && G.L >= h->opts.stream_legs) {
@@ -516,7 +521,7 @@ int build_runs(tb_handle* h, const tb_problem_desc* const* descs, int nruns) {
                     }
                     h->dev_raw.push_back(p);
                     sd.counts = static_cast<unsigned long long*>(p);
-                    TB_CUDA(cudaMemset(sd.counts, 0, sizeof(unsigned long long) * 5));
+                    TB_CUDA(cudaMemsetAsync(sd.counts, 0, sizeof(unsigned long long) * 5, h->stream));
                     G.stream = true;
                     G.layout = TB_LAYOUT_STREAM;
                     G.item_begin = 0;
@@ -689,7 +694,7 @@ static int make_row_sets(tb_handle* h, Take take, bool run_minor, std::vector<Ro
             done[b] = true;
         }
         sets.emplace_back();
-        TB_TRY(build_row_set(A.L, row_form(A.dev), chan, rows, h->ndofs, sets.back(), S));
+        TB_TRY(build_row_set(A.L, row_form(A.dev), chan, rows, h->ndofs, sets.back(), h->stream, S));
     }
     return TB_OK;
 }
@@ -730,7 +735,7 @@ int refresh_row_sets(tb_handle* h) {
             h->d_accr = nullptr;
             return TB_OK;
         }
-        TB_CUDA(cudaMemset(h->d_accr, 0, bytes));
+        TB_CUDA(cudaMemsetAsync(h->d_accr, 0, bytes, h->stream));
         h->n_accr = copies - 1;
     }
     return TB_OK;
@@ -766,10 +771,10 @@ int build_run_states(tb_handle* h) {
             continue;
         }
         for (void* q : p) h->run_allocs.push_back(q);
-        TB_CUDA(cudaMemset(p[0], 0, bytes));
-        TB_CUDA(cudaMemset(p[1], 0, bytes));
-        TB_CUDA(cudaMemcpy(p[2], off.data(), sz[2], cudaMemcpyHostToDevice));
-        TB_CUDA(cudaMemcpy(p[3], run.data(), sz[3], cudaMemcpyHostToDevice));
+        TB_CUDA(cudaMemsetAsync(p[0], 0, bytes, h->stream));
+        TB_CUDA(cudaMemsetAsync(p[1], 0, bytes, h->stream));
+        TB_CUDA(cudaMemcpyAsync(p[2], off.data(), sz[2], cudaMemcpyHostToDevice, h->stream));
+        TB_CUDA(cudaMemcpyAsync(p[3], run.data(), sz[3], cudaMemcpyHostToDevice, h->stream));
         st.fT = static_cast<double*>(p[0]);
         st.accT = static_cast<double*>(p[1]);
         st.dof_off = static_cast<const int64_t*>(p[2]);
@@ -794,7 +799,8 @@ int build_run_states(tb_handle* h) {
     }
     h->run_allocs.push_back(ds);
     h->run_allocs.push_back(dn);
-    TB_CUDA(cudaMemcpy(ds, h->run_states.data(), sizeof(RunState) * h->run_states.size(), cudaMemcpyHostToDevice));
+    TB_CUDA(cudaMemcpyAsync(ds, h->run_states.data(), sizeof(RunState) * h->run_states.size(), cudaMemcpyHostToDevice,
+                            h->stream));
     h->d_run_states = static_cast<RunState*>(ds);
     h->d_run_nf = static_cast<int*>(dn);
     h->n_run_tiles = tiles;
@@ -805,10 +811,21 @@ int build_run_states(tb_handle* h) {
 // fewer accumulators than it would take alone: those of the handle's sets.)
 static int row_one(tb_handle* h, GroupChan& G) {
     if (G.row_one.nblocks > 0) return TB_OK;
-    // the caller may be capturing the handle's stream; the copy is on another
+    // while the caller captures the handle's stream, the set is uploaded on another
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    TB_CUDA(cudaStreamIsCapturing(h->stream, &capture));
     cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
     TB_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
-    const int rc = build_row_set(G.L, row_form(G.dev), {row_chan(G)}, {&G.rows}, h->ndofs, G.row_one, 0, true);
+    cudaStream_t side = nullptr;
+    int rc = TB_OK;
+    if (capture != cudaStreamCaptureStatusNone && cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking) != cudaSuccess) {
+        set_error("stream creation failed");
+        rc = TB_ERR_CUDA;
+    }
+    if (rc == TB_OK)
+        rc = build_row_set(G.L, row_form(G.dev), {row_chan(G)}, {&G.rows}, h->ndofs, G.row_one, side ? side : h->stream, 0,
+                           true);
+    if (side) cudaStreamDestroy(side);
     TB_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
     G.row_one.copies = std::min(G.row_one.copies, h->n_accr + 1);
     return rc;
@@ -1113,7 +1130,8 @@ int dp_alloc(tb_handle* h, int64_t max_dense) {
             h->d_runs = dev_upload_raw(h, h->hruns.data(), h->hruns.size());
             if (!h->d_runs) { set_error("run table allocation failed"); return TB_ERR_OOM; }
         } else {
-            TB_CUDA(cudaMemcpy(h->d_runs, h->hruns.data(), sizeof(RunDev) * h->hruns.size(), cudaMemcpyHostToDevice));
+            TB_CUDA(cudaMemcpyAsync(h->d_runs, h->hruns.data(), sizeof(RunDev) * h->hruns.size(), cudaMemcpyHostToDevice,
+                                    h->stream));
         }
         B.runs = h->d_runs;
         h->dense_cap_alloc = cap;
@@ -1595,7 +1613,7 @@ int tb_set_channel_amplitude_fn(tb_handle* h, int ch, tb_amplitude_fn fn, void* 
                 set_error("amplitude callback failed");
                 return TB_ERR_ARG;
             }
-            TB_CUDA(cudaMemcpy(G.d_tamp + a, fac.data(), sizeof(double) * size_t(m), cudaMemcpyHostToDevice));
+            TB_CUDA(cudaMemcpyAsync(G.d_tamp + a, fac.data(), sizeof(double) * size_t(m), cudaMemcpyHostToDevice, h->stream));
         }
         G.dev.tamp = G.d_tamp;
     }
@@ -1618,8 +1636,9 @@ int tb_set_amplitude(tb_handle* h, int ch, double amplitude) {
     // the kernels read instances from device memory, so a captured graph
     // sees the new value at its next launch
     TB_TRY(stream_wait(h));
-    TB_CUDA(cudaMemcpy(G.d_insts + I.slot, &I.dev, sizeof(InstDev), cudaMemcpyHostToDevice));
-    TB_CUDA(cudaMemcpy(I.d_single, &I.dev, sizeof(InstDev), cudaMemcpyHostToDevice));
+    TB_CUDA(cudaMemcpyAsync(G.d_insts + I.slot, &I.dev, sizeof(InstDev), cudaMemcpyHostToDevice, h->stream));
+    TB_CUDA(cudaMemcpyAsync(I.d_single, &I.dev, sizeof(InstDev), cudaMemcpyHostToDevice, h->stream));
+    TB_TRY(stream_wait(h));
     if (h->graph) { cudaGraphExecDestroy(h->graph); h->graph = nullptr; }  // channel skip set changes
     return TB_OK;
 }

@@ -1063,7 +1063,7 @@ int launch_rows_spread(const RowSet& rs, const RowArgs& A, const FxAcc& fx_amp, 
 }
 
 int build_row_set(int L, int form, const std::vector<RowChan>& chan, const std::vector<const PointRows*>& rows,
-                  int64_t ndofs, RowSet& out, int S, bool whole) {
+                  int64_t ndofs, RowSet& out, cudaStream_t s, int S, bool whole) {
     out.release();
     out.L = L;
     out.form = form;
@@ -1155,7 +1155,8 @@ int build_row_set(int L, int form, const std::vector<RowChan>& chan, const std::
     out.d_work = reinterpret_cast<RowWork*>(base + cb);
     out.d_bounds[0] = reinterpret_cast<int32_t*>(base + cb + wb);
     out.d_bounds[1] = reinterpret_cast<int32_t*>(base + cb + wb + bb);
-    TB_CUDA(cudaMemcpy(base, all.data(), all.size(), cudaMemcpyHostToDevice));
+    TB_CUDA(cudaMemcpyAsync(base, all.data(), all.size(), cudaMemcpyHostToDevice, s));
+    TB_CUDA(cudaStreamSynchronize(s));
     out.nblocks = int(work.size());
     int64_t adds = 0;   // of the channel whose smallest band takes the most for each element
     for (size_t i = 0; i < chan.size(); ++i) {

@@ -106,12 +106,12 @@ struct RunState {
 // Runs per lane group for n runs: the widest of 32, 16 and 8 that pads n least.
 int rows_lane_group(int n);
 
-// Uploads the set for the given channels (rows of channel i in rows[i]) of a
+// Uploads the set (on s, which it waits for) for the given channels (rows of channel i in rows[i]) of a
 // handle with ndofs coefficients;
 // blocks are dealt out by the rows' cost.  whole: every block takes all
 // instances of its channel (a set that is also launched for one instance).
 int build_row_set(int L, int form, const std::vector<RowChan>& chan, const std::vector<const PointRows*>& rows,
-                  int64_t ndofs, RowSet& out, int S = 0, bool whole = false);
+                  int64_t ndofs, RowSet& out, cudaStream_t s, int S = 0, bool whole = false);
 
 // f4[e] = (f0, f1, f2, 0) of every element of the state, u4 of u likewise when
 // it is given; nf[b] != 0 marks an element block with a non-finite coefficient.
