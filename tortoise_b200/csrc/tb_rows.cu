@@ -841,7 +841,8 @@ __global__ void __launch_bounds__(RowCap<L, MODE>::W * 32, 1) k_rows(const RowCh
         const int s = used % ROW_STAGES;
         const int e0_row = e0_next;
         if (r + 1 < r1) e0_next = __ldg(c.row_e0 + r + 1);
-        if (!mbar_wait(&bar[s], uint32_t(used / ROW_STAGES) & 1u, wait_polls)) {
+        // one verdict for the warp: what follows assumes all of its lanes
+        if (!__all_sync(0xffffffffu, mbar_wait(&bar[s], uint32_t(used / ROW_STAGES) & 1u, wait_polls))) {
             // record the failure and give the copies in flight a bounded
             // chance to land before the block releases its shared memory
             if (lane == 0) atomicExch(err_flag, 1);
@@ -1322,7 +1323,8 @@ __global__ void __launch_bounds__(row_shares(L) * 32, 1) k_rows_runs(const RowCh
             const double* p = fl[0] + 3 * S * e0;
             f0 = make_double4(__ldg(p), __ldg(p + S), __ldg(p + 2 * S), 0.0);
         }
-        if (!mbar_wait(&bar[s], uint32_t((r - r0) / ROW_STAGES) & 1u, wait_polls)) {
+        // one verdict for the warp, as in k_rows
+        if (!__all_sync(0xffffffffu, mbar_wait(&bar[s], uint32_t((r - r0) / ROW_STAGES) & 1u, wait_polls))) {
             // record the failure and give the copies in flight a bounded
             // chance to land before the block releases its shared memory
             if (lane == 0) atomicExch(err_flag, 1);
