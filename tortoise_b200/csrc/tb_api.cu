@@ -1219,15 +1219,19 @@ int check_status(tb_handle* h) {
 
 // The input of an operator call on the device and a clean accumulator; with
 // host pointers the result goes to d_out.
-static int host_in(tb_handle* h, const double* f, int flags, const double*& d_in, double*& d_res) {
+static int host_in(tb_handle* h, const double* f, int flags, const double*& d_in, double*& d_res, bool& captured) {
     const size_t bytes = sizeof(double) * size_t(h->ndofs);
     if (flags & TB_PTR_HOST) {
         TB_CUDA(cudaMemcpyAsync(h->d_f, f, bytes, cudaMemcpyHostToDevice, h->stream));
         d_in = h->d_f;
         d_res = h->d_out;
     }
-    if (!h->acc_clean) TB_CUDA(cudaMemsetAsync(h->d_acc, 0, bytes, h->stream));
-    h->acc_clean = false;   // until the call has read and cleared it
+    // a call that the caller captures runs later, whatever is known now
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    TB_CUDA(cudaStreamIsCapturing(h->stream, &capture));
+    captured = capture != cudaStreamCaptureStatusNone;
+    if (captured || !h->acc_clean) TB_CUDA(cudaMemsetAsync(h->d_acc, 0, bytes, h->stream));
+    if (!captured) h->acc_clean = false;   // until the call has read and cleared it
     return TB_OK;
 }
 
@@ -1648,10 +1652,11 @@ static int rhs_common(tb_handle* h, const double* f, double* out, int flags, int
     TB_CUDA(cudaSetDevice(h->device));
     const double* d_in = f;
     double* d_res = out;
-    TB_TRY(host_in(h, f, flags, d_in, d_res));
+    bool captured = false;
+    TB_TRY(host_in(h, f, flags, d_in, d_res, captured));
     TB_TRY(run_rhs_acc(h, d_in, h->d_acc, nullptr, flags, only_inst));
     TB_TRY(launch_inverse_mass(h->ed, h->d_acc, d_res, true, h->stream));
-    h->acc_clean = true;
+    if (!captured) h->acc_clean = true;
     return host_out(h, out, flags);
 }
 
@@ -1671,8 +1676,8 @@ int tb_scattering_rates(tb_handle* h, int ch, int leg, const double* f, double* 
     TB_CUDA(cudaSetDevice(h->device));
     const double* d_in = f;
     double* d_res = rates;
-    TB_TRY(host_in(h, f, flags, d_in, d_res));
-    bool no_drift = false;
+    bool no_drift = false, captured = false;
+    TB_TRY(host_in(h, f, flags, d_in, d_res, captured));
     TB_TRY(launch_row_sets(h, d_in, h->d_acc, nullptr, ch, true, leg, no_drift));
     for (size_t gi = 0; gi < h->groups.size(); ++gi) {
         GroupChan& G = h->groups[gi];
@@ -1698,7 +1703,7 @@ int tb_scattering_rates(tb_handle* h, int ch, int leg, const double* f, double* 
     TB_TRY(launch_fx_flush(h->fx, h->d_acc, h->ndofs, h->stream));
     TB_TRY(shard_allreduce(h, h->d_acc, size_t(h->ndofs)));
     TB_TRY(launch_inverse_mass(h->ed, h->d_acc, d_res, true, h->stream));
-    h->acc_clean = true;
+    if (!captured) h->acc_clean = true;
     return host_out(h, rates, flags);
 }
 
