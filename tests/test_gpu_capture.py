@@ -75,3 +75,23 @@ def test_captured_calls_replay_beside_other_calls(gpu_lib, deterministic):
     finally:
         e.close()
         ref.close()
+
+
+def test_captured_calls_outlive_a_change_of_schedules(gpu_lib):
+    """The row sets that a graph launches stay, although the handle's own calls use others after the change."""
+    mat = _material()
+    f = W.initial_status(mat, seed=1).vec
+    e, ref = E.Engine(mat), E.Engine(mat)
+    try:
+        graphs = [Captured(e, call, f.size) for call, _ in _calls(e)]
+        want = [call(f) for _, call in _calls(ref)]
+        legs = [c.nlegs for c in mat.channels]
+        three, four = legs.index(3), legs.index(4)
+        assert e.schedule(three).get("inside_only") and e.schedule(four).get("inside_only")
+        for ch, kw in ((three, {"pair": 0}), (four, {"inside_only": False}), (three, {"inside_only": True})):
+            e.set_schedule(ch, 0 if "inside_only" in kw else 1, **kw)
+            for (_, call), w, g in zip(_calls(e), want, graphs):
+                assert rel_l2(call(f), w) < TOL and rel_l2(g(f), w) < TOL
+    finally:
+        e.close()
+        ref.close()

@@ -99,7 +99,7 @@ namespace tb {
 int choose_layouts(tb_handle* h);
 int autotune(tb_handle* h);
 int build_run_states(tb_handle* h);
-void release_row_sets(tb_handle* h);
+void retire_row_sets(tb_handle* h);
 }  // namespace tb
 
 namespace tb {
@@ -699,18 +699,23 @@ static int make_row_sets(tb_handle* h, Take take, bool run_minor, std::vector<Ro
     return TB_OK;
 }
 
-void release_row_sets(tb_handle* h) {
+void retire_row_sets(tb_handle* h) {
+    auto retire = [&](RowSet& rs) {
+        if (rs.d_chan) h->retired.push_back(rs.d_chan);   // the allocation's base
+        rs.d_chan = nullptr;
+        rs.release();
+    };
     for (auto* sets : {&h->row_sets, &h->rate_sets, &h->run_sets}) {
-        for (auto& rs : *sets) rs.release();
+        for (auto& rs : *sets) retire(rs);
         sets->clear();
     }
-    for (auto& G : h->groups) G.row_one.release();
+    for (auto& G : h->groups) retire(G.row_one);
 }
 
 int refresh_row_sets(tb_handle* h) {
     // a captured attempt holds the sets' addresses
     if (h->graph) { cudaGraphExecDestroy(h->graph); h->graph = nullptr; }
-    release_row_sets(h);
+    retire_row_sets(h);
     int slots = 0;
     for (auto& G : h->groups) {
         G.gamp0 = slots;
@@ -727,7 +732,7 @@ int refresh_row_sets(tb_handle* h) {
     for (const auto* sets : {&h->row_sets, &h->rate_sets})
         for (const RowSet& rs : *sets) copies = std::max(copies, rs.copies);
     if (copies - 1 > h->n_accr && !h->opts.deterministic) {
-        if (h->d_accr) cudaFree(h->d_accr);
+        if (h->d_accr) h->retired.push_back(h->d_accr);
         h->n_accr = 0;
         const size_t bytes = sizeof(double) * size_t(copies - 1) * size_t(h->ndofs);
         if (cudaMalloc(&h->d_accr, bytes) != cudaSuccess) {
@@ -1319,7 +1324,8 @@ int tb_destroy(tb_handle* h) {
         G.rows.release();
         if (G.d_tamp) cudaFree(G.d_tamp);
     }
-    release_row_sets(h);
+    retire_row_sets(h);
+    for (void* p : h->retired) cudaFree(p);
     for (void* p : h->run_allocs) cudaFree(p);
     if (h->d_accr) cudaFree(h->d_accr);
     for (double* p : h->dev_allocs) cudaFree(p);

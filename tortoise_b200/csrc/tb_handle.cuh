@@ -104,6 +104,9 @@ struct tb_handle {
     tb::RunState* d_run_states = nullptr;
     int* d_run_nf = nullptr;
     int n_run_tiles = 0;
+    // what former row sets held: a graph that the caller captured may still
+    // launch them (a few ten KB for each change of schedules; freed with the handle)
+    std::vector<void*> retired;
     double* d_accr = nullptr;    // further accumulators of the row sets, n_accr of ndofs
     int n_accr = 0;
     double4* d_f4 = nullptr;
