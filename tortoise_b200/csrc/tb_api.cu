@@ -715,17 +715,27 @@ void retire_row_sets(tb_handle* h) {
 int refresh_row_sets(tb_handle* h) {
     // a captured attempt holds the sets' addresses
     if (h->graph) { cudaGraphExecDestroy(h->graph); h->graph = nullptr; }
-    retire_row_sets(h);
     int slots = 0;
     for (auto& G : h->groups) {
         G.gamp0 = slots;
         slots += int(G.insts.size());
     }
-    TB_TRY(make_row_sets(h, [](const GroupChan& G) { return G.run_state < 0; }, false, h->row_sets));
+    // without room for the new sets the former ones stay
+    std::vector<RowSet> row, rate, run;
+    int rc = make_row_sets(h, [](const GroupChan& G) { return G.run_state < 0; }, false, row);
     if (!h->run_states.empty()) {
-        TB_TRY(make_row_sets(h, [](const GroupChan& G) { return G.run_state >= 0; }, false, h->rate_sets));
-        TB_TRY(make_row_sets(h, [](const GroupChan& G) { return G.run_state >= 0; }, true, h->run_sets));
+        if (rc == TB_OK) rc = make_row_sets(h, [](const GroupChan& G) { return G.run_state >= 0; }, false, rate);
+        if (rc == TB_OK) rc = make_row_sets(h, [](const GroupChan& G) { return G.run_state >= 0; }, true, run);
     }
+    if (rc != TB_OK) {
+        for (auto* sets : {&row, &rate, &run})
+            for (auto& rs : *sets) rs.release();
+        return rc;
+    }
+    retire_row_sets(h);
+    h->row_sets = std::move(row);
+    h->rate_sets = std::move(rate);
+    h->run_sets = std::move(run);
     // the further accumulators (not in the deterministic mode, whose adds are
     // exact); without room the blocks share one
     int copies = 1;
@@ -1424,6 +1434,20 @@ int tb_channel_schedule(const tb_handle* h, int ch, int32_t* stages, int32_t* pa
     return TB_OK;
 }
 
+static int run_minor_error() {
+    set_error("the run-minor contraction needs a group of 8..1024 runs with at most 3 legs");
+    return TB_ERR_ARG;
+}
+
+// G over its rows or not; on failure as it was.
+static int switch_rows(tb_handle* h, GroupChan& G, bool rows) {
+    const bool was = G.use_rows;
+    G.use_rows = rows;
+    const int rc = refresh_row_sets(h);
+    if (rc != TB_OK) G.use_rows = was;
+    return rc;
+}
+
 int tb_set_channel_schedule(tb_handle* h, int ch, int32_t stages, int32_t pair) {
     if (!h || ch < 0 || ch >= int(h->insts.size())) { set_error("channel index out of range"); return TB_ERR_ARG; }
     GroupChan& G = h->groups[h->insts[ch].group];
@@ -1442,10 +1466,8 @@ int tb_set_channel_schedule(tb_handle* h, int ch, int32_t stages, int32_t pair) 
         }
         TB_CUDA(cudaSetDevice(h->device));
         TB_CUDA(cudaStreamSynchronize(h->stream));
+        TB_TRY(switch_rows(h, G, pair == 6 && G.rows.blk));
         G.theta.use = pair == 6;
-        G.use_rows = pair == 6 && G.rows.blk;
-        TB_TRY(refresh_row_sets(h));
-        if (h->graph) { cudaGraphExecDestroy(h->graph); h->graph = nullptr; }
         return TB_OK;
     }
     if (G.rows.blk) {   // AUTO's FP64 channel: its rows, or a contraction whose tensor is built now
@@ -1454,21 +1476,21 @@ int tb_set_channel_schedule(tb_handle* h, int ch, int32_t stages, int32_t pair) 
             set_error("stages must be 1..2 and pair 0..5, or stages 0 and pair 6 (packed rows)");
             return TB_ERR_ARG;
         }
+        if (!rows && pair >= 2 && !runs_possible(G.L, int(G.insts.size()))) return run_minor_error();
         TB_CUDA(cudaSetDevice(h->device));
         TB_CUDA(cudaStreamSynchronize(h->stream));
-        if (!rows) TB_TRY(ensure_tensor(h, G));
-        if (rows || pair < 2 || G.tensor.fT) {
-            G.use_rows = rows;
-            TB_TRY(refresh_row_sets(h));
-            if (h->graph) { cudaGraphExecDestroy(h->graph); h->graph = nullptr; }
-            if (rows) return TB_OK;
+        if (rows) return switch_rows(h, G, true);
+        const bool had = G.tensor.d != nullptr;
+        int rc = ensure_tensor(h, G);
+        if (rc == TB_OK && pair >= 2 && !G.tensor.fT) rc = run_minor_error();   // no room for its buffers
+        if (rc == TB_OK) rc = switch_rows(h, G, false);
+        if (rc != TB_OK) {   // refused or failed: as it was
+            if (!had) G.tensor.release();
+            return rc;
         }
     }
     if (stages < 1 || stages > 2 || pair < 0 || pair > 5) { set_error("stages must be 1..2 and pair 0..5"); return TB_ERR_ARG; }
-    if (pair >= 2 && !G.tensor.fT) {
-        set_error("the run-minor contraction needs a group of 8..1024 runs with at most 3 legs");
-        return TB_ERR_ARG;
-    }
+    if (pair >= 2 && !G.tensor.fT) return run_minor_error();
     TB_CUDA(cudaSetDevice(h->device));
     TB_CUDA(cudaStreamSynchronize(h->stream));
     G.tensor.stages = stages;
@@ -1596,11 +1618,15 @@ int tb_set_channel_amplitude_fn(tb_handle* h, int ch, tb_amplitude_fn fn, void* 
     if (G.stream && fn) { set_error("a streamed channel takes no functAmplitude (no per-tuple table)"); return TB_ERR_ARG; }
     const int L = G.L;
     const int64_t n = G.tup.n;
-    if (G.d_tamp) { cudaFree(G.d_tamp); G.d_tamp = nullptr; }
     G.dev.tamp = nullptr;
-    if (G.use_rows) TB_TRY(refresh_row_sets(h));   // the sets hold the table's address
+    if (G.use_rows) {   // the sets hold the table's address
+        const int rc = refresh_row_sets(h);
+        if (rc != TB_OK) { G.dev.tamp = G.d_tamp; return rc; }
+    }
+    if (G.d_tamp) { cudaFree(G.d_tamp); G.d_tamp = nullptr; }
     if (fn && n > 0) {
         if (cudaMalloc(&G.d_tamp, sizeof(double) * size_t(n)) != cudaSuccess) {
+            cudaGetLastError();
             G.d_tamp = nullptr;
             set_error("amplitude table allocation failed");
             return TB_ERR_OOM;

@@ -834,6 +834,7 @@ static int build_t(const ChanDev& c, const int32_t* tup, int64_t stride, int64_t
     const size_t bytes = size_t(tensor_bytes(L, KIND, n));
     T.release();
     if (cudaMalloc(&T.d, bytes) != cudaSuccess) {
+        cudaGetLastError();   // not left for the next launch's check
         T.d = nullptr;
         set_error("moment tensor allocation failed");
         return TB_ERR_OOM;
@@ -982,10 +983,11 @@ static int launch_runs(const ChanDev& c, const InstDev* insts, int n_insts, cons
     return TB_OK;
 }
 
+bool runs_possible(int L, int n_insts) { return L <= 3 && n_insts >= RUNS_MIN && ((n_insts + 31) & ~31) <= RUNS_NP_MAX; }
+
 int prepare_runs(const ChanDev& c, int n_insts, bool distinct_runs, MomentTensor& T, cudaStream_t s, bool exact) {
-    if (c.L > 3 || n_insts < RUNS_MIN || T.fT || !T.d) return TB_OK;
+    if (!runs_possible(c.L, n_insts) || T.fT || !T.d) return TB_OK;
     const int np = (n_insts + 31) & ~31;
-    if (np > RUNS_NP_MAX) return TB_OK;
     int64_t tot = 0;
     for (int l = 0; l < c.L; ++l) {
         T.loff[l] = tot;

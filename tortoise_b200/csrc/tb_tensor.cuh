@@ -48,6 +48,9 @@ int launch_collision_tensor(const ChanDev& c, const InstDev* insts, int n_insts,
                             const int32_t* tup, int64_t stride, int64_t n, const double* f, double* acc,
                             const DPCtl* ctl, cudaStream_t s, int rate_leg = -1, const FxAcc& fx = FxAcc{});
 
+// Whether a group of n_insts instances can take the run-minor contraction.
+bool runs_possible(int L, int n_insts);
+
 // Buffers of the run-minor contraction for a group of n_insts instances
 // (legs <= 3, 8 <= n_insts <= 1024); sets runs = 8 from 16 instances on.
 // exact: also the fixed-point twin of the accumulator (deterministic mode).
