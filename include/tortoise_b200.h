@@ -147,7 +147,9 @@ typedef struct tb_options {
     int32_t device;               /* CUDA device ordinal                            */
     int32_t layout;               /* TB_LAYOUT_*                                    */
     int32_t allow_fp32;           /* AUTO for 2- and 3-leg channels: 0 -> T64, 1 -> T32, 2 -> T40, 3 -> T48 */
-    int64_t tensor_budget_bytes;  /* cap on precomputed-tensor memory (0: 60% free) */
+    int64_t tensor_budget_bytes;  /* cap on the memory of moment tensors and packed rows, all channels
+                                     together (0: 60% of the free memory).  A tensor that
+                                     tb_set_channel_schedule asks for later comes on top. */
     int32_t verbose;
     int32_t autotune;             /* 1: time the contraction schedules at creation, keep the fastest */
     int32_t shard_rank;           /* tuple sharding (tb_shard_connect): this process's part ... */

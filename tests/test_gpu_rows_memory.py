@@ -57,3 +57,32 @@ def test_a_tensor_without_room_is_reported_once(gpu_lib):
         hog = None
         torch.cuda.empty_cache()
         e.close()
+
+
+def _used(mat, cap):
+    """Device memory of a handle, and the bytes of rows that its channels would fill without any padding."""
+    import torch
+    before = _free()
+    e = E.Engine(mat, tensor_budget_bytes=cap)
+    try:
+        f = W.initial_status(mat, kT=0.15, seed=7).vec
+        rows = [max(e.points_inside(c)[0], 0) * 172 for c in range(len(mat.channels))]
+        assert all(e.schedule(c).get("inside_only") for c, n in enumerate(rows) if n)   # every channel has its list
+        return before - _free(), rows, e.rhs(f)
+    finally:
+        e.close()
+        torch.cuda.empty_cache()
+
+
+def test_rows_of_all_channels_stay_within_the_budget(gpu_lib):
+    mat = W.build_material(7, ("P", "D"), (), ee=True, eph=False)   # four-leg channels only
+    _used(mat, 0)   # what the first handle of a process allocates once
+    small, rows, ref = _used(mat, 1)
+    full, _, got = _used(mat, 0)
+    assert len([n for n in rows if n]) > 1 and full - small > 0.9 * sum(rows) > 64 << 20
+    assert rel_l2(got, ref) < TOL
+    cap = int(1.1 * max(rows)) + (4 << 20)
+    assert cap < 0.7 * sum(rows)
+    part, _, got = _used(mat, cap)
+    assert 0 < part - small <= cap + (4 << 20)   # and the row sets and further accumulators, in units of 2 MB
+    assert rel_l2(got, ref) < TOL

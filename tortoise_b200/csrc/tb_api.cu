@@ -571,20 +571,8 @@ int build_runs(tb_handle* h, const tb_problem_desc* const* descs, int nruns) {
     }
     for (auto& G : h->groups) TB_TRY(shard_tuples(h, G));
     {
-        NvtxRange r("tb_create: layouts and moment tensors");
+        NvtxRange r("tb_create: layouts, moment tensors and rows");
         TB_TRY(choose_layouts(h));
-    }
-    {
-        NvtxRange r("tb_create: points inside the simplices");
-        size_t freeb = 0, totalb = 0;
-        cudaMemGetInfo(&freeb, &totalb);
-        const int64_t room = int64_t(double(freeb) * 0.6);   // the most that a channel's rows may take, as for tensors
-        for (auto& G : h->groups)
-            if (G.layout == TB_LAYOUT_MC64) {
-                TB_TRY(build_theta_list(G.dev, G.tup, G.theta, h->stream));
-                if (G.theta.built) TB_TRY(build_rows(G.dev, G.theta, G.rows, room, h->stream));
-                G.use_rows = G.rows.blk != nullptr;
-            }
     }
     h->d_f4 = reinterpret_cast<double4*>(dev_alloc(h, size_t(h->ndofs / 3 * 4)));
     {
@@ -972,7 +960,8 @@ static int tune_rows(tb_handle* h, GroupChan& G) {
     // differently), whose time is only recorded
     const bool choose = !h->opts.deterministic;
     if (choose) {
-        const int rc = ensure_tensor(h, G);
+        const int64_t bytes = tensor_bytes(G.L, TK_F64, G.tup.n);
+        const int rc = G.tensor.d || bytes <= h->budget_left ? ensure_tensor(h, G) : int(TB_ERR_OOM);
         if (rc == TB_ERR_OOM) return TB_OK;   // no room for the tensor: the rows stay
         TB_TRY(rc);
         TB_TRY(tune_tensor(G.dev, G.d_insts, int(G.insts.size()), G.tensor, G.tup.d, G.tup.cap, G.tup.n, h->d_f,
@@ -1005,7 +994,10 @@ static int tune_rows(tb_handle* h, GroupChan& G) {
     G.rows_seconds = 1e-3 * double(ms) / REPS;
     if (!choose) return TB_OK;
     if (G.rows_seconds <= G.tensor.tuned_seconds) G.tensor.release();
-    else G.use_rows = false;
+    else {
+        G.use_rows = false;
+        h->budget_left -= tensor_bytes(G.L, TK_F64, G.tup.n);
+    }
     return TB_OK;
 }
 
@@ -1048,6 +1040,8 @@ int choose_layouts(tb_handle* h) {
     size_t freeb = 0, totalb = 0;
     cudaMemGetInfo(&freeb, &totalb);
     int64_t budget = h->opts.tensor_budget_bytes > 0 ? h->opts.tensor_budget_bytes : int64_t(double(freeb) * 0.6);
+    int64_t left = budget;   // of it, less what tensors and rows take
+    std::vector<bool> over_rows(h->groups.size(), false);
     for (auto& G : h->groups) {
         if (G.stream) continue;   // TB_LAYOUT_STREAM, fixed at creation
         int want = h->opts.layout;
@@ -1074,20 +1068,43 @@ int choose_layouts(tb_handle* h) {
             else budget -= bytes;
         }
         G.layout = want;
-        if (want != TB_LAYOUT_MC64) {
-            const int64_t room = int64_t(double(freeb) * 0.6);   // as for a tensor
-            // AUTO's FP64 channels go over their packed rows; the tensor is
-            // built when a contraction schedule is asked for
-            if (h->opts.layout == TB_LAYOUT_AUTO && want == TB_LAYOUT_T64) {
-                TB_TRY(build_theta_list(G.dev, G.tup, G.theta, h->stream));
-                if (G.theta.built) TB_TRY(build_rows(G.dev, G.theta, G.rows, room, h->stream));
-                G.use_rows = G.rows.blk != nullptr;
-                if (G.use_rows) continue;
-                G.theta.release();
-            }
+        // AUTO's FP64 channels go over their packed rows; the tensor is built
+        // when a contraction schedule is asked for
+        over_rows[size_t(&G - h->groups.data())] = h->opts.layout == TB_LAYOUT_AUTO && want == TB_LAYOUT_T64 && G.dev.nmc <= 64;
+        if (want != TB_LAYOUT_MC64 && !over_rows[size_t(&G - h->groups.data())]) {
             TB_TRY(build_group_tensor(h, G, kind));
+            left -= tensor_bytes(G.L, kind, G.tup.n);
         }
     }
+    // Every channel's point list before any rows: without one a channel visits
+    // every point of every tuple (16x16 e-e: 20.5 ms against 3.6 with the list
+    // and 1.6 over rows).  The rows of all channels share what is left of the
+    // budget, and leave part of the memory that is free now to the rest.
+    NvtxRange r("tb_create: points inside the simplices");
+    for (size_t i = 0; i < h->groups.size(); ++i) {
+        GroupChan& G = h->groups[i];
+        if (G.layout == TB_LAYOUT_MC64 || over_rows[i]) TB_TRY(build_theta_list(G.dev, G.tup, G.theta, h->stream));
+    }
+    cudaMemGetInfo(&freeb, &totalb);
+    left = std::min(left, int64_t(double(freeb) * 0.6));
+    for (bool tensors : {true, false})   // first those that have a tensor's share of the budget
+        for (size_t i = 0; i < h->groups.size(); ++i) {
+            GroupChan& G = h->groups[i];
+            if (G.stream || tensors != over_rows[i] || (!tensors && G.layout != TB_LAYOUT_MC64)) continue;
+            if (G.theta.built) TB_TRY(build_rows(G.dev, G.theta, G.rows, left, h->stream));
+            G.use_rows = G.rows.blk != nullptr;
+            left -= G.rows.bytes;
+            if (!tensors || G.use_rows) continue;
+            const int rc = build_group_tensor(h, G, TK_F64);   // no point inside, or no room for the rows
+            if (rc == TB_ERR_OOM) {
+                G.layout = TB_LAYOUT_MC64;
+                continue;
+            }
+            TB_TRY(rc);
+            G.theta.release();
+            left -= tensor_bytes(G.L, TK_F64, G.tup.n);
+        }
+    h->budget_left = left;
     return TB_OK;
 }
 }  // namespace tb

@@ -109,6 +109,7 @@ struct tb_handle {
     std::vector<void*> retired;
     double* d_accr = nullptr;    // further accumulators of the row sets, n_accr of ndofs
     int n_accr = 0;
+    int64_t budget_left = 0;     // of tensor_budget_bytes (or its default) after creation
     double4* d_f4 = nullptr;
     int* d_nf = nullptr;
     // deterministic mode: the exact accumulator behind d_acc (3 words per

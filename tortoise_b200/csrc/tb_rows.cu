@@ -97,7 +97,7 @@ void PointRows::release() {
     blk = nullptr;
     row_e0 = nullptr;
     perm = nullptr;
-    nrows = n = points = 0;
+    nrows = n = points = bytes = 0;
     cost.clear();
     run_cost.clear();
 }
@@ -243,6 +243,7 @@ int build_rows(const ChanDev& c, const ThetaList& th, PointRows& rows, int64_t m
         rows.run_cost[r + 1] = rows.run_cost[r] + pts[2 * r + 1];
     }
     rows.nrows = nrows;
+    rows.bytes = int64_t(bytes + words);
     rows.n = n;
     rows.points = th.points;
     return TB_OK;

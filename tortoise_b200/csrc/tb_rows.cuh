@@ -23,6 +23,7 @@ struct PointRows {
     int32_t* perm = nullptr;        // [nrows][32] index in the channel's list (padding: -1)
     int64_t nrows = 0;
     int64_t n = 0, points = 0;      // tuples and points inside
+    int64_t bytes = 0;              // device memory of the rows
     std::vector<int64_t> cost;      // [nrows + 1] running cost of the rows (host)
     std::vector<int64_t> run_cost;  // the same, run-minor
     void release();
