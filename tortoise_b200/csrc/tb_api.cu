@@ -763,6 +763,7 @@ int build_run_states(tb_handle* h) {
         st.S = rows_lane_group(st.n);
         st.np = (st.n + st.S - 1) / st.S * st.S;
         st.ndof = h->runs[size_t(run[0])].ndofs;
+        if (st.ndof * st.S > 0x7fffffff) continue;   // k_rows_runs keeps offsets within a group of S runs in 32 bits
         const size_t bytes = sizeof(double) * size_t(st.ndof) * size_t(st.np);
         void* p[4] = {nullptr, nullptr, nullptr, nullptr};
         const size_t sz[4] = {bytes, bytes, sizeof(int64_t) * off.size(), sizeof(int) * run.size()};
