@@ -362,9 +362,12 @@ def ours(args, world, rank, local, pg):
     tp = os.path.join(ROOT, "profiles", "collision_traffic.json")
     if os.path.exists(tp):
         d = json.load(open(tp))
-        key = infos[0]["layout"]
-        if not rows and key in d and d[key].get("bytes_per_tuple"):
-            traffic = d[key]["bytes_per_tuple"] * ntup
+        # per channel: over rows of three legs, or through its tensor
+        part = {ch: (d.get("rows_3legs"), eng.points_inside(ch)[0]) if ch in rows else
+                (d.get(infos[ch]["layout"]), infos[ch]["n_tuples"]) for ch in on}
+        if all(m and m.get("bytes_per_tuple") and (ch not in rows or mat.channels[ch].nlegs == 3)
+               for ch, (m, _) in part.items()):
+            traffic = sum(m["bytes_per_tuple"] * n for m, n in part.values())
     line = {"metric": METRIC, "value": value, "unit": "DP45 steps/s", "n_gpus": world, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": 1e3 * t_max / args.steps, "higher_is_better": True,
             "scaling": "strong" if args.shard else "weak", "vs_baseline": None, "dtype": {None: "f64", "t32": "f32-storage/f64-accumulate",

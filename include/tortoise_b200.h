@@ -146,7 +146,11 @@ typedef struct tb_handle tb_handle;
 typedef struct tb_options {
     int32_t device;               /* CUDA device ordinal                            */
     int32_t layout;               /* TB_LAYOUT_*                                    */
-    int32_t allow_fp32;           /* AUTO for 2- and 3-leg channels: 0 -> T64, 1 -> T32, 2 -> T40, 3 -> T48 */
+    int32_t allow_fp32;           /* AUTO for 2- and 3-leg channels: 0 -> T64, 1 -> T32, 2 -> T40, 3 -> T48.
+                                     1 to 3 contract a moment tensor of fewer bits; 0 goes over
+                                     packed rows (tb_channel_schedule) at full precision, which
+                                     are smaller and faster: one 64x64 e-ph right-hand side
+                                     0.31 ms against 1.09 with T40. */
     int64_t tensor_budget_bytes;  /* cap on the memory of moment tensors and packed rows, all channels
                                      together (0: 60% of the free memory).  A tensor that
                                      tb_set_channel_schedule asks for later comes on top. */
@@ -326,14 +330,15 @@ int tb_dp45_poll(tb_handle* h, tb_dp45_stats* stats);
 int tb_dp45_end(tb_handle* h, double* f_out, double* dense_out, double* dense_times, int64_t max_dense,
                 tb_dp45_stats* stats, int flags);
 
-/* Synchronises the handle's stream; TB_ERR_TIMEOUT when a contraction's
+/* Synchronises the handle's stream; TB_ERR_TIMEOUT when a collision kernel's
  * bounded wait ran out since the last synchronising call. */
 int tb_synchronize(tb_handle* h);
 
-/* Poll limit of the moment-tensor contractions' wait for each staged tile of
- * moments (default 2^22 polls, far above any real copy).  A wait that runs
- * out makes its thread block record the failure, wait (with its own bound)
- * for the copies it still has in flight, and leave its tiles out; the next
+/* Poll limit of the wait for each staged tile of moments (contractions) or row
+ * of tuples (packed rows; default 2^22 polls, far above any real copy).  A wait
+ * that runs out makes its thread block, over rows its warp, record the failure,
+ * wait (with its own bound) for the copies it still has in flight, and leave its
+ * tiles or rows out; the next
  * synchronising call (tb_rhs / tb_scattering_rates with host buffers,
  * tb_synchronize, tb_dp45_poll / tb_dp45_end / tb_dp45_integrate, the
  * adjoint sweeps) returns TB_ERR_TIMEOUT, and the handle stays usable.
@@ -386,8 +391,10 @@ int tb_channel_schedule(const tb_handle* h, int ch, int32_t* stages, int32_t* pa
 
 /* Monte-Carlo channels: the tuples with at least one point inside the
  * simplices and the number of such (tuple, point) pairs, i.e. the work the
- * quadrature does per instance; -1, -1 when the channel has no such list
- * (a moment tensor, or more than 64 Monte-Carlo points).  On a sharded
+ * quadrature does per instance; the same for AUTO's FP64 channels with two or
+ * three legs, also while a contraction is pinned; -1, -1 when the channel has
+ * no such list (an explicit or reduced-precision moment tensor, more than 64
+ * Monte-Carlo points, no tuples, or two or three legs and no point inside).  On a sharded
  * handle, this handle's part.  No counterpart in the reference. */
 int tb_channel_points_inside(const tb_handle* h, int ch, int64_t* n_tuples, int64_t* n_points);
 

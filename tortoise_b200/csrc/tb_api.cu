@@ -619,8 +619,11 @@ constexpr int ROWS_RUN_MINOR = 8;
 // Four legs spread more adds over fewer rows, so run-minor groups pay off later
 // (e-e, us, one by one / run-minor: 6x6 16 runs 248 / 382, 40 runs 612 / 764,
 // 48 runs 748 / 605; 8x8 16 runs 825 / 1296, 32 runs 1661 / 1885, 48 runs 2488 /
-// 2092; 9x9, 2.2 million tuples, 24 runs 2170 / 2844, 32 runs 2898 / 1933; 12x12
-// 16 runs 5900 / 6936, 32 runs 12078 / 8131).
+// 2092; 9x8, 1.7 million tuples, 32 runs 2175 / 2425, 48 runs 3306 / 3183; 9x9,
+// 2.2 million, 24 runs 2129 / 2814, 32 runs 2859 / 1935; 10x9 24 runs 2750 / 3271,
+// 32 runs 3681 / 3373; 12x12 16 runs 5844 / 7146, 24 runs 9053 / 8981, 32 runs
+// 11976 / 8140.  A width that fills its groups gains earlier, 20 runs of 12x12
+// 7513 / 5855 and 40 runs of 4x4 222 / 133; 3x3 never does, 48 runs 87 / 96).
 constexpr int ROWS_RUN_MINOR_4 = 48;
 constexpr int ROWS_RUN_MINOR_4_LARGE = 32;
 constexpr int64_t ROWS_LARGE_4 = 2000000;
@@ -1233,7 +1236,7 @@ namespace tb {
 int status_error(tb_handle* h) {
     if (h->h_status[0]) {
         TB_CUDA(cudaMemsetAsync(h->d_err, 0, sizeof(int), h->stream));
-        set_error("a moment-tensor contraction gave up waiting for its staged tiles; the result is incomplete");
+        set_error("a collision kernel gave up waiting for its staged rows or tiles; the result is incomplete");
         return TB_ERR_TIMEOUT;
     }
     if (h->fx.sat && h->h_status[1]) {

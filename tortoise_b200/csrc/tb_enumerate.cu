@@ -27,7 +27,7 @@
 // item, so that k_enum_write has no test to repeat.  It takes tables of at most
 // 64 points inside the reference domain, and boxes of at most 64 candidates;
 // a channel that does not fit goes through k_enumerate.  Measured, whole
-// tb_create: 64x64 two-band e-ph 97 -> 43 ms (enumeration 72 -> 14), 16x16 e-e
+// tb_create: 64x64 two-band e-ph 97 -> 37 ms (enumeration 72 -> 14), 16x16 e-e
 // 410 -> 105 ms (367 -> 64).
 #include <cub/cub.cuh>
 

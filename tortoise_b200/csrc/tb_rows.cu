@@ -993,7 +993,11 @@ __global__ void __launch_bounds__(1024) k_rows_fold(double* __restrict__ acc, do
 // Measured: 16x16 e-e (239,000 adds an element) 6.6 ms with one copy, 1.79 with
 // 32, 1.71 with 64, 1.58 with 148; an 8x8 e-e integration (29,000) 165 ms with
 // one, 54 with 4, 29 with 16, 23 with 64 and with 148; 64x64 e-ph (900) 324 us
-// with one, 335 with 2, 340 with 8.
+// with one, 335 with 2, 340 with 8.  Around the line, a right-hand side in us with
+// one and with a copy a block: e-ph 40x40 with umklapp (1200 adds) 176 / 160, 96x96
+// (1500) 941 / 1029, 64x64 with umklapp (1900) 537 / 560; e-e 3x3 (1200) 33 / 29, 4x3
+// (2100) 43 / 29, 5x4 (4900) 115 / 27, 6x6 (11,900) 277 / 38; four legs with bosons
+// 8x6 (17,000) 263 / 51.
 constexpr int64_t ROW_ADDS = 2000, ROW_COPY_BYTES = int64_t(64) << 20;
 static int row_copies(int64_t adds_per_element, int nblocks, int64_t ndofs) {
     if (adds_per_element <= ROW_ADDS) return 1;

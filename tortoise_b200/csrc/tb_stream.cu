@@ -101,8 +101,8 @@ __global__ void __launch_bounds__(ST_WARPS * 32, TB_STREAM_MIN_BLOCKS)
     const double inv_fact_nmc = c.fact * double(c.nmc);
     unsigned long long n_pre = 0, n_det = 0, n_surv = 0, n_pts = 0, n_tin = 0;
 
-    int q2n = 0;   // candidates in queue 1 (warp-uniform)
-    int q3n = 0;   // surviving tuples in queue 2 (warp-uniform)
+    int q1n = 0;   // candidates in queue 1 (warp-uniform)
+    int q2n = 0;   // surviving tuples in queue 2 (warp-uniform)
 
     // Stage 1 for `take` candidates of queue 0 from slot `first` on, one per
     // lane: the determinant filter, then the points of the survival table that
@@ -133,12 +133,12 @@ __global__ void __launch_bounds__(ST_WARPS * 32, TB_STREAM_MIN_BLOCKS)
         }
         const unsigned bal = __ballot_sync(full, ok);
         if (ok) {
-            const int pos = q2n + __popc(bal & ((1u << lane) - 1u));
+            const int pos = q1n + __popc(bal & ((1u << lane) - 1u));
 #pragma unroll
             for (int l = 0; l <= L; ++l) s_q[1][warp][l][pos] = l < L ? e[l] : u;
             s_may[warp][pos] = may;
         }
-        q2n += __popc(bal);
+        q1n += __popc(bal);
         __syncwarp();
     };
 
@@ -183,11 +183,11 @@ __global__ void __launch_bounds__(ST_WARPS * 32, TB_STREAM_MIN_BLOCKS)
         n_surv += ok ? 1 : 0;
         const unsigned bal = __ballot_sync(full, ok);
         if (ok) {
-            const int pos = q3n + __popc(bal & ((1u << lane) - 1u));
+            const int pos = q2n + __popc(bal & ((1u << lane) - 1u));
 #pragma unroll
             for (int l = 0; l <= L; ++l) s_q[2][warp][l][pos] = l < L ? e[l] : u;
         }
-        q3n += __popc(bal);
+        q2n += __popc(bal);
         __syncwarp();
     };
 
@@ -338,12 +338,12 @@ __global__ void __launch_bounds__(ST_WARPS * 32, TB_STREAM_MIN_BLOCKS)
                 if (qn >= 32) {
                     stage1(qn - 32, 32);
                     qn -= 32;
-                    if (q2n >= 32) {
-                        survive(q2n - 32, 32);
-                        q2n -= 32;
-                        if (q3n >= 32) {
-                            evaluate(q3n - 32, 32);
-                            q3n -= 32;
+                    if (q1n >= 32) {
+                        survive(q1n - 32, 32);
+                        q1n -= 32;
+                        if (q2n >= 32) {
+                            evaluate(q2n - 32, 32);
+                            q2n -= 32;
                         }
                     }
                     __syncwarp();   // the slots are reused
@@ -355,14 +355,14 @@ __global__ void __launch_bounds__(ST_WARPS * 32, TB_STREAM_MIN_BLOCKS)
     // the queues' remainders, survivors first once queue 1 is empty
     if (qn > 0) stage1(0, qn);
     for (;;) {
-        if (q3n >= 32 || (q2n == 0 && q3n > 0)) {
-            const int t = min(q3n, 32);
-            evaluate(q3n - t, t);
-            q3n -= t;
-        } else if (q2n > 0) {
+        if (q2n >= 32 || (q1n == 0 && q2n > 0)) {
             const int t = min(q2n, 32);
-            survive(q2n - t, t);
+            evaluate(q2n - t, t);
             q2n -= t;
+        } else if (q1n > 0) {
+            const int t = min(q1n, 32);
+            survive(q1n - t, t);
+            q1n -= t;
         } else {
             break;
         }
