@@ -514,6 +514,8 @@ int build_runs(tb_handle* h, const tb_problem_desc* const* descs, int nruns) {
                     }
                     sd.n_items *= int64_t(1) << (G.L - 1);
                     sd.mc_pre = G.d_mc_pre;
+                    for (const double* q : {cd.mc_points, pre})
+                        for (size_t i = 0; i < size_t(cd.n_mc) * c.R; ++i) sd.wide = sd.wide || !(std::fabs(q[i]) <= 1.5);
                     void* p = nullptr;
                     if (cudaMalloc(&p, sizeof(unsigned long long) * 5) != cudaSuccess) {
                         set_error("count buffer allocation failed");

@@ -230,7 +230,7 @@ __global__ void __launch_bounds__(EW_WARPS * 32, 2) k_enum_walk(ChanDev c, Strea
     float* s_fl = reinterpret_cast<float*>(s_pre + (c.nmc * R + 1) / 2 * 2);
     for (int i = threadIdx.x; i < c.nmc * R; i += blockDim.x) {
         s_pre[i] = sd.mc_pre[i];
-        s_fl[i / R * FloatTable<L>::FT + i % R] = float(sd.mc_pre[i]);
+        s_fl[i / R * FloatTable<L>::FT + i % R] = float_point(sd, sd.mc_pre[i]);   // not wide: in_domain
     }
     if (threadIdx.x == 0) {
         const double sqrt2 = 1.4142135623730951;   // sqrt(2.0) correctly rounded

@@ -80,8 +80,8 @@ __global__ void __launch_bounds__(ST_WARPS * 32, TB_STREAM_MIN_BLOCKS)
     for (int i = threadIdx.x; i < c.nmc * R; i += blockDim.x) {
         s_mc[i] = c.mc[i];
         s_pre[i] = sd.mc_pre[i];
-        s_fmc[i / R * FloatTable<L>::FT + i % R] = float(c.mc[i]);
-        s_fpre[i / R * FloatTable<L>::FT + i % R] = float(sd.mc_pre[i]);
+        s_fmc[i / R * FloatTable<L>::FT + i % R] = float_point(sd, c.mc[i]);
+        s_fpre[i / R * FloatTable<L>::FT + i % R] = float_point(sd, sd.mc_pre[i]);
     }
     __syncthreads();
     const unsigned full = 0xffffffffu;

@@ -24,6 +24,7 @@ struct StreamDev {
     int64_t nsec[TB_MAX_LEGS];   // sections of legs 0..L-2 (1 for the others)
     int64_t n_items;             // n_umk * prod nsec * 2^(L-1)
     const double* mc_pre;        // survival-test table (precalculateIndices)
+    bool wide;                   // a coordinate of the channel's point tables lies beyond 1.5: no FP32 pass
     // per evaluation (cleared before each launch): candidates inside the
     // energy window, with a valid determinant, surviving tuples, points
     // inside the simplices, tuples with such points (unsigned long long[5])

@@ -214,18 +214,22 @@ struct FloatTable {
     static constexpr int R = 2 * (L - 2) + 1;
     static constexpr int FT = R <= 1 ? 1 : R <= 4 ? 4 : 8;
 };
+__device__ __forceinline__ float float_point(const StreamDev& sd, double q) {
+    return sd.wide ? __int_as_float(0x7fc00000) : float(q);
+}
 
 // The points that FP32 arithmetic cannot place clearly outside: bit m is clear
 // only where theta_decide is false.  Most points of most tuples are far outside,
 // and FP32 runs beside the FP64 pipe at twice its rate, so the FP64 decisions
 // are left to the set bits (12x10 e-e, streamed: 13.0 -> 10.3 ms; enumeration of
-// 16x16 e-e: 91 -> 62 ms).  With u = 2^-24, B_r = |a0_r| + sum_j |G_rj| and q in
-// [0, 1], the FP32 value of alpha_r (operands rounded to FP32, at most R + 1 fused
-// steps) is within (R + 4) u B_r of the real map, R <= 5, and so within E_r =
+// 16x16 e-e: 91 -> 62 ms).  With u = 2^-24, B_r = |a0_r| + sum_j |G_rj| and |q_j|
+// <= 1.5, the FP32 value of alpha_r (operands rounded to FP32, at most R + 1 fused
+// steps) is within 1.5 (R + 4) u B_r of the real map, R <= 5, and so within E_r =
 // 16 u B_r: a value below -(E_r + 4 mg_r) leaves the FP64 one below -mg_r, and
 // kp0 + alpha_0 or alpha_1 + alpha_2 above their threshold T (outside_thresholds)
 // by those E and 16 u of the operands leaves the FP64 sum above T.  Comparisons
-// with NaN are false, and an infinite bound keeps every point.
+// with NaN are false, and an infinite bound keeps every point: a table with larger
+// coordinates is NaN in FP32 (float_point).
 template <int L>
 __device__ __forceinline__ uint64_t maybe_inside(const AlphaMap<L>& am, const double (&T)[2], const float* tab, int nmc) {
     constexpr int R = AlphaMap<L>::R, FT = FloatTable<L>::FT;
