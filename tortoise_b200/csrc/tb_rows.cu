@@ -736,7 +736,7 @@ template <int L>
 __device__ __noinline__ void spread_nonfinite(const RowChan& c, const InstDev* insts, int n_insts, int64_t t0,
                                               int64_t t1, const double* f, double* acc, const DPCtl* ctl, bool rate,
                                               int rate_leg, const FxAcc& fx, const double* u = nullptr,
-                                              double* gamp = nullptr, const FxAcc& fx_amp = FxAcc{}) {
+                                              double* gamp = nullptr, unsigned int* gamp_poison = nullptr) {
     const double nan = __longlong_as_double(0x7ff8000000000000ll);
     for (int64_t i = t0 + threadIdx.x; i < t1; i += blockDim.x) {
         int e[L];
@@ -754,7 +754,7 @@ __device__ __noinline__ void spread_nonfinite(const RowChan& c, const InstDev* i
                 if (u) all = all || !finite3(u + in.foff[l] + 3 * (int64_t)e[l]);
             }
             if (nbad == 0 && !all) continue;
-            if (u && fx_amp.w) atomicOr(fx_amp.poison, 1u);
+            if (u && gamp_poison) atomicOr(gamp_poison, 1u);
             else if (u) atomicAdd(gamp + k, nan);
 #pragma unroll
             for (int l = 0; l < L; ++l) {
@@ -795,8 +795,8 @@ __global__ void __launch_bounds__(RowCap<L, MODE>::W * 32, 1) k_rows(const RowCh
     for (int i = tid; i < int(sizeof(RowChan) / sizeof(int)); i += blockDim.x)
         reinterpret_cast<int*>(&c)[i] = reinterpret_cast<const int*>(chans + w.chan)[i];
     __syncthreads();
-    const InstDev* insts = one ? one : c.insts + w.i0;
-    const int n_insts = one ? 1 : w.i1 - w.i0;
+    const InstDev* insts = one ? one : c.insts + (MULTI ? w.i0 : 0);
+    const int n_insts = MULTI ? w.i1 - w.i0 : 1;
     if (!VJP) {
         // every instance off or its run finished: nothing to add (an amplitude
         // of 0 still has a gradient)
@@ -830,7 +830,7 @@ __global__ void __launch_bounds__(RowCap<L, MODE>::W * 32, 1) k_rows(const RowCh
     double4 f0 = make_double4(0., 0., 0., 0.), u0 = f0;
     int64_t off[L], el[L];
     double amp = 0.0, ga = 0.0;   // ga: this lane's part of the amplitude gradient
-    if (VJP) gamp += c.gamp0 + w.i0;
+    if (VJP) gamp += c.gamp0 + (MULTI ? w.i0 : 0);
     if (!MULTI) {
 #pragma unroll
         for (int l = 0; l < L; ++l) { off[l] = insts[0].foff[l]; el[l] = off[l] / 3; }
@@ -947,14 +947,14 @@ __global__ void __launch_bounds__(RowCap<L, MODE>::W * 32, 1) k_rows(const RowCh
 template <int L>
 __global__ void __launch_bounds__(256) k_rows_spread(const RowChan* __restrict__ chans, const RowWork* __restrict__ work,
                                                      const double* __restrict__ f, const int* __restrict__ nf, int n_nf,
-                                                     FxAcc fx, const double* __restrict__ u, FxAcc fx_amp) {
+                                                     FxAcc fx, const double* __restrict__ u, unsigned int* gamp_poison) {
     int bad = 0;
     for (int i = threadIdx.x; i < n_nf; i += blockDim.x) bad |= nf[i];
     if (!__syncthreads_or(bad)) return;
     const RowWork w = work[blockIdx.x];
     const RowChan& c = chans[w.chan];
     spread_nonfinite<L>(c, c.insts + w.i0, w.i1 - w.i0, w.t0, w.t1, f, nullptr, nullptr, false, -1, fx, u, nullptr,
-                        fx_amp);
+                        gamp_poison);
 }
 
 // acc += the further accumulators, which are cleared.  A latency chain on the
@@ -1063,7 +1063,7 @@ int launch_rows(const RowSet& rs, const RowArgs& A, cudaStream_t s) {
 int launch_rows_spread(const RowSet& rs, const RowArgs& A, const FxAcc& fx_amp, cudaStream_t s) {
     if (rs.nblocks <= 0) return TB_OK;
     auto kern = rs.L == 2 ? k_rows_spread<2> : rs.L == 3 ? k_rows_spread<3> : k_rows_spread<4>;
-    kern<<<unsigned(rs.nblocks), 256, 0, s>>>(rs.d_chan, rs.d_work, A.f, A.nf, A.ed->nblk, A.fx, A.u, fx_amp);
+    kern<<<unsigned(rs.nblocks), 256, 0, s>>>(rs.d_chan, rs.d_work, A.f, A.nf, A.ed->nblk, A.fx, A.u, fx_amp.poison);
     TB_CUDA(cudaGetLastError());
     return TB_OK;
 }
