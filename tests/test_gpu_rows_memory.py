@@ -86,3 +86,20 @@ def test_rows_of_all_channels_stay_within_the_budget(gpu_lib):
     part, _, got = _used(mat, cap)
     assert 0 < part - small <= cap + (4 << 20)   # and the row sets and further accumulators, in units of 2 MB
     assert rel_l2(got, ref) < TOL
+
+
+def test_changing_factors_again_and_again_keeps_nothing(gpu_lib):
+    """Each change of a channel's factors rebuilds the row sets; what they held before is given back."""
+    mats, states = W.ensemble_runs(1, seed=4, Ns=(16,))
+    e = E.BatchEngine(mats)
+    try:
+        def change(k):
+            e.set_channel_amplitude(0, lambda b: np.full(len(b), 1.0 + 0.01 * k))
+        for k in range(3):
+            change(k)
+        free = _free()
+        for k in range(200):
+            change(k)
+        assert free - _free() <= 2 << 20   # one unit of the allocator; kept sets would take 10 MB
+    finally:
+        e.close()

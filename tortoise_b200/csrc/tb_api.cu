@@ -692,17 +692,36 @@ static int make_row_sets(tb_handle* h, Take take, bool run_minor, std::vector<Ro
     return TB_OK;
 }
 
+constexpr size_t RETIRED_MAX = size_t(64) << 20;
+
+// Device memory that the handle's calls no longer use (the stream is idle).
+static void retire(tb_handle* h, void* p, size_t bytes) {
+    if (!p) return;
+    if (!h->captured) {
+        cudaFree(p);
+        return;
+    }
+    h->retired.emplace_back(p, bytes);
+    size_t total = 0;
+    for (const auto& r : h->retired) total += r.second;
+    while (total > RETIRED_MAX && h->retired.size() > 1) {   // the newest stays
+        total -= h->retired.front().second;
+        cudaFree(h->retired.front().first);
+        h->retired.erase(h->retired.begin());
+    }
+}
+
 void retire_row_sets(tb_handle* h) {
-    auto retire = [&](RowSet& rs) {
-        if (rs.d_chan) h->retired.push_back(rs.d_chan);   // the allocation's base
+    auto retire_set = [&](RowSet& rs) {
+        retire(h, rs.d_chan, rs.bytes);   // the allocation's base
         rs.d_chan = nullptr;
         rs.release();
     };
     for (auto* sets : {&h->row_sets, &h->rate_sets, &h->run_sets}) {
-        for (auto& rs : *sets) retire(rs);
+        for (auto& rs : *sets) retire_set(rs);
         sets->clear();
     }
-    for (auto& G : h->groups) retire(G.row_one);
+    for (auto& G : h->groups) retire_set(G.row_one);
 }
 
 int refresh_row_sets(tb_handle* h) {
@@ -735,7 +754,7 @@ int refresh_row_sets(tb_handle* h) {
     for (const auto* sets : {&h->row_sets, &h->rate_sets})
         for (const RowSet& rs : *sets) copies = std::max(copies, rs.copies);
     if (copies - 1 > h->n_accr && !h->opts.deterministic) {
-        if (h->d_accr) h->retired.push_back(h->d_accr);
+        retire(h, h->d_accr, sizeof(double) * size_t(h->n_accr) * size_t(h->ndofs));
         h->n_accr = 0;
         const size_t bytes = sizeof(double) * size_t(copies - 1) * size_t(h->ndofs);
         if (cudaMalloc(&h->d_accr, bytes) != cudaSuccess) {
@@ -1268,6 +1287,7 @@ static int host_in(tb_handle* h, const double* f, int flags, const double*& d_in
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
     TB_CUDA(cudaStreamIsCapturing(h->stream, &capture));
     captured = capture != cudaStreamCaptureStatusNone;
+    h->captured = h->captured || captured;
     if (captured || !h->acc_clean) TB_CUDA(cudaMemsetAsync(h->d_acc, 0, bytes, h->stream));
     if (!captured) h->acc_clean = false;   // until the call has read and cleared it
     return TB_OK;
@@ -1358,7 +1378,7 @@ int tb_destroy(tb_handle* h) {
         if (G.d_tamp) cudaFree(G.d_tamp);
     }
     retire_row_sets(h);
-    for (void* p : h->retired) cudaFree(p);
+    for (const auto& r : h->retired) cudaFree(r.first);
     for (void* p : h->run_allocs) cudaFree(p);
     if (h->d_accr) cudaFree(h->d_accr);
     for (double* p : h->dev_allocs) cudaFree(p);
@@ -2010,6 +2030,9 @@ int tb_collision_accumulate(tb_handle* h, int ch, const double* f, double* acc) 
     if (!h || !f || !acc) { set_error("null argument"); return TB_ERR_ARG; }
     if (ch < -1 || ch >= int(h->insts.size())) { set_error("channel index out of range"); return TB_ERR_ARG; }
     TB_CUDA(cudaSetDevice(h->device));
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    TB_CUDA(cudaStreamIsCapturing(h->stream, &capture));
+    h->captured = h->captured || capture != cudaStreamCaptureStatusNone;
     return run_rhs_acc(h, f, acc, nullptr, TB_NO_DRIFT, ch);
 }
 

@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "tb_dp45.cuh"
@@ -104,9 +105,11 @@ struct tb_handle {
     tb::RunState* d_run_states = nullptr;
     int* d_run_nf = nullptr;
     int n_run_tiles = 0;
-    // what former row sets held: a graph that the caller captured may still
-    // launch them (a few ten KB for each change of schedules; freed with the handle)
-    std::vector<void*> retired;
+    // what former row sets held, once the caller has captured an operator call:
+    // the graph may still launch them.  A few ten KB for each change of schedules
+    // or factors; beyond RETIRED_MAX the oldest go.
+    bool captured = false;
+    std::vector<std::pair<void*, size_t>> retired;
     double* d_accr = nullptr;    // further accumulators of the row sets, n_accr of ndofs
     int n_accr = 0;
     int64_t budget_left = 0;     // of tensor_budget_bytes (or its default) after creation

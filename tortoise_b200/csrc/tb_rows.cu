@@ -1158,6 +1158,7 @@ int build_row_set(int L, int form, const std::vector<RowChan>& chan, const std::
         return TB_ERR_OOM;
     }
     out.d_chan = reinterpret_cast<RowChan*>(base);
+    out.bytes = all.size();
     out.d_work = reinterpret_cast<RowWork*>(base + cb);
     out.d_bounds[0] = reinterpret_cast<int32_t*>(base + cb + wb);
     out.d_bounds[1] = reinterpret_cast<int32_t*>(base + cb + wb + bb);

@@ -83,6 +83,7 @@ struct RowSet {
     // propagation, and for the kernels that take fewer warps
     int32_t* d_bounds[2] = {nullptr, nullptr};
     int shares[2] = {0, 0};
+    size_t bytes = 0;               // of the allocation behind d_chan
     int nblocks = 0;
     int nmc_max = 0;
     int copies = 1;                 // accumulators that its blocks share out (row_copies)
